@@ -1,0 +1,88 @@
+"""tl_attention against f64 attention at the edges of its kernels: key tiles and splits, query rows per KV head, head
+dimensions, storage types, masks, caches longer than what is read."""
+import numpy as np
+import pytest
+
+from torchlette_b200 import backend as tb
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def be():
+    assert tb.initCuda(0), tb.getCudaInitError()
+    return tb.getBackend()
+
+
+def to_bf16_bits(a):
+    u = np.ascontiguousarray(a, np.float32).view(np.uint32)
+    return ((u + 0x7FFF + ((u >> 16) & 1)) >> 16).astype(np.uint16)
+
+
+def store(be, a, dtype):
+    """The tensor and the values it holds, as f64."""
+    if dtype == "bf16":
+        bits = to_bf16_bits(a)
+        return be.ops.tensorFromArray(bits, list(a.shape), "bf16"), (bits.astype(np.uint32) << 16).view(np.float32).astype(np.float64)
+    a = a.astype(np.float16 if dtype == "f16" else np.float32)
+    return be.ops.tensorFromArray(a, list(a.shape), dtype), a.astype(np.float64)
+
+
+def read(be, t):
+    a = be.ops.read(t)
+    return (a.astype(np.uint32) << 16).view(np.float32) if t.dtype == "bf16" else a
+
+
+def reference(q, k, v, scale, causal, mask):
+    h, s, n, rep = q.shape[1], q.shape[2], k.shape[2], q.shape[1] // k.shape[1]
+    k, v = np.repeat(k, rep, axis=1), np.repeat(v, rep, axis=1)
+    sc = np.matmul(q, k.transpose(0, 1, 3, 2)) * scale
+    if mask is not None:
+        sc = sc + mask
+    if causal:
+        sc = np.where(np.arange(n)[None, :] <= (n - s + np.arange(s))[:, None], sc, -np.inf)
+    p = np.exp(sc - sc.max(-1, keepdims=True))
+    o = np.matmul(p / p.sum(-1, keepdims=True), v)
+    return o.transpose(0, 2, 1, 3).reshape(q.shape[0], s, h * q.shape[3])
+
+
+# one rounding of an output below 2 to the storage type (half an ulp), plus 4e-6: f32 sums over up to 1e3 terms near 1 and
+# probabilities held to 2^-17 or better
+TOL = {"f16": 2.0 ** -11 + 4e-6, "bf16": 2.0 ** -8 + 4e-6, "f32": 4e-6}
+
+
+def check(be, b, heads, kv_heads, d, s, n, dtype, causal=True, masked=False, capacity=None, seed=0):
+    rng = np.random.default_rng(seed + 1000 * n + s)
+    cap = capacity or n + 5
+    q, qr = store(be, rng.standard_normal((b, heads, s, d)), dtype)
+    kf, vf = rng.standard_normal((b, kv_heads, cap, d)), rng.standard_normal((b, kv_heads, cap, d))
+    kf[:, :, n:], vf[:, :, n:] = np.nan, np.inf  # what lies behind the read prefix must not matter
+    k, kr = store(be, kf, dtype)
+    v, vr = store(be, vf, dtype)
+    mask = np.where(rng.random((s, n)) < 0.3, -np.inf, rng.standard_normal((s, n))).astype(np.float32) if masked else None
+    if masked:
+        mask[:, 0] = 0.5  # every query sees something
+    mt = be.ops.tensorFromArray(mask, [s, n], "f32") if masked else None
+    scale = 1.0 / np.sqrt(d)
+    out = be.ops.attention(q, k, v, n, scale, causal=causal, mask=mt)
+    got = read(be, out).astype(np.float64)
+    ref = reference(qr, kr[:, :, :n], vr[:, :, :n], scale, causal, mask)
+    err = np.abs(got - ref) / np.maximum(1.0, np.abs(ref))
+    assert np.isfinite(got).all() and err.max() <= TOL[dtype], (err.max(), np.unravel_index(err.argmax(), err.shape))
+    for t in (q, k, v, out) + ((mt,) if masked else ()):
+        t.destroy()
+
+
+@pytest.mark.parametrize("dtype", ["f16", "bf16", "f32"])
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("b,heads,kv_heads,s,n", [
+    (1, 1, 1, 1, 1), (1, 4, 4, 1, 15), (2, 8, 2, 1, 16), (1, 8, 1, 1, 17), (3, 6, 2, 1, 129), (1, 4, 1, 1, 1000), (1, 16, 8, 1, 2051),
+    (2, 4, 2, 3, 40), (1, 8, 2, 4, 4), (1, 16, 1, 1, 300), (1, 3, 1, 5, 260)])
+def test_decode(be, dtype, d, b, heads, kv_heads, s, n):
+    check(be, b, heads, kv_heads, d, s, n, dtype)
+
+
+@pytest.mark.parametrize("dtype", ["f16", "bf16", "f32"])
+@pytest.mark.parametrize("s,n,causal", [(1, 200, False), (2, 333, True), (4, 70, False)])
+def test_decode_mask(be, dtype, s, n, causal):
+    check(be, 2, 4, 2, 128, s, n, dtype, causal=causal, masked=True)
