@@ -86,3 +86,44 @@ def test_decode(be, dtype, d, b, heads, kv_heads, s, n):
 @pytest.mark.parametrize("s,n,causal", [(1, 200, False), (2, 333, True), (4, 70, False)])
 def test_decode_mask(be, dtype, s, n, causal):
     check(be, 2, 4, 2, 128, s, n, dtype, causal=causal, masked=True)
+
+
+@pytest.mark.parametrize("dtype", ["f16", "bf16", "f32"])
+def test_decode_mask_of_lowest_values(be, dtype):
+    """A row hidden altogether by the lowest f32 is the mean of all values, one hidden in part sees the rest."""
+    rng = np.random.default_rng(7)
+    low = np.finfo(np.float32).min
+    q, qr = store(be, rng.standard_normal((1, 4, 2, 64)), dtype)
+    k, kr = store(be, rng.standard_normal((1, 2, 300, 64)), dtype)
+    v, vr = store(be, rng.standard_normal((1, 2, 300, 64)), dtype)
+    mask = np.full((2, 300), low, np.float32)
+    mask[1, 40:] = 0.0
+    mt = be.ops.tensorFromArray(mask, [2, 300], "f32")
+    out = be.ops.attention(q, k, v, 300, 0.125, causal=False, mask=mt)
+    got = read(be, out).astype(np.float64)
+    ref = np.empty_like(got)
+    ref[:, 0] = np.repeat(vr.mean(2), 2, axis=1).reshape(1, -1)
+    ref[:, 1] = reference(qr[:, :, 1:], kr[:, :, 40:], vr[:, :, 40:], 0.125, False, None)[:, 0]
+    assert (np.abs(got - ref) / np.maximum(1.0, np.abs(ref))).max() <= TOL[dtype]
+    for t in (q, k, v, mt, out):
+        t.destroy()
+
+
+@pytest.mark.parametrize("dtype", ["f16", "bf16", "f32"])
+@pytest.mark.parametrize("s,n", [(3, 37), (3, 200)])
+def test_decode_hidden_values_not_finite(be, dtype, s, n):
+    """What the causal mask hides from a row does not reach it, infinite or not."""
+    rng = np.random.default_rng(n)
+    q, qr = store(be, rng.standard_normal((1, 4, s, 64)), dtype)
+    k, kr = store(be, rng.standard_normal((1, 2, n, 64)), dtype)
+    vf = rng.standard_normal((1, 2, n, 64))
+    vf[:, 0, n - 1, :40], vf[:, 1, n - 1, 5] = np.inf, np.nan
+    v, vr = store(be, vf, dtype)
+    out = be.ops.attention(q, k, v, n, 0.125, causal=True)
+    got = read(be, out).astype(np.float64)
+    ref = reference(qr[:, :, :s - 1], kr[:, :, :n - 1], vr[:, :, :n - 1], 0.125, True, None)
+    assert (np.abs(got[:, :s - 1] - ref) / np.maximum(1.0, np.abs(ref))).max() <= TOL[dtype]
+    last = got[0, s - 1].reshape(4, 64)
+    assert np.isinf(last[:2, :40]).all() and np.isfinite(last[:2, 40:]).all() and np.isnan(last[2:, 5]).all() and np.isfinite(last[2:, 6:]).all()
+    for t in (q, k, v, out):
+        t.destroy()

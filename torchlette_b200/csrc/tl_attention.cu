@@ -15,7 +15,7 @@
 
 #include <cooperative_groups.h>
 
-#include "tl_common.cuh"
+#include "tl_attention.cuh"
 #include "tl_mma_frag.cuh"
 
 namespace cg = cooperative_groups;
@@ -96,11 +96,10 @@ struct DecodeArgs {
   void* out;
   int32_t n_heads, n_kv_heads, rep, q_len, rows, kv_len, splits;  // rows = rep * q_len: query rows of one KV head
   int64_t capacity;
-  float scale_log2;   // scale * log2(e): the softmax runs in base 2
+  float scale;
   const float* mask;  // [q_len, kv_len] or null
   int32_t causal;
 };
-constexpr float kLog2e = 1.4426950408889634f;
 
 // Partials of this CTA's warps -> the cluster's result.  sm: [warps][R] maxima, [warps][R] sums, [warps][R][D]
 // outputs, then the CTA's own merged [R], [R], [R][D].
@@ -122,7 +121,7 @@ __device__ __forceinline__ void decode_merge(const DecodeArgs& p, float* sm, int
 #pragma unroll
     for (int w = 0; w < WARPS; ++w) {
       const float mw = wm[w * R + r];
-      const float f = mw == -INFINITY ? 0.f : exp2f(mw - m);
+      const float f = mw == -INFINITY ? 0.f : exp2f((mw - m) * kLog2e);
       l = fmaf(wl[w * R + r], f, l);
       o = fmaf(wo[(w * R + r) * D + d], f, o);
     }
@@ -133,7 +132,7 @@ __device__ __forceinline__ void decode_merge(const DecodeArgs& p, float* sm, int
   if (p.splits > 1) cluster.sync();
   else __syncthreads();
   const int rank = p.splits > 1 ? int(cluster.block_rank()) : 0;
-  const int total = p.rows * D, per = (total + p.splits - 1) / p.splits;
+  const int total = p.rows * D, per = ((total + p.splits - 1) / p.splits + 31) & ~31;  // a warp's 32 values are one row's
   for (int e = rank * per + threadIdx.x; e < min(total, (rank + 1) * per); e += WARPS * 32) {
     const int r = e / D, d = e - r * D;
     float m = -INFINITY;
@@ -144,13 +143,22 @@ __device__ __forceinline__ void decode_merge(const DecodeArgs& p, float* sm, int
       const float* rl = p.splits > 1 ? cluster.map_shared_rank(cl, s) : cl;
       const float* ro = p.splits > 1 ? cluster.map_shared_rank(co, s) : co;
       const float ms = rm[r];
-      const float f = ms == -INFINITY ? 0.f : exp2f(ms - m);
+      const float f = ms == -INFINITY ? 0.f : exp2f((ms - m) * kLog2e);
       l = fmaf(rl[r], f, l);
       o = fmaf(ro[r * D + d], f, o);
     }
     const int qi = r / p.rep, h = kvh * p.rep + (r - qi * p.rep);
-    const int64_t at = ((int64_t(b) * p.q_len + qi) * p.n_heads + h) * D + d;
-    reinterpret_cast<AT*>(p.out)[at] = DT<AT>::from_f32(o / l);
+    const int64_t at = ((int64_t(b) * p.q_len + qi) * p.n_heads + h) * D;
+    const float v = o / l;
+    if (p.causal && p.q_len > 1 && __any_sync(0xffffffffu, !isfinite(v))) {
+      const int64_t kv = (int64_t(b) * p.n_kv_heads + kvh) * p.capacity * D;
+      attention_row_warp<AT, D>(reinterpret_cast<const AT*>(p.q) + ((int64_t(b) * p.n_heads + h) * p.q_len + qi) * D,
+                                reinterpret_cast<const AT*>(p.k) + kv, reinterpret_cast<const AT*>(p.v) + kv,
+                                reinterpret_cast<AT*>(p.out) + at, p.kv_len - p.q_len + qi + 1, p.scale,
+                                p.mask ? p.mask + int64_t(qi) * p.kv_len : nullptr, d >> 5);
+    } else {
+      reinterpret_cast<AT*>(p.out)[at + d] = DT<AT>::from_f32(v);
+    }
   }
   if (p.splits > 1) cluster.sync();  // no CTA leaves while another reads its shared memory
 }
@@ -158,33 +166,9 @@ template <int D, int R, int WARPS> constexpr size_t decode_smem_bytes() {
   return sizeof(float) * (size_t(WARPS) + 1) * R * (D + 2);
 }
 
-// Two probabilities (of one key, for two query rows) as 16-bit terms whose sum carries (nearly) all 24 bits of
-// each: p rounded, then what is left rounded, then again.  f16 needs two terms (11 bits each), bf16 three (8 bits).
-template <typename AT> struct ProbSplit;
-template <> struct ProbSplit<__half> {
-  static constexpr int kTerms = 2;
-  static constexpr float kBias = 10.f;  // probabilities are held times 2^10: the low term stays clear of f16's subnormals
-  __device__ static void split(float a, float b, uint32_t (&t)[2]) {
-    const __half2 hi = __floats2half2_rn(a, b);
-    const float2 f = __half22float2(hi);
-    const __half2 lo = __floats2half2_rn(a - f.x, b - f.y);
-    t[0] = *reinterpret_cast<const uint32_t*>(&hi);
-    t[1] = *reinterpret_cast<const uint32_t*>(&lo);
-  }
-};
-template <> struct ProbSplit<__nv_bfloat16> {
-  static constexpr int kTerms = 3;
-  static constexpr float kBias = 0.f;
-  __device__ static void split(float a, float b, uint32_t (&t)[3]) {
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-      t[i] = *reinterpret_cast<const uint32_t*>(&h);
-      a -= __uint_as_float(t[i] << 16);
-      b -= __uint_as_float(t[i] & 0xffff0000u);
-    }
-  }
-};
+// Probabilities are held times 2^10 in f16: the low term of their split stays clear of f16's subnormals.
+template <typename AT> constexpr float kProbBias = 0.f;
+template <> constexpr float kProbBias<__half> = 10.f;
 
 __device__ __forceinline__ uint32_t transpose8x8(uint32_t v) {
   uint32_t r;
@@ -280,8 +264,8 @@ __global__ void __launch_bounds__(128, NT == 1 ? 3 : 2) attn_decode_mma_kernel(D
 #pragma unroll
       for (int e = 0; e < 4; ++e) {  // element e: key g + 8 * (e >> 1), query row 2t + (e & 1)
         const int key = key0 + g + 8 * (e >> 1);
-        float x = s[nt][e] * p.scale_log2;
-        if (p.mask) x = fmaf(mrow[nt][e & 1][min(key, last)], kLog2e, x);
+        // natural units up to the difference with the maximum: a mask may hold the lowest f32, which no factor fits
+        const float x = fmaf(s[nt][e], p.scale, p.mask ? mrow[nt][e & 1][min(key, last)] : 0.f);
         s[nt][e] = key < bound[nt][e & 1] ? x : -INFINITY;
       }
       float nm[2];
@@ -297,7 +281,7 @@ __global__ void __launch_bounds__(128, NT == 1 ? 3 : 2) attn_decode_mma_kernel(D
         float f[2];
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
-          f[c] = nm[c] == m[nt][c] ? 1.f : exp2f(m[nt][c] - nm[c]);  // first keys: exp2(-inf) = 0 on zeros
+          f[c] = nm[c] == m[nt][c] ? 1.f : exp2f((m[nt][c] - nm[c]) * kLog2e);  // first keys: exp2(-inf) = 0 on zeros
           l[nt][c] *= f[c];
           m[nt][c] = nm[c];
         }
@@ -310,7 +294,7 @@ __global__ void __launch_bounds__(128, NT == 1 ? 3 : 2) attn_decode_mma_kernel(D
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const float mm = m[nt][e & 1];
-        pr[e] = mm == -INFINITY ? 0.f : exp2f(s[nt][e] - mm + ProbSplit<AT>::kBias);  // no key visible yet: nothing to add
+        pr[e] = mm == -INFINITY ? 0.f : exp2f(fmaf(s[nt][e] - mm, kLog2e, kProbBias<AT>));  // no key visible yet: nothing to add
         l[nt][e & 1] += pr[e];
       }
       uint32_t a[TERMS], c[TERMS];
@@ -413,21 +397,20 @@ __global__ void __launch_bounds__(128) attn_decode_f32_kernel(DecodeArgs p) {
         float x = 0.f;
 #pragma unroll
         for (int i = 0; i < V; ++i) x = fmaf(q[r][i], kf[j][i], x);
-        x = warp_sum(x) * p.scale_log2;
         const int key = tile * KEYS + j;
-        if (p.mask) x = fmaf(mrow[r][min(key, last)], kLog2e, x);
+        x = fmaf(warp_sum(x), p.scale, p.mask ? mrow[r][min(key, last)] : 0.f);
         s[j] = key < bound[r] ? x : -INFINITY;
         nm = fmaxf(nm, s[j]);
       }
       if (nm != -INFINITY) {
-        const float f = exp2f(m[r] - nm);
+        const float f = exp2f((m[r] - nm) * kLog2e);
         m[r] = nm;
         l[r] *= f;
 #pragma unroll
         for (int i = 0; i < V; ++i) o[r][i] *= f;
 #pragma unroll
         for (int j = 0; j < KEYS; ++j) {
-          const float e = exp2f(s[j] - nm);
+          const float e = exp2f((s[j] - nm) * kLog2e);
           l[r] += e;
 #pragma unroll
           for (int i = 0; i < V; ++i) o[r][i] = fmaf(e, vf[j][i], o[r][i]);
@@ -513,7 +496,7 @@ int32_t tl_attention(tl_ctx* ctx, const void* q, const void* k_cache, const void
     p.q = q; p.k = k_cache; p.v = v_cache; p.out = out;
     p.n_heads = int32_t(n_heads); p.n_kv_heads = int32_t(n_kv_heads); p.rep = int32_t(rep); p.q_len = int32_t(q_len);
     p.rows = int32_t(rows); p.kv_len = int32_t(kv_len); p.capacity = kv_capacity;
-    p.scale_log2 = scale * kLog2e; p.mask = mask; p.causal = causal ? 1 : 0;
+    p.scale = scale; p.mask = mask; p.causal = causal ? 1 : 0;
     // Splits (CTAs of a cluster) per KV head: double them while there are fewer than two CTAs per SM and a warp has
     // more than two 16-key tiles; above 8, which needs a non-portable cluster, only if that leaves SMs idle (1
     // sequence, 8 KV heads, 4000 keys: 10.3 us with 8, 9.7 with 16).  Then keep the launch in one wave of three
