@@ -49,6 +49,23 @@ def test_device_quantizer_bit_exact(backend, n, k, group):
     assert np.array_equal(packed, hp) and np.array_equal(scales, hs)
 
 
+@pytest.mark.parametrize("group", [32, 64, 128])
+def test_device_quantizer_at_halves(backend, group):
+    """Values on, just below and just above every half of a whole number, and a count that ends inside a warp's share."""
+    n = 13
+    top = np.array([127.0, 0.02, 1.7, 3e-5, 900.0, 7e-8, 1e-3, 127.0, 254.0, 63.5, 1.0, 5.0, 0.3], np.float32)
+    k = 3 * 128
+    halves = (np.arange(k) % 254 - 127 + 0.5).astype(np.float32)
+    w = np.empty((n, k), np.float32)
+    for i in range(n):
+        step = np.float32(np.float16(top[i])) / np.float32(127)
+        w[i] = np.nextafter(halves * step, np.float32([0, np.inf, -np.inf][i % 3]) if i % 3 else halves * step)
+        w[i, ::group] = top[i]
+    packed, scales = _quantize_on_device(backend, w, group)
+    op, os_ = orc.quantize_linear_weight(w, group)
+    assert np.array_equal(scales, os_) and np.array_equal(packed, op)
+
+
 def test_device_quantizer_argument_errors(backend):
     be = backend
     w = be.ops.tensorFromArray(np.zeros((2, 130), dtype=np.float32), [2, 130], "f32")
