@@ -45,7 +45,7 @@ def _f32(be, arr, shape=None):
     return be.ops.tensorFromArray(arr, list(shape or arr.shape), "f32")
 
 
-@pytest.mark.parametrize("rows,cols", [(1, 4096), (16, 128), (7, 300), (64, 64)])
+@pytest.mark.parametrize("rows,cols", [(1, 4096), (16, 128), (7, 300), (64, 64), (3, 8), (1500, 128), (2, 8192), (2, 8200), (1, 32768), (1, 32776)])
 @pytest.mark.parametrize("dtype", ["f32", "f16"])
 def test_rmsnorm(backend, rows, cols, dtype):
     be = backend
