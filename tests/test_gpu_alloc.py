@@ -1,0 +1,73 @@
+"""tl_alloc / tl_free: blocks are handed out again, but never while anything given to the device before still uses them."""
+import ctypes as C
+
+import numpy as np
+import pytest
+import torch
+
+from torchlette_b200 import backend as tb
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def be():
+    own = tb.CudaBackend(0)  # a context of its own: the refusals below count as its errors
+    yield own
+    own.destroy()
+
+
+class _Memory:
+    def __init__(self, ptr, count):
+        self.__cuda_array_interface__ = {"data": (ptr, False), "shape": (count,), "typestr": "<f4", "version": 2}
+
+
+def test_blocks_are_reused_and_live_ones_do_not_overlap(be):
+    seen, live = set(), []
+    rng = np.random.default_rng(0)
+    again = 0
+    for i in range(600):
+        size = int(rng.choice([1, 100, 512, 4096, 70_000, 3_000_000]))
+        p = be._alloc(size)
+        assert p % 256 == 0
+        again += p in seen
+        seen.add(p)
+        live.append((p, size))
+        spans = sorted(live)
+        assert all(a + s <= b for (a, s), (b, _) in zip(spans, spans[1:]))
+        if len(live) > 5:
+            be._free(live.pop(int(rng.integers(len(live))))[0])
+    for p, _ in live:
+        be._free(p)
+    assert again > 100
+
+
+def test_a_block_given_back_waits_for_other_streams(be):
+    """torch reads the blocks on a stream of its own, long after they were given back; new results must not reach them."""
+    count = 1 << 22
+    side = torch.cuda.Stream()
+    busy = torch.randn(4096, 4096, device="cuda")
+    for _ in range(3):
+        t = be.ops.tensorFromArray(np.full(count, 1.0, np.float32), [count], "f32")
+        be.sync()
+        with torch.cuda.stream(side):
+            for _ in range(30):
+                busy = (busy @ busy).clamp_(-1, 1)
+            copy = torch.as_tensor(_Memory(t.buffer, count), device="cuda").clone()
+        t.destroy()
+        others = [be.ops.tensorFromArray(np.full(count, 2.0, np.float32), [count], "f32") for _ in range(70)]
+        for o in others:
+            o.destroy()
+        side.synchronize()
+        assert bool((copy == 1.0).all())
+
+
+def test_errors(be):
+    p = be._alloc(1000)
+    be._free(p)
+    with pytest.raises(tb.TlError):
+        be._free(p)
+    with pytest.raises(tb.TlError):
+        be._alloc(1 << 50)
+    q = be._alloc(1000)  # neither refusal spoils what follows
+    be._free(q)

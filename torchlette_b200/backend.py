@@ -23,6 +23,7 @@ the CUDA library and an sm_100 GPU, ``initCuda`` raises.
 from __future__ import annotations
 
 import ctypes as C
+import math
 from dataclasses import dataclass, field
 from typing import Optional, Sequence
 
@@ -153,6 +154,7 @@ class CudaTensor:
 
 _NP_OF = {"f32": np.float32, "f16": np.float16, "bf16": np.uint16, "u32": np.uint32, "u16": np.uint16,
           "i8": np.int8}
+_ITEMSIZE = {name: np.dtype(t).itemsize for name, t in _NP_OF.items()}  # np.dtype(...) and np.prod cost microseconds a call
 
 
 class CudaOps:
@@ -173,7 +175,7 @@ class CudaOps:
             host = np.ascontiguousarray(arr)
         else:
             host = np.ascontiguousarray(arr, dtype=_NP_OF[dtype])
-        n = int(np.prod(shape)) if len(shape) else 1
+        n = int(math.prod(shape)) if len(shape) else 1
         if host.size != n:
             raise ValueError(f"tensorFromArray: expected {n} elements, got {host.size}")
         buf = self._b._alloc(host.nbytes)
@@ -181,14 +183,14 @@ class CudaOps:
         return CudaTensor(self._b, shape, dtype, buf, host.nbytes)
 
     def empty(self, shape, dtype="f32") -> CudaTensor:
-        n = int(np.prod(shape)) if len(shape) else 1
-        nbytes = n * np.dtype(_NP_OF[dtype]).itemsize
+        n = int(math.prod(shape)) if len(shape) else 1
+        nbytes = n * _ITEMSIZE[dtype]
         return CudaTensor(self._b, shape, dtype, self._b._alloc(nbytes), nbytes)
 
     def read(self, t: CudaTensor) -> np.ndarray:
         if t.transposed:
             raise ValueError("read: materialize the transposed view first")
-        host = np.empty(int(np.prod(t.shape)) if t.shape else 1, dtype=_NP_OF[t.dtype])
+        host = np.empty(int(math.prod(t.shape)) if t.shape else 1, dtype=_NP_OF[t.dtype])
         self._b._download(host, t.buffer)
         if t.dtype == "f16":
             host = host.view(np.float16)
@@ -196,7 +198,7 @@ class CudaOps:
 
     def reshape(self, t: CudaTensor, shape) -> CudaTensor:
         """A view of a contiguous tensor under another shape (no copy; the buffer stays the owner's)."""
-        if t.transposed or int(np.prod(shape)) != int(np.prod(t.shape)):
+        if t.transposed or int(math.prod(shape)) != int(math.prod(t.shape)):
             raise ValueError("reshape: needs a contiguous tensor and the same element count")
         return CudaTensor(self._b, list(shape), t.dtype, t.buffer, t.nbytes, ownsBuffer=False, format=t.format, scales=t.scales)
 
@@ -212,7 +214,7 @@ class CudaOps:
     def _unary(self, op: int, t: CudaTensor, out_dtype: Optional[str] = None) -> CudaTensor:
         src = self.contiguous(t) if t.transposed else t
         out = self.empty(src.shape, out_dtype or src.dtype)
-        n = int(np.prod(src.shape)) if src.shape else 1
+        n = int(math.prod(src.shape)) if src.shape else 1
         B.check(self._b._ctx, self._b._lib.tl_unary_op(self._b._ctx, op, src.buffer, B.DTYPE_ID[src.dtype], out.buffer,
                                                        B.DTYPE_ID[out.dtype], n))
         if src is not t:
@@ -233,7 +235,7 @@ class CudaOps:
         if a.transposed or b.transposed:
             raise TlError(B.TL_ERR_UNSUPPORTED, f"{name}: materialize transposed views first (contiguous)")
         cols = a.shape[-1]
-        rows = int(np.prod(a.shape[:-1])) if len(a.shape) > 1 else 1
+        rows = int(math.prod(a.shape[:-1])) if len(a.shape) > 1 else 1
         is_row = list(b.shape) == [cols] and len(a.shape) > 1
         if not is_row and list(b.shape) != list(a.shape):
             raise TlError(B.TL_ERR_UNSUPPORTED, f"{name}: b must match a or be its last dim")
@@ -251,7 +253,7 @@ class CudaOps:
         """Materializes a transposed view (a packed weight cannot be: its bytes are not elements)."""
         if t.format is not None and t.format.packing is not None:
             raise TlError(B.TL_ERR_UNSUPPORTED, "contiguous: a packed weight has no element-wise transposition")
-        itemsize = np.dtype(_NP_OF[t.dtype]).itemsize
+        itemsize = _ITEMSIZE[t.dtype]
         if not t.transposed:
             return self._unary(0, t)  # a plain copy
         out = self.empty(t.shape, t.dtype)
@@ -265,7 +267,7 @@ class CudaOps:
         cols = x.shape[-1]
         if list(weight.shape) != [cols]:
             raise TlError(B.TL_ERR_INVALID_ARG, "rmsnorm: weight must be [lastDim]")
-        rows = int(np.prod(x.shape[:-1])) if len(x.shape) > 1 else 1
+        rows = int(math.prod(x.shape[:-1])) if len(x.shape) > 1 else 1
         out = self.empty(x.shape, outputDtype or x.dtype)
         B.check(self._b._ctx, self._b._lib.tl_rmsnorm(self._b._ctx, x.buffer, B.DTYPE_ID[x.dtype], weight.buffer, B.DTYPE_ID[weight.dtype],
                                                       out.buffer, B.DTYPE_ID[out.dtype], rows, cols, float(eps)))
@@ -276,7 +278,7 @@ class CudaOps:
         sinScale (-1: the inverse rotation), cosOffset / sinOffset (element offsets into larger tables)."""
         config = config or {}
         seq, hd = qk.shape[-2], qk.shape[-1]
-        outer = int(np.prod(qk.shape[:-2])) if len(qk.shape) > 2 else 1
+        outer = int(math.prod(qk.shape[:-2])) if len(qk.shape) > 2 else 1
         if cos.dtype != "f32" or sin.dtype != "f32":
             raise TlError(B.TL_ERR_UNSUPPORTED, "fusedRoPE: cos / sin tables are f32")
         out = self.empty(qk.shape, qk.dtype)
@@ -310,7 +312,7 @@ class CudaOps:
     def kvAppend(self, cache: CudaTensor, new: CudaTensor, position: int):
         """cache[:, :, position, :] = new ([B, kvH, 1, D] or [B, kvH, D]): one strided copy (model.ts:240-262)."""
         b, kvh, cap, d = cache.shape
-        esz = np.dtype(_NP_OF[cache.dtype]).itemsize
+        esz = _ITEMSIZE[cache.dtype]
         B.check(self._b._ctx, self._b._lib.tl_copy2d(self._b._ctx, cache.buffer + position * d * esz, cap * d * esz, new.buffer, d * esz, d * esz, b * kvh))
 
     def matmul(self, a: CudaTensor, b: CudaTensor, options: Optional[dict] = None) -> CudaTensor:
@@ -599,7 +601,7 @@ class CudaBackend:
         k, n = b.shape[-2], b.shape[-1]
         if a.shape[-1] != k:
             raise TlError(B.TL_ERR_INVALID_ARG, "matmul dimension mismatch")
-        m = int(np.prod(a.shape[:-1])) if len(a.shape) > 1 else 1
+        m = int(math.prod(a.shape[:-1])) if len(a.shape) > 1 else 1
         epilogue: Optional[EpilogueConfig] = options.get("epilogue")
         epilogueInputs = options.get("epilogueInputs", ())
         out_dtype = epilogue.outputDtype if epilogue is not None else options.get("outputDtype", "f32")
@@ -635,7 +637,7 @@ class CudaBackend:
         if batch_a and batch_b and batch_a != batch_b:
             raise TlError(B.TL_ERR_UNSUPPORTED, "matmul: batch dims must match or be absent on one operand")
         batch_dims = batch_a or batch_b
-        batch = int(np.prod(batch_dims)) if batch_dims else 1
+        batch = int(math.prod(batch_dims)) if batch_dims else 1
         if (a.transposed and batch_a) or (b.transposed and batch_b):
             raise TlError(B.TL_ERR_UNSUPPORTED, "matmul: a transposed view must be a single matrix")
         epilogue: Optional[EpilogueConfig] = options.get("epilogue")
@@ -685,7 +687,10 @@ class CudaBackend:
             chain.append((activation, None))
         if outputDtype != "f32":
             chain.append(("cast", outputDtype))
-        plan = detectMatmulEpilogue(chain)
+        if len(chain) == 1 and chain[0][0] == "cast":  # the plain projection: the fusion pass has nothing to decide
+            plan = EpilogueConfig([{"kind": "cast", "toDtype": outputDtype}], 0, outputDtype), [], 1
+        else:
+            plan = detectMatmulEpilogue(chain)
         wT = self.ops.transpose(weight)
         opts: dict = {"outputDtype": outputDtype}
         if plan is not None:

@@ -1,7 +1,10 @@
 // Context, memory, counters, replay graphs, events, argument validation and the
 // quantized-matmul seam of libtlcuda.
+#include <algorithm>
 #include <cstdlib>
 #include <cstring>
+#include <exception>
+#include <iterator>
 
 #include "tl_common.cuh"
 
@@ -154,6 +157,8 @@ int32_t tl_ctx_destroy(tl_ctx* ctx) {
   DeviceGuard guard(ctx->device);
   if (ctx->nccl_comm) tl_comm_destroy(ctx);
   cudaStreamSynchronize(ctx->stream);
+  ctx->pool.settle();
+  ctx->pool.trim(0);  // blocks still handed out stay the caller's, as before
   if (ctx->scratch) cudaFree(ctx->scratch);
   if (ctx->zscratch) cudaFree(ctx->zscratch);
   for (auto& p : ctx->retired_scratch) cudaFree(p.first);
@@ -231,13 +236,89 @@ int32_t tl_get_option(tl_ctx* ctx, const char* name, int64_t* out_value) {
   return TL_OK;
 }
 
+}  // extern "C"
+
 // ---- memory ---------------------------------------------------------------
+cudaError_t TlBlockPool::settle() {
+  cudaError_t e = cudaDeviceSynchronize();
+  if (e != cudaSuccess) return e;
+  for (auto& w : waiting) ready.emplace(w.second, w.first);
+  ready_bytes += waiting_bytes;
+  waiting.clear();
+  waiting_bytes = 0;
+  return cudaSuccess;
+}
+
+void TlBlockPool::trim(size_t keep) {
+  while (!ready.empty() && ready_bytes > keep) {
+    auto last = std::prev(ready.end());
+    cudaFree(last->second);
+    ready_bytes -= last->first;
+    ready.erase(last);
+  }
+}
+
+cudaError_t TlBlockPool::alloc(size_t bytes, void** out) {
+  // capacities in steps of 512 bytes, or of 1/64 to 1/32 of the size where that is more: sizes that differ a little
+  // from call to call share blocks, and little is lost in weights that stay
+  size_t step = 512;
+  while (bytes <= kLargestBytes && step < bytes / 64) step *= 2;
+  const size_t cap = bytes > SIZE_MAX / 2 ? bytes : std::max<size_t>(1, (bytes + step - 1) / step) * step;
+  std::lock_guard<std::mutex> hold(lock);
+  auto it = ready.lower_bound(cap);
+  if (it != ready.end() && it->first <= cap + cap / 4) {
+    *out = it->second;
+    ready_bytes -= it->first;
+    live[it->second] = it->first;
+    ready.erase(it);
+    return cudaSuccess;
+  }
+  size_t got = cap;
+  cudaError_t e = cudaMalloc(out, cap);
+  if (e == cudaErrorMemoryAllocation) {  // give back what is kept, then ask for no more than was asked for
+    cudaGetLastError();
+    if (settle() == cudaSuccess) trim(0);
+    got = bytes ? bytes : 1;
+    e = cudaMalloc(out, got);
+  }
+  if (e == cudaSuccess) live[*out] = got;
+  return e;
+}
+
+cudaError_t TlBlockPool::free(void* p, bool* known) {
+  std::lock_guard<std::mutex> hold(lock);
+  auto it = live.find(p);
+  *known = it != live.end();
+  if (!*known) {
+    for (auto& w : waiting) *known = *known || w.first == p;
+    for (auto& r : ready) *known = *known || r.second == p;
+    return *known ? cudaErrorInvalidValue : cudaSuccess;  // given back twice, or not from here
+  }
+  const size_t cap = it->second;
+  live.erase(it);
+  if (cap > kLargestBytes) return cudaFree(p);
+  waiting.emplace_back(p, cap);
+  waiting_bytes += cap;
+  if (waiting.size() < kWaitingBlocks && waiting_bytes < kWaitingBytes) return cudaSuccess;
+  cudaError_t e = settle();
+  trim(kKeptBytes - kWaitingBytes);
+  return e;
+}
+
+extern "C" {
+
 int32_t tl_alloc(tl_ctx* ctx, size_t bytes, void** out_dptr) {
   TL_CHECK_CTX(ctx);
   if (!out_dptr) return tl_set_error(ctx, TL_ERR_INVALID_ARG, "tl_alloc: null out pointer");
   *out_dptr = nullptr;
   DeviceGuard guard(ctx->device);
-  cudaError_t e = cudaMalloc(out_dptr, bytes ? bytes : 1);
+  // while a graph is being captured neither pooled nor new memory is given: the graph would keep the address
+  cudaError_t e;
+  try {
+    e = ctx->capturing ? cudaMalloc(out_dptr, bytes ? bytes : 1) : ctx->pool.alloc(bytes, out_dptr);
+  } catch (const std::exception&) {
+    e = cudaErrorMemoryAllocation;  // the host ran out
+  }
   if (e != cudaSuccess) {
     cudaGetLastError();
     return tl_set_error(ctx, e == cudaErrorMemoryAllocation ? TL_ERR_OOM : TL_ERR_CUDA,
@@ -250,6 +331,16 @@ int32_t tl_free(tl_ctx* ctx, void* dptr) {
   TL_CHECK_CTX(ctx);
   if (!dptr) return TL_OK;
   DeviceGuard guard(ctx->device);
+  if (ctx->capturing) TL_CUDA(ctx, cudaStreamSynchronize(ctx->stream));  // refused under capture, as it always was
+  bool known = false;
+  cudaError_t e;
+  try {
+    e = ctx->pool.free(dptr, &known);
+  } catch (const std::exception&) {
+    return tl_set_error(ctx, TL_ERR_OOM, "tl_free: out of host memory");
+  }
+  TL_CUDA(ctx, e);
+  if (known) return TL_OK;
   TL_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   TL_CUDA(ctx, cudaFree(dptr));
   return TL_OK;
