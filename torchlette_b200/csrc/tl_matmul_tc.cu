@@ -66,19 +66,6 @@ __device__ __noinline__ float dense_epilogue_outlined(const EpiParams& e, float 
   return tl_apply_epilogue(e, v, row, col, n);
 }
 
-// MN-major operand descriptor, 128-byte swizzle: the operand is stored [k][n] (n contiguous), staged as
-// 64-column slabs of [64 k x 128 bytes]; 8-k groups 1024 bytes apart (stride offset), slabs `slab_bytes`
-// apart (leading offset).
-__device__ __forceinline__ uint64_t dense_mn_desc(uint32_t smem_addr, uint32_t slab_bytes) {
-  uint64_t d = 0;
-  d |= uint64_t((smem_addr >> 4) & 0x3fffu);
-  d |= uint64_t((slab_bytes >> 4) & 0x3fffu) << 16;
-  d |= uint64_t((1024 >> 4) & 0x3fff) << 32;
-  d |= uint64_t(1) << 46;
-  d |= uint64_t(2) << 61;
-  return d;
-}
-
 // BMN = 1: B is stored [K, N] (the NN layout of matmul(a, b)); its tiles are staged and multiplied MN-major,
 // so no transposed copy of B is made.  BN must then be a multiple of 64.  AMN = 1: the same for an A stored
 // [K, M] (a transposed view of the first operand).
@@ -101,7 +88,7 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
   __shared__ uint32_t tmem_base_smem;
   __shared__ int abort_flag;
   uint8_t* stages = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dense_smem_raw) + 1023) & ~uintptr_t(1023));
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int tiles = p.m_tiles * p.n_tiles;
 
   if (threadIdx.x == 0) {
@@ -159,40 +146,41 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
       }
     }
   } else if (warp == 1) {
-    // ------------------------------ MMA issuer ------------------------------
-    if (lane == 0) {
+    // ------------------------------ MMA issuer: the whole warp, one lane elected ------------------------------
+    {
+      const uint32_t elected = elect_one(), tb = __shfl_sync(0xffffffffu, tmem_base, 0);
       int it = 0, tl = 0;
       for (int t = blockIdx.x; t < tiles && !abort_flag; t += gridDim.x, ++tl) {
         const int acc = tl % kAcc, use = tl / kAcc;
-        if (use >= 1 && !mbar_wait(&tempty_bar[acc], (use - 1) & 1, &abort_flag)) {
-          if (!abort_flag) { abort_flag = 1; atomicExch(p.status, TL_DEV_TIMEOUT_TMEM); }
+        if (use >= 1 && !mbar_wait_warp(&tempty_bar[acc], (use - 1) & 1, &abort_flag)) {
+          if (lane == 0 && !abort_flag) { abort_flag = 1; atomicExch(p.status, TL_DEV_TIMEOUT_TMEM); }
           break;
         }
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + uint32_t(acc * MH * BN);
+        const uint32_t d_tmem = tb + uint32_t(acc * MH * BN);
         bool ok = true;
         for (int ks = 0; ks < p.ksteps; ++ks, ++it) {
           const int s = it % STAGES;
-          if (!mbar_wait(&full_bar[s], (it / STAGES) & 1, &abort_flag)) {
-            if (!abort_flag) { abort_flag = 1; atomicExch(p.status, TL_DEV_TIMEOUT_FULL); }
+          if (!mbar_wait_warp(&full_bar[s], (it / STAGES) & 1, &abort_flag)) {
+            if (lane == 0 && !abort_flag) { abort_flag = 1; atomicExch(p.status, TL_DEV_TIMEOUT_FULL); }
             ok = false;
             break;
           }
           tc_fence_after();
           const uint32_t a_base = smem_u32(stages + size_t(s) * kStageBytes);
           const uint32_t b_base = a_base + kABytes;
+          const uint64_t ad = AMN ? make_mn_desc(a_base, kSlabBytes) : make_b_desc(a_base);
+          const uint64_t bd = BMN ? make_mn_desc(b_base, kSlabBytes) : make_b_desc(b_base);
 #pragma unroll
           for (int h = 0; h < MH; ++h)
 #pragma unroll
             for (int kk = 0; kk < kBK / 16; ++kk)
-              tc_mma_ss(d_tmem + uint32_t(h * BN),
-                        AMN ? dense_mn_desc(a_base + h * (kBM * 128) + kk * 2048, kSlabBytes) : make_b_desc(a_base + h * (kBM * 128) + kk * 32),
-                        BMN ? dense_mn_desc(b_base + kk * 2048, kSlabBytes) : make_b_desc(b_base + kk * 32), kIdesc,
-                        (ks > 0 || kk > 0) ? 1u : 0u);
-          tc_commit(&empty_bar[s]);  // the stage is free once these MMAs have read it
+              tc_mma_ss(d_tmem + uint32_t(h * BN), desc_at(ad, h * (kBM * 128) + kk * (AMN ? 2048 : 32)), desc_at(bd, kk * (BMN ? 2048 : 32)),
+                        kIdesc, (ks > 0 || kk > 0) ? 1u : 0u, elected);
+          tc_commit(&empty_bar[s], elected);  // the stage is free once these MMAs have read it
         }
         if (!ok) break;
-        tc_commit(&tfull_bar[acc]);
+        tc_commit(&tfull_bar[acc], elected);
       }
     }
   } else {

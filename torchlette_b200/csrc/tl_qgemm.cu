@@ -244,7 +244,7 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
   __shared__ uint32_t tmem_base_smem;
   __shared__ int abort_flag;
   uint8_t* stages = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(gemm_smem_raw) + 1023) & ~uintptr_t(1023));
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -299,44 +299,44 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
       }
     }
   } else if (warp == kMmaWarp) {
-    // ------------------------------ MMA issuer ------------------------------
-    if (lane == 0) {
+    // ------------------------------ MMA issuer: the whole warp, one lane elected ------------------------------
+    {
+      const uint32_t elected = elect_one(), tb = __shfl_sync(0xffffffffu, tmem_base, 0);
       int it = 0, tl = 0;
       WorkItem w;
       for (; get_work(p, tl, w) && !abort_flag; ++tl) {
         const int acc = tl & 1;
-        if (tl >= 2 && !mbar_wait(&tempty_bar[acc], ((tl >> 1) - 1) & 1, &abort_flag)) {
-          if (!abort_flag) { abort_flag = 1; atomicExch(p.status, TL_DEV_TIMEOUT_TMEM); }
+        if (tl >= 2 && !mbar_wait_warp(&tempty_bar[acc], ((tl >> 1) - 1) & 1, &abort_flag)) {
+          if (lane == 0 && !abort_flag) { abort_flag = 1; atomicExch(p.status, TL_DEV_TIMEOUT_TMEM); }
           break;
         }
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + uint32_t(acc * BN);
+        const uint32_t d_tmem = tb + uint32_t(acc * BN);
         bool ok = true;
         for (int ks = w.ks0; ks < w.ks0 + w.nks && ok; ++ks, ++it) {
           const int s = it % STAGES, sl = it % TS;
           TL_TR(1, it, 0);
-          ok = mbar_wait(&full_bar[s], (it / STAGES) & 1, &abort_flag);
+          ok = mbar_wait_warp(&full_bar[s], (it / STAGES) & 1, &abort_flag);
           TL_TR(1, it, 1);
-          ok = ok && mbar_wait(&aready_bar[sl], (it / TS) & 1, &abort_flag);
+          ok = ok && mbar_wait_warp(&aready_bar[sl], (it / TS) & 1, &abort_flag);
           TL_TR(1, it, 2);
           if (!ok) {
-            if (!abort_flag) { abort_flag = 1; atomicExch(p.status, TL_DEV_TIMEOUT_FULL); }
+            if (lane == 0 && !abort_flag) { abort_flag = 1; atomicExch(p.status, TL_DEV_TIMEOUT_FULL); }
             break;
           }
           tc_fence_after();
           const uint32_t a_base = smem_u32(stages + size_t(s) * kStageBytes + kWBytes);
-          const uint32_t a_tmem = tmem_base + uint32_t(2 * BN + sl * kSlotCols);
+          const uint32_t a_tmem = tb + uint32_t(2 * BN + sl * kSlotCols);
+          const uint64_t bdesc = make_b_desc(a_base);
 #pragma unroll
-          for (int kk = 0; kk < KSTEP / 16; ++kk) {
-            const uint64_t bdesc = make_b_desc(a_base + (kk >> 2) * kABox + (kk & 3) * 32);
-            tc_mma_ts(d_tmem, a_tmem + kk * 8, bdesc, kIdesc, (ks > w.ks0 || kk > 0) ? 1u : 0u);
-          }
-          tc_commit(&empty_bar[s]);      // the shared-memory stage is free once these MMAs have run
-          tc_commit(&slotfree_bar[sl]);  // and so is the TMEM operand slot
+          for (int kk = 0; kk < KSTEP / 16; ++kk)
+            tc_mma_ts(d_tmem, a_tmem + kk * 8, desc_at(bdesc, (kk >> 2) * kABox + (kk & 3) * 32), kIdesc, (ks > w.ks0 || kk > 0) ? 1u : 0u, elected);
+          tc_commit(&empty_bar[s], elected);      // the shared-memory stage is free once these MMAs have run
+          tc_commit(&slotfree_bar[sl], elected);  // and so is the TMEM operand slot
           TL_TR(1, it, 3);
         }
         if (!ok) break;
-        tc_commit(&tfull_bar[acc]);
+        tc_commit(&tfull_bar[acc], elected);
       }
     }
   } else if (warp < NCW) {
