@@ -127,3 +127,53 @@ def test_decode_hidden_values_not_finite(be, dtype, s, n):
     assert np.isinf(last[:2, :40]).all() and np.isfinite(last[:2, 40:]).all() and np.isnan(last[2:, 5]).all() and np.isfinite(last[2:, 6:]).all()
     for t in (q, k, v, out):
         t.destroy()
+
+
+@pytest.mark.parametrize("dtype", ["f16", "bf16"])
+@pytest.mark.parametrize("b,heads,kv_heads,d,s,n,causal", [
+    (1, 4, 1, 128, 5, 5, True), (1, 8, 8, 64, 17, 17, True), (1, 8, 2, 128, 32, 32, True), (2, 8, 2, 128, 33, 200, True),
+    (1, 4, 4, 64, 128, 128, True), (1, 4, 4, 128, 129, 130, True), (2, 6, 2, 64, 100, 511, True), (1, 3, 1, 128, 257, 300, True),
+    (1, 8, 2, 128, 200, 333, False), (1, 4, 2, 64, 700, 700, True), (3, 14, 2, 128, 40, 1000, True), (2, 32, 8, 128, 640, 641, True),
+    (4, 32, 8, 64, 300, 300, False)])
+def test_prefill(be, dtype, b, heads, kv_heads, d, s, n, causal):
+    check(be, b, heads, kv_heads, d, s, n, dtype, causal=causal)
+
+
+@pytest.mark.parametrize("dtype", ["f16", "bf16"])
+def test_prefill_growing_scores(be, dtype):
+    """Scores that climb from key to key: the running maximum moves at every step, by a little and by far."""
+    rng = np.random.default_rng(3)
+    s = n = 400
+    q = np.abs(rng.standard_normal((1, 4, s, 64)))
+    for slope in (0.01, 0.2):
+        ramp = (np.arange(n) * slope / 8)[None, None, :, None]
+        q_t, qr = store(be, q, dtype)
+        k_t, kr = store(be, rng.standard_normal((1, 2, n, 64)) * 0.1 + ramp, dtype)
+        v_t, vr = store(be, rng.standard_normal((1, 2, n, 64)), dtype)
+        out = be.ops.attention(q_t, k_t, v_t, n, 0.125, causal=True)
+        got = read(be, out).astype(np.float64)
+        ref = reference(qr, kr, vr, 0.125, True, None)
+        # scores up to 64 x 10 x 0.125 x 0.8: f32 products of that size are 2^-24 x 64 off, and exp turns that into a relative error
+        top = (np.abs(qr).sum(-1).max() * np.abs(kr).max()) * 0.125
+        assert (np.abs(got - ref) / np.maximum(1.0, np.abs(ref))).max() <= TOL[dtype] + 4 * top * 2.0 ** -23
+        for t in (q_t, k_t, v_t, out):
+            t.destroy()
+
+
+@pytest.mark.parametrize("dtype", ["f16", "bf16"])
+def test_prefill_hidden_values_not_finite(be, dtype):
+    rng = np.random.default_rng(11)
+    s, n = 70, 150
+    q, qr = store(be, rng.standard_normal((1, 4, s, 128)), dtype)
+    k, kr = store(be, rng.standard_normal((1, 2, n, 128)), dtype)
+    vf = rng.standard_normal((1, 2, n, 128))
+    vf[:, 0, n - 1, :40], vf[:, 1, n - 1, 5] = np.inf, np.nan
+    v, vr = store(be, vf, dtype)
+    out = be.ops.attention(q, k, v, n, 0.1, causal=True)
+    got = read(be, out).astype(np.float64)
+    ref = reference(qr[:, :, :s - 1], kr[:, :, :n - 1], vr[:, :, :n - 1], 0.1, True, None)
+    assert (np.abs(got[:, :s - 1] - ref) / np.maximum(1.0, np.abs(ref))).max() <= TOL[dtype]
+    last = got[0, s - 1].reshape(4, 128)
+    assert np.isinf(last[:2, :40]).all() and np.isfinite(last[:2, 40:]).all() and np.isnan(last[2:, 5]).all() and np.isfinite(last[2:, 6:]).all()
+    for t in (q, k, v, out):
+        t.destroy()

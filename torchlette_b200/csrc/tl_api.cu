@@ -834,8 +834,8 @@ typedef CUresult (*TlEncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_
                                     const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                     CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-bool tl_encode_tmap_2d(CUtensorMap* map, int elem_bytes, const void* base, uint64_t inner, uint64_t outer,
-                       uint64_t row_stride_bytes, uint32_t box_inner, uint32_t box_outer, int swizzle) {
+static bool encode_tmap(CUtensorMap* map, int elem_bytes, const void* base, int rank, const cuuint64_t* dims, const cuuint64_t* strides,
+                        const cuuint32_t* box, int swizzle) {
   static TlEncodeTiledFn fn = nullptr;
   if (!fn) {
     void* p = nullptr;
@@ -849,14 +849,25 @@ bool tl_encode_tmap_2d(CUtensorMap* map, int elem_bytes, const void* base, uint6
   const CUtensorMapDataType dt = elem_bytes == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8
                                  : elem_bytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_UINT16
                                                    : CU_TENSOR_MAP_DATA_TYPE_UINT32;
-  cuuint64_t dims[2] = {inner, outer};
-  cuuint64_t strides[1] = {row_stride_bytes};
-  cuuint32_t box[2] = {box_inner, box_outer};
-  cuuint32_t estr[2] = {1, 1};
+  const cuuint32_t estr[3] = {1, 1, 1};
   const CUtensorMapSwizzle sw = swizzle == 3 ? CU_TENSOR_MAP_SWIZZLE_128B
                                 : swizzle == 2 ? CU_TENSOR_MAP_SWIZZLE_64B
                                 : swizzle == 1 ? CU_TENSOR_MAP_SWIZZLE_32B
                                                : CU_TENSOR_MAP_SWIZZLE_NONE;
-  return fn(map, dt, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
+  return fn(map, dt, cuuint32_t(rank), const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+bool tl_encode_tmap_2d(CUtensorMap* map, int elem_bytes, const void* base, uint64_t inner, uint64_t outer,
+                       uint64_t row_stride_bytes, uint32_t box_inner, uint32_t box_outer, int swizzle) {
+  const cuuint64_t dims[2] = {inner, outer}, strides[1] = {row_stride_bytes};
+  const cuuint32_t box[2] = {box_inner, box_outer};
+  return encode_tmap(map, elem_bytes, base, 2, dims, strides, box, swizzle);
+}
+
+bool tl_encode_tmap_3d(CUtensorMap* map, int elem_bytes, const void* base, uint64_t inner, uint64_t outer, uint64_t slices,
+                       uint64_t row_stride_bytes, uint64_t slice_stride_bytes, uint32_t box_inner, uint32_t box_outer, int swizzle) {
+  const cuuint64_t dims[3] = {inner, outer, slices}, strides[2] = {row_stride_bytes, slice_stride_bytes};
+  const cuuint32_t box[3] = {box_inner, box_outer, 1};
+  return encode_tmap(map, elem_bytes, base, 3, dims, strides, box, swizzle);
 }

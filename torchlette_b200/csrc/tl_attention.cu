@@ -8,6 +8,7 @@
 //            4000 keys x 128 f16 (131 MB): 27.1 us = 4.8 TB/s, about 5 us of it launch, first loads and merging (964 us
 //            one CTA per query head, which read the cache once per query head along a serial chain); 2 x 8 x 700: 6.9
 //            us (171).
+//   prefill  more query rows, f16 / bf16 without a mask tensor: tl_attention_tc.cu.
 //   general  everything else: attention_kernel, one CTA per query row.
 #include <algorithm>
 #include <cfloat>
@@ -155,7 +156,7 @@ __device__ __forceinline__ void decode_merge(const DecodeArgs& p, float* sm, int
       attention_row_warp<AT, D>(reinterpret_cast<const AT*>(p.q) + ((int64_t(b) * p.n_heads + h) * p.q_len + qi) * D,
                                 reinterpret_cast<const AT*>(p.k) + kv, reinterpret_cast<const AT*>(p.v) + kv,
                                 reinterpret_cast<AT*>(p.out) + at, p.kv_len - p.q_len + qi + 1, p.scale,
-                                p.mask ? p.mask + int64_t(qi) * p.kv_len : nullptr, d >> 5);
+                                p.mask ? p.mask + int64_t(qi) * p.kv_len : nullptr, d >> 5, 1);
     } else {
       reinterpret_cast<AT*>(p.out)[at + d] = DT<AT>::from_f32(v);
     }
@@ -510,6 +511,10 @@ int32_t tl_attention(tl_ctx* ctx, const void* q, const void* k_cache, const void
     if (dtype == TL_F32) e = head_dim == 64 ? launch_decode_f32<64>(ctx, p, groups) : launch_decode_f32<128>(ctx, p, groups);
     else if (dtype == TL_F16) e = head_dim == 64 ? launch_decode_mma<__half, 64>(ctx, p, groups) : launch_decode_mma<__half, 128>(ctx, p, groups);
     else e = head_dim == 64 ? launch_decode_mma<__nv_bfloat16, 64>(ctx, p, groups) : launch_decode_mma<__nv_bfloat16, 128>(ctx, p, groups);
+  } else if (tl_attention_tc_applicable(q, k_cache, v_cache, out, dtype, rows, head_dim, scale, mask)) {
+    int32_t rc = tl_launch_attention_tc(ctx, q, k_cache, v_cache, out, dtype, batch, n_heads, n_kv_heads, q_len, head_dim, kv_len, kv_capacity,
+                                        scale, causal);
+    if (rc != TL_OK) return rc;
   } else {
     if (smem > 48 * 1024) cudaFuncSetAttribute(attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     attention_kernel<<<unsigned(batch * n_heads * q_len), 128, smem, ctx->stream>>>(q, k_cache, v_cache, out, dtype, int(n_heads), int(n_kv_heads),

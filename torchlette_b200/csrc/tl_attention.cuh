@@ -11,11 +11,11 @@ constexpr float kLog2e = 1.4426950408889634f;
 
 // The tensor-core kernels multiply whole tiles: a key hidden from a row has probability zero there, and zero times
 // an infinite or NaN value would still poison the row.  A row whose result is not finite is therefore done again
-// here, where hidden keys are never read: two passes, f32, a lane per D / 32 dimensions.  part >= 0: only the
-// dimensions from 32 * part on, 32 of them, are stored.
+// here, where hidden keys are never read: two passes, f32, a lane per D / 32 dimensions.  Only the
+// dimensions from 32 * first on, 32 * count of them, are stored.
 template <typename AT, int D>
 __device__ __noinline__ void attention_row_warp(const AT* q, const AT* k, const AT* v, AT* out, int keys, float scale, const float* mask,
-                                                int part) {
+                                                int first, int count) {
   constexpr int V = D / 32;
   const int lane = threadIdx.x & 31;
   float qf[V], o[V], mx = -FLT_MAX, sum = 0.f;
@@ -44,7 +44,7 @@ __device__ __noinline__ void attention_row_warp(const AT* q, const AT* k, const 
   const float inv = 1.f / sum;
 #pragma unroll
   for (int i = 0; i < V; ++i)
-    if (part < 0 || part == i) out[lane + 32 * i] = DT<AT>::from_f32(o[i] * inv);
+    if (i >= first && i < first + count) out[lane + 32 * i] = DT<AT>::from_f32(o[i] * inv);
 }
 
 // Two probabilities as 16-bit terms whose sum carries (nearly) all 24 bits of each: p rounded, then what is left

@@ -260,6 +260,12 @@ TlDenseTcChoice tl_dense_tc_choose(int64_t m, int64_t n, int64_t k, int sms, int
 int32_t tl_launch_dense_tc(tl_ctx* ctx, const void* a, const void* b, void* out, int64_t m, int64_t n, int64_t k, int32_t dtype,
                            int32_t out_dtype, const struct EpiParams& epi, const void* colscale = nullptr,
                            int32_t colscale_dtype = 0, float colscale_mul = 1.0f, bool b_mn = false, bool a_mn = false);
+// Attention of many query rows (tl_attention_tc.cu): f16 / bf16, head dimension 64 or 128, more than 16 rows per KV head.
+bool tl_attention_tc_applicable(const void* q, const void* k, const void* v, const void* out, int32_t dtype, int64_t rows, int64_t head_dim,
+                                float scale, const float* mask);
+int32_t tl_launch_attention_tc(tl_ctx* ctx, const void* q, const void* k, const void* v, void* out, int32_t dtype, int64_t batch,
+                               int64_t n_heads, int64_t n_kv_heads, int64_t q_len, int64_t head_dim, int64_t kv_len, int64_t capacity,
+                               float scale, int32_t causal);
 bool tl_qgemv_stream_applicable(const tl_variant& v, int64_t m, int64_t k, int32_t a_dtype, const tl_quant_desc& q);
 void tl_qgemv_stream_geometry(tl_ctx* ctx, const tl_variant& v, int32_t m, int64_t tiles, int64_t k, int* grid, int* block,
                               size_t* smem);

@@ -14,6 +14,10 @@
 // swizzle: 0 none, 1 32B, 2 64B, 3 128B.  Returns false on failure.
 bool tl_encode_tmap_2d(CUtensorMap* map, int elem_bytes, const void* base, uint64_t inner, uint64_t outer,
                        uint64_t row_stride_bytes, uint32_t box_inner, uint32_t box_outer, int swizzle);
+// The same over a [slices, outer, inner] array with a pitch of its own between slices: boxes of one slice, zeros
+// beyond a slice's rows.
+bool tl_encode_tmap_3d(CUtensorMap* map, int elem_bytes, const void* base, uint64_t inner, uint64_t outer, uint64_t slices,
+                       uint64_t row_stride_bytes, uint64_t slice_stride_bytes, uint32_t box_inner, uint32_t box_outer, int swizzle);
 
 #ifdef __CUDACC__
 constexpr int kWaitTimeoutIters = 1 << 22;  // each try_wait blocks for a while; this bounds a wait to seconds
@@ -55,6 +59,12 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
       ::"r"(smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+      ::"r"(smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
       : "memory");
 }
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* map) {
