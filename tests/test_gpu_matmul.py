@@ -402,6 +402,37 @@ def test_dense_tensor_core_several_tiles_per_cta(backend, bn, mh):
         t.destroy()
 
 
+@pytest.mark.parametrize("bn", [256, 128])
+@pytest.mark.parametrize("parts", [2, 4, 8])
+@pytest.mark.parametrize("m,k,n,dtype,trans_b", [(40, 512, 72, "f16", True), (130, 1000, 700, "bf16", True), (257, 4096, 520, "f16", False),
+                                                 (64, 960, 264, "bf16", False)])
+def test_dense_tensor_core_cut_along_k(backend, bn, parts, m, k, n, dtype, trans_b):
+    """Tiles whose K is shared by a cluster: ranges of unequal length, ragged rows, columns and k, both layouts of B."""
+    be = backend
+    rng = np.random.default_rng(bn + m + parts)
+    x, x_v = _to_dev(be, rng.uniform(-1, 1, m * k).astype(np.float32), [m, k], dtype)
+    shape = [n, k] if trans_b else [k, n]
+    w, w_v = _to_dev(be, (rng.uniform(-1, 1, n * k) * 0.2).astype(np.float32), shape, dtype)
+    bias_v = rng.uniform(-1, 1, n).astype(np.float32)
+    bias_t = be.ops.tensorFromArray(bias_v, [n], "f32")
+    plan = tb.detectMatmulEpilogue([("add", bias_t), ("silu", None), ("cast", dtype)])
+    op = be.ops.transpose if trans_b else (lambda t: t)
+    ref = (lambda a, b: _ref(a, b.T if trans_b else b))
+    be.forceVariant((B.TL_FAMILY_MATMUL, 2, bn, 0, 1, parts))
+    try:
+        assert be.planMatmul(m, n, k, dtype, dtype, transB=trans_b)["choice"][5] == parts
+        y = be.ops.matmul(x, op(w), {"epilogue": plan[0], "epilogueInputs": plan[1]})
+        assert _rel(_read_f32(be, y), _ref(x_v, w_v.T if trans_b else w_v, bias_v, "silu")) <= 1e-2
+        xp, xp_v = _to_dev(be, _pattern(m * k, 0), [m, k], dtype)  # exactly representable: bit-equal
+        wp, wp_v = _to_dev(be, _pattern(n * k, 3), shape, dtype)
+        yp = be.ops.matmul(xp, op(wp))
+        np.testing.assert_array_equal(_read_f32(be, yp), ref(xp_v, wp_v))
+    finally:
+        be.forceVariant(None)
+    for t in (x, w, bias_t, y, xp, wp, yp):
+        t.destroy()
+
+
 @pytest.mark.parametrize("out_dtype", ["f32", "bf16"])
 @pytest.mark.parametrize("act", ["relu", "silu", "gelu", "gelu_erf", "sigmoid", "tanh"])
 def test_dense_tensor_core_unary_modes_on_two_half_tiles(backend, out_dtype, act):

@@ -267,12 +267,12 @@ extern "C" int32_t tl_matmul(tl_ctx* ctx, const void* a, const void* b, void* ou
       bool ra_mn, rb_mn;
       dense_mn_operands(trans_a != 0, trans_b != 0, m, n, &ra_mn, &rb_mn);
       const TlDenseTcChoice ch = tl_dense_tc_choose(m, n, k, ctx->sm_count, f ? ctx->forced.p0 : 0, f ? ctx->forced.p2 : 0,
-                                                    (ra_mn || rb_mn) ? 64 : 16);
-      receipt_only->choice.p0 = ch.bn; receipt_only->choice.p1 = ch.stages; receipt_only->choice.p2 = ch.mh;
+                                                    (ra_mn || rb_mn) ? 64 : 16, ra_mn ? 1 : f ? std::max(1, ctx->forced.p3) : 0);
+      receipt_only->choice.p0 = ch.bn; receipt_only->choice.p1 = ch.stages; receipt_only->choice.p2 = ch.mh; receipt_only->choice.p3 = ch.parts;
       receipt_only->grid[0] = ch.grid; receipt_only->grid[1] = 1; receipt_only->grid[2] = 1;
       receipt_only->block = 576;
     }
-    receipt_only->split_k = 1;
+    receipt_only->split_k = std::max(1, receipt_only->choice.kernel == kTc ? receipt_only->choice.p3 : 1);
     receipt_only->from_tuning_cache = 0;
     receipt_only->epilogue_engaged = has_ops ? 1 : 0;
     return TL_OK;

@@ -69,7 +69,11 @@ __device__ __noinline__ float dense_epilogue_outlined(const EpiParams& e, float 
 // BMN = 1: B is stored [K, N] (the NN layout of matmul(a, b)); its tiles are staged and multiplied MN-major,
 // so no transposed copy of B is made.  BN must then be a multiple of 64.  AMN = 1: the same for an A stored
 // [K, M] (a transposed view of the first operand).
-template <typename AT, int BN, int STAGES, int MH, int BMN, int AMN>
+// KSP = 1: few tiles, cut along K.  A cluster of CTAs (its size is the launch's) works on one tile, a K range each; the
+// f32 partial tiles meet in distributed shared memory, where the stages were, and each CTA sums, in rank order, and
+// finishes its share of the tile's columns: no scratch, no atomics, and the epilogue is cut with the rest.
+// 256 x 4096 x 4096 occupied 64 of 148 SMs for 64 steps each; see the choice of the tile for the figures.
+template <typename AT, int BN, int STAGES, int MH, int BMN, int AMN, int KSP>
 __global__ void __launch_bounds__(kDenseThreads, 1)
 dense_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap bmap, DenseTcArgs p, EpiParams epi) {
   static_assert(BN % 16 == 0 && BN >= 16 && BN <= 256, "MMA N");
@@ -89,7 +93,12 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
   __shared__ int abort_flag;
   uint8_t* stages = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dense_smem_raw) + 1023) & ~uintptr_t(1023));
   const int warp = warp_index(), lane = threadIdx.x & 31;
+  static_assert(KSP == 0 || (MH == 1 && STAGES * kStageBytes >= kBM * BN * 4), "a cut tile's partial sums fit where the stages were");
   const int tiles = p.m_tiles * p.n_tiles;
+  const int parts = KSP ? int(cluster_size()) : 1, part = KSP ? int(cluster_rank()) : 0;
+  // this CTA's walk over the tiles, and its k steps of each
+  const int first = int(blockIdx.x) / parts, stride = KSP ? tiles : int(gridDim.x);
+  const int per_part = (p.ksteps + parts - 1) / parts, ks_beg = part * per_part, ks_end = KSP ? min(p.ksteps, ks_beg + per_part) : p.ksteps;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -112,15 +121,89 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
   tc_fence_after();
   const uint32_t tmem_base = tmem_base_smem;
 
+  // sixteen outputs of one row, from column col0 on: op chain and store
+  const bool approx = p.out_dtype != TL_F32;
+  enum { kPlain, kGelu, kRelu, kSilu, kUnary, kGeneric };
+  const int fu = epi.fast_unary;
+  const int mode = !epi.fast ? kGeneric
+                 : fu == 0 ? kPlain
+                 : (approx && fu == TL_UNARY_GELU_TANH) ? kGelu
+                 : fu == TL_UNARY_RELU ? kRelu
+                 : (approx && fu == TL_UNARY_SILU) ? kSilu : kUnary;
+  const float* bias = epi.fast ? epi.fast_bias : nullptr;
+  const float alpha = epi.alpha;
+  const int esz = p.out_dtype == TL_F32 ? 4 : 2;
+  const bool vec_ok = (p.n * esz) % 16 == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
+  auto finish16 = [&](int64_t row, int64_t col0, float (&o)[16]) {
+    const int jmax = int(min(int64_t(16), p.n - col0));
+    if (p.colscale) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) o[j] *= j < jmax ? tl_load_scale(p.colscale, p.colscale_dtype, col0 + j) * p.colscale_mul : 0.f;
+    }
+    if (mode != kGeneric) {
+      if (bias) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) o[j] = fmaf(o[j], alpha, j < jmax ? __ldg(bias + col0 + j) : 0.f);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) o[j] *= alpha;
+      }
+      if (mode == kGelu) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+          o[j] = (0.5f * o[j]) * (1.f + tl_tanh_approx(0.7978845608f * (o[j] + 0.044715f * (o[j] * (o[j] * o[j])))));
+      } else if (mode == kRelu) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) o[j] = fmaxf(o[j], 0.f);
+      } else if (mode == kSilu) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) o[j] = __fdividef(o[j], 1.f + __expf(-o[j]));
+      } else if (mode == kUnary) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) o[j] = dense_unary_outlined(fu, approx, o[j]);
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+        if (j < jmax) o[j] = dense_epilogue_outlined(epi, o[j], row, col0 + j, p.n);
+    }
+    uint8_t* optr = reinterpret_cast<uint8_t*>(p.out) + (row * p.n + col0) * esz;
+    if (jmax == 16 && vec_ok) {
+      if (p.out_dtype == TL_F32) {
+#pragma unroll
+        for (int q4 = 0; q4 < 4; ++q4)
+          reinterpret_cast<float4*>(optr)[q4] = make_float4(o[4 * q4], o[4 * q4 + 1], o[4 * q4 + 2], o[4 * q4 + 3]);
+      } else {
+        uint32_t w[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          if (p.out_dtype == TL_F16) {
+            const __half2 h = __floats2half2_rn(o[2 * j], o[2 * j + 1]);
+            w[j] = *reinterpret_cast<const uint32_t*>(&h);
+          } else {
+            const __nv_bfloat162 h = __floats2bfloat162_rn(o[2 * j], o[2 * j + 1]);
+            w[j] = *reinterpret_cast<const uint32_t*>(&h);
+          }
+        }
+        reinterpret_cast<uint4*>(optr)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+        reinterpret_cast<uint4*>(optr)[1] = make_uint4(w[4], w[5], w[6], w[7]);
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+        if (j < jmax) tl_store_out(p.out, p.out_dtype, row * p.n + col0 + j, o[j]);
+    }
+  };
+
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
     if (lane == 0) {
       tma_prefetch_desc(&amap);
       tma_prefetch_desc(&bmap);
       int it = 0;
-      for (int t = blockIdx.x; t < tiles && !abort_flag; t += gridDim.x) {
+      for (int t = first; t < tiles && !abort_flag; t += stride) {
         const int n_tile = t / p.m_tiles, m_tile = t - n_tile * p.m_tiles;
-        for (int ks = 0; ks < p.ksteps; ++ks, ++it) {
+        for (int ks = ks_beg; ks < ks_end; ++ks, ++it) {
           const int s = it % STAGES;
           if (it >= STAGES && !mbar_wait(&empty_bar[s], ((it / STAGES) - 1) & 1, &abort_flag)) {
             if (!abort_flag) { abort_flag = 1; atomicExch(p.status, TL_DEV_TIMEOUT_EMPTY); }
@@ -150,7 +233,7 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
     {
       const uint32_t elected = elect_one(), tb = __shfl_sync(0xffffffffu, tmem_base, 0);
       int it = 0, tl = 0;
-      for (int t = blockIdx.x; t < tiles && !abort_flag; t += gridDim.x, ++tl) {
+      for (int t = first; t < tiles && !abort_flag; t += stride, ++tl) {
         const int acc = tl % kAcc, use = tl / kAcc;
         if (use >= 1 && !mbar_wait_warp(&tempty_bar[acc], (use - 1) & 1, &abort_flag)) {
           if (lane == 0 && !abort_flag) { abort_flag = 1; atomicExch(p.status, TL_DEV_TIMEOUT_TMEM); }
@@ -159,7 +242,7 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
         tc_fence_after();
         const uint32_t d_tmem = tb + uint32_t(acc * MH * BN);
         bool ok = true;
-        for (int ks = 0; ks < p.ksteps; ++ks, ++it) {
+        for (int ks = ks_beg; ks < ks_end; ++ks, ++it) {
           const int s = it % STAGES;
           if (!mbar_wait_warp(&full_bar[s], (it / STAGES) & 1, &abort_flag)) {
             if (lane == 0 && !abort_flag) { abort_flag = 1; atomicExch(p.status, TL_DEV_TIMEOUT_FULL); }
@@ -176,7 +259,7 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
 #pragma unroll
             for (int kk = 0; kk < kBK / 16; ++kk)
               tc_mma_ss(d_tmem + uint32_t(h * BN), desc_at(ad, h * (kBM * 128) + kk * (AMN ? 2048 : 32)), desc_at(bd, kk * (BMN ? 2048 : 32)),
-                        kIdesc, (ks > 0 || kk > 0) ? 1u : 0u, elected);
+                        kIdesc, (ks > ks_beg || kk > 0) ? 1u : 0u, elected);
           tc_commit(&empty_bar[s], elected);  // the stage is free once these MMAs have read it
         }
         if (!ok) break;
@@ -194,20 +277,8 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
     const uint32_t lane_addr = uint32_t(quad * 32) << 16;
     constexpr int kChunksN = BN / 16;
     const int cbeg = cpart * kChunksN / kColParts, cend = (cpart + 1) * kChunksN / kColParts;
-    const bool approx = p.out_dtype != TL_F32;
-    enum { kPlain, kGelu, kRelu, kSilu, kUnary, kGeneric };
-    const int fu = epi.fast_unary;
-    const int mode = !epi.fast ? kGeneric
-                   : fu == 0 ? kPlain
-                   : (approx && fu == TL_UNARY_GELU_TANH) ? kGelu
-                   : fu == TL_UNARY_RELU ? kRelu
-                   : (approx && fu == TL_UNARY_SILU) ? kSilu : kUnary;
-    const float* bias = epi.fast ? epi.fast_bias : nullptr;
-    const float alpha = epi.alpha;
-    const int esz = p.out_dtype == TL_F32 ? 4 : 2;
-    const bool vec_ok = (p.n * esz) % 16 == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
     int tl = 0;
-    for (int t = blockIdx.x; t < tiles; t += gridDim.x, ++tl) {
+    for (int t = first; t < tiles; t += stride, ++tl) {
       const int acc = tl % kAcc;
       const int n_tile = t / p.m_tiles, m_tile = t - n_tile * p.m_tiles;
       const int64_t row = int64_t(m_tile) * kTileM + ehalf * kBM + quad * 32 + lane;  // this thread's output row
@@ -228,65 +299,14 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
 #pragma unroll
         for (int j = 0; j < 16; ++j) o[j] = __uint_as_float(vn[j]);
         if (ch + 1 < cend) tmem_ld16(tmem_base + lane_addr + acc_col + uint32_t((ch + 1) * 16), vn);  // next chunk in flight
+        if (KSP) {  // the partial tile, column by column (the accumulator is complete, so the stages are free)
+          float* sums = reinterpret_cast<float*>(stages) + size_t(ch * 16) * kBM + quad * 32 + lane;
+#pragma unroll
+          for (int j = 0; j < 16; ++j) sums[j * kBM] = o[j];
+          continue;
+        }
         if (!row_ok || col0 >= p.n) continue;
-        const int jmax = int(min(int64_t(16), p.n - col0));
-        if (p.colscale) {
-#pragma unroll
-          for (int j = 0; j < 16; ++j) o[j] *= j < jmax ? tl_load_scale(p.colscale, p.colscale_dtype, col0 + j) * p.colscale_mul : 0.f;
-        }
-        if (mode != kGeneric) {
-          if (bias) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) o[j] = fmaf(o[j], alpha, j < jmax ? __ldg(bias + col0 + j) : 0.f);
-          } else {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) o[j] *= alpha;
-          }
-          if (mode == kGelu) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j)
-              o[j] = (0.5f * o[j]) * (1.f + tl_tanh_approx(0.7978845608f * (o[j] + 0.044715f * (o[j] * (o[j] * o[j])))));
-          } else if (mode == kRelu) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) o[j] = fmaxf(o[j], 0.f);
-          } else if (mode == kSilu) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) o[j] = __fdividef(o[j], 1.f + __expf(-o[j]));
-          } else if (mode == kUnary) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) o[j] = dense_unary_outlined(fu, approx, o[j]);
-          }
-        } else {
-#pragma unroll
-          for (int j = 0; j < 16; ++j)
-            if (j < jmax) o[j] = dense_epilogue_outlined(epi, o[j], row, col0 + j, p.n);
-        }
-        uint8_t* optr = reinterpret_cast<uint8_t*>(p.out) + (row * p.n + col0) * esz;
-        if (jmax == 16 && vec_ok) {
-          if (p.out_dtype == TL_F32) {
-#pragma unroll
-            for (int q4 = 0; q4 < 4; ++q4)
-              reinterpret_cast<float4*>(optr)[q4] = make_float4(o[4 * q4], o[4 * q4 + 1], o[4 * q4 + 2], o[4 * q4 + 3]);
-          } else {
-            uint32_t w[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              if (p.out_dtype == TL_F16) {
-                const __half2 h = __floats2half2_rn(o[2 * j], o[2 * j + 1]);
-                w[j] = *reinterpret_cast<const uint32_t*>(&h);
-              } else {
-                const __nv_bfloat162 h = __floats2bfloat162_rn(o[2 * j], o[2 * j + 1]);
-                w[j] = *reinterpret_cast<const uint32_t*>(&h);
-              }
-            }
-            reinterpret_cast<uint4*>(optr)[0] = make_uint4(w[0], w[1], w[2], w[3]);
-            reinterpret_cast<uint4*>(optr)[1] = make_uint4(w[4], w[5], w[6], w[7]);
-          }
-        } else {
-#pragma unroll
-          for (int j = 0; j < 16; ++j)
-            if (j < jmax) tl_store_out(p.out, p.out_dtype, row * p.n + col0 + j, o[j]);
-        }
+        finish16(row, col0, o);
       }
       tc_fence_before();
       __syncwarp();
@@ -294,6 +314,30 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
     }
   }
 
+  if (KSP) {
+    __syncwarp();
+    cluster_sync_all();
+    if (warp >= kEpiWarp0) {
+      const int quad = warp & 3, cols = BN / parts, n_tile = first / p.m_tiles, m_tile = first - n_tile * p.m_tiles;
+      const int64_t row = int64_t(m_tile) * kTileM + quad * 32 + lane;
+      for (int c = ((warp - kEpiWarp0) >> 2) * 16; c < cols; c += 64) {
+        const int64_t col0 = int64_t(n_tile) * BN + part * cols + c;
+        if (row >= p.m || col0 >= p.n) continue;
+        const float* at = reinterpret_cast<const float*>(stages) + size_t(part * cols + c) * kBM + quad * 32 + lane;
+        float o[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) o[j] = 0.f;
+        for (int r = 0; r < parts; ++r) {
+          const uint32_t from = mapa_u32(at, uint32_t(r));
+#pragma unroll
+          for (int j = 0; j < 16; ++j) o[j] += ld_cluster_f32(from + uint32_t(j * kBM * 4));
+        }
+        finish16(row, col0, o);
+      }
+    }
+    __syncwarp();
+    cluster_sync_all();  // no CTA leaves while another reads its sums
+  }
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {
@@ -302,12 +346,33 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
   }
 }
 
+template <typename AT, int BN, int STAGES, int BMN>
+cudaError_t launch_dense_ksplit(int tiles, int parts, cudaStream_t s, const CUtensorMap& amap, const CUtensorMap& bmap, const DenseTcArgs& p,
+                                const EpiParams& e) {
+  constexpr size_t smem = size_t(STAGES) * (kBM * 128 + BN * 128) + 1024;
+  auto kern = dense_tc_kernel<AT, BN, STAGES, 1, BMN, 0, 1>;
+  cudaError_t rc = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  if (rc != cudaSuccess) return rc;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(unsigned(tiles * parts));
+  cfg.blockDim = dim3(kDenseThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = unsigned(parts);
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, amap, bmap, p, e);
+}
+
 template <typename AT, int BN, int STAGES, int MH, int BMN = 0, int AMN = 0>
 cudaError_t launch_dense(int grid, cudaStream_t s, const CUtensorMap& amap, const CUtensorMap& bmap, const DenseTcArgs& p,
                          const EpiParams& e) {
   constexpr size_t smem = size_t(STAGES) * (kBM * MH * 128 + BN * 128) + 1024;
   static_assert(smem <= 227 * 1024, "shared memory per CTA");
-  auto kern = dense_tc_kernel<AT, BN, STAGES, MH, BMN, AMN>;
+  auto kern = dense_tc_kernel<AT, BN, STAGES, MH, BMN, AMN, 0>;
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
   kern<<<grid, kDenseThreads, smem, s>>>(amap, bmap, p, e);
   return cudaGetLastError();
@@ -339,9 +404,9 @@ constexpr DenseCfg kDenseCfgs[] = {{1, 256, 4, 0.424f}, {1, 224, 5, 0.410f}, {1,
                                    {2, 208, 3, 0.684f}, {2, 192, 4, 0.580f}, {2, 176, 4, 0.586f}, {2, 160, 4, 0.583f}};
 }  // namespace
 
-TlDenseTcChoice tl_dense_tc_choose(int64_t m, int64_t n, int64_t k, int sms, int forced_bn, int forced_mh, int bn_multiple) {
+TlDenseTcChoice tl_dense_tc_choose(int64_t m, int64_t n, int64_t k, int sms, int forced_bn, int forced_mh, int bn_multiple, int forced_parts) {
   const int64_t ksteps = (k + kBK - 1) / kBK;
-  TlDenseTcChoice best{128, 1, 6, 1, 1e300};
+  TlDenseTcChoice best{128, 1, 6, 1, 1, 1e300};
   for (const DenseCfg& c : kDenseCfgs) {
     if (c.bn % bn_multiple != 0) continue;  // an MN-major operand is staged in 64-column slabs
     if (forced_bn > 0) {
@@ -354,7 +419,19 @@ TlDenseTcChoice tl_dense_tc_choose(int64_t m, int64_t n, int64_t k, int sms, int
     const double main_us = double(ksteps) * c.step_us;
     const double tile = c.mh == 1 ? std::max(main_us, 0.012 * c.bn + 0.5) + 0.3 : main_us + 0.0094 * c.bn + 0.5;
     const double cost = double((t + sms - 1) / sms) * tile;
-    if (cost < best.cost_us) best = TlDenseTcChoice{c.bn, c.mh, c.stages, int(std::min<int64_t>(sms, t)), cost};
+    if (cost < best.cost_us && forced_parts <= 1) best = TlDenseTcChoice{c.bn, c.mh, c.stages, 1, int(std::min<int64_t>(sms, t)), cost};
+    // Cut along K (forced_parts 0: free, 1: not, else that many): one wave of clusters (of clusters of 8 about nine fit
+    // at a time), every part some steps; the meeting in shared memory measured 4.5 us.  bf16 + gelu, us uncut / cut:
+    // 256 x 4096 x 4096 28 / 20 (2 ranges), 512 x 1024 x 4096 28 / 16 (4), 100 x 2048 x 8192 48 / 19 (8),
+    // 333 x 4096 x 12288 71 / 50 (2); 700 x 2000 x 3000, whose tiles nearly fill the chip, 25 either way.
+    if (c.mh != 1 || (c.bn != 256 && c.bn != 128)) continue;
+    for (int parts : {2, 4, 8}) {
+      const int64_t per = (ksteps + parts - 1) / parts;
+      if ((parts - 1) * per >= ksteps) continue;  // a part would be empty
+      if (forced_parts > 1 ? parts != forced_parts : (forced_parts == 1 || t * parts > (parts == 8 ? sms / 2 : sms) || per < 4)) continue;
+      const double cut = double(per) * c.step_us + 0.012 * c.bn / parts + 5.0;
+      if (cut < best.cost_us) best = TlDenseTcChoice{c.bn, c.mh, c.stages, parts, int(t) * parts, cut};
+    }
   }
   return best;
 }
@@ -364,9 +441,9 @@ int32_t tl_launch_dense_tc(tl_ctx* ctx, const void* a, const void* b, void* out,
                            bool b_mn, bool a_mn) {
   const bool forced = ctx->has_forced && ctx->forced.family == TL_FAMILY_MATMUL && ctx->forced.kernel == 2 && ctx->forced.p0 > 0;
   const TlDenseTcChoice ch = tl_dense_tc_choose(m, n, k, ctx->sm_count, forced ? ctx->forced.p0 : 0, forced ? ctx->forced.p2 : 0,
-                                                (b_mn || a_mn) ? 64 : 16);
+                                                (b_mn || a_mn) ? 64 : 16, a_mn ? 1 : forced ? std::max(1, ctx->forced.p3) : 0);
   const int bn = ch.bn, mh = ch.mh, grid = ch.grid;
-  if (forced && (bn != ctx->forced.p0 || mh != (ctx->forced.p2 == 2 ? 2 : 1)))
+  if (forced && (bn != ctx->forced.p0 || mh != (ctx->forced.p2 == 2 ? 2 : 1) || (ctx->forced.p3 > 1 && ch.parts != ctx->forced.p3)))
     return tl_set_error(ctx, TL_ERR_INVALID_ARG, "tl_matmul: no tensor-core tile with BN=%d MH=%d", ctx->forced.p0, ctx->forced.p2);
   const int tile_m = kBM * mh;
   DenseTcArgs p{};
@@ -384,11 +461,23 @@ int32_t tl_launch_dense_tc(tl_ctx* ctx, const void* a, const void* b, void* out,
     return tl_set_error(ctx, TL_ERR_CUDA, "tl_matmul: cuTensorMapEncodeTiled failed (m=%lld n=%lld k=%lld)", (long long)m,
                         (long long)n, (long long)k);
   cudaError_t e = cudaErrorInvalidValue;
+#define TL_DENSE_KSPLIT_CASE(BN_, ST_)                                                                                          \
+  if (bn == BN_) {                                                                                                              \
+    if (b_mn)                                                                                                                   \
+      e = dtype == TL_F16 ? launch_dense_ksplit<__half, BN_, ST_, 1>(grid / ch.parts, ch.parts, ctx->stream, amap, bmap, p, epi) \
+                          : launch_dense_ksplit<__nv_bfloat16, BN_, ST_, 1>(grid / ch.parts, ch.parts, ctx->stream, amap, bmap, p, epi); \
+    else                                                                                                                        \
+      e = dtype == TL_F16 ? launch_dense_ksplit<__half, BN_, ST_, 0>(grid / ch.parts, ch.parts, ctx->stream, amap, bmap, p, epi) \
+                          : launch_dense_ksplit<__nv_bfloat16, BN_, ST_, 0>(grid / ch.parts, ch.parts, ctx->stream, amap, bmap, p, epi); \
+  }
 #define TL_DENSE_CASE(MH_, BN_, ST_)                                                                          \
   if (mh == MH_ && bn == BN_)                                                                                \
     e = dtype == TL_F16 ? launch_dense<__half, BN_, ST_, MH_>(grid, ctx->stream, amap, bmap, p, epi)         \
                         : launch_dense<__nv_bfloat16, BN_, ST_, MH_>(grid, ctx->stream, amap, bmap, p, epi);
-  if (b_mn || a_mn) {
+  if (ch.parts > 1) {
+    TL_DENSE_KSPLIT_CASE(256, 4)
+    TL_DENSE_KSPLIT_CASE(128, 6)
+  } else if (b_mn || a_mn) {
 #define TL_DENSE_MN_CASE(MH_, BN_, ST_)                                                                                  \
   if (mh == MH_ && bn == BN_) {                                                                                         \
     if (a_mn && b_mn)                                                                                                   \
@@ -422,6 +511,7 @@ int32_t tl_launch_dense_tc(tl_ctx* ctx, const void* a, const void* b, void* out,
   TL_DENSE_CASE(2, 160, 4)
   }
 #undef TL_DENSE_CASE
+#undef TL_DENSE_KSPLIT_CASE
   if (e != cudaSuccess) {
     ctx->async_errors++;
     return tl_set_error(ctx, TL_ERR_CUDA, "tl_matmul: tensor-core launch failed: %s", cudaGetErrorString(e));
