@@ -271,3 +271,26 @@ def test_qgemm_dequant_dense_graph_replay(backend):
     be.destroyGraph(graph)
     for t in (out, x, w.scales, w):
         t.destroy()
+
+
+@pytest.mark.parametrize("variant", [(2, 0, 192, 128, 3, 8), (2, 0, 64, 128, 6, 8), (2, 0, 192, 64, 6, 4)])
+@pytest.mark.parametrize("group", [16, 48, 64, 128, 192])
+def test_qgemm_group_scales_every_form(backend, variant, group):
+    """Groups shorter and longer than a converter thread's share of a step, and no power of two."""
+    be = backend
+    m, n, k = 70, 300, 1152
+    rng = np.random.default_rng(group)
+    w = (rng.standard_normal((n, k)) * 0.05).astype(np.float32)
+    xb = rng.standard_normal((m, k)).astype(np.float16)
+    packed, scales = be.quantizeLinearWeight(w, group)
+    wt = be.createQuantizedWeight(packed, scales, n, k, tb.StorageFormat("f16", tb.QuantPacking("int8-grouped", group, "f16")))
+    xt = be.ops.tensorFromArray(xb, [m, k], "f16")
+    be.forceVariant(variant)
+    try:
+        y = be.linear(xt, wt)
+    finally:
+        be.forceVariant(None)
+    w16 = orc.dequantize_to_f32(packed, scales, k, group).astype(np.float16).astype(np.float32)
+    assert cases.rel_err(be.ops.read(y), orc.matmul_nt(xb.astype(np.float32), w16)) <= 1e-3
+    for t in (y, xt, wt.scales, wt):
+        t.destroy()
