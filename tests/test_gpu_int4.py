@@ -145,3 +145,29 @@ def test_int4_tensor_core_and_simt_forms_agree(backend, m, g):
     assert cases.rel_err(a, b) <= 1e-4
     for t in (x, y1, y2, w.scales, w):
         t.destroy()
+
+
+@pytest.mark.parametrize("act", ["f16", "bf16"])
+@pytest.mark.parametrize("g", [32, 64, 128, 384, 0])
+@pytest.mark.parametrize("m,n,k", [(1, 1, 128), (1, 17, 384), (2, 500, 1536), (5, 33, 768), (8, 2400, 384), (9, 31, 1152), (16, 1000, 2304)])
+def test_int4_ring_edges(backend, act, g, m, n, k):
+    """Row tiles cut short, fewer k blocks than warps or ring stages, every group form, against the f32 form of the
+    same product.  Both sum the same exact products in f32: K terms of relative size 2^-24 each, four roundings' worth."""
+    be = backend
+    g = g or k
+    if k % g:
+        pytest.skip("K is not whole groups")
+    w, wref, _ = _weight(be, n, k, g, seed=n + m)
+    rng = np.random.default_rng(k + m)
+    xv = rng.uniform(-1, 1, (m, k)).astype(np.float32)
+    if act == "f16":
+        x, xv = be.ops.tensorFromArray(xv.astype(np.float16), [m, k], "f16"), xv.astype(np.float16).astype(np.float64)
+    else:
+        bits = orc.bf16_bits_rne(xv.reshape(-1))
+        x, xv = be.ops.tensorFromArray(bits, [m, k], "bf16"), orc.bf16_bits_to_f32(bits).reshape(m, k).astype(np.float64)
+    y = be.linear(x, w, None, None, "f32")
+    ref = xv @ wref.astype(np.float64).T
+    size = np.abs(xv) @ np.abs(wref.astype(np.float64)).T
+    assert (np.abs(be.ops.read(y) - ref) <= size * 2.0 ** -20).all()
+    for t in (x, y, w.scales, w):
+        t.destroy()

@@ -7,8 +7,8 @@
 //
 //   host quantizer        tl_quantize_linear_weight_int4 (same arithmetic as the int8 quantizer)
 //   explicit dequant      tl_dequant_int4 (f64 through a 16-entry table, one rounding: bit-exact)
-//   small batch, m <= 16  qgemv_int4_mma_kernel (f16 / bf16 activations, K and the group multiples of
-//                         128): mma.sync with the nibbles converted pairwise, see below; else
+//   small batch, m <= 16  qgemv_int4_ring_kernel (f16 / bf16 activations, K a multiple of 128, groups of 32, 64 or
+//                         multiples of 128): mma.sync with the nibbles converted pairwise, see below; else
 //                         qgemv_int4_kernel: warp per R rows, one packed word (8 weights) per lane and
 //                         step -- a warp reads 128 contiguous bytes of each row per step -- nibbles to
 //                         f32 by exponent stuffing, f32 FMA, group scale applied to the group's partial
@@ -26,6 +26,7 @@
 
 #include "tl_common.cuh"
 #include "tl_mma_frag.cuh"
+#include "tl_tma.cuh"
 
 namespace {
 
@@ -213,17 +214,23 @@ void launch_int4_m(tl_ctx* ctx, Int4Args p, const EpiParams& epi, int m) {
 }
 
 // ---------------------------------------------------------------------------
-// Tensor-core form (f16 / bf16 activations, K % 128 == 0, group % 128 == 0): CTA per 16 weight rows,
-// warps interleaved over 128-wide k blocks.  Lane (g, t) loads 16 bytes = 32 nibbles of rows g and
-// g + 8 and the matching 32 activations of batch row g.  (w ^ 0x88888888) turns every nibble into
-// q + 8; a mask and a magic exponent make the pair (q_x + 8, q_{x+4} + 8) 16-bit floats 1024 + .
-// (f16) or 128 + . (bf16), and one subtraction -- or, for the nibbles taken at bits 4-7, one fused
-// multiply-add -- gives (q_x, q_{x+4}) exactly (Nib::quad).  A word of eight
-// nibbles feeds two mma.sync.m16n8k16; the activations are paired the same way with two byte
-// permutes per MMA.  One group per k block: the block's accumulators are folded into the totals
-// with the rows' scales (per-channel scales once at the end).
+// Tensor-core form (f16 / bf16 activations, K % 128 == 0, group 32, 64 or a multiple of 128): CTA per 16 * RT weight
+// rows, warps interleaved over 128-wide k blocks.  Every warp runs its own cp.async ring in shared memory: a stage
+// holds one k block, 64 bytes of each of the tile's rows and 256 bytes of each activation row, so weights AND
+// activations are asked for S blocks ahead and hold no registers while they travel.  A row's 64 bytes are four
+// 16-byte chunks of 32 weights; lane (g, t) reads word t of chunk i of rows g and g + 8 and the matching eight
+// activations, so a chunk's two MMAs cover 32 consecutive k -- one group of the smallest size -- and its sums are
+// folded into the totals with the rows' scales where a group ends (FOLD times a block; 0: scales once at the end).
+// Chunks are swapped by the row (w: (row >> 1) & 3, activations: 4 * (row & 1)) so that neither read has a bank conflict.
+// A mask and an exclusive or with a magic exponent and the sign bits make the pair (q_x + 8, q_{x+4} + 8)
+// 16-bit floats 1024 + . (f16) or 128 + . (bf16), and one subtraction -- or, for the nibbles taken at bits 4-7, one
+// fused multiply-add -- gives (q_x, q_{x+4}) exactly (Nib::quad); the activations are paired the same way.
+// Bound: instruction issue (about 200 a block and warp) ahead of HBM.  14336 x 4096, groups of 128, bias + gelu: 15.8 us
+// at m = 1, 16.0 at 4, 22.7 at 16 (20.3, 21.5, 33.5 with two blocks in registers and the activations met in the loop);
+// groups of 32: 20.3 at m = 1 (they took the CUDA cores' form).
 // ---------------------------------------------------------------------------
-// quad(u, v): the four MMA operand registers of one word u (nibbles already q + 8):
+// quad(u, v): the four MMA operand registers of one packed word u; the exclusive or that sets the exponent also turns
+// the two's complement nibble into n = q + 8:
 //   v[0] = (q0, q4), v[1] = (q1, q5), v[2] = (q2, q6), v[3] = (q3, q7)
 template <typename AT> struct Nib;
 template <> struct Nib<__half> {
@@ -235,8 +242,8 @@ template <> struct Nib<__half> {
     const __half2 k16th = __halves2half2(__ushort_as_half(0x2C00), __ushort_as_half(0x2C00));   // 1/16
     const __half2 km72 = __halves2half2(__ushort_as_half(0xD480), __ushort_as_half(0xD480));    // -72
     const uint32_t u8 = u >> 8;
-    const uint32_t a = (u & 0x000F000Fu) | 0x64006400u, b = (u & 0x00F000F0u) | 0x64006400u;
-    const uint32_t c = (u8 & 0x000F000Fu) | 0x64006400u, d = (u8 & 0x00F000F0u) | 0x64006400u;
+    const uint32_t a = (u & 0x000F000Fu) ^ 0x64086408u, b = (u & 0x00F000F0u) ^ 0x64806480u;
+    const uint32_t c = (u8 & 0x000F000Fu) ^ 0x64086408u, d = (u8 & 0x00F000F0u) ^ 0x64806480u;
     const __half2 r0 = __hsub2(*reinterpret_cast<const __half2*>(&a), k1032);
     const __half2 r1 = __hfma2(*reinterpret_cast<const __half2*>(&b), k16th, km72);
     const __half2 r2 = __hsub2(*reinterpret_cast<const __half2*>(&c), k1032);
@@ -251,154 +258,256 @@ template <> struct Nib<__nv_bfloat16> {
     const uint32_t m = 0x43084308u;  // 136 | 136
 #pragma unroll
     for (int x = 0; x < 4; ++x) {
-      const uint32_t w = ((u >> (4 * x)) & 0x000F000Fu) | 0x43004300u;
+      const uint32_t w = ((u >> (4 * x)) & 0x000F000Fu) ^ 0x43084308u;
       const __nv_bfloat162 r = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&w), *reinterpret_cast<const __nv_bfloat162*>(&m));
       v[x] = *reinterpret_cast<const uint32_t*>(&r);
     }
   }
 };
 
-template <typename AT, int NT, bool GROUPED>
-__global__ void __launch_bounds__(512) qgemv_int4_mma_kernel(Int4Args p, EpiParams epi) {
-  extern __shared__ float red4[];  // [warps][NT][4][32]
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ uint32_t lds32(uint32_t addr) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
+  return v;
+}
+
+template <typename AT, int NT, int RT, int FOLD, int S>
+__global__ void __launch_bounds__(256) qgemv_int4_ring_kernel(Int4Args p, EpiParams epi) {
+  extern __shared__ __align__(128) uint8_t ring4[];
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
-  const int64_t tile_row = int64_t(blockIdx.x) * 16;
-  const int64_t r_lo = min(tile_row + g, int64_t(p.n) - 1), r_hi = min(tile_row + g + 8, int64_t(p.n) - 1);
-  const uint8_t* wb = reinterpret_cast<const uint8_t*>(p.packed);
+  const int64_t tile_row = int64_t(blockIdx.x) * (16 * RT);
   const int64_t row_bytes = p.k >> 1;
-  const uint8_t* w_lo = wb + r_lo * row_bytes + 16 * t;
-  const uint8_t* w_hi = wb + r_hi * row_bytes + 16 * t;
-  const AT* a = reinterpret_cast<const AT*>(p.a);
-  const AT* x_row[NT];
+  const int kblocks = p.k >> 7, mrows = p.m;
+  const uint32_t stage_bytes = uint32_t(RT * 1024 + mrows * 256);
+  const uint32_t ring = smem_u32(ring4) + uint32_t(warp * S) * stage_bytes;
+  int64_t rows[RT][2];
 #pragma unroll
-  for (int nt = 0; nt < NT; ++nt) x_row[nt] = a + int64_t(min(g + 8 * nt, p.m - 1)) * p.k + 32 * t;
-  float total[NT][4];
+  for (int r = 0; r < RT; ++r)
 #pragma unroll
-  for (int nt = 0; nt < NT; ++nt)
+    for (int h = 0; h < 2; ++h) rows[r][h] = min(tile_row + r * 16 + h * 8 + g, int64_t(p.n) - 1);  // tail rows clamp, stores mask
+  const uint32_t w_swz = uint32_t((g >> 1) & 3);
+  auto issue_weights = [&](int s, int kb) {
+    const uint8_t* w = reinterpret_cast<const uint8_t*>(p.packed) + int64_t(kb) * 64 + 16 * t;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) total[nt][i] = 0.f;
-  const int kblocks = p.k >> 7;
-  // one 128-wide k block: 8 MMAs per batch tile, on two accumulators so that only four are dependent
-  auto block = [&](const uint4& wl4, const uint4& wh4, float s_lo, float s_hi, int kb) {
-    const uint32_t wl[4] = {wl4.x ^ 0x88888888u, wl4.y ^ 0x88888888u, wl4.z ^ 0x88888888u, wl4.w ^ 0x88888888u};
-    const uint32_t wh[4] = {wh4.x ^ 0x88888888u, wh4.y ^ 0x88888888u, wh4.z ^ 0x88888888u, wh4.w ^ 0x88888888u};
-    float c[NT][4], d[NT][4];
+    for (int r = 0; r < RT; ++r)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        cp_async16(ring + s * stage_bytes + (r * 16 + h * 8 + g) * 64 + ((t ^ w_swz) << 4), w + rows[r][h] * row_bytes);
+  };
+  const AT* a_lane = reinterpret_cast<const AT*>(p.a) + int64_t(lane >> 4) * p.k + 8 * (lane & 15);
+  const uint32_t a_dst = uint32_t(RT * 1024 + (lane >> 4) * 256 + (((lane & 15) ^ ((lane >> 4) << 2)) << 4));
+  auto issue_acts = [&](int s, int kb) {
+    // lanes 0-15 take even rows, 16-31 odd ones, a 16-byte chunk each
+    const AT* a = a_lane + int64_t(kb) * 128;
+    uint32_t dst = ring + s * stage_bytes + a_dst;
+#pragma unroll
+    for (int r = 0; r < 8 * NT; r += 2) {
+      if (r + (lane >> 4) < mrows) cp_async16(dst, a);
+      a += 2 * int64_t(p.k);
+      dst += 512;
+    }
+  };
+  // group scales, one block ahead of their use
+  constexpr int NF = FOLD > 0 ? FOLD : 1;
+  float sc[RT][2][NF];
+  auto load_scales = [&](int kb) {
+    if (FOLD == 0) return;
+    const int grp = FOLD == 1 ? (kb * 128) / p.group : kb * FOLD;
+#pragma unroll
+    for (int r = 0; r < RT; ++r)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int f = 0; f < NF; ++f) sc[r][h][f] = tl_load_scale(p.scales, p.scales_dtype, rows[r][h] * p.groups_per_row + grp + f);
+  };
+  // the weights do not depend on the kernel before this one: ask for them while it drains
+#pragma unroll
+  for (int s = 0; s < S; ++s)
+    if (warp + s * warps < kblocks) issue_weights(s, warp + s * warps);
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+#pragma unroll
+  for (int s = 0; s < S; ++s) {
+    if (warp + s * warps < kblocks) issue_acts(s, warp + s * warps);
+    cp_async_commit();
+  }
+  if (warp < kblocks) load_scales(warp);
+  if (epi.fast_bias && threadIdx.x < 16 * RT && tile_row + threadIdx.x < p.n)
+    asm volatile("prefetch.global.L1 [%0];" ::"l"(epi.fast_bias + tile_row + threadIdx.x));
+
+  float total[RT][NT][4];
+#pragma unroll
+  for (int r = 0; r < RT; ++r)
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) { c[nt][i] = GROUPED ? 0.f : total[nt][i]; d[nt][i] = 0.f; }
+      for (int i = 0; i < 4; ++i) total[r][nt][i] = 0.f;
+  uint32_t a_off[NT], a_swz[NT];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      uint32_t lo[4], hi[4];
-      Nib<AT>::quad(wl[j], lo);
-      Nib<AT>::quad(wh[j], hi);
-      const uint32_t a00 = lo[0], a01 = hi[0], a02 = lo[1], a03 = hi[1];
-      const uint32_t a10 = lo[2], a11 = hi[2], a12 = lo[3], a13 = hi[3];
+  for (int nt = 0; nt < NT; ++nt) {
+    const int r = min(nt * 8 + g, mrows - 1);
+    a_off[nt] = uint32_t(RT * 1024 + r * 256);
+    a_swz[nt] = uint32_t((r & 1) << 2);
+  }
+  int s = 0;
+  for (int kb = warp; kb < kblocks; kb += warps) {
+    cp_async_wait<S - 1>();
+    __syncwarp();
+    const uint32_t st = ring + s * stage_bytes;
+    float cs[RT][2][NF];
+#pragma unroll
+    for (int r = 0; r < RT; ++r)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int f = 0; f < NF; ++f) cs[r][h][f] = sc[r][h][f];
+    if (kb + warps < kblocks) load_scales(kb + warps);
+    // two accumulators a tile: half as long a chain of dependent MMAs
+    float c[RT][NT][4], d[RT][NT][4];
+#pragma unroll
+    for (int i4 = 0; i4 < 4; ++i4) {
+      if (i4 % (4 / NF) == 0) {
+#pragma unroll
+        for (int r = 0; r < RT; ++r)
+#pragma unroll
+          for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) { c[r][nt][i] = FOLD ? 0.f : total[r][nt][i]; d[r][nt][i] = 0.f; }
+      }
+      uint32_t b[NT][4];
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt) {
-        const uint4 xv = __ldg(reinterpret_cast<const uint4*>(x_row[nt] + int64_t(kb) * 128) + j);  // x0..x7 of this word
-        MmaOps<AT>::mma(c[nt], a00, a01, a02, a03, __byte_perm(xv.x, xv.z, 0x5410), __byte_perm(xv.x, xv.z, 0x7632));
-        MmaOps<AT>::mma(d[nt], a10, a11, a12, a13, __byte_perm(xv.y, xv.w, 0x5410), __byte_perm(xv.y, xv.w, 0x7632));
+        const uint4 xv = lds128(st + a_off[nt] + (((i4 * 4 + t) ^ a_swz[nt]) << 4));  // x0..x7 of this word
+        b[nt][0] = __byte_perm(xv.x, xv.z, 0x5410); b[nt][1] = __byte_perm(xv.x, xv.z, 0x7632);
+        b[nt][2] = __byte_perm(xv.y, xv.w, 0x5410); b[nt][3] = __byte_perm(xv.y, xv.w, 0x7632);
+      }
+#pragma unroll
+      for (int r = 0; r < RT; ++r) {
+        const uint32_t w = st + (r * 16 + g) * 64 + ((i4 ^ w_swz) << 4) + 4 * t;
+        uint32_t lo[4], hi[4];
+        Nib<AT>::quad(lds32(w), lo);
+        Nib<AT>::quad(lds32(w + 512), hi);
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+          MmaOps<AT>::mma_free(c[r][nt], lo[0], hi[0], lo[1], hi[1], b[nt][0], b[nt][1]);
+          MmaOps<AT>::mma_free(d[r][nt], lo[2], hi[2], lo[3], hi[3], b[nt][2], b[nt][3]);
+        }
+      }
+      if ((i4 + 1) % (4 / NF) == 0) {
+        const int f = i4 / (4 / NF);
+#pragma unroll
+        for (int r = 0; r < RT; ++r)
+#pragma unroll
+          for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const float v = c[r][nt][i] + d[r][nt][i];
+              total[r][nt][i] = FOLD ? fmaf(cs[r][i >> 1][f], v, total[r][nt][i]) : v;
+            }
       }
     }
-    if (GROUPED) {
-#pragma unroll
-      for (int nt = 0; nt < NT; ++nt) {
-        total[nt][0] = fmaf(s_lo, c[nt][0] + d[nt][0], total[nt][0]); total[nt][1] = fmaf(s_lo, c[nt][1] + d[nt][1], total[nt][1]);
-        total[nt][2] = fmaf(s_hi, c[nt][2] + d[nt][2], total[nt][2]); total[nt][3] = fmaf(s_hi, c[nt][3] + d[nt][3], total[nt][3]);
-      }
-    } else {
-#pragma unroll
-      for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) total[nt][i] = c[nt][i] + d[nt][i];
+    __syncwarp();  // every lane has read the stage
+    if (kb + S * warps < kblocks) {
+      issue_weights(s, kb + S * warps);
+      issue_acts(s, kb + S * warps);
     }
-  };
-  // Two blocks' weights (and their scales) are always in flight.  (Programmatic dependent launch with
-  // the first loads ahead of griddepcontrol.wait measured slightly slower here, 17.8 against 16.6 us.)
-  // the rows' group scales of a block travel with its weights (loaded in the loop they cost an
-  // exposed L2 / DRAM round trip per block: the scale array is read once, like the weights)
-  const int shift = 31 - __clz(p.group >> 7);  // group = 128 << shift when GROUPED takes this kernel's power-of-two path
-  const bool pow2 = (p.group & (p.group - 1)) == 0;
-  auto scale_of = [&](int64_t row, int kblk) -> float {
-    if (!GROUPED) return 1.f;
-    const int grp = pow2 ? (kblk >> shift) : (kblk * 128) / p.group;
-    return tl_load_scale(p.scales, p.scales_dtype, row * p.groups_per_row + grp);
-  };
-  int kb = warp;
-  bool have0 = kb < kblocks, have1 = kb + warps < kblocks;
-  uint4 l0 = make_uint4(0, 0, 0, 0), h0 = l0, l1 = l0, h1 = l0;
-  float sl0 = 0.f, sh0 = 0.f, sl1 = 0.f, sh1 = 0.f;
-  if (have0) {
-    l0 = __ldg(reinterpret_cast<const uint4*>(w_lo + int64_t(kb) * 64));
-    h0 = __ldg(reinterpret_cast<const uint4*>(w_hi + int64_t(kb) * 64));
-    sl0 = scale_of(r_lo, kb); sh0 = scale_of(r_hi, kb);
+    cp_async_commit();
+    s = (s + 1) % S;
   }
-  if (have1) {
-    l1 = __ldg(reinterpret_cast<const uint4*>(w_lo + int64_t(kb + warps) * 64));
-    h1 = __ldg(reinterpret_cast<const uint4*>(w_hi + int64_t(kb + warps) * 64));
-    sl1 = scale_of(r_lo, kb + warps); sh1 = scale_of(r_hi, kb + warps);
-  }
-  while (have0) {
-    const uint4 cl0 = l0, ch0 = h0, cl1 = l1, ch1 = h1;
-    const float csl0 = sl0, csh0 = sh0, csl1 = sl1, csh1 = sh1;
-    const int kb0 = kb;
-    const bool run1 = have1;
-    kb += 2 * warps;
-    have0 = kb < kblocks;
-    have1 = kb + warps < kblocks;
-    if (have0) {
-      l0 = __ldg(reinterpret_cast<const uint4*>(w_lo + int64_t(kb) * 64));
-      h0 = __ldg(reinterpret_cast<const uint4*>(w_hi + int64_t(kb) * 64));
-      sl0 = scale_of(r_lo, kb); sh0 = scale_of(r_hi, kb);
-    }
-    if (have1) {
-      l1 = __ldg(reinterpret_cast<const uint4*>(w_lo + int64_t(kb + warps) * 64));
-      h1 = __ldg(reinterpret_cast<const uint4*>(w_hi + int64_t(kb + warps) * 64));
-      sl1 = scale_of(r_lo, kb + warps); sh1 = scale_of(r_hi, kb + warps);
-    }
-    block(cl0, ch0, csl0, csh0, kb0);
-    if (run1) block(cl1, ch1, csl1, csh1, kb0 + warps);
-  }
+  cp_async_wait<0>();
+  __syncthreads();  // the rings are done with: the partial tiles meet in their place
+  float* red = reinterpret_cast<float*>(ring4);  // [warps][RT][NT][4][32]
 #pragma unroll
-  for (int nt = 0; nt < NT; ++nt)
+  for (int r = 0; r < RT; ++r)
 #pragma unroll
-    for (int i = 0; i < 4; ++i) red4[((warp * NT + nt) * 4 + i) * 32 + lane] = total[nt][i];
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) red[(((warp * RT + r) * NT + nt) * 4 + i) * 32 + lane] = total[r][nt][i];
   __syncthreads();
-  for (int o = threadIdx.x; o < NT * 128; o += blockDim.x) {
-    const int nt = o >> 7, i = (o >> 5) & 3, ln = o & 31;
-    float v = 0.f;
-    for (int w = 0; w < warps; ++w) v += red4[((w * NT + nt) * 4 + i) * 32 + ln];
-    const int64_t row = tile_row + (ln >> 2) + ((i & 2) ? 8 : 0);
+  for (int o = threadIdx.x; o < RT * NT * 128; o += blockDim.x) {
+    const int tile = o >> 7, i = (o >> 5) & 3, ln = o & 31, r = tile / NT, nt = tile - r * NT;
+    const int64_t row = tile_row + r * 16 + (ln >> 2) + ((i & 2) ? 8 : 0);
     const int col = 8 * nt + 2 * (ln & 3) + (i & 1);
     if (row < p.n && col < p.m) {
-      float sc = p.wscale;
-      if (!GROUPED) sc *= tl_load_scale(p.scales, p.scales_dtype, row);
-      const float r = tl_apply_epilogue(epi, v * sc, col, row, p.n);
-      tl_store_out(p.out, p.out_dtype, int64_t(col) * p.n + row, r);
+      float v = 0.f;
+      for (int w = 0; w < warps; ++w) v += red[((w * RT * NT + tile) * 4 + i) * 32 + ln];
+      float f = p.wscale;
+      if (FOLD == 0) f *= tl_load_scale(p.scales, p.scales_dtype, row);
+      tl_store_out(p.out, p.out_dtype, int64_t(col) * p.n + row, tl_apply_epilogue(epi, v * f, col, row, p.n));
     }
   }
 }
 
-template <typename AT>
-void launch_int4_mma(tl_ctx* ctx, const Int4Args& p, const EpiParams& e, bool grouped) {
-  const int kblocks = p.k >> 7;
-  int warps = kblocks >= 8 ? 8 : kblocks >= 4 ? 4 : kblocks >= 2 ? 2 : 1;  // 8 measured best or equal at m = 1, 8, 16
-  // A/B hook: {TL_FAMILY_QGEMV, 9, warps} forces the CTA width
-  if (ctx->has_forced && ctx->forced.family == TL_FAMILY_QGEMV && ctx->forced.kernel == 9 && ctx->forced.p0 >= 1 && ctx->forced.p0 <= 16 &&
-      (ctx->forced.p0 & (ctx->forced.p0 - 1)) == 0)
-    warps = ctx->forced.p0;
-  const int grid = (p.n + 15) / 16, nt = p.m > 8 ? 2 : 1;
-  const size_t smem = size_t(warps) * nt * 128 * sizeof(float);
-  if (nt == 2) {
-    if (grouped) qgemv_int4_mma_kernel<AT, 2, true><<<grid, warps * 32, smem, ctx->stream>>>(p, e);
-    else qgemv_int4_mma_kernel<AT, 2, false><<<grid, warps * 32, smem, ctx->stream>>>(p, e);
-  } else {
-    if (grouped) qgemv_int4_mma_kernel<AT, 1, true><<<grid, warps * 32, smem, ctx->stream>>>(p, e);
-    else qgemv_int4_mma_kernel<AT, 1, false><<<grid, warps * 32, smem, ctx->stream>>>(p, e);
+inline size_t int4_ring_smem(int warps, int rt, int s, int m) { return size_t(warps) * s * (rt * 1024 + m * 256); }
+
+// Runs the kernel, or (occ != null) asks how many of its CTAs one SM holds.
+template <typename AT, int NT, int RT, int FOLD, int S>
+cudaError_t int4_ring_at(tl_ctx* ctx, const Int4Args& p, const EpiParams& e, int warps, int* occ) {
+  auto kern = qgemv_int4_ring_kernel<AT, NT, RT, FOLD, S>;
+  const size_t smem = int4_ring_smem(warps, RT, S, p.m);
+  if (smem > 48 * 1024) {
+    cudaError_t rc = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    if (rc != cudaSuccess) return rc;
   }
+  if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, kern, warps * 32, smem);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(unsigned((p.n + 16 * RT - 1) / (16 * RT)));
+  cfg.blockDim = dim3(warps * 32);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, p, e);
+}
+template <typename AT, int NT, int RT, int FOLD>
+cudaError_t int4_ring_s(tl_ctx* ctx, const Int4Args& p, const EpiParams& e, int warps, int s, int* occ) {
+  return s == 4 ? int4_ring_at<AT, NT, RT, FOLD, 4>(ctx, p, e, warps, occ) : int4_ring_at<AT, NT, RT, FOLD, 2>(ctx, p, e, warps, occ);
+}
+template <typename AT, int NT, int RT>
+cudaError_t int4_ring_fold(tl_ctx* ctx, const Int4Args& p, const EpiParams& e, int warps, int s, int* occ) {
+  if (p.group == p.k) return int4_ring_s<AT, NT, RT, 0>(ctx, p, e, warps, s, occ);
+  if (p.group % 128 == 0) return int4_ring_s<AT, NT, RT, 1>(ctx, p, e, warps, s, occ);
+  if (p.group == 64) return int4_ring_s<AT, NT, RT, 2>(ctx, p, e, warps, s, occ);
+  return int4_ring_s<AT, NT, RT, 4>(ctx, p, e, warps, s, occ);
+}
+template <typename AT>
+cudaError_t int4_ring(tl_ctx* ctx, const Int4Args& p, const EpiParams& e, int warps, int rt, int s, int* occ) {
+  if (p.m > 8) return rt == 2 ? int4_ring_fold<AT, 2, 2>(ctx, p, e, warps, s, occ) : int4_ring_fold<AT, 2, 1>(ctx, p, e, warps, s, occ);
+  return rt == 2 ? int4_ring_fold<AT, 1, 2>(ctx, p, e, warps, s, occ) : int4_ring_fold<AT, 1, 1>(ctx, p, e, warps, s, occ);
+}
+
+template <typename AT>
+cudaError_t launch_int4_mma(tl_ctx* ctx, const Int4Args& p, const EpiParams& e) {
+  const int kblocks = p.k >> 7;
+  // Eight warps keep a tile's k loop short; where tiles are few their rings are deep, else two stages
+  // leave room for more CTAs.  Two token tiles want 32-row
+  // tiles, which share the activations: four warps where there are several tiles an SM, else eight and deeper rings.
+  int warps = 8, rt = 1, s = p.n <= 2 * 16 * ctx->sm_count ? 4 : 2;
+  if (p.m > 8 && (p.group == p.k || p.group % 128 == 0)) {
+    rt = 2;
+    if (p.n > 2 * 32 * ctx->sm_count) { warps = 4; s = 2; }
+    else s = 4;
+  }
+  while (warps > 2 && warps > kblocks) warps >>= 1;
+  // A/B hook: {TL_FAMILY_QGEMV, 9, warps, row tiles, stages}
+  if (ctx->has_forced && ctx->forced.family == TL_FAMILY_QGEMV && ctx->forced.kernel == 9) {
+    const tl_variant& f = ctx->forced;
+    if (f.p0 >= 1 && f.p0 <= 8 && (f.p0 & (f.p0 - 1)) == 0) warps = f.p0;
+    if (f.p1 == 1 || f.p1 == 2) rt = f.p1;
+    if (f.p2 == 2 || f.p2 == 4) s = f.p2;
+  }
+  cudaError_t rc = int4_ring<AT>(ctx, p, e, warps, rt, s, nullptr);
   ctx->counters[TL_COUNTER_KERNEL_LAUNCHES]++;
+  return rc;
 }
 
 int32_t check_int4(tl_ctx* ctx, const char* who, const void* packed, const void* scales, int64_t n, int64_t k, const tl_quant_desc* q) {
@@ -526,11 +635,12 @@ int32_t tl_int4_matmul(tl_ctx* ctx, const char* who, int route, const void* a, i
     p.wscale = q->scale_convention == TL_SCALE_SNORM127 ? 1.0f / 7.0f : 1.0f;
     // the tensor-core form when its layout conditions hold (and it is not switched off for A/B tests)
     const bool forced_simt = ctx->has_forced && ctx->forced.family == TL_FAMILY_QGEMV && ctx->forced.kernel == 1;
-    const bool mma_ok = !forced_simt && a_dtype != TL_F32 && k % 128 == 0 && q->group_size % 128 == 0 &&
+    const bool mma_ok = !forced_simt && a_dtype != TL_F32 && k % 128 == 0 &&
+                        (q->group_size % 128 == 0 || q->group_size == 64 || q->group_size == 32) &&
                         (reinterpret_cast<uintptr_t>(packed) & 15) == 0;
     p.m = int32_t(m); p.row0 = 0;
-    if (mma_ok && a_dtype == TL_F16) launch_int4_mma<__half>(ctx, p, epi, q->group_size != k);
-    else if (mma_ok) launch_int4_mma<__nv_bfloat16>(ctx, p, epi, q->group_size != k);
+    if (mma_ok && a_dtype == TL_F16) TL_CUDA(ctx, launch_int4_mma<__half>(ctx, p, epi));
+    else if (mma_ok) TL_CUDA(ctx, launch_int4_mma<__nv_bfloat16>(ctx, p, epi));
     else if (a_dtype == TL_F32) launch_int4_m<float>(ctx, p, epi, int(m));
     else if (a_dtype == TL_F16) launch_int4_m<__half>(ctx, p, epi, int(m));
     else launch_int4_m<__nv_bfloat16>(ctx, p, epi, int(m));
