@@ -64,7 +64,7 @@ void quantize_rows_int4(const float* weight, int64_t row0, int64_t row1, int64_t
 template <typename OutT>
 __global__ void __launch_bounds__(256)
 dequant_int4_kernel(const uint32_t* __restrict__ packed, const void* __restrict__ scales, OutT* __restrict__ out, int64_t n_words,
-                    int32_t words_per_row, int32_t group, int32_t groups_per_row, int32_t scales_dtype, int32_t convention) {
+                    int32_t group, int32_t scales_dtype, int32_t convention, int vec) {
   __shared__ double lut[16];  // q/7 (snorm) or q (direct), indexed by the raw nibble
   if (threadIdx.x < 16) {
     const int q = threadIdx.x >= 8 ? int(threadIdx.x) - 16 : int(threadIdx.x);
@@ -72,15 +72,20 @@ dequant_int4_kernel(const uint32_t* __restrict__ packed, const void* __restrict_
   }
   __syncthreads();
   const int64_t stride = int64_t(gridDim.x) * blockDim.x;
+  const int wpg = group >> 3;  // words per group: a word lies in one group, and groups are contiguous across rows
+  const int shift = (wpg & (wpg - 1)) == 0 ? 31 - __clz(wpg) : -1;
   for (int64_t wi = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; wi < n_words; wi += stride) {
-    const int64_t row = wi / words_per_row;
-    const int32_t k0 = int32_t(wi - row * words_per_row) * 8;
     const uint32_t word = __ldg(packed + wi);
-    OutT* o = out + wi * 8;
+    const double s = double(tl_load_scale(scales, scales_dtype, shift >= 0 ? wi >> shift : wi / wpg));
+    alignas(16) OutT o[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const double s = double(tl_load_scale(scales, scales_dtype, row * groups_per_row + (k0 + j) / group));
-      o[j] = DT<OutT>::from_f32(float(lut[(word >> (4 * j)) & 0xfu] * s));
+    for (int j = 0; j < 8; ++j) o[j] = DT<OutT>::from_f32(float(lut[(word >> (4 * j)) & 0xfu] * s));
+    if (vec) {
+#pragma unroll
+      for (int j = 0; j < int(sizeof(o) / 16); ++j) reinterpret_cast<uint4*>(out + wi * 8)[j] = reinterpret_cast<const uint4*>(o)[j];
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) out[wi * 8 + j] = o[j];
     }
   }
 }
@@ -565,14 +570,14 @@ int32_t tl_dequant_int4(tl_ctx* ctx, const void* packed, const void* scales, voi
   if (n_words == 0) return TL_OK;
   DeviceGuard guard(ctx->device);
   const int grid = int(std::min<int64_t>((n_words + 255) / 256, int64_t(ctx->sm_count) * 16));
-  const int32_t wpr = int32_t(k / 8), gpr = int32_t(k / qdesc->group_size);
+  const int vec = (reinterpret_cast<uintptr_t>(out) & 15) == 0;
   const uint32_t* pk = static_cast<const uint32_t*>(packed);
   if (out_dtype == TL_F32)
-    dequant_int4_kernel<float><<<grid, 256, 0, ctx->stream>>>(pk, scales, static_cast<float*>(out), n_words, wpr, qdesc->group_size, gpr, qdesc->scales_dtype, qdesc->scale_convention);
+    dequant_int4_kernel<float><<<grid, 256, 0, ctx->stream>>>(pk, scales, static_cast<float*>(out), n_words, qdesc->group_size, qdesc->scales_dtype, qdesc->scale_convention, vec);
   else if (out_dtype == TL_F16)
-    dequant_int4_kernel<__half><<<grid, 256, 0, ctx->stream>>>(pk, scales, static_cast<__half*>(out), n_words, wpr, qdesc->group_size, gpr, qdesc->scales_dtype, qdesc->scale_convention);
+    dequant_int4_kernel<__half><<<grid, 256, 0, ctx->stream>>>(pk, scales, static_cast<__half*>(out), n_words, qdesc->group_size, qdesc->scales_dtype, qdesc->scale_convention, vec);
   else
-    dequant_int4_kernel<__nv_bfloat16><<<grid, 256, 0, ctx->stream>>>(pk, scales, static_cast<__nv_bfloat16*>(out), n_words, wpr, qdesc->group_size, gpr, qdesc->scales_dtype, qdesc->scale_convention);
+    dequant_int4_kernel<__nv_bfloat16><<<grid, 256, 0, ctx->stream>>>(pk, scales, static_cast<__nv_bfloat16*>(out), n_words, qdesc->group_size, qdesc->scales_dtype, qdesc->scale_convention, vec);
   TL_CUDA(ctx, cudaGetLastError());
   ctx->counters[TL_COUNTER_KERNEL_LAUNCHES]++;
   return TL_OK;

@@ -103,10 +103,12 @@ template <> struct Cvt<__nv_bfloat16> {
 template <typename AT, bool GROUPED>
 __global__ void __launch_bounds__(256)
 dequant_int8_16_kernel(const uint2* __restrict__ packed, const void* __restrict__ scales, int scales_dtype, float wscale, int group,
-                       int groups_per_row, int64_t k, int64_t n_oct, uint4* __restrict__ out) {
+                       int64_t n_oct, uint4* __restrict__ out) {
   // One octet (8 weights: 8 bytes in, 16 bytes out) per thread and step, so that a warp's loads AND its
   // stores are each one contiguous run; four independent steps in flight.
   const int64_t stride = int64_t(gridDim.x) * blockDim.x;
+  const int opg = group >> 3;  // octets per group: groups are contiguous across rows
+  const int shift = (opg & (opg - 1)) == 0 ? 31 - __clz(opg) : -1;
   for (int64_t o0 = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; o0 < n_oct; o0 += 4 * stride) {
     uint2 raw[4];
 #pragma unroll
@@ -118,8 +120,7 @@ dequant_int8_16_kernel(const uint2* __restrict__ packed, const void* __restrict_
       if (o >= n_oct) break;
       uint32_t v[4];
       if (GROUPED) {
-        const int64_t e = o * 8, row = e / k;
-        const float sc = tl_load_scale(scales, scales_dtype, row * groups_per_row + (e - row * k) / group) * wscale;
+        const float sc = tl_load_scale(scales, scales_dtype, shift >= 0 ? o >> shift : o / opg) * wscale;
         const uint32_t w2[2] = {raw[u].x, raw[u].y};
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
@@ -714,20 +715,25 @@ int32_t tl_launch_qgemm(tl_ctx* ctx, const tl_variant& v, const void* a, int32_t
       return tl_set_error(ctx, TL_ERR_INVALID_ARG, "qgemm: weight and activation pointers must be 16-byte aligned");
     void* wbuf = nullptr;
     int32_t rc = tl_ensure_scratch(ctx, size_t(n) * size_t(k) * 2, &wbuf);
-    if (rc != TL_OK) return rc;
+    if (rc != TL_OK) {
+      // No room for the 16-bit copy (or a capture that may not grow it): the fused kernel does without, unless this
+      // route was asked for by name.
+      if (ctx->has_forced && ctx->forced.family == TL_FAMILY_QGEMM && ctx->forced.kernel == kDequantDense) return rc;
+      const tl_variant fused{TL_FAMILY_QGEMM, kTc, 192, 128, 3, 8};
+      return tl_launch_qgemm(ctx, fused, a, a_dtype, packed, scales, out, out_dtype, m, n, k, q, epi, nullptr);
+    }
     const bool grouped = q.group_size != k;
     const float wscale = q.scale_convention == TL_SCALE_SNORM127 ? 1.0f / 127.0f : 1.0f;
     const int64_t n_oct = n * k / 8;
     const int grid = int(std::min<int64_t>((n_oct + 1023) / 1024, int64_t(ctx->sm_count) * 8));
     const uint2* pk = static_cast<const uint2*>(packed);
     uint4* wo = static_cast<uint4*>(wbuf);
-    const int gpr = int(k / q.group_size);
     if (a_dtype == TL_F16) {
-      if (grouped) dequant_int8_16_kernel<__half, true><<<grid, 256, 0, ctx->stream>>>(pk, scales, q.scales_dtype, wscale, q.group_size, gpr, k, n_oct, wo);
-      else dequant_int8_16_kernel<__half, false><<<grid, 256, 0, ctx->stream>>>(pk, scales, q.scales_dtype, wscale, q.group_size, gpr, k, n_oct, wo);
+      if (grouped) dequant_int8_16_kernel<__half, true><<<grid, 256, 0, ctx->stream>>>(pk, scales, q.scales_dtype, wscale, q.group_size, n_oct, wo);
+      else dequant_int8_16_kernel<__half, false><<<grid, 256, 0, ctx->stream>>>(pk, scales, q.scales_dtype, wscale, q.group_size, n_oct, wo);
     } else {
-      if (grouped) dequant_int8_16_kernel<__nv_bfloat16, true><<<grid, 256, 0, ctx->stream>>>(pk, scales, q.scales_dtype, wscale, q.group_size, gpr, k, n_oct, wo);
-      else dequant_int8_16_kernel<__nv_bfloat16, false><<<grid, 256, 0, ctx->stream>>>(pk, scales, q.scales_dtype, wscale, q.group_size, gpr, k, n_oct, wo);
+      if (grouped) dequant_int8_16_kernel<__nv_bfloat16, true><<<grid, 256, 0, ctx->stream>>>(pk, scales, q.scales_dtype, wscale, q.group_size, n_oct, wo);
+      else dequant_int8_16_kernel<__nv_bfloat16, false><<<grid, 256, 0, ctx->stream>>>(pk, scales, q.scales_dtype, wscale, q.group_size, n_oct, wo);
     }
     TL_CUDA(ctx, cudaGetLastError());
     ctx->counters[TL_COUNTER_KERNEL_LAUNCHES]++;
