@@ -299,8 +299,8 @@ __global__ void __launch_bounds__(128, NT == 1 ? 3 : 2) attn_decode_mma_kernel(D
         l[nt][e & 1] += pr[e];
       }
       uint32_t a[TERMS], c[TERMS];
-      ProbSplit<AT>::split(pr[0], pr[1], a);
-      ProbSplit<AT>::split(pr[2], pr[3], c);
+      ProbSplit<AT>::split(make_float2(pr[0], pr[1]), a);
+      ProbSplit<AT>::split(make_float2(pr[2], pr[3]), c);
 #pragma unroll
       for (int i = 0; i < TERMS; ++i) {
         pf[nt][i][0] = transpose8x8(a[i]);

@@ -47,28 +47,43 @@ __device__ __noinline__ void attention_row_warp(const AT* q, const AT* k, const 
     if (i >= first && i < first + count) out[lane + 32 * i] = DT<AT>::from_f32(o[i] * inv);
 }
 
+// Two f32 operations in one instruction
+__device__ __forceinline__ float2 fma_x2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;"
+      : "=l"(reinterpret_cast<uint64_t&>(d))
+      : "l"(reinterpret_cast<const uint64_t&>(a)), "l"(reinterpret_cast<const uint64_t&>(b)), "l"(reinterpret_cast<const uint64_t&>(c)));
+  return d;
+}
+__device__ __forceinline__ float2 add_x2(float2 a, float2 b) {
+  float2 d;
+  asm("add.rn.f32x2 %0, %1, %2;"
+      : "=l"(reinterpret_cast<uint64_t&>(d))
+      : "l"(reinterpret_cast<const uint64_t&>(a)), "l"(reinterpret_cast<const uint64_t&>(b)));
+  return d;
+}
+
 // Two probabilities as 16-bit terms whose sum carries (nearly) all 24 bits of each: p rounded, then what is left
 // rounded, then again.  f16 needs two terms (11 bits each), bf16 three (8 bits).
 template <typename AT> struct ProbSplit;
 template <> struct ProbSplit<__half> {
   static constexpr int kTerms = 2;
-  __device__ static __forceinline__ void split(float a, float b, uint32_t (&t)[2]) {
-    const __half2 hi = __floats2half2_rn(a, b);
-    const float2 f = __half22float2(hi);
-    const __half2 lo = __floats2half2_rn(a - f.x, b - f.y);
+  __device__ static __forceinline__ void split(float2 p, uint32_t (&t)[2]) {
+    const __half2 hi = __floats2half2_rn(p.x, p.y);
+    const float2 rest = fma_x2(__half22float2(hi), make_float2(-1.f, -1.f), p);  // exact
+    const __half2 lo = __floats2half2_rn(rest.x, rest.y);
     t[0] = *reinterpret_cast<const uint32_t*>(&hi);
     t[1] = *reinterpret_cast<const uint32_t*>(&lo);
   }
 };
 template <> struct ProbSplit<__nv_bfloat16> {
   static constexpr int kTerms = 3;
-  __device__ static __forceinline__ void split(float a, float b, uint32_t (&t)[3]) {
+  __device__ static __forceinline__ void split(float2 p, uint32_t (&t)[3]) {
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
-      const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+      const __nv_bfloat162 h = __floats2bfloat162_rn(p.x, p.y);
       t[i] = *reinterpret_cast<const uint32_t*>(&h);
-      a -= __uint_as_float(t[i] << 16);
-      b -= __uint_as_float(t[i] & 0xffff0000u);
+      p = fma_x2(make_float2(__uint_as_float(t[i] << 16), __uint_as_float(t[i] & 0xffff0000u)), make_float2(-1.f, -1.f), p);  // exact
     }
   }
 };

@@ -10,8 +10,9 @@
 // while the other's softmax runs.
 // Bound: the tensor core in principle (three units of work per score in f16: one for q k^T, two for p v), the chain
 // scores -> softmax -> products in practice: tensor pipe 51 % busy, instruction issue 49 %.  1 x 32 (8 KV) heads x 2048
-// x 2048 x 128 causal, f16: 57 us = 600 TFLOP/s of the causal work, 10.3 ms one CTA per query row; 74 us before the MMA
-// warp was kept converged, 89 with one softmax thread a row.
+// x 2048 x 128 causal, in the kernel: f16 51 us = 680 TFLOP/s of the causal work, bf16 62 (10.3 ms one CTA per query row;
+// 67 / 91 with the MMAs issued by one lane of a branch).  The products start on the first half of a step's
+// probabilities and the softmax works on pairs (f32x2): 1000 rows bf16 32.9 -> 30.2, 100 rows x 2000 keys 37.5 -> 35.1.
 #include <algorithm>
 #include <cmath>
 
@@ -66,7 +67,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
   constexpr uint32_t kIdescO = kFmtBits | (uint32_t(D >> 3) << 17) | (1u << 16);   // p v: v as it lies, MN-major
 
   extern __shared__ uint8_t attn_smem_raw[];
-  __shared__ uint64_t kv_full[SLOTS], kv_empty[SLOTS], q_full[MT], s_full[MT], p_full[MT], o_full[MT];
+  __shared__ uint64_t kv_full[SLOTS], kv_empty[SLOTS], q_full[MT], s_full[MT], p_full[MT][2], o_full[MT];
   __shared__ uint32_t tmem_base_smem;
   __shared__ int abort_flag;
   __shared__ float row_half[MT][2][2][128];  // [row block][step parity][half][row]: what a row's two threads tell each other
@@ -93,7 +94,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
     for (int t = 0; t < MT; ++t) {
       mbar_init(&q_full[t], 8);
       mbar_init(&s_full[t], 1);
-      mbar_init(&p_full[t], 8);
+      mbar_init(&p_full[t][0], 8);
+      mbar_init(&p_full[t][1], 8);
       mbar_init(&o_full[t], 1);
     }
     abort_flag = 0;
@@ -157,16 +159,23 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
         const int iv = 2 * j + 1, ik = 2 * j + 2;
 #pragma unroll
         for (int t = 0; t < MT; ++t) {
-          if (j >= steps[t] || !wait(&p_full[t], j & 1, TL_DEV_TIMEOUT_TMEM) || !wait(&kv_full[iv % SLOTS], (iv / SLOTS) & 1, TL_DEV_TIMEOUT_FULL))
-            continue;
-          tc_fence_after();
+          if (j >= steps[t] || !wait(&kv_full[iv % SLOTS], (iv / SLOTS) & 1, TL_DEV_TIMEOUT_FULL)) continue;
           const uint64_t vb = make_mn_desc(slot(iv), BN * 128);
+          // the probabilities come in two parts, the first half of each thread's slices and the rest
 #pragma unroll
-          for (int c = 0; c < BN / 16; ++c)
+          for (int h = 0; h < 2; ++h) {
+            if (!wait(&p_full[t][h], j & 1, TL_DEV_TIMEOUT_TMEM)) break;
+            tc_fence_after();
 #pragma unroll
-            for (int term = 0; term < TERMS; ++term)
-              tc_mma_ts(tb + t * 256, tb + t * 256 + kProb + (c * TERMS + term) * 8, desc_at(vb, c * 2048), kIdescO,
-                        (j > 0 || c > 0 || term > 0) ? 1u : 0u, elected);
+            for (int i = 0; i < BN / 32; ++i) {
+              const int c = (i / (BN / 64)) * (BN / 32) + h * (BN / 64) + i % (BN / 64);
+#pragma unroll
+              for (int term = 0; term < TERMS; ++term)
+                tc_mma_ts(tb + t * 256, tb + t * 256 + kProb + (c * TERMS + term) * 8, desc_at(vb, c * 2048), kIdescO,
+                          (j > 0 || h > 0 || i > 0 || term > 0) ? 1u : 0u, elected);
+            }
+          }
+          if (!ok) continue;
           if (j + 1 == steps[t]) {
             tc_commit(&o_full[t], elected);
           } else if (wait(&kv_full[ik % SLOTS], (ik / SLOTS) & 1, TL_DEV_TIMEOUT_FULL)) {
@@ -214,7 +223,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
     const int bound = p.causal ? p.kv_len - p.q_len + min(warp_row0 + lane, p.rows - 1) / p.rep + 1 : p.kv_len;  // keys this row sees
     const int warp_bound = p.causal ? p.kv_len - p.q_len + min(warp_row0, p.rows - 1) / p.rep + 1 : p.kv_len;
     const float c2 = p.scale_log2, lazy = kLazy / c2;
-    float m = -INFINITY, l[2] = {0.f, 0.f};
+    float m = -INFINITY;
+    float2 l = make_float2(0.f, 0.f);
     bool ok = true;  // a wait that gave up: the loop runs on, so that the other warp of the rows is met, but nothing is stored
     for (int j = 0; j < nsteps; ++j) {
       if (ok && !mbar_wait(&s_full[t], j & 1, &abort_flag)) {
@@ -242,8 +252,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
         const float nm = fmaxf(m, top);
         if (j > 0) {  // the scores' arrival says that the products before them are done
           const float f = ex2((m - nm) * c2);
-          l[0] *= f;
-          l[1] *= f;
+          l.x *= f;
+          l.y *= f;
 #pragma unroll 1
           for (int i = 0; i < HD; i += 16) {
             uint32_t o[16];
@@ -257,29 +267,32 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
         m = nm;
       }
       const float off = AttnTc<AT>::kBias - m * c2;
+      const float2 scale2 = make_float2(c2, c2), off2 = make_float2(off, off);
 #pragma unroll
       for (int c = 0; c < HN / 16; ++c) {
         uint32_t w[TERMS][8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          const float p0 = ex2(fmaf(__uint_as_float(su[c * 16 + 2 * i]), c2, off)), p1 = ex2(fmaf(__uint_as_float(su[c * 16 + 2 * i + 1]), c2, off));
-          l[0] += p0;
-          l[1] += p1;
+          const float2 x = fma_x2(make_float2(__uint_as_float(su[c * 16 + 2 * i]), __uint_as_float(su[c * 16 + 2 * i + 1])), scale2, off2);
+          const float2 pr = make_float2(ex2(x.x), ex2(x.y));
+          l = add_x2(l, pr);
           uint32_t tt[TERMS];
-          ProbSplit<AT>::split(p0, p1, tt);
+          ProbSplit<AT>::split(pr, tt);
 #pragma unroll
           for (int k = 0; k < TERMS; ++k) w[k][i] = tt[k];
         }
 #pragma unroll
         for (int k = 0; k < TERMS; ++k) tmem_st8(tm + kProb + ((half * (HN / 16) + c) * TERMS + k) * 8, w[k]);
+        if (c == HN / 32 - 1 || c == HN / 16 - 1) {  // half of the slices is enough for the product to start on
+          tmem_st_wait();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0 && ok) mbar_arrive(&p_full[t][c == HN / 16 - 1]);
+        }
       }
-      tmem_st_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0 && ok) mbar_arrive(&p_full[t]);
     }
     if (nsteps > 0) {
-      float sum = l[0] + l[1];
+      float sum = l.x + l.y;
       row_half[t][nsteps & 1][half][quad * 32 + lane] = sum;
       meet();
       sum += row_half[t][nsteps & 1][half ^ 1][quad * 32 + lane];
