@@ -282,7 +282,7 @@ __device__ __forceinline__ uint32_t lds32(uint32_t addr) {
 }
 
 template <typename AT, int NT, int RT, int FOLD, int S>
-__global__ void __launch_bounds__(256) qgemv_int4_ring_kernel(Int4Args p, EpiParams epi) {
+__global__ void __launch_bounds__(RT == 2 ? 256 : 512) qgemv_int4_ring_kernel(Int4Args p, EpiParams epi) {
   extern __shared__ __align__(128) uint8_t ring4[];
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -493,21 +493,29 @@ cudaError_t int4_ring(tl_ctx* ctx, const Int4Args& p, const EpiParams& e, int wa
 template <typename AT>
 cudaError_t launch_int4_mma(tl_ctx* ctx, const Int4Args& p, const EpiParams& e) {
   const int kblocks = p.k >> 7;
-  // Eight warps keep a tile's k loop short; where tiles are few their rings are deep, else two stages
-  // leave room for more CTAs.  Two token tiles want 32-row
-  // tiles, which share the activations: four warps where there are several tiles an SM, else eight and deeper rings.
-  int warps = 8, rt = 1, s = p.n <= 2 * 16 * ctx->sm_count ? 4 : 2;
-  if (p.m > 8 && (p.group == p.k || p.group % 128 == 0)) {
+  // A warp takes about a microsecond a block whatever the rest of the chip does, so the fewer the tiles the more warps
+  // share each one's k loop: sixteen up to two tiles an SM, with rings of four stages where shared memory leaves the
+  // tiles resident; else eight with two.  Two token tiles want 32-row tiles, which share the activations, once every SM
+  // has a tile.  us, groups of 128: 1425 x 11008 m = 1 16 warps 7.9, 8 warps 10.5; 4096 x 14336 m = 4 17.0, 22.9; 4096 x 4096
+  // m = 16 32-row tiles 7.6, 16-row 9.6; 14336 x 4096 m = 16 4 warps 22.9, 8 warps 29.5.
+  const int64_t tiles = (p.n + 15) / 16, sms = ctx->sm_count;
+  int warps = 8, rt = 1, s = 2;
+  if (p.m > 8 && tiles > sms && (p.group == p.k || p.group % 128 == 0)) {
     rt = 2;
-    if (p.n > 2 * 32 * ctx->sm_count) { warps = 4; s = 2; }
+    if (tiles > 4 * sms) warps = 4;
     else s = 4;
+  } else if (tiles <= 2 * sms && kblocks >= 16) {
+    warps = 16;
+    if (int4_ring_smem(16, 1, 4, p.m) <= (tiles <= sms ? 220 : 110) * 1024) s = 4;
+  } else if (tiles <= 2 * sms) {
+    s = 4;
   }
   while (warps > 2 && warps > kblocks) warps >>= 1;
   // A/B hook: {TL_FAMILY_QGEMV, 9, warps, row tiles, stages}
   if (ctx->has_forced && ctx->forced.family == TL_FAMILY_QGEMV && ctx->forced.kernel == 9) {
     const tl_variant& f = ctx->forced;
-    if (f.p0 >= 1 && f.p0 <= 8 && (f.p0 & (f.p0 - 1)) == 0) warps = f.p0;
     if (f.p1 == 1 || f.p1 == 2) rt = f.p1;
+    if (f.p0 >= 1 && f.p0 <= (rt == 2 ? 8 : 16) && (f.p0 & (f.p0 - 1)) == 0) warps = f.p0;
     if (f.p2 == 2 || f.p2 == 4) s = f.p2;
   }
   cudaError_t rc = int4_ring<AT>(ctx, p, e, warps, rt, s, nullptr);
