@@ -10,19 +10,16 @@
 //         = TMEM columns; BN a multiple of 16 up to 256), 64 k per pipeline stage (one 128-byte swizzled row
 //         per operand row), 4 MMAs of K = 16 per stage and row half;
 //   MH = 1: two accumulators of BN columns, so the epilogue of tile i overlaps the main loop of tile i+1.
-//   MH = 2: both row halves multiply the SAME B tile in shared memory.  What paces this kernel is the
-//         SM's shared-memory bandwidth (128 bytes per clock), not the tensor pipe: every operand byte is
-//         written once by TMA and read once per MMA that uses it, so a 64-k step of a 128 x 256 tile moves
-//         2 x (16 + 32) KB = 96 KB = 750 clocks for 512 clocks of MMA (measured 0.424 us per step), and a
-//         256 x 256 tile (32 + 32) KB of writes + (32 + 2 x 32) KB of reads = 160 KB for twice the flops
-//         (0.742 us) -- 17 % fewer bytes per flop.  (Sharing B between two SMs with cta_group::2 is the
-//         step that would take the reads down further; this kernel stays within one CTA.)  The two halves
+//   MH = 2: both row halves multiply the SAME B tile in shared memory.  A 256 x 256 tile moves 17 % fewer bytes per
+//         flop through it than a 128 x 256 one, and on large shapes the kernel runs at 0.92 of the fallback cuBLAS rate
+//         (2048 x 4096 x 14336: 1.46 PFLOP/s).  Sharing B between two SMs (cta_group::2) moves fewer bytes still and
+//         measured no faster.  The two halves
 //         fill TMEM (2 x BN columns), so the epilogue (one warp per lane quarter, half and column half)
 //         does not overlap the next tile; it is a few percent when K is in the thousands.
 //         The host picks MH and BN from a per-tile time model times the number of waves (tl_dense_tc_choose);
 //         (Stages of 32 k -- 64-byte-swizzle rows, seven deep in the same shared memory -- computed the same
 //         results 6 to 10 % slower at 256-row tiles.)
-//   warp 0: TMA producer (one elected lane); warp 1: TMEM allocation + MMA issue (one elected lane);
+//   warp 0: TMA producer (one elected lane); warp 1: TMEM allocation + MMA issue (the warp, one lane elected);
 //   warps 2..17: epilogue, four warps per TMEM lane quarter (MH = 1: each takes a quarter of the columns;
 //         MH = 2: a row half and half of the columns) -- the epilogue is a latency-bound instruction
 //         stream, and with K in the low thousands it, not the MMA, paced the tile until it had 16 warps;
@@ -388,20 +385,17 @@ bool tl_dense_tc_applicable(const void* a, const void* b, int64_t m, int64_t n, 
   return true;
 }
 
-// p0 of the receipt: BN (columns per tile); p1: stages; p2: MH (row halves per tile).  The choice minimises
-// waves x tile time, waves = ceil(tiles / SMs), with the tile time taken from measurements on B200 (bf16,
-// shapes from 1024^3 to 8192^3): a 64-k step costs `step_us` whatever the shape -- it follows the bytes the
-// step moves through shared memory (TMA writes + MMA reads, at about 226 KB per us), not the MMA's clocks,
-// which is why 256-row tiles win on large shapes (0.742 us for 256 x 256 against 2 x 0.424 for 128 x 256);
-// the three-stage tiles run a little under that rate, which is why four stages (BN <= 192 at
-// MH = 2) beat three.  With MH = 1 the epilogue hides behind the next tile unless K is short; with MH = 2
-// it adds to every tile.  E.g. m = 2048, n = 14336, k = 4096 on 148 SMs: 128 x 224 tiles run 7 waves of
-// 27 us, 256 x 208 tiles 4 waves of 46 us.
+// p0 of the receipt: BN (columns per tile); p1: stages; p2: MH (row halves per tile); p3: K ranges.  The choice
+// minimises waves x tile time, waves = ceil(tiles / SMs), with the tile time taken from measurements on B200 (bf16 +
+// gelu, whole chip busy): a 64-k step costs `step_us`.  With MH = 1 the epilogue hides behind the next tile unless K is
+// short; with MH = 2 it adds to every tile.  E.g. m = 2048, n = 14336, k = 4096 on 148 SMs: 128 x 224 tiles run 7
+// waves in 174 us, 256 x 208 tiles 4 waves in 191; n = 4096, k = 14336: 256 x 240 tiles one wave in 166 us, 128 x 256 two
+// in 202.
 namespace {
 struct DenseCfg { int mh, bn, stages; float step_us; };
-constexpr DenseCfg kDenseCfgs[] = {{1, 256, 4, 0.424f}, {1, 224, 5, 0.410f}, {1, 192, 5, 0.373f}, {1, 160, 6, 0.358f},
-                                   {1, 128, 6, 0.348f}, {2, 256, 3, 0.742f}, {2, 240, 3, 0.734f}, {2, 224, 3, 0.700f},
-                                   {2, 208, 3, 0.684f}, {2, 192, 4, 0.580f}, {2, 176, 4, 0.586f}, {2, 160, 4, 0.583f}};
+constexpr DenseCfg kDenseCfgs[] = {{1, 256, 4, 0.415f}, {1, 224, 5, 0.385f}, {1, 192, 5, 0.333f}, {1, 160, 6, 0.308f},
+                                   {1, 128, 6, 0.282f}, {2, 256, 3, 0.755f}, {2, 240, 3, 0.745f}, {2, 224, 3, 0.720f},
+                                   {2, 208, 3, 0.700f}, {2, 192, 4, 0.600f}, {2, 176, 4, 0.585f}, {2, 160, 4, 0.550f}};
 }  // namespace
 
 TlDenseTcChoice tl_dense_tc_choose(int64_t m, int64_t n, int64_t k, int sms, int forced_bn, int forced_mh, int bn_multiple, int forced_parts) {
@@ -421,15 +415,15 @@ TlDenseTcChoice tl_dense_tc_choose(int64_t m, int64_t n, int64_t k, int sms, int
     const double cost = double((t + sms - 1) / sms) * tile;
     if (cost < best.cost_us && forced_parts <= 1) best = TlDenseTcChoice{c.bn, c.mh, c.stages, 1, int(std::min<int64_t>(sms, t)), cost};
     // Cut along K (forced_parts 0: free, 1: not, else that many): one wave of clusters (of clusters of 8 about nine fit
-    // at a time), every part some steps; the meeting in shared memory measured 4.5 us.  bf16 + gelu, us uncut / cut:
-    // 256 x 4096 x 4096 28 / 20 (2 ranges), 512 x 1024 x 4096 28 / 16 (4), 100 x 2048 x 8192 48 / 19 (8),
-    // 333 x 4096 x 12288 71 / 50 (2); 700 x 2000 x 3000, whose tiles nearly fill the chip, 25 either way.
+    // at a time), every part some steps, 3.5 us for the meeting of 128-column tiles and 6 for that of wide ones.  bf16 + gelu, us
+    // uncut / cut: 256 x 4096 x 4096 23 / 17 (2 ranges), 512 x 1024 x 4096 23 / 13 (4), 100 x 2048 x 8192 38 / 16 (4),
+    // 333 x 4096 x 12288 56 / 49 (2); 700 x 2000 x 3000, whose tiles nearly fill the chip, 26 / 24.
     if (c.mh != 1 || (c.bn != 256 && c.bn != 128)) continue;
     for (int parts : {2, 4, 8}) {
       const int64_t per = (ksteps + parts - 1) / parts;
       if ((parts - 1) * per >= ksteps) continue;  // a part would be empty
       if (forced_parts > 1 ? parts != forced_parts : (forced_parts == 1 || t * parts > (parts == 8 ? sms / 2 : sms) || per < 4)) continue;
-      const double cut = double(per) * c.step_us + 0.012 * c.bn / parts + 5.0;
+      const double cut = double(per) * c.step_us + (c.bn == 256 ? 6.0 : 3.5);
       if (cut < best.cost_us) best = TlDenseTcChoice{c.bn, c.mh, c.stages, parts, int(t) * parts, cut};
     }
   }
