@@ -644,27 +644,29 @@ int32_t tl_qgemm_default_variant(tl_ctx* ctx, int64_t m, int64_t n, int64_t k, i
     else if (m <= 32) { v.p0 = 32; v.p1 = 128; v.p2 = 8; v.p3 = 8; }
     else if (m <= 64) { v.p0 = 64; v.p1 = 128; v.p2 = 6; v.p3 = 8; }
     else {
-      // 192 tokens x 128 k per step measured ~1.3x the throughput of the 128-token tile per padded
-      // token, so it wins unless it pads the token count by more than that
-      const int64_t pad192 = (m + 191) / 192 * 192, pad128 = (m + 127) / 128 * 128;
-      if (pad192 * 3 <= pad128 * 4) { v.p0 = 192; v.p1 = 128; v.p2 = 3; v.p3 = 8; }
+      // The token tile by modelled time: waves x 128-k steps x the time of a step, a last partial wave cut along K as the
+      // launch does it, 7 us for the meeting of its parts.  Step times on B200: 192 tokens 0.72 us (f16) / 0.78 (bf16) /
+      // 0.95 (group scales), 128 tokens 0.53 / 0.67 / 0.9.  Measured, us, 192 / 128: 2048 x 14336 x 4096 f16 201 / 215, bf16
+      // 217 / 268; 333 x 12288 x 4096 f16 45 / 37, groups of 64 57 / 64; 600 x 14336 x 2048 f16 51 / 38.
+      const int64_t sms = ctx ? ctx->sm_count : 148, ksteps = (k + 127) / 128;
+      const bool grouped = q.group_size != k, half = a_dtype == TL_F16;
+      auto fused_us = [&](int bn, double step) {
+        const int64_t tiles = ((n + kTileRows - 1) / kTileRows) * ((m + bn - 1) / bn), rem = tiles % sms;
+        const int64_t splits = rem ? std::min<int64_t>({sms / rem, 4, ksteps}) : 1;
+        return (double(tiles / sms) + (rem ? 1.0 / double(splits) : 0.0)) * double(ksteps) * step + (splits > 1 ? 7.0 : 0.0);
+      };
+      const double t192 = fused_us(192, grouped ? 0.95 : half ? 0.72 : 0.78), t128 = fused_us(128, grouped ? 0.9 : half ? 0.53 : 0.67);
+      if (t192 <= t128) { v.p0 = 192; v.p1 = 128; v.p2 = 3; v.p3 = 8; }
       else { v.p0 = 128; v.p1 = 128; v.p2 = 4; v.p3 = 8; }
       // With many tokens per weight byte, writing the weight out once as a 16-bit matrix and running the
       // dense kernel (whose operands both come from shared memory at its full tile sizes) beats converting
-      // on the operand path: compare the modelled times.  Fused: 0.87 us per 128-k step of a 128 x 192 tile
-      // (measured; 1.4 us with group scales), the last partial wave cut along K; dequantization: 3 bytes of
-      // HBM traffic per weight (the pass alone runs at the copy peak, 27 us for 14336 x 4096; the model charges 4 TB/s
-      // because the dense kernel that follows reads a freshly written operand and runs a little slower for it).  E.g. 2048 tokens: n = 4096,
-      // k = 14336 runs 200 us this way against 229 us fused, n = 14336, k = 4096 228 against 229 (stays fused),
-      // the same with groups of 128 218 against 368; 8192 tokens x 4096 x 4096: 231 against 284.
-      tl_variant dd{TL_FAMILY_QGEMM, kDequantDense, 0, 0, 0, 0};
-      if (v.p0 == 192 && tl_qgemm_variant_applicable(dd, m, n, k, a_dtype, q)) {
-        const int sms = ctx ? ctx->sm_count : 148;
-        const double tiles = double((n + kTileRows - 1) / kTileRows) * double((m + 191) / 192);
-        const double waves = std::max(1.0, std::ceil(tiles / sms * 4.0) / 4.0);
-        const double fused_us = waves * double((k + 127) / 128) * (q.group_size != k ? 1.4 : 0.87);  // group scales: an f32 multiply per weight
-        const double dense_us = tl_dense_tc_choose(m, n, k, sms).cost_us + double(n) * double(k) * 3.0 / 4.0e6 + 6.0;
-        if (dense_us < 0.92 * fused_us) v = dd;
+      // on the operand path: the dense kernel's modelled time, the pass at 6 TB/s (3 bytes a weight) and 4 us for the second
+      // launch.  Measured, us, fused / this way: 2048 tokens, n = 4096, k = 14336 bf16 222 / 190; n = 14336, k = 4096
+      // 217 / 223 (stays fused), with groups of 128 249 / 215; 700 x 4096 x 4096, groups of 64, 37 / 37.
+      const tl_variant dd{TL_FAMILY_QGEMM, kDequantDense, 0, 0, 0, 0};
+      if (m > 128 && tl_qgemm_variant_applicable(dd, m, n, k, a_dtype, q)) {
+        const double dense_us = tl_dense_tc_choose(m, n, k, int(sms)).cost_us + double(n) * double(k) * 3.0 / 6.0e6 + 4.0;
+        if (dense_us < 0.95 * std::min(t192, t128)) v = dd;
       }
     }
   } else {
