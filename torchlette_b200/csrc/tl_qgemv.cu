@@ -1882,7 +1882,12 @@ int32_t tl_qgemv_default_variant(tl_ctx* ctx, int32_t m, int64_t n, int64_t k, i
     ring_pick_shape(ctx, false, a_dtype, m, q.group_size != k, tiles, k, &w, &d, &wide);
     v.p0 = w; v.p1 = d; v.p2 = wide ? 2 : 0;
   } else if (k % 16 == 0 && q.group_size % 16 == 0) {
-    v.kernel = kSimt; v.p0 = 8; v.p1 = 2;
+    // Rows a warp: four share an activation load where that leaves enough CTAs, the more so the more batch rows there are
+    // (12288 x 4096, f32, us with 2 / 4 rows: 20 / 16 at m = 1, 58 / 40 at m = 4, 231 / 158 at m = 16; 4096 x 12288: 20 / 33,
+    // 56 / 45, 222 / 174); one where rows are few (1000 x 1024: 2.9 / 2.9 / 3.6 us with 1 / 2 / 4 at m = 1, 4.6 / 5.1 / 6.6 at 4).
+    const int64_t sms = ctx ? ctx->sm_count : 148;
+    v.kernel = kSimt; v.p0 = 4;
+    v.p1 = n >= (m <= 2 ? 48 : 24) * sms ? 4 : n >= 12 * sms ? 2 : 1;
   } else {
     v.kernel = kScalar; v.p0 = 8;
   }
