@@ -282,11 +282,13 @@ __global__ void __launch_bounds__(256) quantize_kernel(const float* __restrict__
 
 // Groups of 32, 64 or 128 (LANES = group / 4 lanes of a warp, a float4 each): the weight is read once, and the f64
 // arithmetic runs only where it can change the result.  Bound: HBM and, close behind, the instructions of the rounding;
-// 12288 x 4096 with groups of 64: 62 us = 4.1 TB/s (234 us a warp per group, all in f64, the weight read twice).
-//   x = w * inv in f32 is off by less than 2^-22 |x| < 1e-4 (two roundings, |x| < 256: the scale's f16 bits are at
-//   least half of the group's maximum, or zero); the rounding to a whole number can differ from the f64 one only if
-//   x lies that close to a half, and those values are done again in f64.  Rounding adds 1.5 * 2^23, whose low byte is
-//   then the two's complement; a clamp to +-127 before it gives what the clamp after it gave.
+// 12288 x 4096 with groups of 64: 51 us = 5.0 TB/s (234 us a warp per group, all in f64, the weight read twice; 62
+// with an exact division and conversion for every scale).
+//   x = w * inv in f32 is off by at most 3e-7 |x| < 8e-5 (a quotient good to 2 units in the last place and one rounding; |x| <
+//   256: the scale's f16 bits are at least half of the group's maximum, or zero); the rounding to a whole number can
+//   differ from the f64 one only if x lies that close to a half, and those values, and what is NaN, are done again in f64.
+//   Rounding adds 1.5 * 2^23, whose low byte is then the two's complement; a clamp to +-127 before it gives what the
+//   clamp after it gave.
 template <int LANES>
 __global__ void __launch_bounds__(256) quantize_group_kernel(const float4* __restrict__ weight, int64_t n_words, uint32_t* __restrict__ packed,
                                                              uint16_t* __restrict__ scales) {
@@ -310,21 +312,21 @@ __global__ void __launch_bounds__(256) quantize_group_kernel(const float4* __res
       for (int b = 0; b < 4; ++b) amax = fmaxf(amax, fabsf(f[b]));  // the number where the other is NaN: NaN is skipped
 #pragma unroll
       for (int o = LANES / 2; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-      const uint32_t sbits = dev_f32_to_f16_bits(amax);
+      // f16's normal range rounds to nearest even like the converter; below it the converter rounds halves up
+      const uint32_t sbits = amax >= 6.103515625e-5f ? uint32_t(__half_as_ushort(__float2half_rn(amax))) : dev_f32_to_f16_bits(amax);
       const float sc = __half2float(__ushort_as_half(uint16_t(sbits)));
-      const float inv = sc > 0.f ? 127.f / sc : 0.f;
+      const float inv = sc > 0.f ? __fdividef(127.f, sc) : 0.f;
       uint32_t q[4];
-      bool near_half = false;
+      bool again = false;
 #pragma unroll
       for (int b = 0; b < 4; ++b) {
-        float x = f[b] * inv;
-        x = x == x ? fminf(fmaxf(x, -127.f), 127.f) : 0.f;
+        const float raw = f[b] * inv, x = fminf(fmaxf(raw, -127.f), 127.f);
         const float r = x + 12582912.f;
         q[b] = __float_as_uint(r);
-        near_half = near_half || fabsf(fabsf(x - (r - 12582912.f)) - 0.5f) < 1e-4f;
+        again = again || !(fabsf(x - (r - 12582912.f)) <= 0.4999f) || raw != raw;
       }
-      if (near_half) {
-        const double inv64 = 127.0 / double(sc);  // sc > 0: a zero scale leaves zeros, far from a half
+      if (again) {
+        const double inv64 = sc > 0.f ? 127.0 / double(sc) : 0.0;
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
           const double x = double(f[b]) * inv64;
