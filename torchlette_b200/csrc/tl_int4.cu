@@ -440,8 +440,13 @@ __global__ void __launch_bounds__(RT == 2 ? 256 : 512) qgemv_int4_ring_kernel(In
     const int64_t row = tile_row + r * 16 + (ln >> 2) + ((i & 2) ? 8 : 0);
     const int col = 8 * nt + 2 * (ln & 3) + (i & 1);
     if (row < p.n && col < p.m) {
-      float v = 0.f;
-      for (int w = 0; w < warps; ++w) v += red[((w * RT * NT + tile) * 4 + i) * 32 + ln];
+      // four short sums instead of one long one: sixteen warps' partial tiles add up as exactly as eight did
+      float part[4] = {0.f, 0.f, 0.f, 0.f};
+      for (int w = 0; w < warps; w += 4)
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (w + e < warps) part[e] += red[(((w + e) * RT * NT + tile) * 4 + i) * 32 + ln];
+      const float v = (part[0] + part[1]) + (part[2] + part[3]);
       float f = p.wscale;
       if (FOLD == 0) f *= tl_load_scale(p.scales, p.scales_dtype, row);
       tl_store_out(p.out, p.out_dtype, int64_t(col) * p.n + row, tl_apply_epilogue(epi, v * f, col, row, p.n));
