@@ -73,6 +73,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
   __shared__ float row_half[MT][2][2][128];  // [row block][step parity][half][row]: what a row's two threads tell each other
   uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(attn_smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* kv_sm = sm + MT * kQBytes;
+  pdl_launch_dependents();
   const int warp = warp_index(), lane = threadIdx.x & 31;
   // longest rows first: with a causal mask the last row blocks see the most keys
   const int mblk = p.m_blocks - 1 - int(blockIdx.x) / p.groups, bkv = int(blockIdx.x) % p.groups;
@@ -109,6 +110,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = tmem_base_smem;
+  pdl_wait();
 
   if (warp == 0) {
     // ------------------------------ TMA producer: k 0, v 0, k 1, v 1, ... ------------------------------
@@ -352,8 +354,15 @@ cudaError_t launch(tl_ctx* ctx, const CUtensorMap& kmap, const CUtensorMap& vmap
   auto kern = attn_tc_kernel<AT, D, MT>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
   if (e != cudaSuccess) return e;
-  kern<<<unsigned(p.m_blocks) * unsigned(p.groups), 64 + 256 * MT, smem, ctx->stream>>>(kmap, vmap, p);
-  return cudaGetLastError();
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(unsigned(p.m_blocks) * unsigned(p.groups));
+  cfg.blockDim = dim3(64 + 256 * MT);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute attr[1] = {tl_pdl_attribute()};
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, kmap, vmap, p);
 }
 template <typename AT, int D>
 cudaError_t launch_mt(tl_ctx* ctx, const CUtensorMap& kmap, const CUtensorMap& vmap, const AttnTcArgs& p) {

@@ -89,6 +89,7 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
   __shared__ uint32_t tmem_base_smem;
   __shared__ int abort_flag;
   uint8_t* stages = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dense_smem_raw) + 1023) & ~uintptr_t(1023));
+  pdl_launch_dependents();
   const int warp = warp_index(), lane = threadIdx.x & 31;
   static_assert(KSP == 0 || (MH == 1 && STAGES * kStageBytes >= kBM * BN * 4), "a cut tile's partial sums fit where the stages were");
   const int tiles = p.m_tiles * p.n_tiles;
@@ -117,6 +118,7 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = tmem_base_smem;
+  pdl_wait();
 
   // sixteen outputs of one row, from column col0 on: op chain and store
   const bool approx = p.out_dtype != TL_F32;
@@ -370,9 +372,17 @@ cudaError_t launch_dense(int grid, cudaStream_t s, const CUtensorMap& amap, cons
   constexpr size_t smem = size_t(STAGES) * (kBM * MH * 128 + BN * 128) + 1024;
   static_assert(smem <= 227 * 1024, "shared memory per CTA");
   auto kern = dense_tc_kernel<AT, BN, STAGES, MH, BMN, AMN, 0>;
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-  kern<<<grid, kDenseThreads, smem, s>>>(amap, bmap, p, e);
-  return cudaGetLastError();
+  cudaError_t rc = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  if (rc != cudaSuccess) return rc;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(unsigned(grid));
+  cfg.blockDim = dim3(kDenseThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1] = {tl_pdl_attribute()};
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, amap, bmap, p, e);
 }
 
 }  // namespace
