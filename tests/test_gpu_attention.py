@@ -129,6 +129,37 @@ def test_decode_hidden_values_not_finite(be, dtype, s, n):
         t.destroy()
 
 
+@pytest.mark.parametrize("dtype", ["f16", "bf16", "f32"])
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("s,n,causal,masked", [(1, 1, False, False), (1, 16, False, False), (1, 17, False, False), (1, 64, True, False),
+                                               (1, 333, False, True), (2, 50, False, False), (2, 64, False, True), (3, 37, True, False),
+                                               (4, 600, True, False)])
+@pytest.mark.parametrize("where", ["first", "middle", "last"])
+def test_decode_visible_values_not_finite(be, dtype, d, s, n, causal, masked, where):
+    """An infinite or NaN value of a key that every row sees comes out as what it is, wherever the key lies in its tile, and
+    leaves the other dimensions and heads alone."""
+    rng = np.random.default_rng(n + s)
+    q, qr = store(be, rng.standard_normal((1, 4, s, d)), dtype)
+    k, kr = store(be, rng.standard_normal((1, 2, n, d)), dtype)
+    seen = n - s if causal else n - 1  # the last key that the first row sees
+    vf = rng.standard_normal((1, 2, n, d))
+    v_t, vr = store(be, vf, dtype)
+    v_t.destroy()
+    at = {"first": 0, "middle": seen // 2, "last": seen}[where]
+    vf[:, 0, at, :20], vf[:, 0, at, 20:30], vf[:, 0, at, 30:33] = np.inf, -np.inf, np.nan
+    v, _ = store(be, vf, dtype)
+    mask = rng.standard_normal((s, n)).astype(np.float32) if masked else None
+    mt = be.ops.tensorFromArray(mask, [s, n], "f32") if masked else None
+    out = be.ops.attention(q, k, v, n, 0.125, causal=causal, mask=mt)
+    got = read(be, out).astype(np.float64).reshape(s, 4, d)
+    ref = reference(qr, kr, vr, 0.125, causal, mask).reshape(s, 4, d)  # of finite values: the other dimensions' results
+    assert np.isposinf(got[:, :2, :20]).all() and np.isneginf(got[:, :2, 20:30]).all() and np.isnan(got[:, :2, 30:33]).all()
+    for g, r in ((got[:, :2, 33:], ref[:, :2, 33:]), (got[:, 2:], ref[:, 2:])):
+        assert (np.abs(g - r) / np.maximum(1.0, np.abs(r))).max() <= TOL[dtype]
+    for t in (q, k, v, out) + ((mt,) if masked else ()):
+        t.destroy()
+
+
 @pytest.mark.parametrize("dtype", ["f16", "bf16"])
 @pytest.mark.parametrize("b,heads,kv_heads,d,s,n,causal", [
     (1, 4, 1, 128, 5, 5, True), (1, 8, 8, 64, 17, 17, True), (1, 8, 2, 128, 32, 32, True), (2, 8, 2, 128, 33, 200, True),

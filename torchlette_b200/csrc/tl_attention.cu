@@ -151,11 +151,13 @@ __device__ __forceinline__ void decode_merge(const DecodeArgs& p, float* sm, int
     const int qi = r / p.rep, h = kvh * p.rep + (r - qi * p.rep);
     const int64_t at = ((int64_t(b) * p.q_len + qi) * p.n_heads + h) * D;
     const float v = o / l;
-    if (p.causal && p.q_len > 1 && __any_sync(0xffffffffu, !isfinite(v))) {
+    // Not finite: a probability times an infinite value went through the split terms (or a key past the end, clamped to the
+    // last one, met it with probability zero), or it is what the row sees.  The redo tells them apart.
+    if (__any_sync(0xffffffffu, !isfinite(v))) {
       const int64_t kv = (int64_t(b) * p.n_kv_heads + kvh) * p.capacity * D;
       attention_row_warp<AT, D>(reinterpret_cast<const AT*>(p.q) + ((int64_t(b) * p.n_heads + h) * p.q_len + qi) * D,
                                 reinterpret_cast<const AT*>(p.k) + kv, reinterpret_cast<const AT*>(p.v) + kv,
-                                reinterpret_cast<AT*>(p.out) + at, p.kv_len - p.q_len + qi + 1, p.scale,
+                                reinterpret_cast<AT*>(p.out) + at, p.causal ? p.kv_len - p.q_len + qi + 1 : p.kv_len, p.scale,
                                 p.mask ? p.mask + int64_t(qi) * p.kv_len : nullptr, d >> 5, 1);
     } else {
       reinterpret_cast<AT*>(p.out)[at + d] = DT<AT>::from_f32(v);

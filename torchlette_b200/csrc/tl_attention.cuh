@@ -9,10 +9,11 @@
 #ifdef __CUDACC__
 constexpr float kLog2e = 1.4426950408889634f;
 
-// The tensor-core kernels multiply whole tiles: a key hidden from a row has probability zero there, and zero times
-// an infinite or NaN value would still poison the row.  A row whose result is not finite is therefore done again
-// here, where hidden keys are never read: two passes, f32, a lane per D / 32 dimensions.  Only the
-// dimensions from 32 * first on, 32 * count of them, are stored.
+// The fast kernels multiply whole tiles and split probabilities into terms: a key hidden from a row (or past the end) has
+// probability zero there, and zero times an infinite or NaN value would still poison the row; a visible infinite value meets
+// a low term that is zero or negative, and infinity becomes NaN.  A row whose result is not finite is therefore done again
+// here, over exactly the keys that it sees and with whole probabilities: two passes, f32, a lane per D / 32 dimensions.  Only
+// the dimensions from 32 * first on, 32 * count of them, are stored.
 template <typename AT, int D>
 __device__ __noinline__ void attention_row_warp(const AT* q, const AT* k, const AT* v, AT* out, int keys, float scale, const float* mask,
                                                 int first, int count) {
