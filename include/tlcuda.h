@@ -136,8 +136,8 @@ TL_API int32_t tl_get_option(tl_ctx* ctx, const char* name, int64_t* out_value);
 /* ---- memory: tensorFromArray / read / destroy (src/backend/types.ts:341-345,
  * :666) ---------------------------------------------------------------------- */
 /* tl_free keeps the block for a later tl_alloc (at most 1 GiB in all; blocks above 256 MB go straight back), which gets
- * it only after a device-wide synchronization that came after the tl_free: no stream can still be using the old
- * contents.  What is kept is given back when memory runs short and by tl_ctx_destroy. */
+ * it only after all that any stream of the device had been given by the tl_free is over.  A tl_free that fails leaves the
+ * block with the caller.  What is kept is given back when a tl_alloc runs short and by tl_ctx_destroy. */
 TL_API int32_t tl_alloc(tl_ctx* ctx, size_t bytes, void** out_dptr);
 TL_API int32_t tl_free(tl_ctx* ctx, void* dptr);
 TL_API int32_t tl_upload(tl_ctx* ctx, void* dst_dptr, const void* src_host, size_t bytes);

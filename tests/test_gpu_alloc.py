@@ -1,5 +1,5 @@
 """tl_alloc / tl_free: blocks are handed out again, but never while anything given to the device before still uses them."""
-import ctypes as C
+import threading
 
 import numpy as np
 import pytest
@@ -71,3 +71,75 @@ def test_errors(be):
         be._alloc(1 << 50)
     q = be._alloc(1000)  # neither refusal spoils what follows
     be._free(q)
+
+
+class _Capture(threading.Thread):
+    """A capture on a thread of its own that stays open until `close`."""
+
+    def __init__(self, begin, work, end):
+        super().__init__()
+        self.steps, self.opened, self.may_end, self.error, self.graph = (begin, work, end), threading.Event(), threading.Event(), None, None
+
+    def run(self):
+        begin, work, end = self.steps
+        try:
+            begin()
+            self.opened.set()
+            try:
+                assert self.may_end.wait(60)
+                work()
+            finally:
+                self.graph = end()
+        except Exception as e:  # handed to the test
+            self.error = e
+        finally:
+            self.opened.set()
+
+    def close(self):
+        self.may_end.set()
+        self.join()
+
+
+@pytest.mark.parametrize("size,count", [(100, 200), (30 << 20, 20)])
+@pytest.mark.parametrize("other", ["context", "torch"])
+def test_freeing_leaves_the_captures_of_others_alone(be, other, size, count):
+    """More blocks than wait for one synchronization, given back while another context or torch captures on this device."""
+    if other == "context":
+        be2 = tb.CudaBackend(0)
+        cache = be2.ops.tensorFromArray(np.zeros((1, 1, 4, 64), np.float32), [1, 1, 4, 64], "f32")
+        new = be2.ops.tensorFromArray(np.full((1, 1, 1, 64), 3.0, np.float32), [1, 1, 1, 64], "f32")
+        be2.sync()
+        cap = _Capture(be2.beginCapture, lambda: be2.ops.kvAppend(cache, new, 2), be2.endCapture)
+    else:
+        stream, graph, x = torch.cuda.Stream(), torch.cuda.CUDAGraph(), torch.zeros(64, device="cuda")
+        torch.cuda.synchronize()
+
+        def begin():
+            torch.cuda.set_stream(stream)
+            graph.capture_begin(capture_error_mode="thread_local")
+
+        cap = _Capture(begin, lambda: x.add_(3.0), graph.capture_end)
+    blocks = [be._alloc(size) for _ in range(count)]
+    cap.start()
+    cap.opened.wait()
+    try:
+        for p in blocks:
+            be._free(p)
+        blocks = [be._alloc(size) for _ in range(count)]
+    finally:
+        cap.close()
+    assert cap.error is None
+    for p in blocks:
+        be._free(p)
+    if other == "context":
+        be2.replay(cap.graph)
+        got = be2.ops.read(cache)
+        assert (got[0, 0, 2] == 3.0).all() and (got[0, 0, [0, 1, 3]] == 0.0).all()
+        be2.destroyGraph(cap.graph)
+        for t in (cache, new):
+            t.destroy()
+        be2.destroy()
+    else:
+        graph.replay()
+        torch.cuda.synchronize()
+        assert bool((x == 3.0).all())

@@ -1,10 +1,8 @@
 // Context, memory, counters, replay graphs, events, argument validation and the
 // quantized-matmul seam of libtlcuda.
-#include <algorithm>
 #include <cstdlib>
 #include <cstring>
 #include <exception>
-#include <iterator>
 
 #include "tl_common.cuh"
 
@@ -157,8 +155,7 @@ int32_t tl_ctx_destroy(tl_ctx* ctx) {
   DeviceGuard guard(ctx->device);
   if (ctx->nccl_comm) tl_comm_destroy(ctx);
   cudaStreamSynchronize(ctx->stream);
-  ctx->pool.settle();
-  ctx->pool.trim(0);  // blocks still handed out stay the caller's, as before
+  ctx->pool.release();  // blocks still handed out stay the caller's, as before
   if (ctx->scratch) cudaFree(ctx->scratch);
   if (ctx->zscratch) cudaFree(ctx->zscratch);
   for (auto& p : ctx->retired_scratch) cudaFree(p.first);
@@ -236,77 +233,7 @@ int32_t tl_get_option(tl_ctx* ctx, const char* name, int64_t* out_value) {
   return TL_OK;
 }
 
-}  // extern "C"
-
 // ---- memory ---------------------------------------------------------------
-cudaError_t TlBlockPool::settle() {
-  cudaError_t e = cudaDeviceSynchronize();
-  if (e != cudaSuccess) return e;
-  for (auto& w : waiting) ready.emplace(w.second, w.first);
-  ready_bytes += waiting_bytes;
-  waiting.clear();
-  waiting_bytes = 0;
-  return cudaSuccess;
-}
-
-void TlBlockPool::trim(size_t keep) {
-  while (!ready.empty() && ready_bytes > keep) {
-    auto last = std::prev(ready.end());
-    cudaFree(last->second);
-    ready_bytes -= last->first;
-    ready.erase(last);
-  }
-}
-
-cudaError_t TlBlockPool::alloc(size_t bytes, void** out) {
-  // capacities in steps of 512 bytes, or of 1/64 to 1/32 of the size where that is more: sizes that differ a little
-  // from call to call share blocks, and little is lost in weights that stay
-  size_t step = 512;
-  while (bytes <= kLargestBytes && step < bytes / 64) step *= 2;
-  const size_t cap = bytes > SIZE_MAX / 2 ? bytes : std::max<size_t>(1, (bytes + step - 1) / step) * step;
-  std::lock_guard<std::mutex> hold(lock);
-  auto it = ready.lower_bound(cap);
-  if (it != ready.end() && it->first <= cap + cap / 4) {
-    *out = it->second;
-    ready_bytes -= it->first;
-    live[it->second] = it->first;
-    ready.erase(it);
-    return cudaSuccess;
-  }
-  size_t got = cap;
-  cudaError_t e = cudaMalloc(out, cap);
-  if (e == cudaErrorMemoryAllocation) {  // give back what is kept, then ask for no more than was asked for
-    cudaGetLastError();
-    if (settle() == cudaSuccess) trim(0);
-    got = bytes ? bytes : 1;
-    e = cudaMalloc(out, got);
-  }
-  if (e == cudaSuccess) live[*out] = got;
-  return e;
-}
-
-cudaError_t TlBlockPool::free(void* p, bool* known) {
-  std::lock_guard<std::mutex> hold(lock);
-  auto it = live.find(p);
-  *known = it != live.end();
-  if (!*known) {
-    for (auto& w : waiting) *known = *known || w.first == p;
-    for (auto& r : ready) *known = *known || r.second == p;
-    return *known ? cudaErrorInvalidValue : cudaSuccess;  // given back twice, or not from here
-  }
-  const size_t cap = it->second;
-  live.erase(it);
-  if (cap > kLargestBytes) return cudaFree(p);
-  waiting.emplace_back(p, cap);
-  waiting_bytes += cap;
-  if (waiting.size() < kWaitingBlocks && waiting_bytes < kWaitingBytes) return cudaSuccess;
-  cudaError_t e = settle();
-  trim(kKeptBytes - kWaitingBytes);
-  return e;
-}
-
-extern "C" {
-
 int32_t tl_alloc(tl_ctx* ctx, size_t bytes, void** out_dptr) {
   TL_CHECK_CTX(ctx);
   if (!out_dptr) return tl_set_error(ctx, TL_ERR_INVALID_ARG, "tl_alloc: null out pointer");
@@ -339,6 +266,7 @@ int32_t tl_free(tl_ctx* ctx, void* dptr) {
   } catch (const std::exception&) {
     return tl_set_error(ctx, TL_ERR_OOM, "tl_free: out of host memory");
   }
+  if (e != cudaSuccess) cudaGetLastError();  // reported here, not at the next launch
   TL_CUDA(ctx, e);
   if (known) return TL_OK;
   TL_CUDA(ctx, cudaStreamSynchronize(ctx->stream));

@@ -10,12 +10,12 @@
 #include <cstdint>
 #include <cstdio>
 #include <map>
-#include <mutex>
 #include <string>
 #include <utility>
 #include <vector>
 
 #include "../../include/tlcuda.h"
+#include "tl_pool.cuh"
 
 // ---------------------------------------------------------------------------
 // Context
@@ -32,28 +32,6 @@ struct TuneKey {
     if (scales_dtype != o.scales_dtype) return scales_dtype < o.scales_dtype;
     return convention < o.convention;
   }
-};
-
-// Device blocks behind tl_alloc / tl_free.  cudaMalloc and cudaFree map and unmap memory and stop the device: 1.5 ms
-// a call that returns 50 MB, 0.5 ms a decoder layer with its fourteen results.  A block that was given back is kept
-// and handed out again, but only after a device-wide synchronization that came after it was given back, the
-// promise that cudaFree makes: whatever any stream still does with the old contents is over by then.  One
-// synchronization serves many blocks (kWaitingBlocks, kWaitingBytes).
-struct TlBlockPool {
-  static constexpr size_t kKeptBytes = size_t(1) << 30;       // blocks kept in all, waiting ones included
-  static constexpr size_t kLargestBytes = size_t(1) << 28;    // larger blocks go straight back
-  static constexpr size_t kWaitingBytes = size_t(1) << 28;
-  static constexpr size_t kWaitingBlocks = 64;
-  std::mutex lock;                            // tl_alloc and tl_free may come from several threads
-  std::map<void*, size_t> live;               // handed out: capacity
-  std::multimap<size_t, void*> ready;         // free and synchronized, by capacity
-  std::vector<std::pair<void*, size_t>> waiting;  // given back since the last device-wide synchronization
-  size_t ready_bytes = 0, waiting_bytes = 0;
-  cudaError_t alloc(size_t bytes, void** out);
-  // *known: the block is one of the pool's (a pointer from elsewhere is left to the caller)
-  cudaError_t free(void* p, bool* known);
-  cudaError_t settle();   // synchronizes the device: waiting blocks become ready
-  void trim(size_t keep); // gives ready blocks back until at most `keep` bytes of them are left, the largest first
 };
 
 struct tl_ctx {
