@@ -143,3 +143,60 @@ def test_freeing_leaves_the_captures_of_others_alone(be, other, size, count):
         graph.replay()
         torch.cuda.synchronize()
         assert bool((x == 3.0).all())
+
+
+@pytest.mark.parametrize("mode", ["thread_local", "relaxed"])
+def test_a_capture_that_a_program_began_on_the_stream_refuses(be, mode):
+    """The context's stream captured without tl_graph_begin: a block handed out or taken back there could be another tensor's
+    by the time the graph runs."""
+    from cuda.bindings import driver as cu
+
+    kinds = cu.CUstreamCaptureMode
+    mode = {"thread_local": kinds.CU_STREAM_CAPTURE_MODE_THREAD_LOCAL, "relaxed": kinds.CU_STREAM_CAPTURE_MODE_RELAXED}[mode]
+    held, kept = [be._alloc(1000) for _ in range(3)], [be._alloc(1000) for _ in range(70)]
+    for p in kept:
+        be._free(p)  # some are ready to be handed out again
+    be.sync()
+
+    def capture(call):
+        assert cu.cuStreamBeginCapture(be.stream(), mode)[0] == cu.CUresult.CUDA_SUCCESS
+        try:
+            call()
+        finally:
+            err, graph = cu.cuStreamEndCapture(be.stream())
+            if err == cu.CUresult.CUDA_SUCCESS:
+                cu.cuGraphDestroy(graph)
+
+    def free():
+        with pytest.raises(tb.TlError):
+            be._free(held[0])
+
+    def alloc():
+        if mode == kinds.CU_STREAM_CAPTURE_MODE_RELAXED:  # new memory is allowed there, another tensor's is not
+            p = be._alloc(1000)
+            assert p not in kept
+            held.append(p)
+        else:
+            with pytest.raises(tb.TlError):
+                be._alloc(1000)
+
+    capture(free)
+    capture(alloc)
+    assert not set(be._alloc(1000) for _ in range(3)) & set(held)  # what was refused is still the caller's
+    for p in held:
+        be._free(p)
+
+
+def test_a_graph_of_this_thread_on_another_context_refuses(be):
+    be2 = tb.CudaBackend(0)
+    p = be._alloc(1000)
+    be2.beginCapture()
+    with pytest.raises(tb.TlError):
+        be._free(p)
+    with pytest.raises(tb.TlError):
+        be._alloc(1000)
+    with pytest.raises(tb.TlError):  # what a cudaMalloc in the capturing thread does to the capture
+        be2.endCapture()
+    assert be._alloc(1000) != p
+    be._free(p)
+    be2.destroy()

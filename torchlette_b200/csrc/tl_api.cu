@@ -88,6 +88,8 @@ TlProfileScope::~TlProfileScope() {
     fprintf(stderr, "[tl profile] %s m=%lld n=%lld k=%lld: %.2f us\n", label, (long long)m, (long long)n, (long long)k, ms * 1e3);
 }
 
+static thread_local int t_captures = 0;  // graphs that this thread has open (tl_graph_begin), on whatever context
+
 extern "C" {
 
 int32_t tl_ctx_create(int32_t device_ordinal, tl_ctx** out_ctx) {
@@ -154,6 +156,7 @@ int32_t tl_ctx_destroy(tl_ctx* ctx) {
   TL_CHECK_CTX(ctx);
   DeviceGuard guard(ctx->device);
   if (ctx->nccl_comm) tl_comm_destroy(ctx);
+  if (ctx->capturing && t_captures > 0) --t_captures;
   cudaStreamSynchronize(ctx->stream);
   ctx->pool.release();  // blocks still handed out stay the caller's, as before
   if (ctx->scratch) cudaFree(ctx->scratch);
@@ -234,15 +237,23 @@ int32_t tl_get_option(tl_ctx* ctx, const char* name, int64_t* out_value) {
 }
 
 // ---- memory ---------------------------------------------------------------
+// A graph is being captured, on the context's stream (by tl_graph_begin or by a program that took the stream from
+// tl_ctx_stream) or by this thread: it would keep the addresses of blocks that the pool hands to others later.
+static bool capture_open(tl_ctx* ctx) {
+  if (ctx->capturing || t_captures > 0) return true;
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(ctx->stream, &status) != cudaSuccess || status != cudaStreamCaptureStatusNone;
+}
+
 int32_t tl_alloc(tl_ctx* ctx, size_t bytes, void** out_dptr) {
   TL_CHECK_CTX(ctx);
   if (!out_dptr) return tl_set_error(ctx, TL_ERR_INVALID_ARG, "tl_alloc: null out pointer");
   *out_dptr = nullptr;
   DeviceGuard guard(ctx->device);
-  // while a graph is being captured neither pooled nor new memory is given: the graph would keep the address
   cudaError_t e;
   try {
-    e = ctx->capturing ? cudaMalloc(out_dptr, bytes ? bytes : 1) : ctx->pool.alloc(bytes, out_dptr);
+    // under capture CUDA says whether there may be memory; the pool has none to give
+    e = capture_open(ctx) ? cudaMalloc(out_dptr, bytes ? bytes : 1) : ctx->pool.alloc(bytes, out_dptr);
   } catch (const std::exception&) {
     e = cudaErrorMemoryAllocation;  // the host ran out
   }
@@ -258,7 +269,12 @@ int32_t tl_free(tl_ctx* ctx, void* dptr) {
   TL_CHECK_CTX(ctx);
   if (!dptr) return TL_OK;
   DeviceGuard guard(ctx->device);
-  if (ctx->capturing) TL_CUDA(ctx, cudaStreamSynchronize(ctx->stream));  // refused under capture, as it always was
+  if (capture_open(ctx)) {
+    const cudaError_t refused = cudaStreamSynchronize(ctx->stream);
+    if (refused != cudaSuccess) cudaGetLastError();
+    TL_CUDA(ctx, refused);
+    if (t_captures > 0) return tl_set_error(ctx, TL_ERR_CUDA, "tl_free: not while this thread captures a graph on another context");
+  }
   bool known = false;
   cudaError_t e;
   try {
@@ -361,6 +377,7 @@ int32_t tl_graph_begin(tl_ctx* ctx) {
   DeviceGuard guard(ctx->device);
   TL_CUDA(ctx, cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
   ctx->capturing = true;
+  ++t_captures;
   for (int i = 0; i < TL_COUNTER_COUNT; ++i) g_capture_base[i] = ctx->counters[i];
   return TL_OK;
 }
@@ -371,6 +388,7 @@ int32_t tl_graph_end(tl_ctx* ctx, tl_graph** out_graph) {
   if (!out_graph) return tl_set_error(ctx, TL_ERR_INVALID_ARG, "tl_graph_end: null out pointer");
   DeviceGuard guard(ctx->device);
   ctx->capturing = false;
+  if (t_captures > 0) --t_captures;  // a capture ends on the thread that began it
   tl_graph* g = new tl_graph();
   cudaError_t e = cudaStreamEndCapture(ctx->stream, &g->graph);
   if (e != cudaSuccess || !g->graph) {
