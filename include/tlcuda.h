@@ -137,7 +137,8 @@ TL_API int32_t tl_get_option(tl_ctx* ctx, const char* name, int64_t* out_value);
  * :666) ---------------------------------------------------------------------- */
 /* tl_free keeps the block for a later tl_alloc (at most 1 GiB in all; blocks above 256 MB go straight back), which gets
  * it only after all that any stream of the device had been given by the tl_free is over.  A tl_free that fails leaves the
- * block with the caller.  What is kept is given back when a tl_alloc runs short and by tl_ctx_destroy. */
+ * block with the caller.  What is kept is given back when the library runs short of memory, in whichever context of the device, and by
+ * tl_ctx_destroy. */
 TL_API int32_t tl_alloc(tl_ctx* ctx, size_t bytes, void** out_dptr);
 TL_API int32_t tl_free(tl_ctx* ctx, void* dptr);
 TL_API int32_t tl_upload(tl_ctx* ctx, void* dst_dptr, const void* src_host, size_t bytes);

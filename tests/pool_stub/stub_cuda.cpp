@@ -12,11 +12,15 @@ static std::map<uintptr_t, size_t> device;  // what is allocated
 static uintptr_t next_address = 1 << 20;
 static int mallocs = 0, frees = 0;
 static cudaError_t fail_malloc = cudaSuccess, fail_free = cudaSuccess;  // every call fails with this
+static size_t memory = SIZE_MAX;  // cudaMalloc fails beyond this
 
 extern "C" {
 cudaError_t cudaMalloc(void** out, size_t bytes) {
   ++mallocs;
   if (fail_malloc != cudaSuccess) return fail_malloc;
+  size_t used = 0;
+  for (const auto& d : device) used += d.second;
+  if (bytes > memory || used > memory - bytes) return cudaErrorMemoryAllocation;
   *out = reinterpret_cast<void*>(next_address);
   device[next_address] = bytes;
   next_address += (bytes + 511) / 512 * 512 + 512;
@@ -127,9 +131,30 @@ static void bounds() {
   CHECK(device.empty());
 }
 
+// memory is short: what every pool of the device keeps goes back, for the library's own buffers as for blocks
+static void short_of_memory() {
+  for (int own = 0; own < 2; ++own) {
+    TlBlockPool a, b, other;
+    a.device = b.device = 0;
+    other.device = 1;
+    void* still = take(a, 10 << 20);
+    for (TlBlockPool* p : {&a, &b, &other}) give(*p, take(*p, 100 << 20));
+    memory = size_t(320) << 20;
+    void* p = nullptr;
+    const cudaError_t e = own ? b.device_malloc(&p, 200 << 20) : b.alloc(200 << 20, &p);
+    CHECK(e == cudaSuccess && p && device.count(reinterpret_cast<uintptr_t>(still)));
+    CHECK(a.waiting_bytes + a.ready_bytes == 0 && b.waiting_bytes + b.ready_bytes == 0 && other.waiting_bytes + other.ready_bytes > 0);
+    CHECK((own ? a.device_malloc(&p, 200 << 20) : a.alloc(200 << 20, &p)) == cudaErrorMemoryAllocation);
+    memory = SIZE_MAX;
+    device.clear();
+    a.live.clear(); b.live.clear(); other.waiting.clear();
+  }
+}
+
 int main(int, char** argv) {
   const struct { const char* name; void (*run)(); } tests[] = {
-      {"reuse", reuse}, {"failing_fence", failing_fence}, {"no_memory_for_the_fence", no_memory_for_the_fence}, {"bounds", bounds}};
+      {"reuse", reuse}, {"failing_fence", failing_fence}, {"no_memory_for_the_fence", no_memory_for_the_fence}, {"bounds", bounds},
+      {"short_of_memory", short_of_memory}};
   for (const auto& t : tests)
     if (!strcmp(t.name, argv[1])) { t.run(); return 0; }
   return 2;

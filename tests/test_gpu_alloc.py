@@ -200,3 +200,48 @@ def test_a_graph_of_this_thread_on_another_context_refuses(be):
     assert be._alloc(1000) != p
     be._free(p)
     be2.destroy()
+
+
+def _int4(be, n, k, seed):
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    packed = torch.randint(-2 ** 31, 2 ** 31 - 1, (n, k // 8), dtype=torch.int32, device="cuda", generator=gen)
+    scales = torch.full((n, k // 128), 0.01, dtype=torch.float16, device="cuda")
+    st = tb.CudaTensor(be, [n, k // 128], "u16", scales.data_ptr(), scales.nbytes, ownsBuffer=False)
+    w = tb.CudaTensor(be, [n, k], "f16", packed.data_ptr(), packed.nbytes, ownsBuffer=False, scales=st,
+                      format=tb.StorageFormat("f16", tb.QuantPacking("int4-grouped", 128, "f16")))
+    x = torch.randn(20, k, device="cuda", generator=gen).half()
+    xt = tb.CudaTensor(be, [20, k], "f16", x.data_ptr(), x.nbytes, ownsBuffer=False)
+    y = torch.empty(20, n, device="cuda", dtype=torch.float32)
+    yt = tb.CudaTensor(be, [20, n], "f32", y.data_ptr(), y.nbytes, ownsBuffer=False)
+    torch.cuda.synchronize()
+
+    def run():
+        be.ops.matmul(xt, be.ops.transpose(w), {"outBuffer": yt})
+        be.sync()
+        return y
+    run.keep = packed, scales, x
+    return run
+
+
+def test_scratch_takes_the_memory_that_freed_blocks_hold():
+    """A nearly full GPU: the library's own scratch grows into what tl_free kept."""
+    n, k = 16384, 16384  # 512 MB of scratch for the 16-bit copy
+    own, hog = tb.CudaBackend(0), None
+    try:
+        _int4(own, 256, 256, 0)()  # its kernels are loaded
+        run = _int4(own, n, k, 1)
+        torch.cuda.empty_cache()
+        blocks = [own._alloc(200 << 20) for _ in range(4)]
+        for p in blocks:
+            own._free(p)
+        free = torch.cuda.mem_get_info()[0]
+        hog = torch.empty(free - (256 << 20), dtype=torch.uint8, device="cuda")
+        got = run().clone()
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+        own.destroy()
+    plenty = tb.CudaBackend(0)
+    ref = _int4(plenty, n, k, 1)()
+    plenty.destroy()
+    assert bool(torch.isfinite(got).all()) and torch.equal(got, ref)

@@ -18,6 +18,6 @@ def harness(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("name", ["reuse", "failing_fence", "no_memory_for_the_fence", "bounds"])
+@pytest.mark.parametrize("name", ["reuse", "failing_fence", "no_memory_for_the_fence", "bounds", "short_of_memory"])
 def test_block_pool(harness, name):
     subprocess.run([harness, name], check=True)

@@ -33,7 +33,7 @@ int32_t tl_ensure_scratch(tl_ctx* ctx, size_t bytes, void** out) {
       ctx->scratch_bytes = 0;
     }
     size_t want = bytes < (size_t(1) << 20) ? (size_t(1) << 20) : bytes;
-    cudaError_t e = cudaMalloc(&ctx->scratch, want);
+    cudaError_t e = ctx->pool.device_malloc(&ctx->scratch, want);
     if (e != cudaSuccess) {
       cudaGetLastError();
       return tl_set_error(ctx, TL_ERR_OOM, "scratch allocation of %zu bytes failed: %s", want,
@@ -59,7 +59,7 @@ int32_t tl_ensure_zeroed_scratch(tl_ctx* ctx, size_t bytes, void** out) {
       ctx->zscratch_bytes = 0;
     }
     size_t want = bytes < (size_t(1) << 20) ? (size_t(1) << 20) : bytes;
-    cudaError_t e = cudaMalloc(&ctx->zscratch, want);
+    cudaError_t e = ctx->pool.device_malloc(&ctx->zscratch, want);
     if (e != cudaSuccess) {
       cudaGetLastError();
       return tl_set_error(ctx, TL_ERR_OOM, "scratch allocation of %zu bytes failed: %s", want,
@@ -115,6 +115,7 @@ int32_t tl_ctx_create(int32_t device_ordinal, tl_ctx** out_ctx) {
                         device_ordinal, prop.major, prop.minor);
   tl_ctx* ctx = new tl_ctx();
   ctx->device = device_ordinal;
+  ctx->pool.device = device_ordinal;
   ctx->sm_count = prop.multiProcessorCount;
   ctx->l2_bytes = prop.l2CacheSize;
   DeviceGuard guard(device_ordinal);
@@ -126,7 +127,7 @@ int32_t tl_ctx_create(int32_t device_ordinal, tl_ctx** out_ctx) {
   // one small block: the status word, then (from byte 64) the eight flag words of the timed
   // weight prefetch, which start out raised ("no launch is streaming")
   const uint32_t ones[8] = {1, 1, 1, 1, 1, 1, 1, 1};
-  if (cudaMalloc(&ctx->dev_status, 128) != cudaSuccess || cudaMemset(ctx->dev_status, 0, 128) != cudaSuccess ||
+  if (ctx->pool.device_malloc(reinterpret_cast<void**>(&ctx->dev_status), 128) != cudaSuccess || cudaMemset(ctx->dev_status, 0, 128) != cudaSuccess ||
       cudaMemcpy(reinterpret_cast<uint8_t*>(ctx->dev_status) + 64, ones, sizeof(ones), cudaMemcpyHostToDevice) != cudaSuccess) {
     cudaGetLastError();
     cudaStreamDestroy(ctx->stream);

@@ -113,8 +113,8 @@ int32_t tl_pretune(tl_ctx* ctx, const tl_shape* shapes, int32_t n_shapes, int32_
     auto cleanup = [&]() {
       cudaFree(w); cudaFree(s); cudaFree(a); cudaFree(o);
     };
-    if (cudaMalloc(&w, wbytes * copies) != cudaSuccess || cudaMalloc(&s, sbytes * copies) != cudaSuccess ||
-        cudaMalloc(&a, abytes) != cudaSuccess || cudaMalloc(&o, obytes) != cudaSuccess) {
+    if (ctx->pool.device_malloc(&w, wbytes * copies) != cudaSuccess || ctx->pool.device_malloc(&s, sbytes * copies) != cudaSuccess ||
+        ctx->pool.device_malloc(&a, abytes) != cudaSuccess || ctx->pool.device_malloc(&o, obytes) != cudaSuccess) {
       cudaGetLastError();
       cleanup();
       return tl_set_error(ctx, TL_ERR_OOM, "tl_pretune: cannot allocate bench buffers for %lldx%lldx%lld",

@@ -340,7 +340,7 @@ int32_t tl_p2p_create(tl_ctx* ctx, size_t max_bytes, void* out_handle64) {
   DeviceGuard guard(ctx->device);
   max_bytes = (max_bytes + 255) & ~size_t(255);
   void* p = nullptr;
-  cudaError_t e = cudaMalloc(&p, p2p_total_bytes(max_bytes));
+  cudaError_t e = ctx->pool.device_malloc(&p, p2p_total_bytes(max_bytes));
   if (e != cudaSuccess) {
     cudaGetLastError();
     return tl_set_error(ctx, TL_ERR_OOM, "tl_p2p_create: %s", cudaGetErrorString(e));

@@ -5,6 +5,35 @@
 #include <cstdint>
 #include <iterator>
 
+namespace {
+std::mutex pools_lock;  // taken before a pool's own
+std::vector<TlBlockPool*> pools;
+}  // namespace
+
+TlBlockPool::TlBlockPool() {
+  std::lock_guard<std::mutex> hold(pools_lock);
+  pools.push_back(this);
+}
+
+TlBlockPool::~TlBlockPool() {
+  std::lock_guard<std::mutex> hold(pools_lock);
+  pools.erase(std::find(pools.begin(), pools.end(), this));
+}
+
+void TlBlockPool::release_device() {
+  std::lock_guard<std::mutex> hold(pools_lock);
+  for (TlBlockPool* p : pools)
+    if (p->device == device) p->release();
+}
+
+cudaError_t TlBlockPool::device_malloc(void** out, size_t bytes) {
+  cudaError_t e = cudaMalloc(out, bytes);
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  release_device();
+  return cudaMalloc(out, bytes);
+}
+
 void TlBlockPool::fenced() {
   while (!waiting.empty()) {
     const auto w = waiting.back();
@@ -61,7 +90,7 @@ cudaError_t TlBlockPool::alloc(size_t bytes, void** out) {
   if (e == cudaErrorMemoryAllocation) {  // give back what is kept, then ask for no more than was asked for
     cudaGetLastError();
     hold.unlock();
-    release();
+    release_device();
     hold.lock();
     got = bytes ? bytes : 1;
     e = cudaMalloc(out, got);

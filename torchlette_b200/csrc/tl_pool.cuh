@@ -18,6 +18,10 @@
 #include <vector>
 
 struct TlBlockPool {
+  TlBlockPool();
+  ~TlBlockPool();
+  TlBlockPool(const TlBlockPool&) = delete;
+  TlBlockPool& operator=(const TlBlockPool&) = delete;
   static constexpr size_t kKeptBytes = size_t(1) << 30;       // blocks kept in all, waiting ones included
   static constexpr size_t kLargestBytes = size_t(1) << 28;    // larger blocks go straight back
   static constexpr size_t kWaitingBytes = size_t(1) << 28;
@@ -32,9 +36,14 @@ struct TlBlockPool {
   // *known: the block is one of the pool's (a pointer from elsewhere is left to the caller).  After an error the block is
   // still the caller's.
   cudaError_t free(void* p, bool* known);
+  // cudaMalloc for the library itself (scratch, schedules): where memory is short, what the device's pools keep goes
+  // back first
+  cudaError_t device_malloc(void** out, size_t bytes);
   void release();  // gives back all that is kept
+  int device = -1;
 
  private:
+  void release_device();   // of every context of the device (not with `lock` held)
   void fenced();           // a fence has just passed: waiting blocks become ready
   void trim(size_t keep);  // gives ready blocks back until at most `keep` bytes of them are left, the largest first
 };

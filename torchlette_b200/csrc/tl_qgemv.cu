@@ -2885,7 +2885,7 @@ extern "C" int32_t tl_qgemv_chain_create(tl_ctx* ctx, const tl_chain_phase* phas
     return tl_set_error(ctx, TL_ERR_CUDA, "tl_qgemv_chain_create: occupancy query failed: %s", cudaGetErrorString(e));
   }
   ch->grid = ctx->sm_count * per_sm;  // all of them co-resident: the launch is cooperative
-  e = cudaMalloc(&ch->d_epi, epis.size() * sizeof(EpiParams));
+  e = ctx->pool.device_malloc(reinterpret_cast<void**>(&ch->d_epi), epis.size() * sizeof(EpiParams));
   if (e == cudaSuccess) e = cudaMemcpy(ch->d_epi, epis.data(), epis.size() * sizeof(EpiParams), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) {
     tl_qgemv_chain_destroy(ctx, ch);
@@ -2934,8 +2934,8 @@ extern "C" int32_t tl_qgemv_chain_create(tl_ctx* ctx, const tl_chain_phase* phas
   flat.resize(lists.size() * size_t(ch->stride));
   for (size_t cta = 0; cta < lists.size(); ++cta)
     std::copy(lists[cta].begin(), lists[cta].end(), flat.begin() + cta * size_t(ch->stride));
-  e = cudaMalloc(&ch->d_sched, flat.size() * sizeof(ChainTile));
-  if (e == cudaSuccess) e = cudaMalloc(&ch->d_bar, size_t(n_phases + 1) * sizeof(unsigned));
+  e = ctx->pool.device_malloc(reinterpret_cast<void**>(&ch->d_sched), flat.size() * sizeof(ChainTile));
+  if (e == cudaSuccess) e = ctx->pool.device_malloc(reinterpret_cast<void**>(&ch->d_bar), size_t(n_phases + 1) * sizeof(unsigned));
   if (e == cudaSuccess) e = cudaMemcpy(ch->d_sched, flat.data(), flat.size() * sizeof(ChainTile), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) {
     tl_qgemv_chain_destroy(ctx, ch);

@@ -639,7 +639,7 @@ int32_t tl_launch_qgemv_stream(tl_ctx* ctx, const tl_variant& v, const void* a, 
     const size_t bytes = size_t(ctx->sm_count) * 2 * 2 * 128 * sizeof(float) + size_t(ctx->sm_count) * sizeof(unsigned);
     if (ctx->capturing)
       return tl_set_error(ctx, TL_ERR_UNSUPPORTED, "qgemv: the stream kernel's scratch must exist before graph capture; run the call once first");
-    TL_CUDA(ctx, cudaMalloc(&ctx->stream_scratch, bytes));
+    TL_CUDA(ctx, ctx->pool.device_malloc(&ctx->stream_scratch, bytes));
     TL_CUDA(ctx, cudaMemset(ctx->stream_scratch, 0, bytes));
   }
   p.a = a;
