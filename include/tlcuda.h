@@ -129,13 +129,16 @@ TL_API int32_t tl_device_sm_count(tl_ctx* ctx, int32_t* out_sms);
  *                            at 2^22).
  *   "push_poll_ranks"        reduce-on-read (tl_qgemv_nt_push's consumer): how many ranks' words a
  *                            summing thread requests together before it checks them, 1..4
- *                            (default 4; 1 polls the ranks one after the other). */
+ *                            (default 4; 1 polls the ranks one after the other).
+ *   "kept_bytes"             upper bound of the memory that tl_free keeps for later tl_alloc calls
+ *                            (default 2^30; 0 gives every block straight back).  Setting it gives
+ *                            back what is kept, for a host that is short of memory itself. */
 TL_API int32_t tl_set_option(tl_ctx* ctx, const char* name, int64_t value);
 TL_API int32_t tl_get_option(tl_ctx* ctx, const char* name, int64_t* out_value);
 
 /* ---- memory: tensorFromArray / read / destroy (src/backend/types.ts:341-345,
  * :666) ---------------------------------------------------------------------- */
-/* tl_free keeps the block for a later tl_alloc (at most 1 GiB in all; blocks above 256 MB go straight back), which gets
+/* tl_free keeps the block for a later tl_alloc (option "kept_bytes", 1 GiB in all; blocks above a quarter of it go straight back), which gets
  * it only after all that any stream of the device had been given by the tl_free is over.  A tl_free that fails leaves the
  * block with the caller.  What is kept is given back when the library runs short of memory, in whichever context of the device, and by
  * tl_ctx_destroy. */

@@ -122,6 +122,19 @@ static void bounds() {
     give(pool, q);
     CHECK(pool.ready_bytes + pool.waiting_bytes <= TlBlockPool::kKeptBytes);
   }
+  pool.keep_at_most(size_t(100) << 20);
+  CHECK(device.size() == pool.live.size() && pool.ready_bytes + pool.waiting_bytes == 0);  // all that was kept went back
+  held.clear();
+  for (int i = 0; i < 20; ++i) held.push_back(take(pool, size_t(20) << 20));
+  for (void* q : held) {
+    give(pool, q);
+    CHECK(pool.ready_bytes + pool.waiting_bytes <= size_t(100) << 20);
+  }
+  CHECK(pool.ready_bytes + pool.waiting_bytes > 0);
+  pool.keep_at_most(0);
+  give(pool, take(pool, 1));
+  CHECK(device.empty());
+  pool.keep_at_most(TlBlockPool::kKeptBytes);
   bool known = false;
   p = take(pool, 100);
   give(pool, p);

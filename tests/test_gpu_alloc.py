@@ -202,6 +202,23 @@ def test_a_graph_of_this_thread_on_another_context_refuses(be):
     be2.destroy()
 
 
+def test_kept_bytes(be):
+    """A program that needs the memory elsewhere: what is kept goes back at once, and with 0 nothing is kept."""
+    assert be.getOption("kept_bytes") == 1 << 30
+    blocks = [be._alloc(100 << 20) for _ in range(3)]
+    for p in blocks:
+        be._free(p)
+    held = torch.cuda.mem_get_info()[0]
+    be.setOption("kept_bytes", 0)
+    assert torch.cuda.mem_get_info()[0] >= held + (300 << 20)
+    free = torch.cuda.mem_get_info()[0]
+    be._free(be._alloc(100 << 20))
+    assert torch.cuda.mem_get_info()[0] >= free
+    with pytest.raises(tb.TlError):
+        be.setOption("kept_bytes", -1)
+    be.setOption("kept_bytes", 1 << 30)
+
+
 def _int4(be, n, k, seed):
     gen = torch.Generator(device="cuda").manual_seed(seed)
     packed = torch.randint(-2 ** 31, 2 ** 31 - 1, (n, k // 8), dtype=torch.int32, device="cuda", generator=gen)

@@ -70,6 +70,12 @@ void TlBlockPool::release() {
   if (mark && cudaFree(mark) == cudaSuccess) mark = nullptr;
 }
 
+void TlBlockPool::keep_at_most(size_t bytes) {
+  release();
+  std::lock_guard<std::mutex> hold(lock);
+  keep = bytes;
+}
+
 cudaError_t TlBlockPool::alloc(size_t bytes, void** out) {
   // capacities in steps of 512 bytes, or of 1/64 to 1/32 of the size where that is more: sizes that differ a little
   // from call to call share blocks, and little is lost in weights that stay
@@ -116,8 +122,9 @@ cudaError_t TlBlockPool::free(void* p, bool* known) {
     return *known ? cudaErrorInvalidValue : cudaSuccess;  // given back twice, or not from here
   }
   const size_t cap = it->second;
-  const bool full = waiting.size() + 1 >= kWaitingBlocks || waiting_bytes + cap >= kWaitingBytes;
-  bool kept = cap <= kLargestBytes;
+  const size_t part = keep / 4;  // kLargestBytes and kWaitingBytes
+  const bool full = waiting.size() + 1 >= kWaitingBlocks || waiting_bytes + cap >= part;
+  bool kept = cap <= part;
   if (kept && full) {
     cudaError_t e = mark ? cudaSuccess : cudaMalloc(&mark, 256);
     if (e == cudaErrorMemoryAllocation) {
@@ -146,6 +153,6 @@ cudaError_t TlBlockPool::free(void* p, bool* known) {
     live.erase(it);
     return cudaSuccess;
   }
-  trim(kKeptBytes - kWaitingBytes);
+  trim(keep - part);
   return cudaSuccess;
 }

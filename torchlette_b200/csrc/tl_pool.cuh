@@ -22,9 +22,9 @@ struct TlBlockPool {
   ~TlBlockPool();
   TlBlockPool(const TlBlockPool&) = delete;
   TlBlockPool& operator=(const TlBlockPool&) = delete;
-  static constexpr size_t kKeptBytes = size_t(1) << 30;       // blocks kept in all, waiting ones included
-  static constexpr size_t kLargestBytes = size_t(1) << 28;    // larger blocks go straight back
-  static constexpr size_t kWaitingBytes = size_t(1) << 28;
+  static constexpr size_t kKeptBytes = size_t(1) << 30;     // blocks kept in all, waiting ones included
+  static constexpr size_t kLargestBytes = kKeptBytes / 4;   // larger blocks go straight back
+  static constexpr size_t kWaitingBytes = kKeptBytes / 4;
   static constexpr size_t kWaitingBlocks = 64;
   std::mutex lock;                            // tl_alloc and tl_free may come from several threads
   std::map<void*, size_t> live;               // handed out: capacity
@@ -40,7 +40,9 @@ struct TlBlockPool {
   // back first
   cudaError_t device_malloc(void** out, size_t bytes);
   void release();  // gives back all that is kept
+  void keep_at_most(size_t bytes);  // in place of kKeptBytes; 0: tl_free gives every block straight back
   int device = -1;
+  size_t keep = kKeptBytes;
 
  private:
   void release_device();   // of every context of the device (not with `lock` held)
