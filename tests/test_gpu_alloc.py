@@ -262,3 +262,40 @@ def test_scratch_takes_the_memory_that_freed_blocks_hold():
     ref = _int4(plenty, n, k, 1)()
     plenty.destroy()
     assert bool(torch.isfinite(got).all()) and torch.equal(got, ref)
+
+
+def test_dequantize_dense_without_memory_is_the_fused_kernel():
+    """No room for the 16-bit copy of the weight: the fused kernel computes the call, unless the route was asked for by name."""
+    m, n, k = 300, 16384, 16384
+    gen = torch.Generator(device="cuda").manual_seed(2)
+    q = torch.randint(-127, 128, (n, k), dtype=torch.int8, device="cuda", generator=gen)
+    scales = torch.full((n, 1), 1e-3, device="cuda")
+    x, y = torch.randn(m, k, device="cuda", generator=gen).half(), torch.empty(m, n, device="cuda")
+    own, hog = tb.CudaBackend(0), None
+    wrap = lambda t, dtype, **more: tb.CudaTensor(own, list(t.shape), dtype, t.data_ptr(), t.nbytes, ownsBuffer=False, **more)  # noqa: E731
+    fmt = tb.perChannelFormat(k)
+    w = own.ops.transpose(wrap(q, "f16", format=fmt, scales=wrap(scales, "f32")))
+    xt, yt = wrap(x, "f16"), wrap(y, "f32")
+    dense = (2, 2, 0, 0, 0, 0)
+
+    def run(variant):
+        own.forceVariant(variant)
+        own.ops.matmul(xt, w, {"outBuffer": yt})
+        own.sync()
+        return y.clone()
+
+    torch.cuda.synchronize()
+    try:
+        fused = [run((2, 0, 192, 128, 3, 8)), run((2, 0, 128, 128, 4, 8))]
+        own.forceVariant(None)
+        own.seedPerShapeMatmulChoice(m, n, k, "f16", fmt.packing, dense)
+        torch.cuda.empty_cache()
+        hog = torch.empty(torch.cuda.mem_get_info()[0] - (256 << 20), dtype=torch.uint8, device="cuda")
+        with pytest.raises(tb.TlError, match="scratch"):
+            run(dense)
+        got = run(None)
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+        own.destroy()
+    assert any(torch.equal(got, r) for r in fused)

@@ -294,3 +294,35 @@ def test_qgemm_group_scales_every_form(backend, variant, group):
     assert cases.rel_err(be.ops.read(y), orc.matmul_nt(xb.astype(np.float32), w16)) <= 1e-3
     for t in (y, xt, wt.scales, wt):
         t.destroy()
+
+
+def test_qgemm_dequant_dense_without_scratch_is_the_fused_default():
+    """A capture that may not grow the scratch: the fused kernel with the tile that the rule picks for these tokens (which here
+    needs no scratch of its own), to the bit."""
+    m, n, k = 300, 4096, 4096
+    cs = cases.per_channel_case(n, k, m, seed=9, act_dtype="f16")
+    fmt = tb.perChannelFormat(k)
+    outs = []
+    for captured in (False, True):
+        be = tb.CudaBackend(0)
+        w = be.createQuantizedWeight(cs["packed"], cs["scales"], n, k, fmt)
+        x = be.ops.tensorFromArray(cs["x_bits"], [m, k], "f16")
+        out = be.ops.empty([m, n], "f32")
+        if captured:
+            be.seedPerShapeMatmulChoice(m, n, k, "f16", fmt.packing, DEQUANT_DENSE)
+            be.beginCapture()
+            try:
+                be.ops.matmul(x, be.ops.transpose(w), {"outBuffer": out})
+            finally:
+                graph = be.endCapture()
+            be.replay(graph)
+            outs.append(be.ops.read(out))
+            be.destroyGraph(graph)
+        else:
+            assert be.planQuantizedMatmul(m, n, k, "f16", "f32", fmt.packing)["choice"][2] == 128
+            be.ops.matmul(x, be.ops.transpose(w), {"outBuffer": out})
+            outs.append(be.ops.read(out))
+        for t in (x, out, w.scales, w):
+            t.destroy()
+        be.destroy()
+    np.testing.assert_array_equal(outs[0], outs[1])

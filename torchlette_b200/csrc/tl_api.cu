@@ -720,6 +720,10 @@ static int32_t qmatmul_impl(tl_ctx* ctx, const char* who, int route /*0 auto,1 g
       if (has_ops) ctx->counters[TL_COUNTER_QGEMV_EPILOGUE]++;
     }
   } else {
+    if (!receipt_only && !(ctx->has_forced && ctx->forced.family == TL_FAMILY_QGEMM)) {
+      rc = tl_qgemm_secure_scratch(ctx, &v, m, n, k, a_dtype, *qdesc);
+      if (rc != TL_OK) return rc;
+    }
     rc = tl_launch_qgemm(ctx, v, a, a_dtype, packed, scales, out, out_dtype, m, n, k, *qdesc, epi,
                          receipt_only);
     if (rc == TL_OK && !receipt_only) ctx->counters[TL_COUNTER_QGEMM]++;

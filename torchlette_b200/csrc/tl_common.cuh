@@ -256,6 +256,7 @@ int32_t tl_qgemv_default_variant(tl_ctx* ctx, int32_t m, int64_t n, int64_t k, i
                                  const tl_quant_desc& q, tl_variant* out);
 int32_t tl_qgemv_candidates(tl_ctx* ctx, int32_t m, int64_t n, int64_t k, int32_t a_dtype,
                             const tl_quant_desc& q, std::vector<tl_variant>* out);
+int32_t tl_qgemm_secure_scratch(tl_ctx* ctx, tl_variant* v, int64_t m, int64_t n, int64_t k, int32_t a_dtype, const tl_quant_desc& q);
 int32_t tl_qgemm_default_variant(tl_ctx* ctx, int64_t m, int64_t n, int64_t k, int32_t a_dtype,
                                  const tl_quant_desc& q, tl_variant* out);
 int32_t tl_qgemm_candidates(tl_ctx* ctx, int64_t m, int64_t n, int64_t k, int32_t a_dtype,

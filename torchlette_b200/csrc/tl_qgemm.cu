@@ -634,45 +634,64 @@ bool tl_qgemm_variant_applicable(const tl_variant& v, int64_t m, int64_t n, int6
   return (a_dtype == TL_F16 || a_dtype == TL_BF16) && k % 16 == 0 && q.group_size % 16 == 0 && tc_config_known(v);
 }
 
+namespace {
+// The fused kernel's tile, by the token count, and (*us) its modelled time above 64 tokens.  Only for what the fused kernel
+// takes: 16-bit activations, k and groups of whole 16s.
+tl_variant fused_tile(tl_ctx* ctx, int64_t m, int64_t n, int64_t k, int32_t a_dtype, const tl_quant_desc& q, double* us) {
+  *us = 0;
+  if (m <= 16) return tl_variant{TL_FAMILY_QGEMM, kTc, 16, 128, 8, 8};
+  if (m <= 32) return tl_variant{TL_FAMILY_QGEMM, kTc, 32, 128, 8, 8};
+  if (m <= 64) return tl_variant{TL_FAMILY_QGEMM, kTc, 64, 128, 6, 8};
+  // The token tile by modelled time: waves x 128-k steps x the time of a step, a last partial wave cut along K as the
+  // launch does it, 7 us for the meeting of its parts.  Step times on B200: 192 tokens 0.72 us (f16) / 0.78 (bf16) /
+  // 0.95 (group scales), 128 tokens 0.53 / 0.67 / 0.9.  Measured, us, 192 / 128: 2048 x 14336 x 4096 f16 201 / 215, bf16
+  // 217 / 268; 333 x 12288 x 4096 f16 45 / 37, groups of 64 57 / 64; 600 x 14336 x 2048 f16 51 / 38.
+  const int64_t sms = ctx ? ctx->sm_count : 148, ksteps = (k + 127) / 128;
+  const bool grouped = q.group_size != k, half = a_dtype == TL_F16;
+  auto fused_us = [&](int bn, double step) {
+    const int64_t tiles = ((n + kTileRows - 1) / kTileRows) * ((m + bn - 1) / bn), rem = tiles % sms;
+    const int64_t splits = rem ? std::min<int64_t>({sms / rem, 4, ksteps}) : 1;
+    return (double(tiles / sms) + (rem ? 1.0 / double(splits) : 0.0)) * double(ksteps) * step + (splits > 1 ? 7.0 : 0.0);
+  };
+  const double t192 = fused_us(192, grouped ? 0.95 : half ? 0.72 : 0.78), t128 = fused_us(128, grouped ? 0.9 : half ? 0.53 : 0.67);
+  *us = std::min(t192, t128);
+  return t192 <= t128 ? tl_variant{TL_FAMILY_QGEMM, kTc, 192, 128, 3, 8} : tl_variant{TL_FAMILY_QGEMM, kTc, 128, 128, 4, 8};
+}
+}  // namespace
+
 int32_t tl_qgemm_default_variant(tl_ctx* ctx, int64_t m, int64_t n, int64_t k, int32_t a_dtype,
                                  const tl_quant_desc& q, tl_variant* out) {
   tl_variant v{};
   v.family = TL_FAMILY_QGEMM;
   if ((a_dtype == TL_F16 || a_dtype == TL_BF16) && k % 16 == 0 && q.group_size % 16 == 0) {
-    v.kernel = kTc;
-    if (m <= 16) { v.p0 = 16; v.p1 = 128; v.p2 = 8; v.p3 = 8; }
-    else if (m <= 32) { v.p0 = 32; v.p1 = 128; v.p2 = 8; v.p3 = 8; }
-    else if (m <= 64) { v.p0 = 64; v.p1 = 128; v.p2 = 6; v.p3 = 8; }
-    else {
-      // The token tile by modelled time: waves x 128-k steps x the time of a step, a last partial wave cut along K as the
-      // launch does it, 7 us for the meeting of its parts.  Step times on B200: 192 tokens 0.72 us (f16) / 0.78 (bf16) /
-      // 0.95 (group scales), 128 tokens 0.53 / 0.67 / 0.9.  Measured, us, 192 / 128: 2048 x 14336 x 4096 f16 201 / 215, bf16
-      // 217 / 268; 333 x 12288 x 4096 f16 45 / 37, groups of 64 57 / 64; 600 x 14336 x 2048 f16 51 / 38.
-      const int64_t sms = ctx ? ctx->sm_count : 148, ksteps = (k + 127) / 128;
-      const bool grouped = q.group_size != k, half = a_dtype == TL_F16;
-      auto fused_us = [&](int bn, double step) {
-        const int64_t tiles = ((n + kTileRows - 1) / kTileRows) * ((m + bn - 1) / bn), rem = tiles % sms;
-        const int64_t splits = rem ? std::min<int64_t>({sms / rem, 4, ksteps}) : 1;
-        return (double(tiles / sms) + (rem ? 1.0 / double(splits) : 0.0)) * double(ksteps) * step + (splits > 1 ? 7.0 : 0.0);
-      };
-      const double t192 = fused_us(192, grouped ? 0.95 : half ? 0.72 : 0.78), t128 = fused_us(128, grouped ? 0.9 : half ? 0.53 : 0.67);
-      if (t192 <= t128) { v.p0 = 192; v.p1 = 128; v.p2 = 3; v.p3 = 8; }
-      else { v.p0 = 128; v.p1 = 128; v.p2 = 4; v.p3 = 8; }
-      // With many tokens per weight byte, writing the weight out once as a 16-bit matrix and running the
-      // dense kernel (whose operands both come from shared memory at its full tile sizes) beats converting
-      // on the operand path: the dense kernel's modelled time, the pass at 6 TB/s (3 bytes a weight) and 4 us for the second
-      // launch.  Measured, us, fused / this way: 2048 tokens, n = 4096, k = 14336 bf16 222 / 190; n = 14336, k = 4096
-      // 217 / 223 (stays fused), with groups of 128 249 / 215; 700 x 4096 x 4096, groups of 64, 37 / 37.
-      const tl_variant dd{TL_FAMILY_QGEMM, kDequantDense, 0, 0, 0, 0};
-      if (m > 128 && tl_qgemm_variant_applicable(dd, m, n, k, a_dtype, q)) {
-        const double dense_us = tl_dense_tc_choose(m, n, k, int(sms)).cost_us + double(n) * double(k) * 3.0 / 6.0e6 + 4.0;
-        if (dense_us < 0.95 * std::min(t192, t128)) v = dd;
-      }
+    double fused_us = 0;
+    v = fused_tile(ctx, m, n, k, a_dtype, q, &fused_us);
+    // With many tokens per weight byte, writing the weight out once as a 16-bit matrix and running the
+    // dense kernel (whose operands both come from shared memory at its full tile sizes) beats converting
+    // on the operand path: the dense kernel's modelled time, the pass at 6 TB/s (3 bytes a weight) and 4 us for the second
+    // launch.  Measured, us, fused / this way: 2048 tokens, n = 4096, k = 14336 bf16 222 / 190; n = 14336, k = 4096
+    // 217 / 223 (stays fused), with groups of 128 249 / 215; 700 x 4096 x 4096, groups of 64, 37 / 37.
+    const tl_variant dd{TL_FAMILY_QGEMM, kDequantDense, 0, 0, 0, 0};
+    if (m > 128 && tl_qgemm_variant_applicable(dd, m, n, k, a_dtype, q)) {
+      const double dense_us = tl_dense_tc_choose(m, n, k, ctx ? ctx->sm_count : 148).cost_us + double(n) * double(k) * 3.0 / 6.0e6 + 4.0;
+      if (dense_us < 0.95 * fused_us) v = dd;
     }
   } else {
     v.kernel = kSliced;  // f32 activations or odd K: sixteen-row slices through the small-batch kernels
   }
   *out = v;
+  return TL_OK;
+}
+
+// Dequantize + dense needs a 16-bit copy of the weight in scratch.  Where that is not to be had (memory is short, or a capture
+// may not grow it) *v becomes the fused kernel, which does without; any other failure is the call's.
+int32_t tl_qgemm_secure_scratch(tl_ctx* ctx, tl_variant* v, int64_t m, int64_t n, int64_t k, int32_t a_dtype, const tl_quant_desc& q) {
+  if (v->kernel != kDequantDense) return TL_OK;
+  void* wbuf = nullptr;
+  const int32_t rc = tl_ensure_scratch(ctx, size_t(n) * size_t(k) * 2, &wbuf);
+  if (rc != TL_ERR_OOM && !(rc == TL_ERR_UNSUPPORTED && ctx->capturing)) return rc;
+  double us;
+  *v = fused_tile(ctx, m, n, k, a_dtype, q, &us);
   return TL_OK;
 }
 
@@ -717,13 +736,7 @@ int32_t tl_launch_qgemm(tl_ctx* ctx, const tl_variant& v, const void* a, int32_t
       return tl_set_error(ctx, TL_ERR_INVALID_ARG, "qgemm: weight and activation pointers must be 16-byte aligned");
     void* wbuf = nullptr;
     int32_t rc = tl_ensure_scratch(ctx, size_t(n) * size_t(k) * 2, &wbuf);
-    if (rc != TL_OK) {
-      // No room for the 16-bit copy (or a capture that may not grow it): the fused kernel does without, unless this
-      // route was asked for by name.
-      if (ctx->has_forced && ctx->forced.family == TL_FAMILY_QGEMM && ctx->forced.kernel == kDequantDense) return rc;
-      const tl_variant fused{TL_FAMILY_QGEMM, kTc, 192, 128, 3, 8};
-      return tl_launch_qgemm(ctx, fused, a, a_dtype, packed, scales, out, out_dtype, m, n, k, q, epi, nullptr);
-    }
+    if (rc != TL_OK) return rc;
     const bool grouped = q.group_size != k;
     const float wscale = q.scale_convention == TL_SCALE_SNORM127 ? 1.0f / 127.0f : 1.0f;
     const int64_t n_oct = n * k / 8;
