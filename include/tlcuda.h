@@ -328,7 +328,8 @@ TL_API int32_t tl_decode_attention(tl_ctx* ctx, const void* q, const void* k_cac
  *  src/backend/webgpu/matmul/variants.ts:54-260) ------------------------------ */
 /* Kernel ids and parameters by family (tl_variant_name prints them):
  *   TL_FAMILY_QGEMV  (m <= 16): 0 scalar, 1 simt, 2 mma, 3 sk, 4 ring (default; p0 warps, p1 k blocks in flight,
- *                    p2 = 2: 32-row tiles), 5 tma, 6 bulk, 7 chain, 8 stream, 9 int4
+ *                    p2 = 2: 32-row tiles), 5 tma, 6 bulk, 7 chain, 8 stream, 9 int4 (tensor-core form: p0 warps, p1 row
+ *                    tiles of 16 per CTA, p2 stages; all 0: CUDA cores, and the receipt is the first launch)
  *   TL_FAMILY_QGEMM  (m > 16): 0 tcgen05 with the int8 -> 16-bit conversion on the operand path (p0 token tile,
  *                    p1 k per stage, p2 stages, p3 converter warps); 1 sliced (sixteen-row slices through the
  *                    small-batch kernels: f32 activations, odd K); 2 dequant+dense (the weight written once as a

@@ -6,6 +6,7 @@ import numpy as np
 import pytest
 
 import cases
+from launches import launches
 from oracle import oracle as orc
 from torchlette_b200 import backend as tb
 
@@ -169,5 +170,22 @@ def test_int4_ring_edges(backend, act, g, m, n, k):
     ref = xv @ wref.astype(np.float64).T
     size = np.abs(xv) @ np.abs(wref.astype(np.float64)).T
     assert (np.abs(be.ops.read(y) - ref) <= size * 2.0 ** -20).all()
+    for t in (x, y, w.scales, w):
+        t.destroy()
+
+
+@pytest.mark.parametrize("act", ["f16", "f32"])
+@pytest.mark.parametrize("m,n,k,g", [(1, 1000, 4096, 128), (4, 3000, 2048, 128), (4, 12000, 1024, 128), (16, 3000, 2048, 128), (16, 12000, 1024, 1024),
+                                     (16, 12000, 1024, 32), (1, 300, 128, 128), (3, 40, 136, 8)])
+def test_int4_receipt_is_the_launch(backend, act, m, n, k, g):
+    be = backend
+    packing = tb.QuantPacking("int4-grouped", g, "f16")
+    w = be.ops.empty([n, k // 8], "u32")
+    w.scales = be.ops.empty([n, k // g], "u16")
+    w.shape, w.dtype, w.format = [n, k], "f16", tb.StorageFormat("f16", packing)
+    x, y = be.ops.empty([m, k], act), be.ops.empty([m, n], "f32")
+    plan = be.planQuantizedMatmul(m, n, k, act, "f32", packing)
+    got = launches(be, lambda: be.ops.matmul(x, be.ops.transpose(w), {"outBuffer": y}))
+    assert (plan["grid"], plan["block"]) == got[0]
     for t in (x, y, w.scales, w):
         t.destroy()

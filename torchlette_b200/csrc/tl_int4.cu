@@ -193,13 +193,14 @@ __global__ void __launch_bounds__(256) qgemv_int4_kernel(Int4Args p, EpiParams e
   }
 }
 
+constexpr int kSimtWarps = 8;
+constexpr int simt_batch(int m) { return m >= 4 ? 4 : m >= 2 ? 2 : 1; }   // batch rows of a launch
+constexpr int simt_rows(int batch) { return batch >= 4 ? 2 : 4; }         // weight rows of a warp
+
 template <typename AT, int MT>
 void launch_int4(tl_ctx* ctx, const Int4Args& p, const EpiParams& e) {
-  constexpr int R = MT >= 4 ? 2 : 4;
-  const int warps = 8;
-  const int64_t rows_per_cta = int64_t(warps) * R;
-  const int grid = int((p.n + rows_per_cta - 1) / rows_per_cta);
-  qgemv_int4_kernel<AT, MT, R><<<grid, warps * 32, 0, ctx->stream>>>(p, e);
+  constexpr int R = simt_rows(MT), kRows = kSimtWarps * R;
+  qgemv_int4_kernel<AT, MT, R><<<(p.n + kRows - 1) / kRows, kSimtWarps * 32, 0, ctx->stream>>>(p, e);
 }
 
 template <typename AT>
@@ -207,7 +208,7 @@ void launch_int4_m(tl_ctx* ctx, Int4Args p, const EpiParams& epi, int m) {
   const uint8_t* a0 = static_cast<const uint8_t*>(p.a);
   // column tiles of 4, 2 and 1 batch rows (each launch re-reads the weights: FMA-bound territory anyway)
   for (int m0 = 0; m0 < m;) {
-    const int mt = m - m0 >= 4 ? 4 : m - m0 >= 2 ? 2 : 1;
+    const int mt = simt_batch(m - m0);
     p.a = a0 + size_t(m0) * p.k * sizeof(AT);
     p.row0 = m0; p.m = mt;
     if (mt == 4) launch_int4<AT, 4>(ctx, p, epi);
@@ -495,23 +496,24 @@ cudaError_t int4_ring(tl_ctx* ctx, const Int4Args& p, const EpiParams& e, int wa
   return rt == 2 ? int4_ring_fold<AT, 1, 2>(ctx, p, e, warps, s, occ) : int4_ring_fold<AT, 1, 1>(ctx, p, e, warps, s, occ);
 }
 
-template <typename AT>
-cudaError_t launch_int4_mma(tl_ctx* ctx, const Int4Args& p, const EpiParams& e) {
-  const int kblocks = p.k >> 7;
+struct RingShape { int warps, row_tiles, stages; };
+
+RingShape int4_ring_shape(const tl_ctx* ctx, int m, int64_t n, int64_t k, int group) {
+  const int kblocks = int(k >> 7);
   // A warp takes about a microsecond a block whatever the rest of the chip does, so the fewer the tiles the more warps
   // share each one's k loop: sixteen up to two tiles an SM, with rings of four stages where shared memory leaves the
   // tiles resident; else eight with two.  Two token tiles want 32-row tiles, which share the activations, once every SM
   // has a tile.  us, groups of 128: 1425 x 11008 m = 1 16 warps 7.9, 8 warps 10.5; 4096 x 14336 m = 4 17.0, 22.9; 4096 x 4096
   // m = 16 32-row tiles 7.6, 16-row 9.6; 14336 x 4096 m = 16 4 warps 22.9, 8 warps 29.5.
-  const int64_t tiles = (p.n + 15) / 16, sms = ctx->sm_count;
+  const int64_t tiles = (n + 15) / 16, sms = ctx->sm_count;
   int warps = 8, rt = 1, s = 2;
-  if (p.m > 8 && tiles > sms && (p.group == p.k || p.group % 128 == 0)) {
+  if (m > 8 && tiles > sms && (group == k || group % 128 == 0)) {
     rt = 2;
     if (tiles > 4 * sms) warps = 4;
     else s = 4;
   } else if (tiles <= 2 * sms && kblocks >= 16) {
     warps = 16;
-    if (int4_ring_smem(16, 1, 4, p.m) <= (tiles <= sms ? 220 : 110) * 1024) s = 4;
+    if (int4_ring_smem(16, 1, 4, m) <= (tiles <= sms ? 220 : 110) * 1024) s = 4;
   } else if (tiles <= 2 * sms) {
     s = 4;
   }
@@ -523,7 +525,19 @@ cudaError_t launch_int4_mma(tl_ctx* ctx, const Int4Args& p, const EpiParams& e) 
     if (f.p0 >= 1 && f.p0 <= (rt == 2 ? 8 : 16) && (f.p0 & (f.p0 - 1)) == 0) warps = f.p0;
     if (f.p2 == 2 || f.p2 == 4) s = f.p2;
   }
-  cudaError_t rc = int4_ring<AT>(ctx, p, e, warps, rt, s, nullptr);
+  return RingShape{warps, rt, s};
+}
+
+// The tensor-core form, when its layout conditions hold (and it is not switched off for A/B tests)
+bool int4_ring_applies(const tl_ctx* ctx, int32_t a_dtype, int64_t k, int group) {
+  const bool forced_simt = ctx->has_forced && ctx->forced.family == TL_FAMILY_QGEMV && ctx->forced.kernel == 1;
+  return !forced_simt && a_dtype != TL_F32 && k % 128 == 0 && (group % 128 == 0 || group == 64 || group == 32);
+}
+
+template <typename AT>
+cudaError_t launch_int4_mma(tl_ctx* ctx, const Int4Args& p, const EpiParams& e) {
+  const RingShape r = int4_ring_shape(ctx, p.m, p.n, p.k, p.group);
+  cudaError_t rc = int4_ring<AT>(ctx, p, e, r.warps, r.row_tiles, r.stages, nullptr);
   ctx->counters[TL_COUNTER_KERNEL_LAUNCHES]++;
   return rc;
 }
@@ -634,8 +648,20 @@ int32_t tl_int4_matmul(tl_ctx* ctx, const char* who, int route, const void* a, i
     memset(receipt_only, 0, sizeof(*receipt_only));
     receipt_only->choice.family = gemv ? TL_FAMILY_QGEMV : TL_FAMILY_QGEMM;
     receipt_only->choice.kernel = gemv ? 9 : 2;  // "int4" / "dequant+dense"
-    receipt_only->grid[0] = gemv ? int32_t((n + 15) / 16) : 0;
-    receipt_only->block = gemv ? 256 : 0;
+    if (gemv && m > 0 && n > 0) {
+      int64_t rows = 0;  // of a CTA
+      if (int4_ring_applies(ctx, a_dtype, k, q->group_size)) {
+        const RingShape r = int4_ring_shape(ctx, int(m), n, k, q->group_size);
+        receipt_only->choice.p0 = r.warps; receipt_only->choice.p1 = r.row_tiles; receipt_only->choice.p2 = r.stages;
+        rows = 16 * r.row_tiles;
+        receipt_only->block = 32 * r.warps;
+      } else {  // the first of its launches, if the batch rows take several
+        rows = kSimtWarps * simt_rows(simt_batch(int(m)));
+        receipt_only->block = 32 * kSimtWarps;
+      }
+      receipt_only->grid[0] = int32_t((n + rows - 1) / rows);
+      receipt_only->grid[1] = receipt_only->grid[2] = 1;
+    }
     receipt_only->split_k = 1;
     receipt_only->epilogue_engaged = has_ops ? 1 : 0;
     return TL_OK;
@@ -651,11 +677,7 @@ int32_t tl_int4_matmul(tl_ctx* ctx, const char* who, int route, const void* a, i
     p.group = q->group_size; p.groups_per_row = int32_t(k / q->group_size);
     p.scales_dtype = q->scales_dtype; p.out_dtype = out_dtype;
     p.wscale = q->scale_convention == TL_SCALE_SNORM127 ? 1.0f / 7.0f : 1.0f;
-    // the tensor-core form when its layout conditions hold (and it is not switched off for A/B tests)
-    const bool forced_simt = ctx->has_forced && ctx->forced.family == TL_FAMILY_QGEMV && ctx->forced.kernel == 1;
-    const bool mma_ok = !forced_simt && a_dtype != TL_F32 && k % 128 == 0 &&
-                        (q->group_size % 128 == 0 || q->group_size == 64 || q->group_size == 32) &&
-                        (reinterpret_cast<uintptr_t>(packed) & 15) == 0;
+    const bool mma_ok = int4_ring_applies(ctx, a_dtype, k, q->group_size) && (reinterpret_cast<uintptr_t>(packed) & 15) == 0;
     p.m = int32_t(m); p.row0 = 0;
     if (mma_ok && a_dtype == TL_F16) TL_CUDA(ctx, launch_int4_mma<__half>(ctx, p, epi));
     else if (mma_ok) TL_CUDA(ctx, launch_int4_mma<__nv_bfloat16>(ctx, p, epi));
