@@ -333,10 +333,12 @@ TL_API int32_t tl_decode_attention(tl_ctx* ctx, const void* q, const void* k_cac
  *   TL_FAMILY_QGEMM  (m > 16): 0 tcgen05 with the int8 -> 16-bit conversion on the operand path (p0 token tile,
  *                    p1 k per stage, p2 stages, p3 converter warps); 1 sliced (sixteen-row slices through the
  *                    small-batch kernels: f32 activations, odd K); 2 dequant+dense (the weight written once as a
- *                    16-bit matrix into scratch, then the dense tcgen05 kernel; receipt: p0 BN, p1 stages, p2 MH)
+ *                    16-bit matrix into scratch, then the dense tcgen05 kernel; receipt: p0 BN, p1 stages, p2 MH,
+ *                    p3 K ranges)
  *   TL_FAMILY_MATMUL (dense): 0 tiled (CUDA cores, always applicable), 1 gemv (m <= 16 NT; p0 warps),
  *                    2 tc (tcgen05, both operands from shared memory; p0 BN columns per tile, p1 stages,
- *                    p2 MH = row halves of 128 per tile; forcing with p0 = 0 leaves the tile to the library) */
+ *                    p2 MH = row halves of 128 per tile, p3 K ranges of a tile that a cluster shares: forced 0 and 1 mean
+ *                    one; forcing with p0 = 0 leaves the tile to the library) */
 enum { TL_FAMILY_QGEMV = 1, TL_FAMILY_QGEMM = 2, TL_FAMILY_MATMUL = 3 };
 typedef struct tl_variant {
   int32_t family;   /* TL_FAMILY_* */

@@ -10,6 +10,7 @@ import numpy as np
 import pytest
 
 import cases
+from launches import launches
 from oracle import oracle as orc
 from torchlette_b200 import backend as tb
 from torchlette_b200 import binding as B
@@ -326,3 +327,25 @@ def test_qgemm_dequant_dense_without_scratch_is_the_fused_default():
             t.destroy()
         be.destroy()
     np.testing.assert_array_equal(outs[0], outs[1])
+
+
+def test_qgemm_dequant_dense_receipt_is_the_launch(backend):
+    """Few tiles, so that the dense kernel cuts them along K."""
+    be = backend
+    m, n, k = 300, 512, 4096
+    packing = tb.perChannelFormat(k).packing
+    w = be.ops.empty([n, k // 4], "u32")
+    w.scales = be.ops.empty([n, 1], "f32")
+    w.shape, w.dtype, w.format = [n, k], "f16", tb.perChannelFormat(k)
+    x, y = be.ops.empty([m, k], "bf16"), be.ops.empty([m, n], "f32")
+    be.forceVariant(DEQUANT_DENSE)
+    try:
+        be.ops.matmul(x, be.ops.transpose(w), {"outBuffer": y})  # sizes the scratch outside the capture
+        plan = be.planQuantizedMatmul(m, n, k, "bf16", "f32", packing)
+        got = launches(be, lambda: be.ops.matmul(x, be.ops.transpose(w), {"outBuffer": y}))
+    finally:
+        be.forceVariant(None)
+    assert (plan["grid"], plan["block"]) == got[1]
+    assert plan["splitK"] == plan["choice"][5] > 1
+    for t in (x, y, w.scales, w):
+        t.destroy()

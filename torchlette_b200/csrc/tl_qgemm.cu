@@ -729,7 +729,7 @@ int32_t tl_launch_qgemm(tl_ctx* ctx, const tl_variant& v, const void* a, int32_t
       const TlDenseTcChoice ch = tl_dense_tc_choose(m, n, k, ctx->sm_count);
       receipt->choice.p0 = ch.bn; receipt->choice.p1 = ch.stages; receipt->choice.p2 = ch.mh; receipt->choice.p3 = ch.parts;
       receipt->grid[0] = ch.grid; receipt->grid[1] = 1; receipt->grid[2] = 1;
-      receipt->block = 576; receipt->split_k = 1;
+      receipt->block = 576; receipt->split_k = ch.parts;
       return TL_OK;
     }
     if ((reinterpret_cast<uintptr_t>(packed) & 15) || (reinterpret_cast<uintptr_t>(a) & 15))
