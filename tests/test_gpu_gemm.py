@@ -349,3 +349,18 @@ def test_qgemm_dequant_dense_receipt_is_the_launch(backend):
     assert plan["splitK"] == plan["choice"][5] > 1
     for t in (x, y, w.scales, w):
         t.destroy()
+
+
+@pytest.mark.parametrize("m", [129, 255])
+def test_qgemm_tuning_measures_both_routes(backend, m, monkeypatch, capfd):
+    be = backend
+    monkeypatch.setenv("TORCHLETTE_DEBUG_AUTOTUNE", "1")  # a line for every candidate on stderr
+    was = be.isAutotuneEnabled()
+    be.setAutotuneEnabled(True)
+    try:
+        be.pretuneMatmulShapes([(m, 512, 1024)], "f16", "f32", tb.perChannelFormat(1024).packing)
+    finally:
+        be.setAutotuneEnabled(was)
+        be.clearPerShapeMatmulChoices()
+    said = capfd.readouterr().err
+    assert "dequant+dense" in said and "tcgen05" in said

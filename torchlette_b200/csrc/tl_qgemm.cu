@@ -704,7 +704,7 @@ int32_t tl_qgemm_candidates(tl_ctx* ctx, int64_t m, int64_t n, int64_t k, int32_
   if (d.kernel == kSliced) return TL_OK;
   {
     tl_variant dd{TL_FAMILY_QGEMM, kDequantDense, 0, 0, 0, 0};
-    if (d.kernel != kDequantDense && m >= 256 && tl_qgemm_variant_applicable(dd, m, n, k, a_dtype, q)) out->push_back(dd);
+    if (d.kernel != kDequantDense && m > 128 && tl_qgemm_variant_applicable(dd, m, n, k, a_dtype, q)) out->push_back(dd);
   }
   for (const auto& c : kTcConfigs) {
     if (c.bn < 64 && m > 4 * c.bn) continue;  // narrow token tiles re-stream the weight too often
