@@ -457,16 +457,14 @@ __global__ void __launch_bounds__(RT == 2 ? 256 : 512) qgemv_int4_ring_kernel(In
 
 inline size_t int4_ring_smem(int warps, int rt, int s, int m) { return size_t(warps) * s * (rt * 1024 + m * 256); }
 
-// Runs the kernel, or (occ != null) asks how many of its CTAs one SM holds.
 template <typename AT, int NT, int RT, int FOLD, int S>
-cudaError_t int4_ring_at(tl_ctx* ctx, const Int4Args& p, const EpiParams& e, int warps, int* occ) {
+cudaError_t int4_ring_at(tl_ctx* ctx, const Int4Args& p, const EpiParams& e, int warps) {
   auto kern = qgemv_int4_ring_kernel<AT, NT, RT, FOLD, S>;
   const size_t smem = int4_ring_smem(warps, RT, S, p.m);
   if (smem > 48 * 1024) {
     cudaError_t rc = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     if (rc != cudaSuccess) return rc;
   }
-  if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, kern, warps * 32, smem);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(unsigned((p.n + 16 * RT - 1) / (16 * RT)));
   cfg.blockDim = dim3(warps * 32);
@@ -480,20 +478,20 @@ cudaError_t int4_ring_at(tl_ctx* ctx, const Int4Args& p, const EpiParams& e, int
   return cudaLaunchKernelEx(&cfg, kern, p, e);
 }
 template <typename AT, int NT, int RT, int FOLD>
-cudaError_t int4_ring_s(tl_ctx* ctx, const Int4Args& p, const EpiParams& e, int warps, int s, int* occ) {
-  return s == 4 ? int4_ring_at<AT, NT, RT, FOLD, 4>(ctx, p, e, warps, occ) : int4_ring_at<AT, NT, RT, FOLD, 2>(ctx, p, e, warps, occ);
+cudaError_t int4_ring_s(tl_ctx* ctx, const Int4Args& p, const EpiParams& e, int warps, int s) {
+  return s == 4 ? int4_ring_at<AT, NT, RT, FOLD, 4>(ctx, p, e, warps) : int4_ring_at<AT, NT, RT, FOLD, 2>(ctx, p, e, warps);
 }
 template <typename AT, int NT, int RT>
-cudaError_t int4_ring_fold(tl_ctx* ctx, const Int4Args& p, const EpiParams& e, int warps, int s, int* occ) {
-  if (p.group == p.k) return int4_ring_s<AT, NT, RT, 0>(ctx, p, e, warps, s, occ);
-  if (p.group % 128 == 0) return int4_ring_s<AT, NT, RT, 1>(ctx, p, e, warps, s, occ);
-  if (p.group == 64) return int4_ring_s<AT, NT, RT, 2>(ctx, p, e, warps, s, occ);
-  return int4_ring_s<AT, NT, RT, 4>(ctx, p, e, warps, s, occ);
+cudaError_t int4_ring_fold(tl_ctx* ctx, const Int4Args& p, const EpiParams& e, int warps, int s) {
+  if (p.group == p.k) return int4_ring_s<AT, NT, RT, 0>(ctx, p, e, warps, s);
+  if (p.group % 128 == 0) return int4_ring_s<AT, NT, RT, 1>(ctx, p, e, warps, s);
+  if (p.group == 64) return int4_ring_s<AT, NT, RT, 2>(ctx, p, e, warps, s);
+  return int4_ring_s<AT, NT, RT, 4>(ctx, p, e, warps, s);
 }
 template <typename AT>
-cudaError_t int4_ring(tl_ctx* ctx, const Int4Args& p, const EpiParams& e, int warps, int rt, int s, int* occ) {
-  if (p.m > 8) return rt == 2 ? int4_ring_fold<AT, 2, 2>(ctx, p, e, warps, s, occ) : int4_ring_fold<AT, 2, 1>(ctx, p, e, warps, s, occ);
-  return rt == 2 ? int4_ring_fold<AT, 1, 2>(ctx, p, e, warps, s, occ) : int4_ring_fold<AT, 1, 1>(ctx, p, e, warps, s, occ);
+cudaError_t int4_ring(tl_ctx* ctx, const Int4Args& p, const EpiParams& e, int warps, int rt, int s) {
+  if (p.m > 8) return rt == 2 ? int4_ring_fold<AT, 2, 2>(ctx, p, e, warps, s) : int4_ring_fold<AT, 2, 1>(ctx, p, e, warps, s);
+  return rt == 2 ? int4_ring_fold<AT, 1, 2>(ctx, p, e, warps, s) : int4_ring_fold<AT, 1, 1>(ctx, p, e, warps, s);
 }
 
 struct RingShape { int warps, row_tiles, stages; };
@@ -537,7 +535,7 @@ bool int4_ring_applies(const tl_ctx* ctx, int32_t a_dtype, int64_t k, int group)
 template <typename AT>
 cudaError_t launch_int4_mma(tl_ctx* ctx, const Int4Args& p, const EpiParams& e) {
   const RingShape r = int4_ring_shape(ctx, p.m, p.n, p.k, p.group);
-  cudaError_t rc = int4_ring<AT>(ctx, p, e, r.warps, r.row_tiles, r.stages, nullptr);
+  cudaError_t rc = int4_ring<AT>(ctx, p, e, r.warps, r.row_tiles, r.stages);
   ctx->counters[TL_COUNTER_KERNEL_LAUNCHES]++;
   return rc;
 }
