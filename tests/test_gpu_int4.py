@@ -189,3 +189,22 @@ def test_int4_receipt_is_the_launch(backend, act, m, n, k, g):
     assert (plan["grid"], plan["block"]) == got[0]
     for t in (x, y, w.scales, w):
         t.destroy()
+
+
+@pytest.mark.parametrize("m,n,k", [(11, 300, 1024), (16, 300, 1024), (16, 300, 4096)])
+@pytest.mark.parametrize("warps,row_tiles,stages", [(16, 0, 0), (16, 1, 4), (8, 2, 4), (1, 2, 2)])
+def test_int4_forced_shapes_run(backend, m, n, k, warps, row_tiles, stages):
+    """Every forced CTA width, with stages to fit: the default's result up to the order of f32 sums."""
+    be = backend
+    w, wref, _ = _weight(be, n, k, 128, seed=m)
+    xv = np.random.default_rng(k).uniform(-1, 1, (m, k)).astype(np.float16)
+    x = be.ops.tensorFromArray(xv, [m, k], "f16")
+    be.forceVariant((1, 9, warps, row_tiles, stages, 0))
+    try:
+        y = be.linear(x, w, None, None, "f32")
+    finally:
+        be.forceVariant(None)
+    size = np.abs(xv.astype(np.float64)) @ np.abs(wref.astype(np.float64)).T
+    assert (np.abs(be.ops.read(y) - xv.astype(np.float64) @ wref.astype(np.float64).T) <= size * 2.0 ** -20).all()
+    for t in (x, y, w.scales, w):
+        t.destroy()

@@ -522,6 +522,7 @@ RingShape int4_ring_shape(const tl_ctx* ctx, int m, int64_t n, int64_t k, int gr
     if (f.p1 == 1 || f.p1 == 2) rt = f.p1;
     if (f.p0 >= 1 && f.p0 <= (rt == 2 ? 8 : 16) && (f.p0 & (f.p0 - 1)) == 0) warps = f.p0;
     if (f.p2 == 2 || f.p2 == 4) s = f.p2;
+    if (int4_ring_smem(warps, rt, s, m) > 220 * 1024) s = 2;  // sixteen warps of many tokens: what a CTA may have
   }
   return RingShape{warps, rt, s};
 }
