@@ -67,9 +67,9 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
   constexpr uint32_t kIdescO = kFmtBits | (uint32_t(D >> 3) << 17) | (1u << 16);   // p v: v as it lies, MN-major
 
   extern __shared__ uint8_t attn_smem_raw[];
-  __shared__ uint64_t kv_full[SLOTS], kv_empty[SLOTS], q_full[MT], s_full[MT], p_full[MT][2], o_full[MT];
+  __shared__ uint64_t kv_full[SLOTS], kv_empty[SLOTS], q_full[MT], s_full[MT], p_full[MT][2], o_full[MT], drained;
   __shared__ uint32_t tmem_base_smem;
-  __shared__ int abort_flag;
+  __shared__ int abort_flag, issued;  // issued: key and value tiles that were asked for
   __shared__ float row_half[MT][2][2][128];  // [row block][step parity][half][row]: what a row's two threads tell each other
   uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(attn_smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* kv_sm = sm + MT * kQBytes;
@@ -99,7 +99,9 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
       mbar_init(&p_full[t][1], 8);
       mbar_init(&o_full[t], 1);
     }
+    mbar_init(&drained, 1);
     abort_flag = 0;
+    issued = 2 * most;
     mbar_fence_init();
   }
   if (warp == 1) {
@@ -121,6 +123,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
         const int s = i % SLOTS;
         if (i >= SLOTS && !mbar_wait(&kv_empty[s], ((i / SLOTS) - 1) & 1, &abort_flag)) {
           if (!abort_flag) { abort_flag = 1; atomicExch(p.status, TL_DEV_TIMEOUT_EMPTY); }
+          issued = i;
           break;
         }
         mbar_expect_tx(&kv_full[s], kSlotBytes);
@@ -341,6 +344,10 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
 
   tc_fence_before();
   __syncthreads();
+  if (abort_flag) {
+    if (warp == 0 && lane == 0) tma_drain(kv_full, SLOTS, issued);
+    if (warp == 1) tc_drain(&drained);
+  }
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, kTmemCols);

@@ -85,9 +85,9 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
   constexpr int kSlabBytes = kBK * 128;  // one 64-column slab of an MN-major B stage
 
   extern __shared__ uint8_t dense_smem_raw[];
-  __shared__ uint64_t full_bar[STAGES], empty_bar[STAGES], tfull_bar[2], tempty_bar[2];
+  __shared__ uint64_t full_bar[STAGES], empty_bar[STAGES], tfull_bar[2], tempty_bar[2], drained;
   __shared__ uint32_t tmem_base_smem;
-  __shared__ int abort_flag;
+  __shared__ int abort_flag, issued;  // issued: stages that were asked for
   uint8_t* stages = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dense_smem_raw) + 1023) & ~uintptr_t(1023));
   pdl_launch_dependents();
   const int warp = warp_index(), lane = threadIdx.x & 31;
@@ -107,6 +107,7 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
       mbar_init(&tfull_bar[b], 1);
       mbar_init(&tempty_bar[b], kEpiWarps);
     }
+    mbar_init(&drained, 1);
     abort_flag = 0;
     mbar_fence_init();
   }
@@ -226,6 +227,7 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
           }
         }
       }
+      issued = it;
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer: the whole warp, one lane elected ------------------------------
@@ -339,6 +341,10 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant_
   }
   tc_fence_before();
   __syncthreads();
+  if (abort_flag) {
+    if (warp == 0 && lane == 0) tma_drain(full_bar, STAGES, issued);
+    if (warp == 1) tc_drain(&drained);
+  }
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, kTmemCols);

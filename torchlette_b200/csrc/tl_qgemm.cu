@@ -240,10 +240,10 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
                               (uint32_t(kTileRows >> 4) << 24);
 
   extern __shared__ uint8_t gemm_smem_raw[];
-  __shared__ uint64_t full_bar[STAGES], empty_bar[STAGES], aready_bar[TS], slotfree_bar[TS], tfull_bar[2], tempty_bar[2], esync_bar[2];
+  __shared__ uint64_t full_bar[STAGES], empty_bar[STAGES], aready_bar[TS], slotfree_bar[TS], tfull_bar[2], tempty_bar[2], esync_bar[2], drained;
   __shared__ int split_last;
   __shared__ uint32_t tmem_base_smem;
-  __shared__ int abort_flag;
+  __shared__ int abort_flag, issued;  // issued: stages that were asked for
   uint8_t* stages = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(gemm_smem_raw) + 1023) & ~uintptr_t(1023));
   const int warp = warp_index(), lane = threadIdx.x & 31;
 
@@ -261,6 +261,7 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
       mbar_init(&tempty_bar[b], kEpiWarps);
       mbar_init(&esync_bar[b], kEpiWarps);
     }
+    mbar_init(&drained, 1);
     abort_flag = 0;
     mbar_fence_init();
   }
@@ -298,6 +299,7 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
           TL_TR(0, it, 1);
         }
       }
+      issued = it;
     }
   } else if (warp == kMmaWarp) {
     // ------------------------------ MMA issuer: the whole warp, one lane elected ------------------------------
@@ -559,6 +561,10 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
 
   tc_fence_before();
   __syncthreads();
+  if (abort_flag) {
+    if (warp == kProducerWarp && lane == 0) tma_drain(full_bar, STAGES, issued);
+    if (warp == kMmaWarp) tc_drain(&drained);
+  }
   if (warp == kMmaWarp) {
     tc_fence_after();
     tmem_dealloc(tmem_base, kTmemCols);

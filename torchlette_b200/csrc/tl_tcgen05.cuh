@@ -37,6 +37,11 @@ __device__ __forceinline__ void tc_commit(uint64_t* bar, uint32_t elected) {
                "r"(elected)
                : "memory");
 }
+// The same by the issuing warp: its MMAs are over before their TMEM is freed.  `bar` is used for nothing else.
+__device__ __forceinline__ void tc_drain(uint64_t* bar) {
+  tc_commit(bar, elect_one());  // the lane that issued them: the election is always the same
+  mbar_drain(bar, 0);
+}
 // D[tmem] (+)= A[tmem] * B[smem descriptor]
 __device__ __forceinline__ void tc_mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate, uint32_t elected) {
   asm volatile(

@@ -68,6 +68,16 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   return false;
 }
 
+// A wait that the abort flag does not end, still bounded.
+__device__ __forceinline__ void mbar_drain(uint64_t* bar, uint32_t parity) {
+  for (int it = 0; it < kWaitTimeoutIters && !mbar_try_wait(bar, parity); ++it) {}
+}
+// After a wait that gave up, by the producer: no copy into this CTA's shared memory is in flight when the CTA ends.  `issued`
+// copies went round `stages` barriers.
+__device__ __forceinline__ void tma_drain(uint64_t* full, int stages, int issued) {
+  for (int i = issued > stages ? issued - stages : 0; i < issued; ++i) mbar_drain(&full[i % stages], (i / stages) & 1);
+}
+
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
