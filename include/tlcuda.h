@@ -302,7 +302,8 @@ TL_API int32_t tl_transpose2d(tl_ctx* ctx, const void* in, void* out, int64_t ba
  *   [batch, n_heads, head_dim], the caches are [batch, n_kv_heads, kv_capacity, head_dim] of which the
  *   first kv_len positions are read; query head h reads kv head h / (n_heads / n_kv_heads) (the order of
  *   expandKV, model.ts:171-180); out[b,h,:] = softmax_j(q . k_j * scale + mask[j]) . v; mask is f32
- *   [kv_len] or NULL.  kv_len <= 51200 per launch.  (Appending this step's k / v at a position is
+ *   [kv_len] or NULL.  kv_len <= 51200 (what the general kernel's shared memory holds; the same
+ *   for every kernel, so that a call's shape does not decide).  (Appending this step's k / v at a position is
  *   tl_copy2d; the residual adds are tl_binary_op; silu(gate) * up rides in an epilogue.) */
 TL_API int32_t tl_rmsnorm(tl_ctx* ctx, const void* x, int32_t x_dtype, const void* weight, int32_t weight_dtype,
                           void* out, int32_t out_dtype, int64_t rows, int64_t cols, float eps);

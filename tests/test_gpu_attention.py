@@ -46,8 +46,8 @@ def reference(q, k, v, scale, causal, mask):
     return o.transpose(0, 2, 1, 3).reshape(q.shape[0], s, h * q.shape[3])
 
 
-# one rounding of an output below 2 to the storage type (half an ulp), plus 4e-6: f32 sums over up to 1e3 terms near 1 and
-# probabilities held to 2^-17 or better
+# one rounding of an output below 2 to the storage type (half an ulp), plus 4e-6: f32 sums over up to 1e3 terms near 1, of which
+# probabilities held to 23 bits (f16) or 24 are the smallest part
 TOL = {"f16": 2.0 ** -11 + 4e-6, "bf16": 2.0 ** -8 + 4e-6, "f32": 4e-6}
 
 

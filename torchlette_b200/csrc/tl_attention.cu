@@ -4,7 +4,8 @@
 // [B, kvH, capacity, D], the output is [B, S, H, D] -- the permute in front of o_proj folded into the store.
 //
 //   decode   up to 16 query rows per KV head (query positions x query heads that share it): attn_decode_mma_kernel
-//            (f16 / bf16) and attn_decode_f32_kernel.  Bound: HBM (the cache is read once).  8 sequences x 8 KV heads x
+//            (f16 / bf16) and attn_decode_f32_kernel.  Bound: HBM (the cache is read once), by the loads that twelve warps
+//            an SM have in flight (DRAM pipe 54 % busy, long scoreboard the first stall).  8 sequences x 8 KV heads x
 //            4000 keys x 128 f16 (131 MB): 27.1 us = 4.8 TB/s, about 5 us of it launch, first loads and merging (964 us
 //            one CTA per query head, which read the cache once per query head along a serial chain); 2 x 8 x 700: 6.9
 //            us (171).

@@ -64,8 +64,8 @@ __device__ __forceinline__ float2 add_x2(float2 a, float2 b) {
   return d;
 }
 
-// Two probabilities as 16-bit terms whose sum carries (nearly) all 24 bits of each: p rounded, then what is left
-// rounded, then again.  f16 needs two terms (11 bits each), bf16 three (8 bits).
+// Two probabilities as 16-bit terms whose sum carries nearly or quite all 24 bits of each: p rounded, then what is left
+// rounded, then again.  Two f16 terms (11 bits each and the sign of the second) carry 23, three bf16 ones (8 bits) all.
 template <typename AT> struct ProbSplit;
 template <> struct ProbSplit<__half> {
   static constexpr int kTerms = 2;

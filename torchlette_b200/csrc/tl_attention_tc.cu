@@ -5,7 +5,7 @@
 // A CTA owns one or two blocks of 128 query rows of one KV head; a row is a (position, head of the group) pair, so the
 // heads that share keys share the K and V tiles.  Scores and output accumulate in TMEM (256 columns a block); the
 // probabilities take the scores' place there as the A operand of the second product, two 16-bit terms in f16, three
-// in bf16, so that they keep the 24 bits they were computed with.  The maximum that a row is scaled by moves only when it is
+// in bf16: 23 and all 24 of the bits they were computed with.  The maximum that a row is scaled by moves only when it is
 // passed by 2^8 (the output is then rescaled in TMEM): a step rarely waits for that.  With two blocks one is multiplied
 // while the other's softmax runs.
 // Bound: the tensor core in principle (three units of work per score in f16: one for q k^T, two for p v), the chain

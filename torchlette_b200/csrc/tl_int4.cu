@@ -231,9 +231,10 @@ void launch_int4_m(tl_ctx* ctx, Int4Args p, const EpiParams& epi, int m) {
 // A mask and an exclusive or with a magic exponent and the sign bits make the pair (q_x + 8, q_{x+4} + 8)
 // 16-bit floats 1024 + . (f16) or 128 + . (bf16), and one subtraction -- or, for the nibbles taken at bits 4-7, one
 // fused multiply-add -- gives (q_x, q_{x+4}) exactly (Nib::quad); the activations are paired the same way.
-// Bound: instruction issue (about 200 a block and warp) ahead of HBM.  14336 x 4096, groups of 128, bias + gelu: 15.8 us
-// at m = 1, 16.0 at 4, 22.7 at 16 (20.3, 21.5, 33.5 with two blocks in registers and the activations met in the loop);
-// groups of 32: 20.3 at m = 1 (they took the CUDA cores' form).
+// Bound: instruction issue (65 % of the slots, the ALU pipe 58 %; 337 instructions a 16 x 128 block, prologue and epilogue
+// shared out) and a second wave that fills half the chip, ahead of HBM.  14336 x 4096, groups of 128, bias + gelu, replayed:
+// 15.4 us at m = 1, 15.7 at 4, 21.8 at 16 (20.3, 21.5, 33.5 with two blocks in registers and the activations met in the
+// loop); groups of 32: 18.4, 18.6, 30.1 (they took the CUDA cores' form).
 // ---------------------------------------------------------------------------
 // quad(u, v): the four MMA operand registers of one packed word u; the exclusive or that sets the exponent also turns
 // the two's complement nibble into n = q + 8:
@@ -502,7 +503,7 @@ RingShape int4_ring_shape(const tl_ctx* ctx, int m, int64_t n, int64_t k, int gr
   // share each one's k loop: sixteen up to two tiles an SM, with rings of four stages where shared memory leaves the
   // tiles resident; else eight with two.  Two token tiles want 32-row tiles, which share the activations, once every SM
   // has a tile.  us, groups of 128: 1425 x 11008 m = 1 16 warps 7.9, 8 warps 10.5; 4096 x 14336 m = 4 17.0, 22.9; 4096 x 4096
-  // m = 16 32-row tiles 7.6, 16-row 9.6; 14336 x 4096 m = 16 4 warps 22.9, 8 warps 29.5.
+  // m = 16 32-row tiles 7.6, 16-row 9.6; 14336 x 4096 m = 16 4 warps 21.8 to 22.9, 8 warps 29.5.
   const int64_t tiles = (n + 15) / 16, sms = ctx->sm_count;
   int warps = 8, rt = 1, s = 2;
   if (m > 8 && tiles > sms && (group == k || group % 128 == 0)) {

@@ -11,8 +11,8 @@
 //         per operand row), 4 MMAs of K = 16 per stage and row half;
 //   MH = 1: two accumulators of BN columns, so the epilogue of tile i overlaps the main loop of tile i+1.
 //   MH = 2: both row halves multiply the SAME B tile in shared memory.  A 256 x 256 tile moves 17 % fewer bytes per
-//         flop through it than a 128 x 256 one, and on large shapes the kernel runs at 0.92 of the fallback cuBLAS rate
-//         (2048 x 4096 x 14336: 1.46 PFLOP/s).  Sharing B between two SMs (cta_group::2) moves fewer bytes still and
+//         flop through it than a 128 x 256 one, and on large shapes the kernel runs at 0.89 of the measured cuBLAS burst rate
+//         (2048 x 4096 x 14336: 1.46 of 1.64 PFLOP/s).  Sharing B between two SMs (cta_group::2) moves fewer bytes still and
 //         measured no faster.  The two halves
 //         fill TMEM (2 x BN columns), so the epilogue (one warp per lane quarter, half and column half)
 //         does not overlap the next tile; it is a few percent when K is in the thousands.
@@ -431,9 +431,9 @@ TlDenseTcChoice tl_dense_tc_choose(int64_t m, int64_t n, int64_t k, int sms, int
     const double cost = double((t + sms - 1) / sms) * tile;
     if (cost < best.cost_us && forced_parts <= 1) best = TlDenseTcChoice{c.bn, c.mh, c.stages, 1, int(std::min<int64_t>(sms, t)), cost};
     // Cut along K (forced_parts 0: free, 1: not, else that many): one wave of clusters (of clusters of 8 about nine fit
-    // at a time), every part some steps, 3.5 us for the meeting of 128-column tiles and 6 for that of wide ones.  bf16 + gelu, us
-    // uncut / cut: 256 x 4096 x 4096 23 / 17 (2 ranges), 512 x 1024 x 4096 23 / 13 (4), 100 x 2048 x 8192 38 / 16 (4),
-    // 333 x 4096 x 12288 56 / 49 (2); 700 x 2000 x 3000, whose tiles nearly fill the chip, 26 / 24.
+    // at a time), every part some steps, 3.5 us for the meeting of 128-column tiles and 6 for that of wide ones.  bf16, bias
+    // + gelu, us, the best uncut tile / cut: 256 x 4096 x 4096 22 / 17 (2 ranges), 512 x 1024 x 4096 21 / 13 (4), 100 x 2048 x
+    // 8192 37 / 17 (4), 333 x 4096 x 12288 55 / 49 (2); 700 x 2000 x 3000, whose tiles nearly fill the chip, stays uncut.
     if (c.mh != 1 || (c.bn != 256 && c.bn != 128)) continue;
     for (int parts : {2, 4, 8}) {
       const int64_t per = (ksteps + parts - 1) / parts;

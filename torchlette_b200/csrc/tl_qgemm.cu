@@ -651,7 +651,7 @@ tl_variant fused_tile(tl_ctx* ctx, int64_t m, int64_t n, int64_t k, int32_t a_dt
   // The token tile by modelled time: waves x 128-k steps x the time of a step, a last partial wave cut along K as the
   // launch does it, 7 us for the meeting of its parts.  Step times on B200: 192 tokens 0.72 us (f16) / 0.78 (bf16) /
   // 0.95 (group scales), 128 tokens 0.53 / 0.67 / 0.9.  Measured, us, 192 / 128: 2048 x 14336 x 4096 f16 201 / 215, bf16
-  // 217 / 268; 333 x 12288 x 4096 f16 45 / 37, groups of 64 57 / 64; 600 x 14336 x 2048 f16 51 / 38.
+  // 217 / 268; 333 x 12288 x 4096 f16 47 / 38, groups of 64 58 / 65; 600 x 14336 x 2048 f16 50 / 38.
   const int64_t sms = ctx ? ctx->sm_count : 148, ksteps = (k + 127) / 128;
   const bool grouped = q.group_size != k, half = a_dtype == TL_F16;
   auto fused_us = [&](int bn, double step) {
@@ -675,8 +675,10 @@ int32_t tl_qgemm_default_variant(tl_ctx* ctx, int64_t m, int64_t n, int64_t k, i
     // With many tokens per weight byte, writing the weight out once as a 16-bit matrix and running the
     // dense kernel (whose operands both come from shared memory at its full tile sizes) beats converting
     // on the operand path: the dense kernel's modelled time, the pass at 6 TB/s (3 bytes a weight) and 4 us for the second
-    // launch.  Measured, us, fused / this way: 2048 tokens, n = 4096, k = 14336 bf16 222 / 190; n = 14336, k = 4096
-    // 217 / 223 (stays fused), with groups of 128 249 / 215; 700 x 4096 x 4096, groups of 64, 37 / 37.
+    // launch.  Measured, us a call among others, fused / this way: 2048 tokens, n = 4096, k = 14336 bf16 243 / 204; n = 14336,
+    // k = 4096 with groups of 128 279 / 209; 700 x 4096 x 4096, groups of 64, f16 40 / 41; 333 x 12288 x 4096, groups of 64, 60 /
+    // 76; 1024 x 14336 x 4096 bf16 131 / 139.  Where the model errs: 2048 x 14336 x 4096 bf16 per channel measures 223 / 205
+    // (gelu; 217 / 201 without an epilogue), the model says 215 / 208 and the margin keeps the fused kernel.
     const tl_variant dd{TL_FAMILY_QGEMM, kDequantDense, 0, 0, 0, 0};
     if (m > 128 && tl_qgemm_variant_applicable(dd, m, n, k, a_dtype, q)) {
       const double dense_us = tl_dense_tc_choose(m, n, k, ctx ? ctx->sm_count : 148).cost_us + double(n) * double(k) * 3.0 / 6.0e6 + 4.0;
