@@ -7,22 +7,25 @@
 
 namespace {
 std::mutex pools_lock;  // taken before a pool's own
-std::vector<TlBlockPool*> pools;
+std::vector<TlBlockPool*>& pools() {
+  static auto* all = new std::vector<TlBlockPool*>;  // never destroyed: a context may go after the library's statics
+  return *all;
+}
 }  // namespace
 
 TlBlockPool::TlBlockPool() {
   std::lock_guard<std::mutex> hold(pools_lock);
-  pools.push_back(this);
+  pools().push_back(this);
 }
 
 TlBlockPool::~TlBlockPool() {
   std::lock_guard<std::mutex> hold(pools_lock);
-  pools.erase(std::find(pools.begin(), pools.end(), this));
+  pools().erase(std::find(pools().begin(), pools().end(), this));
 }
 
 void TlBlockPool::release_device() {
   std::lock_guard<std::mutex> hold(pools_lock);
-  for (TlBlockPool* p : pools)
+  for (TlBlockPool* p : pools())
     if (p->device == device) p->release();
 }
 
