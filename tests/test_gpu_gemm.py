@@ -300,7 +300,7 @@ def test_qgemm_group_scales_every_form(backend, variant, group):
 def test_qgemm_dequant_dense_without_scratch_is_the_fused_default():
     """A capture that may not grow the scratch: the fused kernel with the tile that the rule picks for these tokens (which here
     needs no scratch of its own), to the bit."""
-    m, n, k = 300, 4096, 4096
+    m, n, k = 333, 12288, 512
     cs = cases.per_channel_case(n, k, m, seed=9, act_dtype="f16")
     fmt = tb.perChannelFormat(k)
     outs = []
@@ -364,3 +364,40 @@ def test_qgemm_tuning_measures_both_routes(backend, m, monkeypatch, capfd):
         be.clearPerShapeMatmulChoices()
     said = capfd.readouterr().err
     assert "dequant+dense" in said and "tcgen05" in said
+
+
+@pytest.mark.parametrize("m,n,k,group,act", [(170, 576, 512, 0, "f16"), (366, 1296, 512, 64, "f16"), (300, 4096, 4096, 0, "f16"), (170, 2944, 896, 0, "f16"),
+                                             (150, 700, 2048, 0, "bf16"), (500, 1000, 1536, 128, "f16"), (1000, 512, 1024, 0, "f16")])
+def test_qgemm_default_sums_as_exactly_as_the_fused_tiles(backend, m, n, k, group, act):
+    """The tensor core's f32 sums lose bits with their length: the default's distance from 64 bits is that of the better of the two
+    fused tiles, whose K is cut where they leave SMs idle (2 % for the order of the partial sums)."""
+    be = backend
+    group = group or k
+    rng = np.random.default_rng(m)
+    xv = rng.standard_normal((m, k)).astype(np.float32)
+    if act == "f16":
+        x, xv = be.ops.tensorFromArray(xv.astype(np.float16), [m, k], "f16"), xv.astype(np.float16).astype(np.float64)
+    else:
+        bits = orc.bf16_bits_rne(xv.reshape(-1))
+        x, xv = be.ops.tensorFromArray(bits, [m, k], "bf16"), orc.bf16_bits_to_f32(bits).reshape(m, k).astype(np.float64)
+    if group == k:
+        q = rng.integers(-127, 128, (n, k), dtype=np.int8)
+        scales = rng.uniform(0.001, 0.01, (n, 1)).astype(np.float32)
+        w, wv = be.createQuantizedWeight(cases.pack_int8(q), scales, n, k, tb.perChannelFormat(k)), q * scales.astype(np.float64)
+    else:
+        packed, scales = be.quantizeLinearWeight((rng.standard_normal((n, k)) * 0.05).astype(np.float32), group)
+        w = be.createQuantizedWeight(packed, scales, n, k, tb.StorageFormat("f16", tb.QuantPacking("int8-grouped", group, "f16")))
+        wv = orc.dequantize_to_f32(packed, scales, k, group).astype(np.float16).astype(np.float64)  # the operand
+    ref = xv @ wv.T
+    err = []
+    for variant in (None, (2, 0, 192, 128, 3, 8), (2, 0, 128, 128, 4, 8)):
+        be.forceVariant(variant)
+        try:
+            y = be.linear(x, w)
+        finally:
+            be.forceVariant(None)
+        err.append(np.linalg.norm(be.ops.read(y) - ref))
+        y.destroy()
+    assert err[0] <= 1.02 * min(err[1:]), err
+    for t in (x, w.scales, w):
+        t.destroy()

@@ -641,10 +641,11 @@ bool tl_qgemm_variant_applicable(const tl_variant& v, int64_t m, int64_t n, int6
 }
 
 namespace {
-// The fused kernel's tile, by the token count, and (*us) its modelled time above 64 tokens.  Only for what the fused kernel
-// takes: 16-bit activations, k and groups of whole 16s.
-tl_variant fused_tile(tl_ctx* ctx, int64_t m, int64_t n, int64_t k, int32_t a_dtype, const tl_quant_desc& q, double* us) {
+// The fused kernel's tile, by the token count, and above 64 tokens its modelled time and the longest sum in one accumulator
+// (*chain, in k).  Only for what the fused kernel takes: 16-bit activations, k and groups of whole 16s.
+tl_variant fused_tile(tl_ctx* ctx, int64_t m, int64_t n, int64_t k, int32_t a_dtype, const tl_quant_desc& q, double* us, int64_t* chain) {
   *us = 0;
+  *chain = k;
   if (m <= 16) return tl_variant{TL_FAMILY_QGEMM, kTc, 16, 128, 8, 8};
   if (m <= 32) return tl_variant{TL_FAMILY_QGEMM, kTc, 32, 128, 8, 8};
   if (m <= 64) return tl_variant{TL_FAMILY_QGEMM, kTc, 64, 128, 6, 8};
@@ -654,14 +655,21 @@ tl_variant fused_tile(tl_ctx* ctx, int64_t m, int64_t n, int64_t k, int32_t a_dt
   // 217 / 268; 333 x 12288 x 4096 f16 47 / 38, groups of 64 58 / 65; 600 x 14336 x 2048 f16 50 / 38.
   const int64_t sms = ctx ? ctx->sm_count : 148, ksteps = (k + 127) / 128;
   const bool grouped = q.group_size != k, half = a_dtype == TL_F16;
-  auto fused_us = [&](int bn, double step) {
+  // Before the time comes the sum: the tensor core's f32 accumulator loses bits with every product it takes (170 x 576 x 512 f16,
+  // f32 output, against 64 bits: 1.0e-7 with K cut in four, 4.3e-7 uncut), so where one wave's tiles are all cut, the
+  // tile that is cut more is taken.  With several waves most sums go over all of K in any case.
+  auto fused_us = [&](int bn, double step, int64_t* longest) {
     const int64_t tiles = ((n + kTileRows - 1) / kTileRows) * ((m + bn - 1) / bn), rem = tiles % sms;
     const int64_t splits = rem ? std::min<int64_t>({sms / rem, 4, ksteps}) : 1;
+    *longest = tiles < sms ? std::min(k, (ksteps + splits - 1) / splits * 128) : k;
     return (double(tiles / sms) + (rem ? 1.0 / double(splits) : 0.0)) * double(ksteps) * step + (splits > 1 ? 7.0 : 0.0);
   };
-  const double t192 = fused_us(192, grouped ? 0.95 : half ? 0.72 : 0.78), t128 = fused_us(128, grouped ? 0.9 : half ? 0.53 : 0.67);
-  *us = std::min(t192, t128);
-  return t192 <= t128 ? tl_variant{TL_FAMILY_QGEMM, kTc, 192, 128, 3, 8} : tl_variant{TL_FAMILY_QGEMM, kTc, 128, 128, 4, 8};
+  int64_t c192, c128;
+  const double t192 = fused_us(192, grouped ? 0.95 : half ? 0.72 : 0.78, &c192), t128 = fused_us(128, grouped ? 0.9 : half ? 0.53 : 0.67, &c128);
+  const bool wide = c192 != c128 ? c192 < c128 : t192 <= t128;
+  *us = wide ? t192 : t128;
+  *chain = wide ? c192 : c128;
+  return wide ? tl_variant{TL_FAMILY_QGEMM, kTc, 192, 128, 3, 8} : tl_variant{TL_FAMILY_QGEMM, kTc, 128, 128, 4, 8};
 }
 }  // namespace
 
@@ -671,7 +679,8 @@ int32_t tl_qgemm_default_variant(tl_ctx* ctx, int64_t m, int64_t n, int64_t k, i
   v.family = TL_FAMILY_QGEMM;
   if ((a_dtype == TL_F16 || a_dtype == TL_BF16) && k % 16 == 0 && q.group_size % 16 == 0) {
     double fused_us = 0;
-    v = fused_tile(ctx, m, n, k, a_dtype, q, &fused_us);
+    int64_t chain = 0;
+    v = fused_tile(ctx, m, n, k, a_dtype, q, &fused_us, &chain);
     // With many tokens per weight byte, writing the weight out once as a 16-bit matrix and running the
     // dense kernel (whose operands both come from shared memory at its full tile sizes) beats converting
     // on the operand path: the dense kernel's modelled time, the pass at 6 TB/s (3 bytes a weight) and 4 us for the second
@@ -681,8 +690,10 @@ int32_t tl_qgemm_default_variant(tl_ctx* ctx, int64_t m, int64_t n, int64_t k, i
     // (gelu; 217 / 201 without an epilogue), the model says 215 / 208 and the margin keeps the fused kernel.
     const tl_variant dd{TL_FAMILY_QGEMM, kDequantDense, 0, 0, 0, 0};
     if (m > 128 && tl_qgemm_variant_applicable(dd, m, n, k, a_dtype, q)) {
-      const double dense_us = tl_dense_tc_choose(m, n, k, ctx ? ctx->sm_count : 148).cost_us + double(n) * double(k) * 3.0 / 6.0e6 + 4.0;
-      if (dense_us < 0.95 * fused_us) v = dd;
+      const TlDenseTcChoice dense = tl_dense_tc_choose(m, n, k, ctx ? ctx->sm_count : 148);
+      const double dense_us = dense.cost_us + double(n) * double(k) * 3.0 / 6.0e6 + 4.0;
+      const int64_t steps64 = (k + 63) / 64, dense_chain = std::min(k, (steps64 + dense.parts - 1) / dense.parts * 64);
+      if (dense_us < 0.95 * fused_us && dense_chain <= chain) v = dd;  // not for longer sums either
     }
   } else {
     v.kernel = kSliced;  // f32 activations or odd K: sixteen-row slices through the small-batch kernels
@@ -699,7 +710,8 @@ int32_t tl_qgemm_secure_scratch(tl_ctx* ctx, tl_variant* v, int64_t m, int64_t n
   const int32_t rc = tl_ensure_scratch(ctx, size_t(n) * size_t(k) * 2, &wbuf);
   if (rc != TL_ERR_OOM && !(rc == TL_ERR_UNSUPPORTED && ctx->capturing)) return rc;
   double us;
-  *v = fused_tile(ctx, m, n, k, a_dtype, q, &us);
+  int64_t chain;
+  *v = fused_tile(ctx, m, n, k, a_dtype, q, &us, &chain);
   return TL_OK;
 }
 
