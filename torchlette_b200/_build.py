@@ -2,18 +2,21 @@
 
 ``python -m torchlette_b200._build`` compiles every translation unit under
 ``csrc/`` to an object file (in parallel) and links the shared library next to
-the sources, where the ctypes binding looks for it.
+the sources, where the ctypes binding looks for it; ``tl_pycall.cpp`` becomes the
+extension module ``_tlcall.so`` beside it.
 """
 from __future__ import annotations
 
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(CSRC, "libtlcuda.so")
+PYCALL = os.path.join(CSRC, "_tlcall.so")
 SOURCES = ["tl_api.cu", "tl_pool.cu", "tl_quantize.cu", "tl_qgemv.cu", "tl_qgemv_stream.cu", "tl_qgemm.cu", "tl_matmul.cu", "tl_matmul_tc.cu", "tl_elementwise.cu", "tl_decode_ops.cu", "tl_attention.cu", "tl_attention_tc.cu", "tl_int4.cu", "tl_autotune.cu", "tl_comm.cu"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = [
@@ -50,13 +53,16 @@ def build(force: bool = False, verbose: bool = False) -> str:
         if r.returncode != 0 or verbose:
             sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
         if r.returncode != 0:
-            raise RuntimeError(f"nvcc failed for {cmd[-3]}")
+            raise RuntimeError(f"{os.path.basename(cmd[0])} failed for {cmd[-3] if cmd[0] == NVCC else cmd[-1]}")
 
     if jobs:
         with ThreadPoolExecutor(max_workers=min(8, len(jobs))) as ex:
             list(ex.map(run, jobs))
     if jobs or _stale(LIB, objs):
         run([NVCC, "-shared", "-o", LIB, *objs, "-cudart", "static", "-ldl"])
+    pysrc = os.path.join(CSRC, "tl_pycall.cpp")
+    if force or _stale(PYCALL, [pysrc, headers[-1]]):
+        run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", "-I", sysconfig.get_paths()["include"], "-o", PYCALL, pysrc])
     return LIB
 
 

@@ -145,7 +145,7 @@ class CudaTensor:
 
     def destroy(self):
         if self.ownsBuffer and self.buffer:
-            self.backend._free(self.buffer)
+            self.backend._calls.tl_free(self.backend._handle, self.buffer)
         self.buffer = None
 
     def toArray(self):
@@ -183,9 +183,8 @@ class CudaOps:
         return CudaTensor(self._b, shape, dtype, buf, host.nbytes)
 
     def empty(self, shape, dtype="f32") -> CudaTensor:
-        n = int(math.prod(shape)) if len(shape) else 1
-        nbytes = n * _ITEMSIZE[dtype]
-        return CudaTensor(self._b, shape, dtype, self._b._alloc(nbytes), nbytes)
+        nbytes = int(math.prod(shape)) * _ITEMSIZE[dtype]
+        return CudaTensor(self._b, shape, dtype, self._b._calls.tl_alloc(self._b._handle, nbytes), nbytes)
 
     def read(self, t: CudaTensor) -> np.ndarray:
         if t.transposed:
@@ -198,9 +197,9 @@ class CudaOps:
 
     def reshape(self, t: CudaTensor, shape) -> CudaTensor:
         """A view of a contiguous tensor under another shape (no copy; the buffer stays the owner's)."""
-        if t.transposed or int(math.prod(shape)) != int(math.prod(t.shape)):
+        if t.transposed or math.prod(shape) != math.prod(t.shape):
             raise ValueError("reshape: needs a contiguous tensor and the same element count")
-        return CudaTensor(self._b, list(shape), t.dtype, t.buffer, t.nbytes, ownsBuffer=False, format=t.format, scales=t.scales)
+        return CudaTensor(self._b, shape, t.dtype, t.buffer, t.nbytes, ownsBuffer=False, format=t.format, scales=t.scales)
 
     def transpose(self, t: CudaTensor, dim0: int = -2, dim1: int = -1) -> CudaTensor:
         nd = len(t.shape)
@@ -215,8 +214,8 @@ class CudaOps:
         src = self.contiguous(t) if t.transposed else t
         out = self.empty(src.shape, out_dtype or src.dtype)
         n = int(math.prod(src.shape)) if src.shape else 1
-        B.check(self._b._ctx, self._b._lib.tl_unary_op(self._b._ctx, op, src.buffer, B.DTYPE_ID[src.dtype], out.buffer,
-                                                       B.DTYPE_ID[out.dtype], n))
+        self._b._calls.tl_unary_op(self._b._handle, op, src.buffer, B.DTYPE_ID[src.dtype], out.buffer,
+                                                       B.DTYPE_ID[out.dtype], n)
         if src is not t:
             src.destroy()
         return out
@@ -240,9 +239,9 @@ class CudaOps:
         if not is_row and list(b.shape) != list(a.shape):
             raise TlError(B.TL_ERR_UNSUPPORTED, f"{name}: b must match a or be its last dim")
         out = self.empty(a.shape, a.dtype)
-        B.check(self._b._ctx, self._b._lib.tl_binary_op(self._b._ctx, B.TL_BINARY[name], a.buffer, B.DTYPE_ID[a.dtype], b.buffer,
+        self._b._calls.tl_binary_op(self._b._handle, B.TL_BINARY[name], a.buffer, B.DTYPE_ID[a.dtype], b.buffer,
                                                         B.DTYPE_ID[b.dtype], out.buffer, B.DTYPE_ID[out.dtype], rows, cols,
-                                                        1 if is_row else 0))
+                                                        1 if is_row else 0)
         return out
 
     def add(self, a, b): return self._binary("add", a, b)
@@ -269,8 +268,8 @@ class CudaOps:
             raise TlError(B.TL_ERR_INVALID_ARG, "rmsnorm: weight must be [lastDim]")
         rows = int(math.prod(x.shape[:-1])) if len(x.shape) > 1 else 1
         out = self.empty(x.shape, outputDtype or x.dtype)
-        B.check(self._b._ctx, self._b._lib.tl_rmsnorm(self._b._ctx, x.buffer, B.DTYPE_ID[x.dtype], weight.buffer, B.DTYPE_ID[weight.dtype],
-                                                      out.buffer, B.DTYPE_ID[out.dtype], rows, cols, float(eps)))
+        self._b._calls.tl_rmsnorm(self._b._handle, x.buffer, B.DTYPE_ID[x.dtype], weight.buffer, B.DTYPE_ID[weight.dtype],
+                                                      out.buffer, B.DTYPE_ID[out.dtype], rows, cols, float(eps))
         return out
 
     def fusedRoPE(self, qk: CudaTensor, cos: CudaTensor, sin: CudaTensor, config: Optional[dict] = None) -> CudaTensor:
@@ -282,8 +281,8 @@ class CudaOps:
         if cos.dtype != "f32" or sin.dtype != "f32":
             raise TlError(B.TL_ERR_UNSUPPORTED, "fusedRoPE: cos / sin tables are f32")
         out = self.empty(qk.shape, qk.dtype)
-        B.check(self._b._ctx, self._b._lib.tl_rope(self._b._ctx, qk.buffer, B.DTYPE_ID[qk.dtype], cos.buffer, sin.buffer, out.buffer, outer, seq, hd,
-                                                   float(config.get("sinScale", 1.0)), int(config.get("cosOffset", 0)), int(config.get("sinOffset", 0))))
+        self._b._calls.tl_rope(self._b._handle, qk.buffer, B.DTYPE_ID[qk.dtype], cos.buffer, sin.buffer, out.buffer, outer, seq, hd,
+                                                   float(config.get("sinScale", 1.0)), int(config.get("cosOffset", 0)), int(config.get("sinOffset", 0)))
         return out
 
     def decodeAttention(self, q: CudaTensor, kCache: CudaTensor, vCache: CudaTensor, kvLen: int, scale: float,
@@ -293,8 +292,8 @@ class CudaOps:
         b, h, d = q.shape[0], q.shape[1], q.shape[-1]
         kvh, cap = kCache.shape[1], kCache.shape[2]
         out = self.empty([b, 1, h * d], q.dtype)
-        B.check(self._b._ctx, self._b._lib.tl_decode_attention(self._b._ctx, q.buffer, kCache.buffer, vCache.buffer, out.buffer, B.DTYPE_ID[q.dtype], b, h,
-                                                               kvh, d, kvLen, cap, float(scale), mask.buffer if mask is not None else None))
+        self._b._calls.tl_decode_attention(self._b._handle, q.buffer, kCache.buffer, vCache.buffer, out.buffer, B.DTYPE_ID[q.dtype], b, h,
+                                                               kvh, d, kvLen, cap, float(scale), mask.buffer if mask is not None else None)
         return out
 
     def attention(self, q: CudaTensor, kCache: CudaTensor, vCache: CudaTensor, kvLen: int, scale: float, causal: bool = True,
@@ -304,16 +303,16 @@ class CudaOps:
         keys up to kvLen - S + s (prefill: kvLen == S)."""
         b, h, sq, d = q.shape
         out = self.empty([b, sq, h * d], q.dtype)
-        B.check(self._b._ctx, self._b._lib.tl_attention(self._b._ctx, q.buffer, kCache.buffer, vCache.buffer, out.buffer, B.DTYPE_ID[q.dtype], b, h,
+        self._b._calls.tl_attention(self._b._handle, q.buffer, kCache.buffer, vCache.buffer, out.buffer, B.DTYPE_ID[q.dtype], b, h,
                                                         kCache.shape[1], sq, d, kvLen, kCache.shape[2], float(scale),
-                                                        mask.buffer if mask is not None else None, 1 if causal else 0))
+                                                        mask.buffer if mask is not None else None, 1 if causal else 0)
         return out
 
     def kvAppend(self, cache: CudaTensor, new: CudaTensor, position: int):
         """cache[:, :, position, :] = new ([B, kvH, 1, D] or [B, kvH, D]): one strided copy (model.ts:240-262)."""
         b, kvh, cap, d = cache.shape
         esz = _ITEMSIZE[cache.dtype]
-        B.check(self._b._ctx, self._b._lib.tl_copy2d(self._b._ctx, cache.buffer + position * d * esz, cap * d * esz, new.buffer, d * esz, d * esz, b * kvh))
+        self._b._calls.tl_copy2d(self._b._handle, cache.buffer + position * d * esz, cap * d * esz, new.buffer, d * esz, d * esz, b * kvh)
 
     def matmul(self, a: CudaTensor, b: CudaTensor, options: Optional[dict] = None) -> CudaTensor:
         """Backend matmul; the storage-format seam (matmul-ops.ts:42-59)."""
@@ -332,6 +331,8 @@ class CudaBackend:
         ctx = C.c_void_p()
         B.check(None, self._lib.tl_ctx_create(device, C.byref(ctx)))
         self._ctx = ctx
+        self._handle = ctx.value  # the same for the native calls
+        self._calls = B.calls()
         self.device = device
         self.ops = CudaOps(self)
 
@@ -339,7 +340,7 @@ class CudaBackend:
     def destroy(self):
         if self._ctx:
             self._lib.tl_ctx_destroy(self._ctx)
-            self._ctx = None
+            self._ctx = self._handle = None
 
     def sync(self):
         B.check(self._ctx, self._lib.tl_sync(self._ctx))
@@ -359,12 +360,10 @@ class CudaBackend:
 
     # -- raw memory ---------------------------------------------------------
     def _alloc(self, nbytes: int) -> int:
-        p = C.c_void_p()
-        B.check(self._ctx, self._lib.tl_alloc(self._ctx, nbytes, C.byref(p)))
-        return p.value
+        return self._calls.tl_alloc(self._handle, nbytes)
 
     def _free(self, ptr: int):
-        B.check(self._ctx, self._lib.tl_free(self._ctx, C.c_void_p(ptr)))
+        self._calls.tl_free(self._handle, ptr)
 
     def _upload(self, ptr: int, host: np.ndarray):
         B.check(self._ctx, self._lib.tl_upload(self._ctx, C.c_void_p(ptr), host.ctypes.data_as(C.c_void_p),
@@ -414,7 +413,7 @@ class CudaBackend:
             raise TlError(B.TL_ERR_INVALID_ARG, f"quantize: K={k} must be divisible by groupSize={g}")
         wt = self.ops.empty([n, k // 4], "u32")
         st = self.ops.empty([n, k // g], "u16")
-        B.check(self._ctx, self._lib.tl_quantize_linear_weight_device(self._ctx, weight.buffer, n, k, g, wt.buffer, st.buffer))
+        self._calls.tl_quantize_linear_weight_device(self._handle, weight.buffer, n, k, g, wt.buffer, st.buffer)
         wt.shape = [n, k]
         wt.dtype = format.elementType
         wt.format = format
@@ -455,47 +454,54 @@ class CudaBackend:
         return wt
 
     # -- descriptors ----------------------------------------------------------
-    @staticmethod
-    def _qdesc(packing: QuantPacking) -> B.QuantDesc:
+    def _quant(self, packing: QuantPacking) -> bytes:
+        """The packing as the bytes of a tl_quant_desc."""
         if packing.scheme not in _VALUES_PER_WORD:
             raise TlError(B.TL_ERR_UNSUPPORTED, f"matmulQuantizedB: unsupported scheme {packing.scheme}")
-        return B.QuantDesc(B.TL_SCHEME_INT8_GROUPED if packing.scheme == "int8-grouped" else B.TL_SCHEME_INT4_GROUPED, packing.groupSize, B.DTYPE_ID[packing.scalesDtype],
-                           B.TL_SCALE_SNORM127 if packing.scaleConvention == "snorm127" else B.TL_SCALE_DIRECT)
+        return self._calls.quant(B.TL_SCHEME_INT8_GROUPED if packing.scheme == "int8-grouped" else B.TL_SCHEME_INT4_GROUPED, packing.groupSize,
+                                 B.DTYPE_ID[packing.scalesDtype], B.TL_SCALE_SNORM127 if packing.scaleConvention == "snorm127" else B.TL_SCALE_DIRECT)
 
-    @staticmethod
-    def _epilogue(epilogue: Optional[EpilogueConfig], epilogueInputs: Sequence[CudaTensor]):
+    def _qdesc(self, packing: QuantPacking) -> B.QuantDesc:
+        return B.QuantDesc.from_buffer_copy(self._quant(packing))
+
+    def _epilogueBytes(self, epilogue: Optional[EpilogueConfig], epilogueInputs: Sequence[CudaTensor]) -> Optional[bytes]:
+        """The op chain as the bytes of a tl_epilogue."""
         if epilogue is None:
             return None
-        e = B.Epilogue()
         if len(epilogue.ops) > B.TL_EPI_MAX_OPS:
             raise TlError(B.TL_ERR_INVALID_ARG, "epilogue: too many ops")
         if len(epilogueInputs) > B.TL_EPI_MAX_INPUTS:
             raise TlError(B.TL_ERR_INVALID_ARG, "epilogue: at most 4 extra inputs")
-        e.n_ops = len(epilogue.ops)
-        for i, op in enumerate(epilogue.ops):
+        ops = []
+        for op in epilogue.ops:
             kind = op["kind"]
             if kind == "none":
-                e.ops[i] = B.EpilogueOp(B.TL_EPI_NONE, 0, 0, 0)
+                ops.append((B.TL_EPI_NONE, 0, 0, 0))
             elif kind == "bias":
-                e.ops[i] = B.EpilogueOp(B.TL_EPI_BIAS, 0, op["inputIndex"], 0)
+                ops.append((B.TL_EPI_BIAS, 0, op["inputIndex"], 0))
             elif kind == "unary":
                 if op["op"] not in B.TL_UNARY:
                     raise TlError(B.TL_ERR_UNSUPPORTED, f"epilogue: unsupported unary op {op['op']}")
-                e.ops[i] = B.EpilogueOp(B.TL_EPI_UNARY, B.TL_UNARY[op["op"]], 0, 0)
+                ops.append((B.TL_EPI_UNARY, B.TL_UNARY[op["op"]], 0, 0))
             elif kind == "binary":
                 if op["op"] not in B.TL_BINARY:
                     raise TlError(B.TL_ERR_UNSUPPORTED, f"epilogue: unsupported binary op {op['op']}")
-                e.ops[i] = B.EpilogueOp(B.TL_EPI_BINARY, B.TL_BINARY[op["op"]], op["inputIndex"], 0)
+                ops.append((B.TL_EPI_BINARY, B.TL_BINARY[op["op"]], op["inputIndex"], 0))
             elif kind == "cast":
-                e.ops[i] = B.EpilogueOp(B.TL_EPI_CAST, 0, 0, B.DTYPE_ID[op["toDtype"]])
+                ops.append((B.TL_EPI_CAST, 0, 0, B.DTYPE_ID[op["toDtype"]]))
             else:
                 raise TlError(B.TL_ERR_INVALID_ARG, f"epilogue: unknown op kind {kind}")
-        e.n_inputs = len(epilogueInputs)
-        for i, t in enumerate(epilogueInputs):
+        inputs = []
+        for t in epilogueInputs:
             if t.dtype != "f32":
                 raise TlError(B.TL_ERR_UNSUPPORTED, "epilogue inputs must be f32")
-            e.inputs[i] = t.buffer
-        return e
+            at = t.buffer
+            inputs.append(at if at is None or isinstance(at, int) else C.cast(at, C.c_void_p).value)
+        return self._calls.epilogue(tuple(ops), tuple(inputs))
+
+    def _epilogue(self, epilogue: Optional[EpilogueConfig], epilogueInputs: Sequence[CudaTensor]):
+        e = self._epilogueBytes(epilogue, epilogueInputs)
+        return None if e is None else B.Epilogue.from_buffer_copy(e)
 
     # -- the hot path ---------------------------------------------------------
     def dispatchQuantizedGemvNT(self, aBuffer: CudaTensor, packedWeight: CudaTensor, scales: CudaTensor,
@@ -607,11 +613,10 @@ class CudaBackend:
         out_dtype = epilogue.outputDtype if epilogue is not None else options.get("outputDtype", "f32")
         out_shape = (a.shape[:-1] if len(a.shape) > 1 else [1]) + [n]
         out = options.get("outBuffer") or self.ops.empty(out_shape, out_dtype)
-        q = self._qdesc(packing)
-        e = self._epilogue(epilogue, epilogueInputs)
-        B.check(self._ctx, self._lib.tl_qmatmul_nt(
-            self._ctx, a.buffer, B.DTYPE_ID[a.dtype], b.buffer, scales.buffer, out.buffer, B.DTYPE_ID[out_dtype],
-            m, n, k, C.byref(q), float(options.get("alpha", 1.0)), C.byref(e) if e is not None else None))
+        q = self._quant(packing)
+        e = self._epilogueBytes(epilogue, epilogueInputs)
+        self._calls.tl_qmatmul_nt(self._handle, a.buffer, B.DTYPE_ID[a.dtype], b.buffer, scales.buffer, out.buffer, B.DTYPE_ID[out_dtype],
+                                  m, n, k, q, float(options.get("alpha", 1.0)), e)
         return out
 
     def dispatchMatmul(self, a: CudaTensor, b: CudaTensor, options: dict) -> CudaTensor:
@@ -647,15 +652,14 @@ class CudaBackend:
         if batch > 1 and not batch_b and not a.transposed:
             m, batch = m * batch, 1
         out = options.get("outBuffer") or self.ops.empty(list(batch_dims) + [a_shape[-2], n], out_dtype)
-        e = self._epilogue(epilogue, epilogueInputs)
+        e = self._epilogueBytes(epilogue, epilogueInputs)
         cast = {None: -1, "f16": B.TL_F16, "bf16": B.TL_BF16}
-        B.check(self._ctx, self._lib.tl_matmul(
-            self._ctx, a.buffer, b.buffer, out.buffer, m, n, k, batch,
+        self._calls.tl_matmul(
+            self._handle, a.buffer, b.buffer, out.buffer, m, n, k, batch,
             m * k if (batch_a and batch > 1) else 0, k * n if (batch_b and batch > 1) else 0, m * n,
             1 if a.transposed else 0, 1 if b.transposed else 0, float(options.get("alpha", 1.0)),
             B.DTYPE_ID[a.dtype], B.DTYPE_ID[b.dtype], B.DTYPE_ID[out_dtype],
-            cast[options.get("inputCastA")], cast[options.get("inputCastB")],
-            C.byref(e) if e is not None else None, None))
+            cast[options.get("inputCastA")], cast[options.get("inputCastB")], e, None)
         return out
 
     def planMatmul(self, m, n, k, aDtype, bDtype, *, batch=1, transA=False, transB=False,
@@ -704,9 +708,11 @@ class CudaBackend:
         result, cast] -- the multiply rides in the second product's store loop.  Both weights may be
         packed (either scheme) or dense."""
         u = self.linear(x, up, None, None, "f32")
-        chain = [("silu", None), ("mul", u)] + ([("cast", outputDtype)] if outputDtype != "f32" else [])
-        plan = detectMatmulEpilogue(chain)
-        h = self.ops.matmul(x, self.ops.transpose(gate), {"epilogue": plan[0], "epilogueInputs": plan[1], "outputDtype": outputDtype})
+        # what the fusion pass decides for the chain silu, mul by u, cast: all of it fuses
+        ops = [{"kind": "unary", "op": "silu"}, {"kind": "binary", "op": "mul", "inputIndex": 0}]
+        if outputDtype != "f32":
+            ops.append({"kind": "cast", "toDtype": outputDtype})
+        h = self.ops.matmul(x, self.ops.transpose(gate), {"epilogue": EpilogueConfig(ops, 1, outputDtype), "epilogueInputs": [u]})
         u.destroy()
         return h
 

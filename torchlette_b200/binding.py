@@ -7,10 +7,13 @@ when a context is created, the call raises.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.machinery
+import importlib.util
 import os
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.environ.get("TLCUDA_LIB") or os.path.join(_HERE, "csrc", "libtlcuda.so")
+PYCALL_PATH = os.path.join(_HERE, "csrc", "_tlcall.so")
 
 TL_OK = 0
 TL_ERR_INVALID_ARG, TL_ERR_UNSUPPORTED, TL_ERR_CUDA, TL_ERR_NCCL = -1, -2, -3, -4
@@ -193,6 +196,42 @@ def load():
         fn.argtypes = args
     _lib = lib
     return lib
+
+
+class _Calls:
+    """The calls of the hot paths, one attribute per function of ``csrc/tl_pycall.cpp``: native argument conversion, an
+    exception instead of a status, ``tl_alloc(ctx, nbytes)`` with the address as its result.  ``quant`` and ``epilogue`` make the
+    descriptors those calls take (bytes)."""
+
+
+_calls = None
+
+
+def calls() -> _Calls:
+    global _calls
+    if _calls is not None:
+        return _calls
+    lib = load()
+    if not os.path.exists(PYCALL_PATH):
+        raise ImportError(f"{PYCALL_PATH} is missing: build it with `python -m torchlette_b200._build`")
+    loader = importlib.machinery.ExtensionFileLoader("_tlcall", PYCALL_PATH)
+    native = importlib.util.module_from_spec(importlib.util.spec_from_loader("_tlcall", loader))
+    loader.exec_module(native)
+
+    def through_ctypes(fn, kinds):
+        """The same call where an argument is not a plain number or address: ctypes' own rules, descriptors as structures again."""
+        def call(*args):
+            return fn(*(C.byref(kind._type_.from_buffer_copy(a)) if isinstance(a, bytes) and hasattr(kind, "_type_") and kind is not C.c_void_p else a
+                        for a, kind in zip(args, kinds)), *args[len(kinds):])
+        return call
+
+    c = _Calls()
+    for name in native.names:
+        fn = getattr(lib, name)
+        setattr(c, name, native.bind(name, C.cast(fn, C.c_void_p).value, through_ctypes(fn, SIGNATURES[name][1]), check))
+    c.quant, c.epilogue = native.quant, native.epilogue
+    _calls = c
+    return c
 
 
 def check(ctx, status: int):
