@@ -287,8 +287,13 @@ __global__ void __launch_bounds__(256) quantize_kernel(const float* __restrict__
 //   x = w * inv in f32 is off by at most 3e-7 |x| < 8e-5 (a quotient good to 2 units in the last place and one rounding; |x| <
 //   256: the scale's f16 bits are at least half of the group's maximum, or zero); the rounding to a whole number can
 //   differ from the f64 one only if x lies that close to a half, and those values, and what is NaN, are done again in f64.
-//   Rounding adds 1.5 * 2^23, whose low byte is then the two's complement; a clamp to +-127 before it gives what the
-//   clamp after it gave.
+//   Rounding is a multiply-add of 1.5 * 2^23, whose low byte is then the two's complement, and a second one gives what was rounded
+//   off.  The clamp to +-127 can only act where the scale is a subnormal f16: a group that passes 127.4 goes to f64 too.
+__device__ __forceinline__ float max_nan(float a, float b) {  // NaN if either is
+  float y;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(y) : "f"(a), "f"(b));
+  return y;
+}
 template <int LANES>
 __global__ void __launch_bounds__(256) quantize_group_kernel(const float4* __restrict__ weight, int64_t n_words, uint32_t* __restrict__ packed,
                                                              uint16_t* __restrict__ scales) {
@@ -317,15 +322,14 @@ __global__ void __launch_bounds__(256) quantize_group_kernel(const float4* __res
       const float sc = __half2float(__ushort_as_half(uint16_t(sbits)));
       const float inv = sc > 0.f ? __fdividef(127.f, sc) : 0.f;
       uint32_t q[4];
-      bool again = false;
+      float off = 0.f;
 #pragma unroll
       for (int b = 0; b < 4; ++b) {
-        const float raw = f[b] * inv, x = fminf(fmaxf(raw, -127.f), 127.f);
-        const float r = x + 12582912.f;
+        const float r = fmaf(f[b], inv, 12582912.f);
         q[b] = __float_as_uint(r);
-        again = again || !(fabsf(x - (r - 12582912.f)) <= 0.4999f) || raw != raw;
+        off = max_nan(off, fabsf(fmaf(f[b], inv, 12582912.f - r)));
       }
-      if (again) {
+      if (!(off <= 0.4999f && amax * inv < 127.4f)) {
         const double inv64 = sc > 0.f ? 127.0 / double(sc) : 0.0;
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
