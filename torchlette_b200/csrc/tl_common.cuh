@@ -362,4 +362,23 @@ __device__ __forceinline__ void tl_store_out(void* out, int out_dtype, int64_t i
   else if (out_dtype == TL_F16) reinterpret_cast<__half*>(out)[idx] = __float2half_rn(v);
   else reinterpret_cast<__nv_bfloat16*>(out)[idx] = __float2bfloat16_rn(v);
 }
+
+// The small ops of a step (norms, rotations, residual adds) are launched so that their CTAs may be set up while a kernel in front
+// that allows it drains; each waits for all of it before it reads or writes anything (every thread, or the kernel behind
+// could start before that one has ended), and allows no early start itself: the kernels behind prefetch what they take
+// for constant (weights, scales, biases), and that may be what an op has just made.
+__device__ __forceinline__ void tl_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <typename... P, typename... A>
+cudaError_t tl_launch_waiting(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t stream, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
 #endif  // __CUDACC__

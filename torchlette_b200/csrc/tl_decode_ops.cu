@@ -54,15 +54,17 @@ template <int CH>
 __global__ void __launch_bounds__(1024) rmsnorm_vec_kernel(const void* x, int x_dtype, const void* w, int w_dtype, void* out, int out_dtype,
                                                            int64_t rows, int cols, float eps) {
   __shared__ float part[32];
+  tl_pdl_wait();
   const int64_t row = int64_t(blockIdx.x) * blockDim.y + threadIdx.y;
   const bool here = row < rows;
   const int64_t base = row * cols;
-  float v[CH][8], ss = 0.f;
+  float v[CH][8], g0[8], ss = 0.f;
 #pragma unroll
   for (int c = 0; c < CH; ++c) {
     const int i = (c * int(blockDim.x) + int(threadIdx.x)) * 8;
     if (here && i < cols) {
       load8_any(x, x_dtype, base + i, v[c]);
+      if (CH == 1) load8_any(w, w_dtype, i, g0);  // on its way during the reduction
 #pragma unroll
       for (int e = 0; e < 8; ++e) ss = fmaf(v[c][e], v[c][e], ss);
     }
@@ -80,9 +82,9 @@ __global__ void __launch_bounds__(1024) rmsnorm_vec_kernel(const void* x, int x_
     const int i = (c * int(blockDim.x) + int(threadIdx.x)) * 8;
     if (here && i < cols) {
       float g[8];
-      load8_any(w, w_dtype, i, g);
+      if (CH > 1) load8_any(w, w_dtype, i, g);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) g[e] = v[c][e] * inv * g[e];
+      for (int e = 0; e < 8; ++e) g[e] = v[c][e] * inv * (CH == 1 ? g0[e] : g[e]);
       if (out_dtype == TL_F32) store8(reinterpret_cast<float*>(out) + base + i, g);
       else if (out_dtype == TL_F16) store8(reinterpret_cast<__half*>(out) + base + i, g);
       else store8(reinterpret_cast<__nv_bfloat16*>(out) + base + i, g);
@@ -93,6 +95,7 @@ __global__ void __launch_bounds__(1024) rmsnorm_vec_kernel(const void* x, int x_
 __global__ void __launch_bounds__(128) rmsnorm_kernel(const void* x, int x_dtype, const void* w, int w_dtype, void* out, int out_dtype,
                                                       int64_t rows, int cols, float eps) {
   __shared__ float part[4];
+  tl_pdl_wait();
   const int64_t row = blockIdx.x;
   if (row >= rows) return;
   const int64_t base = row * cols;
@@ -116,6 +119,7 @@ __global__ void __launch_bounds__(128) rmsnorm_kernel(const void* x, int x_dtype
 __global__ void __launch_bounds__(256) rope_kernel(const void* qk, int dtype, const float* cos_t, const float* sin_t, void* out,
                                                    int64_t total, int seq_len, int head_dim, float sin_scale, int64_t cos_offset,
                                                    int64_t sin_offset) {
+  tl_pdl_wait();
   const int64_t stride = int64_t(gridDim.x) * blockDim.x;
   const int half = head_dim >> 1;
   for (int64_t idx = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; idx < total; idx += stride) {
@@ -153,12 +157,12 @@ int32_t tl_rmsnorm(tl_ctx* ctx, const void* x, int32_t x_dtype, const void* weig
     const int per_cta = threads == 32 && rows >= 8 * int64_t(ctx->sm_count) ? 8 : 1;
     const dim3 block(threads, per_cta);
     const unsigned grid = unsigned((rows + per_cta - 1) / per_cta);
-    if (vecs <= 1024) rmsnorm_vec_kernel<1><<<grid, block, 0, ctx->stream>>>(x, x_dtype, weight, weight_dtype, out, out_dtype, rows, int(cols), eps);
-    else rmsnorm_vec_kernel<4><<<grid, block, 0, ctx->stream>>>(x, x_dtype, weight, weight_dtype, out, out_dtype, rows, int(cols), eps);
+    TL_CUDA(ctx, tl_launch_waiting(vecs <= 1024 ? rmsnorm_vec_kernel<1> : rmsnorm_vec_kernel<4>, dim3(grid), block, ctx->stream, x, x_dtype, weight,
+                                   weight_dtype, out, out_dtype, rows, cols, eps));
   } else {
-    rmsnorm_kernel<<<unsigned(rows), 128, 0, ctx->stream>>>(x, x_dtype, weight, weight_dtype, out, out_dtype, rows, int(cols), eps);
+    TL_CUDA(ctx, tl_launch_waiting(rmsnorm_kernel, dim3(unsigned(rows)), dim3(128), ctx->stream, x, x_dtype, weight, weight_dtype, out, out_dtype, rows,
+                                   cols, eps));
   }
-  TL_CUDA(ctx, cudaGetLastError());
   ctx->counters[TL_COUNTER_KERNEL_LAUNCHES]++;
   return TL_OK;
 }
@@ -176,9 +180,8 @@ int32_t tl_rope(tl_ctx* ctx, const void* qk, int32_t dtype, const float* cos_tab
     return tl_set_error(ctx, TL_ERR_INVALID_ARG, "tl_rope: null or aliased pointers (an element reads its partner: not in place)");
   DeviceGuard guard(ctx->device);
   const int grid = int(std::min<int64_t>((total + 255) / 256, int64_t(ctx->sm_count) * 8));
-  rope_kernel<<<grid, 256, 0, ctx->stream>>>(qk, dtype, cos_table, sin_table, out, total, int(seq_len), int(head_dim), sin_scale, cos_offset,
-                                             sin_offset);
-  TL_CUDA(ctx, cudaGetLastError());
+  TL_CUDA(ctx, tl_launch_waiting(rope_kernel, dim3(unsigned(grid)), dim3(256), ctx->stream, qk, dtype, cos_table, sin_table, out, total, seq_len,
+                                 head_dim, sin_scale, cos_offset, sin_offset));
   ctx->counters[TL_COUNTER_KERNEL_LAUNCHES]++;
   return TL_OK;
 }

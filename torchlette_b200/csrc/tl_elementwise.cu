@@ -17,6 +17,7 @@ __device__ __forceinline__ float ld_as_f32(const void* p, int dtype, int64_t i) 
 
 // out[i] = op(in[i]) with a cast on either side; op 0 is the plain cast / copy
 __global__ void __launch_bounds__(256) unary_kernel(const void* in, int in_dtype, void* out, int out_dtype, int op, int64_t count, int vec) {
+  tl_pdl_wait();
   const int64_t stride = int64_t(gridDim.x) * blockDim.x;
   const int64_t tid = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (vec) {  // f32 -> f32, both pointers 16-byte aligned
@@ -38,6 +39,7 @@ __global__ void __launch_bounds__(256) unary_kernel(const void* in, int in_dtype
 // out[r, c] = a[r, c] (op) b[b_rows == 1 ? 0 : r, c]
 __global__ void __launch_bounds__(256) binary_kernel(const void* a, int a_dtype, const void* b, int b_dtype, void* out, int out_dtype,
                                                      int op, int64_t rows, int64_t cols, int b_broadcast) {
+  tl_pdl_wait();
   const int64_t count = rows * cols, stride = int64_t(gridDim.x) * blockDim.x;
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += stride) {
     const float x = ld_as_f32(a, a_dtype, i);
@@ -77,8 +79,8 @@ int32_t tl_unary_op(tl_ctx* ctx, int32_t op, const void* in, int32_t in_dtype, v
   if (count == 0) return TL_OK;
   DeviceGuard guard(ctx->device);
   const bool vec = in_dtype == TL_F32 && out_dtype == TL_F32 && !((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15);
-  unary_kernel<<<grid_for(ctx, vec ? count / 4 + 1 : count), 256, 0, ctx->stream>>>(in, in_dtype, out, out_dtype, op, count, vec ? 1 : 0);
-  TL_CUDA(ctx, cudaGetLastError());
+  TL_CUDA(ctx, tl_launch_waiting(unary_kernel, dim3(unsigned(grid_for(ctx, vec ? count / 4 + 1 : count))), dim3(256), ctx->stream, in, in_dtype, out,
+                                 out_dtype, op, count, vec ? 1 : 0));
   ctx->counters[TL_COUNTER_KERNEL_LAUNCHES]++;
   return TL_OK;
 }
@@ -91,8 +93,8 @@ int32_t tl_binary_op(tl_ctx* ctx, int32_t op, const void* a, int32_t a_dtype, co
   if (op != TL_BINARY_ADD && op != TL_BINARY_SUB && op != TL_BINARY_MUL) return tl_set_error(ctx, TL_ERR_UNSUPPORTED, "tl_binary_op: unknown op %d", op);
   if (rows * cols == 0) return TL_OK;
   DeviceGuard guard(ctx->device);
-  binary_kernel<<<grid_for(ctx, rows * cols), 256, 0, ctx->stream>>>(a, a_dtype, b, b_dtype, out, out_dtype, op, rows, cols, b_is_row ? 1 : 0);
-  TL_CUDA(ctx, cudaGetLastError());
+  TL_CUDA(ctx, tl_launch_waiting(binary_kernel, dim3(unsigned(grid_for(ctx, rows * cols))), dim3(256), ctx->stream, a, a_dtype, b, b_dtype, out, out_dtype,
+                                 op, rows, cols, b_is_row ? 1 : 0));
   ctx->counters[TL_COUNTER_KERNEL_LAUNCHES]++;
   return TL_OK;
 }
