@@ -229,7 +229,11 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
   static_assert(TS >= 2, "TMEM operand ring");
   constexpr uint32_t kTmemCols = pow2_at_least(2 * BN + TS * kSlotCols);
   static_assert(kTmemCols <= 512, "TMEM budget");
-  constexpr int kParts = NCW / 4;                   // converter threads per weight row
+  // Sixteen converter warps are two groups on alternate k steps: a step's chain of wait, load, convert, store and signal is
+  // longer than its MMAs, whatever its arithmetic.
+  constexpr int kGroups = NCW == 16 ? 2 : 1;
+  constexpr int kGroupWarps = NCW / kGroups;
+  constexpr int kParts = kGroupWarps / 4;           // converter threads per weight row
   constexpr int kChunks = KSTEP / 16 / kParts;      // 16-byte chunks per converter thread and stage
   constexpr int kEpiWarp0 = NCW, kEpiWarps = 8, kProducerWarp = NCW + 8, kMmaWarp = NCW + 9;
   // Both operands carry the activation type: kind::f16 with an f16 weight operand against
@@ -253,7 +257,7 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
       mbar_init(&empty_bar[s], 1);
     }
     for (int s = 0; s < TS; ++s) {
-      mbar_init(&aready_bar[s], NCW);
+      mbar_init(&aready_bar[s], kGroupWarps);
       mbar_init(&slotfree_bar[s], 1);
     }
     for (int b = 0; b < 2; ++b) {
@@ -344,7 +348,7 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
     }
   } else if (warp < NCW) {
     // ------------------------------ converters ------------------------------
-    const int quad = warp & 3, part = warp >> 2;
+    const int quad = warp & 3, part = (warp >> 2) % kParts, group = warp / kGroupWarps;
     const int r = quad * 32 + lane;  // weight row inside the tile = TMEM lane
     const uint32_t swz = KSTEP == 128 ? uint32_t(r & 7) : uint32_t((r >> 1) & 3);
     const uint32_t row_off = uint32_t(r) * KSTEP;
@@ -375,7 +379,7 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
 #pragma unroll
       for (int i = 0; i < kChunks; ++i) raw[i] = lds128(wb + ((uint32_t(part * kChunks + i) ^ swz) << 4));
       const float sc_one = sc_next;
-      if (GROUPED && one_scale) sc_next = scale_at(n_tile, (ks + 1) * KSTEP + part * kChunks * 16);
+      if (GROUPED && one_scale) sc_next = scale_at(n_tile, (ks + kGroups) * KSTEP + part * kChunks * 16);
 #pragma unroll
       for (int i = 0; i < kChunks; ++i) {
         const int c = part * kChunks + i;
@@ -408,8 +412,9 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
     WorkItem w;
     for (int wi = 0; ok && get_work(p, wi, w); ++wi) {
       const int n_tile = w.tile / p.m_tiles;
-      if (GROUPED && one_scale) sc_next = scale_at(n_tile, w.ks0 * KSTEP + part * kChunks * 16);
+      if (GROUPED && one_scale) sc_next = scale_at(n_tile, (w.ks0 + (kGroups - 1) * ((it ^ group) & 1)) * KSTEP + part * kChunks * 16);
       for (int ks = w.ks0; ks < w.ks0 + w.nks; ++ks, ++it) {
+        if (kGroups == 2 && ((it ^ group) & 1)) continue;  // the other group's
         const int sl = it % TS;
         if (!convert(it, ks, n_tile)) { ok = false; break; }
         if (warp == 0 && lane == 0) TL_TR(2, it, 2);
@@ -580,7 +585,8 @@ struct TcConfig { int bn, kstep, stages, ncw; };
 // the instantiated tile configurations (tl_variant p0..p3)
 const TcConfig kTcConfigs[] = {{192, 64, 6, 4}, {192, 64, 6, 8}, {128, 64, 8, 4}, {128, 64, 8, 8},
                                {64, 128, 6, 8}, {32, 128, 8, 8}, {16, 128, 8, 8},
-                               {128, 128, 4, 8}, {192, 128, 3, 8}, {128, 128, 4, 16}, {192, 128, 3, 16}};
+                               {128, 128, 4, 8}, {192, 128, 3, 8}, {128, 128, 4, 16}, {192, 128, 3, 16},
+                               {64, 128, 6, 16}, {32, 128, 8, 16}};
 
 bool tc_config_known(const tl_variant& v) {
   for (const auto& c : kTcConfigs)
@@ -622,6 +628,8 @@ cudaError_t launch_tc_cfg(const tl_variant& v, bool grouped, int grid, cudaStrea
   TL_TC_CASE(192, 128, 3, 8)
   TL_TC_CASE(128, 128, 4, 16)
   TL_TC_CASE(192, 128, 3, 16)
+  TL_TC_CASE(64, 128, 6, 16)
+  TL_TC_CASE(32, 128, 8, 16)
 #undef TL_TC_CASE
   return cudaErrorInvalidValue;
 }
@@ -646,15 +654,20 @@ namespace {
 tl_variant fused_tile(tl_ctx* ctx, int64_t m, int64_t n, int64_t k, int32_t a_dtype, const tl_quant_desc& q, double* us, int64_t* chain) {
   *us = 0;
   *chain = k;
+  // Sixteen converter warps where the weights have group scales, whose conversion is the longer chain (us, 8 / 16 warps: 30 x 12288 x
+  // 4096 groups of 64 31.5 / 27.6, 64 tokens 32.7 / 28.6, 250 51.0 / 47.4, 400 x 4096 x 4096 34.2 / 31.0; per channel 64 x 12288 x
+  // 4096 17.6 / 19.2, 30 x 4096 x 4096 11.6 / 12.5).  Tiles of 192 tokens gain only over several waves (1500 x 12288 x 4096 168 / 161, 900 x 4096 x
+  // 4096 54.2 / 56.0).
+  const bool grouped = q.group_size != k, half = a_dtype == TL_F16;
+  const int32_t ncw = grouped ? 16 : 8;
   if (m <= 16) return tl_variant{TL_FAMILY_QGEMM, kTc, 16, 128, 8, 8};
-  if (m <= 32) return tl_variant{TL_FAMILY_QGEMM, kTc, 32, 128, 8, 8};
-  if (m <= 64) return tl_variant{TL_FAMILY_QGEMM, kTc, 64, 128, 6, 8};
+  if (m <= 32) return tl_variant{TL_FAMILY_QGEMM, kTc, 32, 128, 8, ncw};
+  if (m <= 64) return tl_variant{TL_FAMILY_QGEMM, kTc, 64, 128, 6, ncw};
   // The token tile by modelled time: waves x 128-k steps x the time of a step, a last partial wave cut along K as the
   // launch does it, 7 us for the meeting of its parts.  Step times on B200: 192 tokens 0.72 us (f16) / 0.78 (bf16) /
-  // 0.95 (group scales), 128 tokens 0.53 / 0.67 / 0.9.  Measured, us, 192 / 128: 2048 x 14336 x 4096 f16 201 / 215, bf16
-  // 217 / 268; 333 x 12288 x 4096 f16 47 / 38, groups of 64 58 / 65; 600 x 14336 x 2048 f16 50 / 38.
+  // 0.95 (group scales; 0.92 over several waves), 128 tokens 0.53 / 0.67 / 0.76.  Measured, us, 192 / 128: 2048 x 14336 x 4096 f16 201 / 215, bf16
+  // 217 / 268; 333 x 12288 x 4096 f16 47 / 38, groups of 64 56 / 54 over rotating copies, 60 / 62 on one; 600 x 14336 x 2048 f16 50 / 38.
   const int64_t sms = ctx ? ctx->sm_count : 148, ksteps = (k + 127) / 128;
-  const bool grouped = q.group_size != k, half = a_dtype == TL_F16;
   // Before the time comes the sum: the tensor core's f32 accumulator loses bits with every product it takes (170 x 576 x 512 f16,
   // f32 output, against 64 bits: 1.0e-7 with K cut in four, 4.3e-7 uncut), so where one wave's tiles are all cut, the
   // tile that is cut more is taken.  With several waves most sums go over all of K in any case.
@@ -665,11 +678,12 @@ tl_variant fused_tile(tl_ctx* ctx, int64_t m, int64_t n, int64_t k, int32_t a_dt
     return (double(tiles / sms) + (rem ? 1.0 / double(splits) : 0.0)) * double(ksteps) * step + (splits > 1 ? 7.0 : 0.0);
   };
   int64_t c192, c128;
-  const double t192 = fused_us(192, grouped ? 0.95 : half ? 0.72 : 0.78, &c192), t128 = fused_us(128, grouped ? 0.9 : half ? 0.53 : 0.67, &c128);
+  const bool waves = ((n + kTileRows - 1) / kTileRows) * ((m + 191) / 192) >= 3 * sms;
+  const double t192 = fused_us(192, grouped ? (waves ? 0.92 : 0.95) : half ? 0.72 : 0.78, &c192), t128 = fused_us(128, grouped ? 0.76 : half ? 0.53 : 0.67, &c128);
   const bool wide = c192 != c128 ? c192 < c128 : t192 <= t128;
   *us = wide ? t192 : t128;
   *chain = wide ? c192 : c128;
-  return wide ? tl_variant{TL_FAMILY_QGEMM, kTc, 192, 128, 3, 8} : tl_variant{TL_FAMILY_QGEMM, kTc, 128, 128, 4, 8};
+  return wide ? tl_variant{TL_FAMILY_QGEMM, kTc, 192, 128, 3, grouped && waves ? 16 : 8} : tl_variant{TL_FAMILY_QGEMM, kTc, 128, 128, 4, ncw};
 }
 }  // namespace
 
