@@ -71,6 +71,14 @@ __device__ __forceinline__ uint4 ldg_stream(const void* p) {
   return v;
 }
 
+__device__ __forceinline__ void cp_async16(uint32_t smem_addr, const void* gptr) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr), "l"(gptr) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -144,48 +152,26 @@ __device__ __forceinline__ void bytes_to_f32(uint32_t word, float (&f)[4]) {
   f[3] = __uint_as_float(__byte_perm(x, 0x4B000000u, 0x7653)) - 8388736.f;
 }
 
-template <typename AT> struct ActChunk;  // 16 activations of one batch row as f32
-template <> struct ActChunk<float> {
-  __device__ static void load(const float* p, float (&x)[16]) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float4 v = __ldg(reinterpret_cast<const float4*>(p) + i);
-      x[4 * i] = v.x; x[4 * i + 1] = v.y; x[4 * i + 2] = v.z; x[4 * i + 3] = v.w;
-    }
-  }
-};
-template <> struct ActChunk<__half> {
-  __device__ static void load(const __half* p, float (&x)[16]) {
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const uint4 v = __ldg(reinterpret_cast<const uint4*>(p) + i);
-      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[j]));
-        x[8 * i + 2 * j] = f.x; x[8 * i + 2 * j + 1] = f.y;
-      }
-    }
-  }
-};
-template <> struct ActChunk<__nv_bfloat16> {
-  __device__ static void load(const __nv_bfloat16* p, float (&x)[16]) {
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const uint4 v = __ldg(reinterpret_cast<const uint4*>(p) + i);
-      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        x[8 * i + 2 * j] = __uint_as_float(w[j] << 16);
-        x[8 * i + 2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u);
-      }
-    }
-  }
-};
+// Four activations as f32.
+__device__ __forceinline__ float4 act4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
+__device__ __forceinline__ float4 act4(const __half* p) {
+  const uint2 v = __ldg(reinterpret_cast<const uint2*>(p));
+  const float2 lo = __half22float2(*reinterpret_cast<const __half2*>(&v.x)), hi = __half22float2(*reinterpret_cast<const __half2*>(&v.y));
+  return make_float4(lo.x, lo.y, hi.x, hi.y);
+}
+__device__ __forceinline__ float4 act4(const __nv_bfloat16* p) {
+  const uint2 v = __ldg(reinterpret_cast<const uint2*>(p));
+  return make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16), __uint_as_float(v.y & 0xffff0000u));
+}
 
-// MT batch rows, R output rows per warp.  Lane l handles 16-byte chunks l, l+32, ...
-template <typename AT, int MT, int R, bool GROUPED>
-__global__ void __launch_bounds__(256) qgemv_simt_kernel(GemvArgs p, EpiParams epi) {
+// Both forms: R output rows per warp, lane l handles the 16-byte chunks l, l + 32, ... of each.  Bound: memory, with the conversion (2
+// operations a weight) and the FMA behind it.
+//
+// One batch row, four weight rows a warp, on tall matrices: the activations straight from L1, shared by four rows.  12288 x 4096, groups of
+// 64: 15.7 us (17.2 staged: what a CTA stages, 768 CTAs stage).
+template <typename AT, bool GROUPED>
+__global__ void __launch_bounds__(256) qgemv_simt_tall_kernel(GemvArgs p, EpiParams epi) {
+  constexpr int R = 4;
   const int warps = blockDim.x >> 5, lane = threadIdx.x & 31;
   const int64_t row_base = (int64_t(blockIdx.x) * warps + (threadIdx.x >> 5)) * R;
   if (row_base >= p.n) return;
@@ -195,42 +181,28 @@ __global__ void __launch_bounds__(256) qgemv_simt_kernel(GemvArgs p, EpiParams e
   int64_t rows[R];
 #pragma unroll
   for (int r = 0; r < R; ++r) rows[r] = min(row_base + r, int64_t(p.n) - 1);  // tail rows clamp, stores mask
-  float acc[R][MT];
-#pragma unroll
-  for (int r = 0; r < R; ++r)
-#pragma unroll
-    for (int i = 0; i < MT; ++i) acc[r][i] = 0.f;
-
+  float acc[R] = {};
   for (int c = lane; c < chunks; c += 32) {
     uint4 wv[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) wv[r] = ldg_stream(wbytes + rows[r] * p.k + int64_t(c) * 16);
-    float x[MT][16];
+    float4 x[4];
 #pragma unroll
-    for (int i = 0; i < MT; ++i) ActChunk<AT>::load(a + int64_t(i) * p.k + int64_t(c) * 16, x[i]);
+    for (int j = 0; j < 4; ++j) x[j] = act4(a + int64_t(c) * 16 + 4 * j);
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       const uint32_t w4[4] = {wv[r].x, wv[r].y, wv[r].z, wv[r].w};
-      float part[MT];
-#pragma unroll
-      for (int i = 0; i < MT; ++i) part[i] = GROUPED ? 0.f : acc[r][i];
+      float part = GROUPED ? 0.f : acc[r];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         float f[4];
         bytes_to_f32(w4[j], f);
-#pragma unroll
-        for (int b = 0; b < 4; ++b)
-#pragma unroll
-          for (int i = 0; i < MT; ++i) part[i] = fmaf(f[b], x[i][4 * j + b], part[i]);
+        part = fmaf(f[0], x[j].x, part);
+        part = fmaf(f[1], x[j].y, part);
+        part = fmaf(f[2], x[j].z, part);
+        part = fmaf(f[3], x[j].w, part);
       }
-      if (GROUPED) {
-        const float s = tl_load_scale(p.scales, p.scales_dtype, rows[r] * p.groups_per_row + (c * 16) / p.group);
-#pragma unroll
-        for (int i = 0; i < MT; ++i) acc[r][i] = fmaf(s, part[i], acc[r][i]);
-      } else {
-#pragma unroll
-        for (int i = 0; i < MT; ++i) acc[r][i] = part[i];
-      }
+      acc[r] = GROUPED ? fmaf(tl_load_scale(p.scales, p.scales_dtype, rows[r] * p.groups_per_row + (c * 16) / p.group), part, acc[r]) : part;
     }
   }
 #pragma unroll
@@ -238,6 +210,126 @@ __global__ void __launch_bounds__(256) qgemv_simt_kernel(GemvArgs p, EpiParams e
     const int64_t row = row_base + r;
     float s = p.wscale;
     if (!GROUPED) s *= tl_load_scale(p.scales, p.scales_dtype, rows[r]);
+    const float v = warp_sum(acc[r]) * s;
+    if (lane == 0 && row < p.n) tl_store_out(p.out, p.out_dtype, int64_t(p.row0) * p.n + row, tl_apply_epilogue(epi, v, p.row0, row, p.n));
+  }
+}
+
+// MT batch rows.  D steps of 512 weights of each row (and their scales) are in registers ahead of their use: for one token and K = 4096
+// half of all that the launch reads is asked for at once, before the kernel in front of this one has ended.  The activations go
+// through shared memory as f32, in two buffers of `slice` steps each, the next slice on its way while the CTA's warps work on this one: a
+// lane's sixteen are 64 contiguous bytes, which straight from global memory are four 16-byte loads that touch four times the
+// lines they need (a 4096-row launch spent 8000 of its clocks on L1 wavefronts for them); here the quarters of a chunk are
+// swapped by the chunk ((c >> 1) & 3), so that no read has a bank conflict.
+// 4096 x 4096 with groups of 64, replayed: 7.1 us at m = 1 (9.9 with the activations met in the loop), 12.2 at 4 (16.9), 46 at 16 (65); 513 x 14336 16.8 (24.2).
+// Steps of a slice, a multiple of D: all of K in one if that takes 32 KB, else two buffers of 16 to 32 KB (of 32 for one row, three CTAs fit an
+// SM and 4096 x 12288 took 29 us, the last of its 512 CTAs alone).
+constexpr int simt_slice(int mt, int steps) { return mt >= 3 ? 4 : mt == 2 ? (steps <= 8 ? 8 : 4) : steps <= 16 ? 16 : 8; }
+
+template <typename AT> __device__ __forceinline__ void stage4(float* dst, const AT* src) { *reinterpret_cast<float4*>(dst) = act4(src); }
+__device__ __forceinline__ void stage4(float* dst, const float* src) { cp_async16(uint32_t(__cvta_generic_to_shared(dst)), src); }
+
+template <typename AT, int MT, int R, int D, bool GROUPED>
+__global__ void __launch_bounds__(256, D == 8 ? 4 : 1) qgemv_simt_kernel(GemvArgs p, EpiParams epi, int slice) {
+  extern __shared__ __align__(16) uint8_t simt_smem[];  // [2][MT][slice * 32 chunks][16] f32
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int warps = blockDim.x >> 5, lane = threadIdx.x & 31;
+  const int64_t row_base = (int64_t(blockIdx.x) * warps + (threadIdx.x >> 5)) * R;
+  const AT* a = reinterpret_cast<const AT*>(p.a);
+  const int chunks = p.k >> 4, steps = (chunks + 31) >> 5;
+  const uint8_t* wrow[R];
+  int64_t srow[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int64_t row = min(row_base + r, int64_t(p.n) - 1);  // tail rows clamp, stores mask
+    wrow[r] = reinterpret_cast<const uint8_t*>(p.packed) + row * p.k;
+    srow[r] = row * p.groups_per_row;
+  }
+  const int gshift = (p.group & (p.group - 1)) == 0 ? 31 - __clz(p.group) : -1;
+  uint4 wv[D][R];
+  float sv[D][R];
+  auto fetch = [&](int d, int step) {
+    const int c = step * 32 + lane;
+    if (c >= chunks) return;
+#pragma unroll
+    for (int r = 0; r < R; ++r) wv[d][r] = ldg_stream(wrow[r] + int64_t(c) * 16);
+    if (GROUPED) {
+      const int g = gshift >= 0 ? (c * 16) >> gshift : (c * 16) / p.group;
+#pragma unroll
+      for (int r = 0; r < R; ++r) sv[d][r] = tl_load_scale(p.scales, p.scales_dtype, srow[r] + g);
+    }
+  };
+  // weights and scales do not depend on the kernel before this one
+#pragma unroll
+  for (int d = 0; d < D; ++d) fetch(d, d);
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  float* xs = reinterpret_cast<float*>(simt_smem);
+  const int row_floats = slice * 512, swz = (lane >> 1) & 3;
+  auto stage = [&](int s0, float* to) {
+    const int quads = min(row_floats, p.k - s0 * 512) >> 2;
+#pragma unroll
+    for (int i = 0; i < MT; ++i)
+      for (int q = threadIdx.x; q < quads; q += blockDim.x)
+        stage4(to + i * row_floats + (q >> 2) * 16 + (((q & 3) ^ ((q >> 3) & 3)) << 2), a + int64_t(i) * p.k + s0 * 512 + 4 * q);
+    cp_async_commit();
+  };
+  stage(0, xs);
+  float acc[R][MT];
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+#pragma unroll
+    for (int i = 0; i < MT; ++i) acc[r][i] = 0.f;
+
+  int buf = 0;
+  for (int s0 = 0; s0 < steps; s0 += slice, buf ^= 1) {
+    cp_async_wait<0>();
+    __syncthreads();  // the slice is there for all, and all are done with the one before
+    if (s0 + slice < steps) stage(s0 + slice, xs + (buf ^ 1) * MT * row_floats);
+    const float* xb = xs + buf * MT * row_floats;
+    const int s1 = min(steps, s0 + slice);
+    for (int st = s0; st < s1; st += D) {
+#pragma unroll
+      for (int d = 0; d < D; ++d) {
+        const int c = (st + d) * 32 + lane;
+        if (c < chunks) {
+          const float* x = xb + (c - s0 * 32) * 16;
+          float part[R][MT];
+#pragma unroll
+          for (int r = 0; r < R; ++r)
+#pragma unroll
+            for (int i = 0; i < MT; ++i) part[r][i] = GROUPED ? 0.f : acc[r][i];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            float4 xv[MT];
+#pragma unroll
+            for (int i = 0; i < MT; ++i) xv[i] = *reinterpret_cast<const float4*>(x + i * row_floats + ((j ^ swz) << 2));
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+              float f[4];
+              bytes_to_f32(j == 0 ? wv[d][r].x : j == 1 ? wv[d][r].y : j == 2 ? wv[d][r].z : wv[d][r].w, f);
+#pragma unroll
+              for (int i = 0; i < MT; ++i) {
+                part[r][i] = fmaf(f[0], xv[i].x, part[r][i]);
+                part[r][i] = fmaf(f[1], xv[i].y, part[r][i]);
+                part[r][i] = fmaf(f[2], xv[i].z, part[r][i]);
+                part[r][i] = fmaf(f[3], xv[i].w, part[r][i]);
+              }
+            }
+          }
+#pragma unroll
+          for (int r = 0; r < R; ++r)
+#pragma unroll
+            for (int i = 0; i < MT; ++i) acc[r][i] = GROUPED ? fmaf(sv[d][r], part[r][i], acc[r][i]) : part[r][i];
+        }
+        fetch(d, st + d + D);
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int64_t row = row_base + r;
+    float s = p.wscale;
+    if (!GROUPED) s *= tl_load_scale(p.scales, p.scales_dtype, min(row, int64_t(p.n) - 1));
 #pragma unroll
     for (int i = 0; i < MT; ++i) {
       const float v = warp_sum(acc[r][i]) * s;
@@ -572,13 +664,6 @@ __global__ void __launch_bounds__(256) qgemv_sk_kernel(GemvArgs p, EpiParams epi
 // (so that many are resident per SM) an SM keeps ~100 KB of loads outstanding,
 // which is what it takes to cover HBM latency at full bandwidth.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void cp_async16(uint32_t smem_addr, const void* gptr) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr), "l"(gptr) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
 
 __device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
 
@@ -1815,10 +1900,40 @@ void launch_sk(bool m16, bool grouped, int depth, int grid, cudaStream_t s, cons
   }
 }
 
+template <typename AT, int MT, int R, int D, bool GROUPED>
+void launch_simt_staged(int grid, int block, cudaStream_t s, const GemvArgs& p, const EpiParams& e) {
+  const int steps = (p.k / 16 + 31) / 32, slice = std::min(simt_slice(MT, steps), (steps + D - 1) / D * D);
+  const size_t smem = (steps > slice ? 2 : 1) * size_t(MT) * slice * 512 * sizeof(float);
+  auto kern = qgemv_simt_kernel<AT, MT, R, D, GROUPED>;
+  if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return;  // the caller asks for the error
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(unsigned(grid));
+  cfg.blockDim = dim3(unsigned(block));
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kern, p, e, slice);
+}
+template <typename AT, int MT, int R, bool GROUPED>
+void launch_simt_g(int grid, int block, cudaStream_t s, const GemvArgs& p, const EpiParams& e) {
+  if constexpr (MT == 1 && R == 4) {
+    qgemv_simt_tall_kernel<AT, GROUPED><<<grid, block, 0, s>>>(p, e);
+  } else if constexpr (MT == 1 && R == 1) {
+    // eight steps ahead where K is long enough for them (513 x 14336: 21.5 -> 18.8 us; 4096 x 4096, whose eight steps they are: 7.4 -> 10.2)
+    if (p.k >= 8192) launch_simt_staged<AT, MT, R, 8, GROUPED>(grid, block, s, p, e);
+    else launch_simt_staged<AT, MT, R, 4, GROUPED>(grid, block, s, p, e);
+  } else {
+    launch_simt_staged<AT, MT, R, R == 4 ? 2 : 4, GROUPED>(grid, block, s, p, e);
+  }
+}
 template <typename AT, int MT, int R>
 void launch_simt(bool grouped, int grid, int block, cudaStream_t s, const GemvArgs& p, const EpiParams& e) {
-  if (grouped) qgemv_simt_kernel<AT, MT, R, true><<<grid, block, 0, s>>>(p, e);
-  else qgemv_simt_kernel<AT, MT, R, false><<<grid, block, 0, s>>>(p, e);
+  if (grouped) launch_simt_g<AT, MT, R, true>(grid, block, s, p, e);
+  else launch_simt_g<AT, MT, R, false>(grid, block, s, p, e);
 }
 template <typename AT, int R>
 void launch_simt_m(int mt, bool grouped, int grid, int block, cudaStream_t s, const GemvArgs& p, const EpiParams& e) {
@@ -1895,12 +2010,25 @@ int32_t tl_qgemv_default_variant(tl_ctx* ctx, int32_t m, int64_t n, int64_t k, i
     ring_pick_shape(ctx, false, a_dtype, m, q.group_size != k, tiles, k, &w, &d, &wide);
     v.p0 = w; v.p1 = d; v.p2 = wide ? 2 : 0;
   } else if (k % 16 == 0 && q.group_size % 16 == 0) {
-    // Rows a warp: four share an activation load where that leaves enough CTAs, the more so the more batch rows there are
-    // (12288 x 4096, f32, us with 2 / 4 rows: 20 / 16 at m = 1, 58 / 40 at m = 4, 231 / 158 at m = 16; 4096 x 12288: 20 / 33,
-    // 56 / 45, 222 / 174); one where rows are few (1000 x 1024: 2.9 / 2.9 / 3.6 us with 1 / 2 / 4 at m = 1, 4.6 / 5.1 / 6.6 at 4).
     const int64_t sms = ctx ? ctx->sm_count : 148;
-    v.kernel = kSimt; v.p0 = 4;
-    v.p1 = n >= (m <= 2 ? 48 : 24) * sms ? 4 : n >= 12 * sms ? 2 : 1;
+    v.kernel = kSimt;
+    // Rows a warp: the more, the fewer reads of the staged activations; the fewer, the more CTAs, as long as one wave holds them (three
+    // or four of eight warps an SM).  us with 1 / 2 / 4 rows and eight warps (f32, groups of 64): 4096 x 4096 m = 1 7.3 / 8.2 / 11.5, m = 3
+    // 11.7 / 10.9 / 15.1, m = 4 20.6 / 12.2 / 14.4; 7000 x 2048 m = 1 7.0 / 5.2 / 8.0, m = 3 11.0 / 10.8 / 9.6, m = 4 13.3 / 13.6 / 18.0 and 10.6 with
+    // four warps of four rows; 12288 x 4096 m = 1 19.1 / 16.8 / 15.4 (four warps, the tall form), m = 2 23.8 / 24.9 / 24.0, m = 3 30.4 / 30.5 / 27.4,
+    // m = 4 42.2 / 34.2 / 41.6; 1024 x 4096 m = 1 5.1 / 5.8 / 9.4, m = 16 41.8 / 39.2 / 48.8; 1000 x 1024 m = 4 4.0 / 4.5 / 6.6.
+    const bool tall = n >= 48 * sms;
+    v.p0 = 8;
+    if (m == 1) {
+      v.p1 = tall ? 4 : n > 28 * sms ? 2 : 1;
+      if (tall) v.p0 = 4;
+    } else if (m <= 3) {
+      v.p1 = n > 28 * sms ? 4 : m == 3 && n >= 12 * sms ? 2 : 1;
+    } else if (n > 36 * sms && !tall) {
+      v.p0 = v.p1 = 4;
+    } else {
+      v.p1 = m >= 8 || n >= 12 * sms ? 2 : 1;
+    }
   } else {
     v.kernel = kScalar; v.p0 = 8;
   }
