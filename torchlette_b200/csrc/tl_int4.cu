@@ -513,13 +513,17 @@ RingShape int4_ring_shape(const tl_ctx* ctx, int m, int64_t n, int64_t k, int gr
   // share each one's k loop: sixteen up to two tiles an SM, with rings of four stages where shared memory leaves the
   // tiles resident; else eight with two.  Two token tiles want 32-row tiles, which share the activations, once every SM
   // has a tile.  us, groups of 128: 1425 x 11008 m = 1 16 warps 7.9, 8 warps 10.5; 4096 x 14336 m = 4 17.0, 22.9; 4096 x 4096
-  // m = 16 32-row tiles 7.6, 16-row 9.6; 14336 x 4096 m = 16 4 warps 21.8 to 22.9, 8 warps 29.5.
+  // m = 16 32-row tiles 7.6, 16-row 9.6; 14336 x 4096 m = 16 4 warps 21.8 to 22.9, 8 warps 29.5.  Groups of 32: 30000 x 1024 m = 1 4 warps
+  // 10.3, 8 warps 13.3, m = 16 16.6, 22.7; 14336 x 4096 m = 16 28.8, 30.6; 4096 x 12288 m = 16 32-row tiles 22.8, sixteen warps 26.7.
   const int64_t tiles = (n + 15) / 16, sms = ctx->sm_count;
   int warps = 8, rt = 1, s = 2;
-  if (m > 8 && tiles > sms && (group == k || group % 128 == 0)) {
+  const bool folds_once = group == k || group % 128 == 0;
+  if (m > 8 && tiles > sms && (folds_once || tiles <= 2 * sms)) {
     rt = 2;
     if (tiles > 4 * sms) warps = 4;
     else s = 4;
+  } else if (tiles > 4 * sms && (m > 8 || kblocks <= 8)) {
+    warps = 4;  // several waves: short k loops, or the registers of two token tiles whose scales fold several times a block
   } else if (tiles <= 2 * sms && kblocks >= 16) {
     warps = 16;
     if (int4_ring_smem(16, 1, 4, m) <= (tiles <= sms ? 220 : 110) * 1024) s = 4;
