@@ -281,9 +281,9 @@ __global__ void __launch_bounds__(256) quantize_kernel(const float* __restrict__
 }
 
 // Groups of 32, 64 or 128 (LANES = group / 4 lanes of a warp, a float4 each): the weight is read once, and the f64
-// arithmetic runs only where it can change the result.  Bound: the instructions of the rounding (issue slots 67 %, ALU pipe
-// 66 %) ahead of HBM; 12288 x 4096 with groups of 64: 51 us = 5.0 TB/s (234 us a warp per group, all in f64, the weight read twice; 62
-// with an exact division and conversion for every scale).
+// arithmetic runs only where it can change the result.  Bound: HBM, the instructions of the rounding close behind; 12288 x 4096 with
+// groups of 64, replayed: 45 us = 5.6 TB/s (51 with a product, a clamp, two additions and a comparison a value; 62 with an exact
+// division and conversion for every scale; 234 a warp per group, all in f64, the weight read twice).
 //   x = w * inv in f32 is off by at most 3e-7 |x| < 8e-5 (a quotient good to 2 units in the last place and one rounding; |x| <
 //   256: the scale's f16 bits are at least half of the group's maximum, or zero); the rounding to a whole number can
 //   differ from the f64 one only if x lies that close to a half, and those values, and what is NaN, are done again in f64.
