@@ -893,13 +893,11 @@ __device__ __forceinline__ void ring_tile(const GemvArgs& p, const EpiParams& ep
   }
   // The tile's per-channel scales and bias entries are read in the epilogue, at the very end of a
   // one-wave launch: a cold line there is an exposed DRAM round trip on every launch.  Ask for the
-  // lines now (scales and bias are inputs, never a predecessor's output); no register stays live.
-  if (tid == 0) {
-    if (!GROUPED) prefetch_l1(reinterpret_cast<const uint8_t*>(p.scales) + size_t(tile_row) * (p.scales_dtype == TL_F32 ? 4 : 2));
-    if (epi.fast_bias) prefetch_l1(epi.fast_bias + tile_row);
-  }
-  // weights never depend on the previous kernel; activations (its output) and our own stores do
+  // lines early; no register stays live.
+  if (tid == 0 && !GROUPED) prefetch_l1(reinterpret_cast<const uint8_t*>(p.scales) + size_t(tile_row) * (p.scales_dtype == TL_F32 ? 4 : 2));
+  // weights and scales never depend on the previous kernel; activations (its output), a bias that may be one and our own stores do
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (tid == 0 && epi.fast_bias) prefetch_l1(epi.fast_bias + tile_row);
   if (rin) reduce_in_prologue(*rin);  // the activations are written by CTAs of THIS grid: read them through L2
   uint32_t push2_half = 0, push2_epoch = 0;
   if (PUSH == 2) {
@@ -1136,11 +1134,10 @@ __device__ __forceinline__ void ring_tile2(const GemvArgs& p, const EpiParams& e
     }
     cp_async_commit();
   }
-  if (tid == 0) {  // the epilogue's scales and bias entries: see ring_tile
-    if (!GROUPED) prefetch_l1(reinterpret_cast<const uint8_t*>(p.scales) + size_t(tile_row) * (p.scales_dtype == TL_F32 ? 4 : 2));
-    if (epi.fast_bias) prefetch_l1(epi.fast_bias + tile_row);
-  }
+  // the epilogue's scales and bias entries: see ring_tile
+  if (tid == 0 && !GROUPED) prefetch_l1(reinterpret_cast<const uint8_t*>(p.scales) + size_t(tile_row) * (p.scales_dtype == TL_F32 ? 4 : 2));
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (tid == 0 && epi.fast_bias) prefetch_l1(epi.fast_bias + tile_row);
 
   float total[2][NT][4];
 #pragma unroll
