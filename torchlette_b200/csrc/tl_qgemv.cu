@@ -230,7 +230,7 @@ template <typename AT> __device__ __forceinline__ void stage4(float* dst, const 
 __device__ __forceinline__ void stage4(float* dst, const float* src) { cp_async16(uint32_t(__cvta_generic_to_shared(dst)), src); }
 
 template <typename AT, int MT, int R, int D, bool GROUPED>
-__global__ void __launch_bounds__(256, D == 8 ? 4 : 1) qgemv_simt_kernel(GemvArgs p, EpiParams epi, int slice) {
+__global__ void __launch_bounds__(256) qgemv_simt_kernel(GemvArgs p, EpiParams epi, int slice) {
   extern __shared__ __align__(16) uint8_t simt_smem[];  // [2][MT][slice * 32 chunks][16] f32
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int warps = blockDim.x >> 5, lane = threadIdx.x & 31;
@@ -1920,8 +1920,9 @@ void launch_simt_g(int grid, int block, cudaStream_t s, const GemvArgs& p, const
   if constexpr (MT == 1 && R == 4) {
     qgemv_simt_tall_kernel<AT, GROUPED><<<grid, block, 0, s>>>(p, e);
   } else if constexpr (MT == 1 && R == 1) {
-    // eight steps ahead where K is long enough for them (513 x 14336: 21.5 -> 18.8 us; 4096 x 4096, whose eight steps they are: 7.4 -> 10.2)
-    if (p.k >= 8192) launch_simt_staged<AT, MT, R, 8, GROUPED>(grid, block, s, p, e);
+    // Eight steps ahead where K is long enough for them (513 x 14336: 21.5 -> 18.8 us; 4096 x 4096, whose eight steps they are: 7.4 -> 10.2)
+    // and, with the registers of as many scales, where one wave still holds the CTAs (4096 x 12288, groups of 64, 512 of them: 31 us).
+    if (p.k >= 8192 && (!GROUPED || grid <= 384)) launch_simt_staged<AT, MT, R, 8, GROUPED>(grid, block, s, p, e);
     else launch_simt_staged<AT, MT, R, 4, GROUPED>(grid, block, s, p, e);
   } else {
     launch_simt_staged<AT, MT, R, R == 4 ? 2 : 4, GROUPED>(grid, block, s, p, e);
