@@ -29,6 +29,7 @@
 #include <type_traits>
 
 #include "tl_common.cuh"
+#include "tl_qgemm_ring.h"
 #include "tl_tcgen05.cuh"
 #include "tl_tma.cuh"
 
@@ -224,14 +225,14 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
   constexpr int kSlotCols = KSTEP / 2;              // TMEM columns of one dequantized operand slot
   // The shared-memory ring (STAGES deep) has to cover the TMA round trip; the TMEM operand
   // ring only has to cover conversion -> MMA, so it is sized by what TMEM has left (TS slots).
-  constexpr int kFreeCols = 512 - 2 * BN;
-  constexpr int TS = (kFreeCols / kSlotCols) < STAGES ? (kFreeCols / kSlotCols) : STAGES;
+  constexpr TcRing kRing = tl_tc_ring({BN, KSTEP, STAGES, NCW});
+  constexpr int TS = kRing.slots;
   static_assert(TS >= 2, "TMEM operand ring");
   constexpr uint32_t kTmemCols = pow2_at_least(2 * BN + TS * kSlotCols);
   static_assert(kTmemCols <= 512, "TMEM budget");
   // Sixteen converter warps are two groups on alternate k steps: a step's chain of wait, load, convert, store and signal is
-  // longer than its MMAs, whatever its arithmetic.
-  constexpr int kGroups = NCW == 16 ? 2 : 1;
+  // longer than its MMAs, whatever its arithmetic.  When such a group may look at a stage: tl_tc_ring.
+  constexpr int kGroups = kRing.groups;
   constexpr int kGroupWarps = NCW / kGroups;
   constexpr int kParts = kGroupWarps / 4;           // converter threads per weight row
   constexpr int kChunks = KSTEP / 16 / kParts;      // 16-byte chunks per converter thread and stage
@@ -369,8 +370,10 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
       const int grp = gshift >= 0 ? k >> gshift : k / p.group;
       return (grp < p.groups_per_row ? tl_load_scale(p.scales, p.scales_dtype, grow * p.groups_per_row + grp) : 0.f) * p.wscale;
     };
+    auto slot_free = [&](int it) -> bool { return it < TS || mbar_wait(&slotfree_bar[it % TS], ((it / TS) - 1) & 1, &abort_flag); };
     auto convert = [&](int it, int ks, int n_tile) -> bool {
       const int s = it % STAGES;
+      if (kRing.slot_first && !slot_free(it)) return false;
       if (warp == 0 && lane == 0) TL_TR(2, it, 0);
       if (!mbar_wait(&full_bar[s], (it / STAGES) & 1, &abort_flag)) return false;
       if (warp == 0 && lane == 0) TL_TR(2, it, 1);
@@ -418,7 +421,7 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
         const int sl = it % TS;
         if (!convert(it, ks, n_tile)) { ok = false; break; }
         if (warp == 0 && lane == 0) TL_TR(2, it, 2);
-        if (it >= TS && !mbar_wait(&slotfree_bar[sl], ((it / TS) - 1) & 1, &abort_flag)) { ok = false; break; }
+        if (!kRing.slot_first && !slot_free(it)) { ok = false; break; }
         if (warp == 0 && lane == 0) TL_TR(2, it, 3);
         tc_fence_after();
         const uint32_t slot = tmem_base + lane_addr + uint32_t(2 * BN + sl * kSlotCols);
@@ -581,13 +584,6 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
 // ---------------------------------------------------------------------------
 constexpr int kTc = 0, kSliced = 1, kDequantDense = 2;
 
-struct TcConfig { int bn, kstep, stages, ncw; };
-// the instantiated tile configurations (tl_variant p0..p3)
-const TcConfig kTcConfigs[] = {{192, 64, 6, 4}, {192, 64, 6, 8}, {128, 64, 8, 4}, {128, 64, 8, 8},
-                               {64, 128, 6, 8}, {32, 128, 8, 8}, {16, 128, 8, 8},
-                               {128, 128, 4, 8}, {192, 128, 3, 8}, {128, 128, 4, 16}, {192, 128, 3, 16},
-                               {64, 128, 6, 16}, {32, 128, 8, 16}};
-
 bool tc_config_known(const tl_variant& v) {
   for (const auto& c : kTcConfigs)
     if (c.bn == v.p0 && c.kstep == v.p1 && c.stages == v.p2 && c.ncw == v.p3) return true;
@@ -654,10 +650,12 @@ namespace {
 tl_variant fused_tile(tl_ctx* ctx, int64_t m, int64_t n, int64_t k, int32_t a_dtype, const tl_quant_desc& q, double* us, int64_t* chain) {
   *us = 0;
   *chain = k;
-  // Sixteen converter warps where the weights have group scales, whose conversion is the longer chain (us, 8 / 16 warps: 30 x 12288 x
-  // 4096 groups of 64 31.5 / 27.6, 64 tokens 32.7 / 28.6, 250 51.0 / 47.4, 400 x 4096 x 4096 34.2 / 31.0; per channel 64 x 12288 x
-  // 4096 17.6 / 19.2, 30 x 4096 x 4096 11.6 / 12.5).  Tiles of 192 tokens gain only over several waves (1500 x 12288 x 4096 168 / 161, 900 x 4096 x
-  // 4096 54.2 / 56.0).
+  // Sixteen converter warps where the weights have group scales, whose conversion is the longer chain, for every group size and both types
+  // (us, 8 / 16 warps, n = 12288, k = 4096, f16: 30 tokens groups of 16 52.4 / 41.1, 32 46.1 / 36.9, 48 53.2 / 39.0, 64 32.8 / 28.7,
+  // 128 30.8 / 27.3, 256 30.8 / 26.7; 250 tokens 69.8 / 57.4, 67.6 / 55.7, 75.7 / 58.7, 50.9 / 47.0, 49.0 / 45.1, 47.5 / 44.7; bf16 within 0.3 of these
+  // but for 30 tokens in groups of 16, 49.1 / 39.0).  Per channel eight (64 x 12288 x 4096 17.6 / 19.2, 30 x 4096 x 4096 11.6 / 12.5), and eight for
+  // tiles of 192 tokens, on whose three-stage ring a converter of two groups waits for its slot before it reads (groups of 64: 1500 x 12288 x 4096
+  // 168.5 / 168.0, 900 x 12288 x 1024 43.7 / 49.2, 333 x 12288 x 4096 55.4 / 57.3).
   const bool grouped = q.group_size != k, half = a_dtype == TL_F16;
   const int32_t ncw = grouped ? 16 : 8;
   if (m <= 16) return tl_variant{TL_FAMILY_QGEMM, kTc, 16, 128, 8, 8};
@@ -665,7 +663,7 @@ tl_variant fused_tile(tl_ctx* ctx, int64_t m, int64_t n, int64_t k, int32_t a_dt
   if (m <= 64) return tl_variant{TL_FAMILY_QGEMM, kTc, 64, 128, 6, ncw};
   // The token tile by modelled time: waves x 128-k steps x the time of a step, a last partial wave cut along K as the
   // launch does it, 7 us for the meeting of its parts.  Step times on B200: 192 tokens 0.72 us (f16) / 0.78 (bf16) /
-  // 0.95 (group scales; 0.92 over several waves), 128 tokens 0.53 / 0.67 / 0.76.  Measured, us, 192 / 128: 2048 x 14336 x 4096 f16 201 / 215, bf16
+  // 0.95 (group scales), 128 tokens 0.53 / 0.67 / 0.76.  Measured, us, 192 / 128: 2048 x 14336 x 4096 f16 201 / 215, bf16
   // 217 / 268; 333 x 12288 x 4096 f16 47 / 38, groups of 64 56 / 54 over rotating copies, 60 / 62 on one; 600 x 14336 x 2048 f16 50 / 38.
   const int64_t sms = ctx ? ctx->sm_count : 148, ksteps = (k + 127) / 128;
   // Before the time comes the sum: the tensor core's f32 accumulator loses bits with every product it takes (170 x 576 x 512 f16,
@@ -678,12 +676,11 @@ tl_variant fused_tile(tl_ctx* ctx, int64_t m, int64_t n, int64_t k, int32_t a_dt
     return (double(tiles / sms) + (rem ? 1.0 / double(splits) : 0.0)) * double(ksteps) * step + (splits > 1 ? 7.0 : 0.0);
   };
   int64_t c192, c128;
-  const bool waves = ((n + kTileRows - 1) / kTileRows) * ((m + 191) / 192) >= 3 * sms;
-  const double t192 = fused_us(192, grouped ? (waves ? 0.92 : 0.95) : half ? 0.72 : 0.78, &c192), t128 = fused_us(128, grouped ? 0.76 : half ? 0.53 : 0.67, &c128);
+  const double t192 = fused_us(192, grouped ? 0.95 : half ? 0.72 : 0.78, &c192), t128 = fused_us(128, grouped ? 0.76 : half ? 0.53 : 0.67, &c128);
   const bool wide = c192 != c128 ? c192 < c128 : t192 <= t128;
   *us = wide ? t192 : t128;
   *chain = wide ? c192 : c128;
-  return wide ? tl_variant{TL_FAMILY_QGEMM, kTc, 192, 128, 3, grouped && waves ? 16 : 8} : tl_variant{TL_FAMILY_QGEMM, kTc, 128, 128, 4, ncw};
+  return wide ? tl_variant{TL_FAMILY_QGEMM, kTc, 192, 128, 3, 8} : tl_variant{TL_FAMILY_QGEMM, kTc, 128, 128, 4, ncw};
 }
 }  // namespace
 
