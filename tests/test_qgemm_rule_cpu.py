@@ -1,0 +1,59 @@
+"""The route of a quantized product with many tokens, as the default rule chooses it for 148 SMs, without a GPU: a program linked against the
+library's objects asks the rule itself."""
+import glob
+import os
+import subprocess
+
+import pytest
+
+from torchlette_b200 import _build
+
+ASK = """
+#include <cstdio>
+#include "tl_common.cuh"
+int main() {
+  long long m, n, k;
+  int group, bf16;
+  while (std::scanf("%lld %lld %lld %d %d", &m, &n, &k, &group, &bf16) == 5) {
+    tl_quant_desc q{};
+    q.scheme = TL_SCHEME_INT8_GROUPED;
+    q.group_size = group ? group : int(k);
+    q.scales_dtype = TL_F16;
+    tl_variant v;
+    tl_qgemm_default_variant(nullptr, m, n, k, bf16 ? TL_BF16 : TL_F16, q, &v);
+    std::printf("%d %d %d %d %d %d\\n", v.kernel, v.p0, v.p1, v.p2, v.p3, tl_dense_tc_choose(m, n, k, 148).parts);
+  }
+}
+"""
+FUSED, DEQUANT_DENSE = 0, 2
+
+
+@pytest.fixture(scope="module")
+def rule(tmp_path_factory):
+    _build.build()
+    d = tmp_path_factory.mktemp("rule")
+    src, exe = d / "ask.cpp", d / "ask"
+    src.write_text(ASK)
+    cuda = os.path.dirname(os.path.dirname(_build.NVCC))
+    subprocess.run(["g++", "-std=c++17", "-I", _build.CSRC, "-I", os.path.join(cuda, "include"), str(src), *glob.glob(os.path.join(_build.CSRC, "*.o")),
+                    "-L", os.path.join(cuda, "lib64"), "-lcudart_static", "-ldl", "-lpthread", "-lrt", "-o", str(exe)], check=True)
+
+    def ask(*shapes):
+        text = "".join(" ".join(map(str, s)) + "\n" for s in shapes)
+        return [tuple(map(int, line.split())) for line in subprocess.run([str(exe)], input=text, check=True, capture_output=True, text=True).stdout.splitlines()]
+    return ask
+
+
+# m, n, k, group, bf16: dequantize + dense cuts K in two to eight; the fused kernel, which the faster converters make the quicker one by up to
+# an eighth, would sum over all of K or over more of it
+@pytest.mark.parametrize("shape", [(1999, 793, 4992, 64, 0), (445, 2130, 11136, 16, 1), (470, 4160, 13824, 64, 0), (177, 909, 9344, 64, 0),
+                                   (224, 4976, 13312, 128, 1), (510, 3832, 10032, 48, 0), (250, 791, 9216, 64, 1), (233, 513, 8320, 32, 0)])
+def test_a_faster_fused_kernel_takes_no_longer_sums(rule, shape):
+    kernel, *_, parts = rule(shape)[0]
+    assert kernel == DEQUANT_DENSE and parts > 1
+
+
+def test_tiles_of_192_tokens_keep_eight_converter_warps(rule):
+    got = rule((180, 100352, 4096, 64, 0), (150, 151936, 1024, 64, 1), (333, 12288, 4096, 0, 0))
+    assert [g[:5] for g in got[:2]] == [(FUSED, 192, 128, 3, 8)] * 2
+    assert got[2][4] == 8

@@ -645,10 +645,10 @@ bool tl_qgemm_variant_applicable(const tl_variant& v, int64_t m, int64_t n, int6
 }
 
 namespace {
-// The fused kernel's tile, by the token count, and above 64 tokens its modelled time and the longest sum in one accumulator
-// (*chain, in k).  Only for what the fused kernel takes: 16-bit activations, k and groups of whole 16s.
-tl_variant fused_tile(tl_ctx* ctx, int64_t m, int64_t n, int64_t k, int32_t a_dtype, const tl_quant_desc& q, double* us, int64_t* chain) {
-  *us = 0;
+// The fused kernel's tile, by the token count, and above 64 tokens its modelled time (*us8: of the better tile with eight converter
+// warps) and the longest sum in one accumulator (*chain, in k).  Only for what the fused kernel takes: 16-bit activations, k and groups of whole 16s.
+tl_variant fused_tile(tl_ctx* ctx, int64_t m, int64_t n, int64_t k, int32_t a_dtype, const tl_quant_desc& q, double* us, double* us8, int64_t* chain) {
+  *us = *us8 = 0;
   *chain = k;
   // Sixteen converter warps where the weights have group scales, whose conversion is the longer chain, for every group size and both types
   // (us, 8 / 16 warps, n = 12288, k = 4096, f16: 30 tokens groups of 16 52.4 / 41.1, 32 46.1 / 36.9, 48 53.2 / 39.0, 64 32.8 / 28.7,
@@ -663,8 +663,8 @@ tl_variant fused_tile(tl_ctx* ctx, int64_t m, int64_t n, int64_t k, int32_t a_dt
   if (m <= 64) return tl_variant{TL_FAMILY_QGEMM, kTc, 64, 128, 6, ncw};
   // The token tile by modelled time: waves x 128-k steps x the time of a step, a last partial wave cut along K as the
   // launch does it, 7 us for the meeting of its parts.  Step times on B200: 192 tokens 0.72 us (f16) / 0.78 (bf16) /
-  // 0.95 (group scales), 128 tokens 0.53 / 0.67 / 0.76.  Measured, us, 192 / 128: 2048 x 14336 x 4096 f16 201 / 215, bf16
-  // 217 / 268; 333 x 12288 x 4096 f16 47 / 38, groups of 64 56 / 54 over rotating copies, 60 / 62 on one; 600 x 14336 x 2048 f16 50 / 38.
+  // 0.95 (group scales), 128 tokens 0.53 / 0.67 / 0.76 (0.9 with eight converter warps).  Measured, us, 192 / 128: 2048 x 14336 x 4096
+  // f16 201 / 215, bf16 217 / 268; 333 x 12288 x 4096 f16 47 / 38, groups of 64 56 / 54 over rotating copies, 60 / 62 on one; 600 x 14336 x 2048 f16 50 / 38.
   const int64_t sms = ctx ? ctx->sm_count : 148, ksteps = (k + 127) / 128;
   // Before the time comes the sum: the tensor core's f32 accumulator loses bits with every product it takes (170 x 576 x 512 f16,
   // f32 output, against 64 bits: 1.0e-7 with K cut in four, 4.3e-7 uncut), so where one wave's tiles are all cut, the
@@ -678,7 +678,9 @@ tl_variant fused_tile(tl_ctx* ctx, int64_t m, int64_t n, int64_t k, int32_t a_dt
   int64_t c192, c128;
   const double t192 = fused_us(192, grouped ? 0.95 : half ? 0.72 : 0.78, &c192), t128 = fused_us(128, grouped ? 0.76 : half ? 0.53 : 0.67, &c128);
   const bool wide = c192 != c128 ? c192 < c128 : t192 <= t128;
+  const double t128_8 = grouped ? fused_us(128, 0.9, &c128) : t128;
   *us = wide ? t192 : t128;
+  *us8 = (c192 != c128 ? wide : t192 <= t128_8) ? t192 : t128_8;
   *chain = wide ? c192 : c128;
   return wide ? tl_variant{TL_FAMILY_QGEMM, kTc, 192, 128, 3, 8} : tl_variant{TL_FAMILY_QGEMM, kTc, 128, 128, 4, ncw};
 }
@@ -689,9 +691,9 @@ int32_t tl_qgemm_default_variant(tl_ctx* ctx, int64_t m, int64_t n, int64_t k, i
   tl_variant v{};
   v.family = TL_FAMILY_QGEMM;
   if ((a_dtype == TL_F16 || a_dtype == TL_BF16) && k % 16 == 0 && q.group_size % 16 == 0) {
-    double fused_us = 0;
+    double fused_us = 0, fair_us = 0;
     int64_t chain = 0;
-    v = fused_tile(ctx, m, n, k, a_dtype, q, &fused_us, &chain);
+    v = fused_tile(ctx, m, n, k, a_dtype, q, &fused_us, &fair_us, &chain);
     // With many tokens per weight byte, writing the weight out once as a 16-bit matrix and running the
     // dense kernel (whose operands both come from shared memory at its full tile sizes) beats converting
     // on the operand path: the dense kernel's modelled time, the pass at 6 TB/s (3 bytes a weight) and 4 us for the second
@@ -704,7 +706,10 @@ int32_t tl_qgemm_default_variant(tl_ctx* ctx, int64_t m, int64_t n, int64_t k, i
       const TlDenseTcChoice dense = tl_dense_tc_choose(m, n, k, ctx ? ctx->sm_count : 148);
       const double dense_us = dense.cost_us + double(n) * double(k) * 3.0 / 6.0e6 + 4.0;
       const int64_t steps64 = (k + 63) / 64, dense_chain = std::min(k, (steps64 + dense.parts - 1) / dense.parts * 64);
-      if (dense_us < 0.95 * fused_us && dense_chain <= chain) v = dd;  // not for longer sums either
+      // The sums are not to be longer for it, on either route: this way only where its own are no longer, and where they are shorter
+      // against the time that the fused kernel takes for longer ones with eight converter warps (fair_us), since sixteen made it faster
+      // but no more exact: 1999 x 793 x 4992, groups of 64, cut in two this way, uncut in the fused kernel.
+      if (dense_us < 0.95 * (dense_chain < chain ? fair_us : fused_us) && dense_chain <= chain) v = dd;
     }
   } else {
     v.kernel = kSliced;  // f32 activations or odd K: sixteen-row slices through the small-batch kernels
@@ -720,9 +725,9 @@ int32_t tl_qgemm_secure_scratch(tl_ctx* ctx, tl_variant* v, int64_t m, int64_t n
   void* wbuf = nullptr;
   const int32_t rc = tl_ensure_scratch(ctx, size_t(n) * size_t(k) * 2, &wbuf);
   if (rc != TL_ERR_OOM && !(rc == TL_ERR_UNSUPPORTED && ctx->capturing)) return rc;
-  double us;
+  double us, us8;
   int64_t chain;
-  *v = fused_tile(ctx, m, n, k, a_dtype, q, &us, &chain);
+  *v = fused_tile(ctx, m, n, k, a_dtype, q, &us, &us8, &chain);
   return TL_OK;
 }
 
