@@ -208,3 +208,47 @@ def test_int4_forced_shapes_run(backend, m, n, k, warps, row_tiles, stages):
     assert (np.abs(be.ops.read(y) - xv.astype(np.float64) @ wref.astype(np.float64).T) <= size * 2.0 ** -20).all()
     for t in (x, y, w.scales, w):
         t.destroy()
+
+
+@pytest.mark.parametrize("out", ["f16", "bf16", "f32"])
+@pytest.mark.parametrize("m,n,k,g", [(9, 2400, 384, 32), (16, 2400, 1152, 64), (16, 4700, 256, 32), (9, 4700, 2304, 64), (1, 9500, 1024, 32), (1, 9500, 1024, 64),
+                                     (1, 9500, 1024, 128), (16, 9500, 1024, 32), (16, 9500, 1024, 64), (16, 9500, 640, 128), (8, 9480, 128, 64)])
+def test_int4_ring_of_few_warps(backend, out, m, n, k, g):
+    """Tiles of 32 rows whose scales fold several times a block, and four warps a tile (16-bit outputs; f32 takes more warps), where rows,
+    blocks and warps end.  Sums as above; a 16-bit result is rounded once more."""
+    be = backend
+    w, wref, _ = _weight(be, n, k, g, seed=n + m)
+    xv = np.random.default_rng(k + m).uniform(-1, 1, (m, k)).astype(np.float32)
+    if out == "bf16":
+        bits = orc.bf16_bits_rne(xv.reshape(-1))
+        x, xv = be.ops.tensorFromArray(bits, [m, k], "bf16"), orc.bf16_bits_to_f32(bits).reshape(m, k).astype(np.float64)
+    else:
+        x, xv = be.ops.tensorFromArray(xv.astype(np.float16), [m, k], "f16"), xv.astype(np.float16).astype(np.float64)
+    y = be.linear(x, w, None, None, out)
+    got = be.ops.read(y)
+    got = orc.bf16_bits_to_f32(got.reshape(-1)).reshape(m, n) if out == "bf16" else np.asarray(got, np.float64)
+    ref = xv @ wref.astype(np.float64).T
+    bound = np.abs(xv) @ np.abs(wref.astype(np.float64)).T * 2.0 ** -20
+    bound += {"f16": 2.0 ** -11, "bf16": 2.0 ** -8, "f32": 0.0}[out] * (np.abs(ref) + bound) + (2.0 ** -25 if out == "f16" else 0.0)
+    assert (np.abs(got - ref) <= bound).all()
+    for t in (x, y, w.scales, w):
+        t.destroy()
+
+
+@pytest.mark.parametrize("g", [32, 64, 0])
+@pytest.mark.parametrize("m,n,k", [(5, 100, 640), (16, 300, 1024)])
+@pytest.mark.parametrize("warps,row_tiles,stages", [(16, 1, 4), (8, 2, 4), (4, 1, 2), (1, 2, 2)])
+def test_int4_forced_shapes_with_other_groups(backend, g, m, n, k, warps, row_tiles, stages):
+    be = backend
+    w, wref, _ = _weight(be, n, k, g or k, seed=m)
+    xv = np.random.default_rng(k).uniform(-1, 1, (m, k)).astype(np.float16)
+    x = be.ops.tensorFromArray(xv, [m, k], "f16")
+    be.forceVariant((1, 9, warps, row_tiles, stages, 0))
+    try:
+        y = be.linear(x, w, None, None, "f32")
+    finally:
+        be.forceVariant(None)
+    size = np.abs(xv.astype(np.float64)) @ np.abs(wref.astype(np.float64)).T
+    assert (np.abs(be.ops.read(y) - xv.astype(np.float64) @ wref.astype(np.float64).T) <= size * 2.0 ** -20).all()
+    for t in (x, y, w.scales, w):
+        t.destroy()

@@ -1,5 +1,5 @@
-"""The route of a quantized product with many tokens, as the default rule chooses it for 148 SMs, without a GPU: a program linked against the
-library's objects asks the rule itself."""
+"""The forms that the default rules choose for quantized products on 148 SMs, without a GPU: a program linked against the library's objects asks
+the rules themselves."""
 import glob
 import os
 import subprocess
@@ -7,15 +7,27 @@ import subprocess
 import pytest
 
 from torchlette_b200 import _build
+from torchlette_b200 import binding as B
 
 ASK = """
 #include <cstdio>
 #include "tl_common.cuh"
 int main() {
   long long m, n, k;
-  int group, bf16;
-  while (std::scanf("%lld %lld %lld %d %d", &m, &n, &k, &group, &bf16) == 5) {
+  int group, bf16, int4_out;
+  while (std::scanf("%lld %lld %lld %d %d %d", &m, &n, &k, &group, &bf16, &int4_out) == 6) {
     tl_quant_desc q{};
+    if (int4_out >= 0) {  // a receipt of an int4 product
+      tl_ctx ctx;
+      ctx.sm_count = 148;
+      q.scheme = TL_SCHEME_INT4_GROUPED;
+      q.group_size = group ? group : int(k);
+      q.scales_dtype = TL_F16;
+      tl_plan_receipt r;
+      if (tl_plan_qmatmul(&ctx, m, n, k, bf16 ? TL_BF16 : TL_F16, int4_out, &q, nullptr, &r) != TL_OK) return 1;
+      std::printf("%d %d %d\\n", r.choice.p0, r.choice.p1, r.choice.p2);
+      continue;
+    }
     q.scheme = TL_SCHEME_INT8_GROUPED;
     q.group_size = group ? group : int(k);
     q.scales_dtype = TL_F16;
@@ -39,7 +51,7 @@ def rule(tmp_path_factory):
                     "-L", os.path.join(cuda, "lib64"), "-lcudart_static", "-ldl", "-lpthread", "-lrt", "-o", str(exe)], check=True)
 
     def ask(*shapes):
-        text = "".join(" ".join(map(str, s)) + "\n" for s in shapes)
+        text = "".join(" ".join(map(str, s if len(s) == 6 else s + (-1,))) + "\n" for s in shapes)
         return [tuple(map(int, line.split())) for line in subprocess.run([str(exe)], input=text, check=True, capture_output=True, text=True).stdout.splitlines()]
     return ask
 
@@ -57,3 +69,11 @@ def test_tiles_of_192_tokens_keep_eight_converter_warps(rule):
     got = rule((180, 100352, 4096, 64, 0), (150, 151936, 1024, 64, 1), (333, 12288, 4096, 0, 0))
     assert [g[:5] for g in got[:2]] == [(FUSED, 192, 128, 3, 8)] * 2
     assert got[2][4] == 8
+
+
+@pytest.mark.parametrize("n,k,group,m,fewer,warps", [(2400, 4096, 32, 16, (8, 2), 16), (4700, 12288, 64, 9, (8, 2), 16), (4096, 1536, 32, 12, (8, 2), 8),
+                                                     (9500, 4096, 64, 16, (4, 1), 8), (9500, 1024, 128, 1, (4, 1), 8), (30000, 1024, 32, 16, (4, 1), 8)])
+def test_an_int4_product_with_f32_output_keeps_its_short_sums(rule, n, k, group, m, fewer, warps):
+    """The forms with fewer warps a tile, hence longer sums, are for 16-bit outputs."""
+    wide, half, bf16 = (r[:2] for r in rule((m, n, k, group, 0, B.DTYPE_ID["f32"]), (m, n, k, group, 0, B.DTYPE_ID["f16"]), (m, n, k, group, 1, B.DTYPE_ID["bf16"])))
+    assert half == bf16 == fewer and wide == (warps, 1)

@@ -452,7 +452,7 @@ __global__ void __launch_bounds__(RT == 2 ? 256 : 512) qgemv_int4_ring_kernel(In
     const int64_t row = tile_row + r * 16 + (ln >> 2) + ((i & 2) ? 8 : 0);
     const int col = 8 * nt + 2 * (ln & 3) + (i & 1);
     if (row < p.n && col < p.m) {
-      // four short sums instead of one long one: sixteen warps' partial tiles add up as exactly as eight did
+      // four short sums instead of one long one, whatever the number of warps
       float part[4] = {0.f, 0.f, 0.f, 0.f};
       for (int w = 0; w < warps; w += 4)
 #pragma unroll
@@ -507,22 +507,25 @@ cudaError_t int4_ring(tl_ctx* ctx, const Int4Args& p, const EpiParams& e, int wa
 
 struct RingShape { int warps, row_tiles, stages; };
 
-RingShape int4_ring_shape(const tl_ctx* ctx, int m, int64_t n, int64_t k, int group) {
+RingShape int4_ring_shape(const tl_ctx* ctx, int m, int64_t n, int64_t k, int group, int32_t out_dtype) {
   const int kblocks = int(k >> 7);
   // A warp takes about a microsecond a block whatever the rest of the chip does, so the fewer the tiles the more warps
   // share each one's k loop: sixteen up to two tiles an SM, with rings of four stages where shared memory leaves the
   // tiles resident; else eight with two.  Two token tiles want 32-row tiles, which share the activations, once every SM
-  // has a tile.  us, groups of 128: 1425 x 11008 m = 1 16 warps 7.9, 8 warps 10.5; 4096 x 14336 m = 4 17.0, 22.9; 4096 x 4096
-  // m = 16 32-row tiles 7.6, 16-row 9.6; 14336 x 4096 m = 16 4 warps 21.8 to 22.9, 8 warps 29.5.  Groups of 32: 30000 x 1024 m = 1 4 warps
-  // 10.3, 8 warps 13.3, m = 16 16.6, 22.7; 14336 x 4096 m = 16 28.8, 30.6; 4096 x 12288 m = 16 32-row tiles 22.8, sixteen warps 26.7.
+  // has a tile -- with groups below 128, whose folds take the registers, up to two tiles an SM.  us, groups of 128: 1425 x 11008 m = 1
+  // 16 warps 7.9, 8 warps 10.5; 4096 x 14336 m = 4 17.0, 22.9; 4096 x 4096 m = 16 32-row tiles 7.6, 16-row 9.6; 14336 x 4096 m = 16
+  // 4 warps 21.8 to 22.9, 8 warps 29.5.  Groups of 32: 30000 x 1024 m = 1 4 warps 10.3, 8 warps 13.3, m = 16 16.6, 22.7; 14336 x 4096 m = 16 28.8,
+  // 30.6; 4096 x 12288 m = 16 32-row tiles 22.8, sixteen warps 26.7.
+  // Fewer warps are longer f32 sums (against 64 bits, 16 x 4096 x 12288 in groups of 32: 1.07e-7 with sixteen, 1.34e-7 with eight): an f32
+  // output keeps the warps that the small groups and short k loops would give up; a 16-bit one, off by 2.1e-4 either way, does not.
   const int64_t tiles = (n + 15) / 16, sms = ctx->sm_count;
   int warps = 8, rt = 1, s = 2;
-  const bool folds_once = group == k || group % 128 == 0;
-  if (m > 8 && tiles > sms && (folds_once || tiles <= 2 * sms)) {
+  const bool folds_once = group == k || group % 128 == 0, fewer = out_dtype != TL_F32;
+  if (m > 8 && tiles > sms && (folds_once || (fewer && tiles <= 2 * sms))) {
     rt = 2;
     if (tiles > 4 * sms) warps = 4;
     else s = 4;
-  } else if (tiles > 4 * sms && (m > 8 || kblocks <= 8)) {
+  } else if (fewer && tiles > 4 * sms && (m > 8 || kblocks <= 8)) {
     warps = 4;  // several waves: short k loops, or the registers of two token tiles whose scales fold several times a block
   } else if (tiles <= 2 * sms && kblocks >= 16) {
     warps = 16;
@@ -550,7 +553,7 @@ bool int4_ring_applies(const tl_ctx* ctx, int32_t a_dtype, int64_t k, int group)
 
 template <typename AT>
 cudaError_t launch_int4_mma(tl_ctx* ctx, const Int4Args& p, const EpiParams& e) {
-  const RingShape r = int4_ring_shape(ctx, p.m, p.n, p.k, p.group);
+  const RingShape r = int4_ring_shape(ctx, p.m, p.n, p.k, p.group, p.out_dtype);
   cudaError_t rc = int4_ring<AT>(ctx, p, e, r.warps, r.row_tiles, r.stages);
   ctx->counters[TL_COUNTER_KERNEL_LAUNCHES]++;
   return rc;
@@ -665,7 +668,7 @@ int32_t tl_int4_matmul(tl_ctx* ctx, const char* who, int route, const void* a, i
     if (gemv && m > 0 && n > 0) {
       int64_t rows = 0;  // of a CTA
       if (int4_ring_applies(ctx, a_dtype, k, q->group_size)) {
-        const RingShape r = int4_ring_shape(ctx, int(m), n, k, q->group_size);
+        const RingShape r = int4_ring_shape(ctx, int(m), n, k, q->group_size, out_dtype);
         receipt_only->choice.p0 = r.warps; receipt_only->choice.p1 = r.row_tiles; receipt_only->choice.p2 = r.stages;
         rows = 16 * r.row_tiles;
         receipt_only->block = 32 * r.warps;
