@@ -119,7 +119,10 @@ TL_API int64_t tl_async_error_count(tl_ctx* ctx);
  * a context when ctx is NULL).  Valid until the next call on the same thread. */
 TL_API const char* tl_last_error(tl_ctx* ctx);
 /* The CUDA stream every enqueue goes to (a cudaStream_t), so a host framework
- * can order its own work or record its own events on it. */
+ * can order its own work or record its own events on it.  Small-batch products start while the kernels in front of them drain and may
+ * ask for packed weights and scales (not for activations or epilogue inputs) before they wait for those.  Behind the calls of this
+ * library that write these, and after this call, the next one does not.  So a program whose own kernel writes a packed weight or
+ * its scales on the stream takes the stream, by this call, before that kernel or after it, each time. */
 TL_API int32_t tl_ctx_stream(tl_ctx* ctx, void** out_stream);
 TL_API int32_t tl_device_sm_count(tl_ctx* ctx, int32_t* out_sms);
 /* Per-context settings by name, the analogue of the reference's single ENV accessor

@@ -200,6 +200,7 @@ int32_t tl_ctx_stream(tl_ctx* ctx, void** out_stream) {
   TL_CHECK_CTX(ctx);
   if (!out_stream) return tl_set_error(ctx, TL_ERR_INVALID_ARG, "tl_ctx_stream: null out pointer");
   *out_stream = (void*)ctx->stream;
+  ctx->fresh_weights = true;  // for kernels of the program's own
   return TL_OK;
 }
 
@@ -396,6 +397,7 @@ int32_t tl_graph_end(tl_ctx* ctx, tl_graph** out_graph) {
   ctx->capturing = false;
   if (t_captures > 0) --t_captures;  // a capture ends on the thread that began it
   tl_graph* g = new tl_graph();
+  ctx->fresh_weights = true;  // the capture's launches have not run behind what had been enqueued before it
   cudaError_t e = cudaStreamEndCapture(ctx->stream, &g->graph);
   if (e != cudaSuccess || !g->graph) {
     delete g;
@@ -425,6 +427,7 @@ int32_t tl_graph_launch(tl_ctx* ctx, tl_graph* graph) {
   if (!graph || !graph->exec) return tl_set_error(ctx, TL_ERR_INVALID_ARG, "tl_graph_launch: null graph");
   DeviceGuard guard(ctx->device);
   TL_CUDA(ctx, cudaGraphLaunch(graph->exec, ctx->stream));
+  ctx->fresh_weights = true;  // its last kernel may have written some
   for (int i = 0; i < TL_COUNTER_COUNT; ++i) ctx->counters[i] += graph->counter_delta[i];
   return TL_OK;
 }

@@ -527,6 +527,7 @@ int32_t tl_attention(tl_ctx* ctx, const void* q, const void* k_cache, const void
   }
   TL_CUDA(ctx, e);
   ctx->counters[TL_COUNTER_KERNEL_LAUNCHES]++;
+  tl_wrote(ctx, out, batch * q_len * n_heads * head_dim * tl_dtype_size(dtype));
   return TL_OK;
 }
 

@@ -128,6 +128,7 @@ int32_t tl_allgather_cols(tl_ctx* ctx, const void* local, void* out, int64_t m, 
   if (!ctx->nccl_comm) return tl_set_error(ctx, TL_ERR_NCCL, "tl_allgather_cols: communicator not initialised");
   if (m == 1) {
     TL_NCCL(ctx, nccl().AllGather(local, out, count, nccl_dtype(dtype), (ncclComm_t)ctx->nccl_comm, ctx->stream));
+    tl_wrote_some(ctx);
     return TL_OK;
   }
   void* stage = nullptr;
@@ -141,6 +142,7 @@ int32_t tl_allgather_cols(tl_ctx* ctx, const void* local, void* out, int64_t m, 
   else interleave_cols_kernel<uint16_t><<<grid, block, 0, ctx->stream>>>((const uint16_t*)stage, (uint16_t*)out, m, n_local, ctx->world);
   TL_CUDA(ctx, cudaGetLastError());
   ctx->counters[TL_COUNTER_KERNEL_LAUNCHES]++;
+  tl_wrote_some(ctx);
   return TL_OK;
 }
 
@@ -152,6 +154,7 @@ int32_t tl_allreduce_sum(tl_ctx* ctx, void* buf, int64_t count, int32_t dtype) {
   if (!ctx->nccl_comm) return tl_set_error(ctx, TL_ERR_NCCL, "tl_allreduce_sum: communicator not initialised");
   DeviceGuard guard(ctx->device);
   TL_NCCL(ctx, nccl().AllReduce(buf, buf, size_t(count), nccl_dtype(dtype), ncclSum, (ncclComm_t)ctx->nccl_comm, ctx->stream));
+  tl_wrote_some(ctx);
   return TL_OK;
 }
 
@@ -452,6 +455,7 @@ static int32_t p2p_allreduce_impl(tl_ctx* ctx, const char* who, const void* src,
   else cudaLaunchKernelEx(&cfg, p2p_allreduce_kernel<__nv_bfloat16>, a);
   TL_CUDA(ctx, cudaGetLastError());
   ctx->counters[TL_COUNTER_KERNEL_LAUNCHES]++;
+  tl_wrote_some(ctx);
   return TL_OK;
 }
 

@@ -6,6 +6,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdarg>
 #include <cstdint>
 #include <cstdio>
@@ -79,6 +80,11 @@ struct tl_ctx {
   std::map<TuneKey, tl_variant> class_tuned;
   std::map<int, int> ring_occupancy;  // resident CTAs per SM of each ring kernel shape (queried once)
   bool capturing = false;
+  // what an early launch may have to wait for (tl_early_stream): a kernel that wrote packed weights, and recent outputs
+  static constexpr int kWritten = 16;
+  struct { const uint8_t *begin, *end; } written[kWritten];
+  int n_written = 0;
+  bool fresh_weights = false;
   // TORCHLETTE_CUDA_PROFILE=1: CUDA events around every product call, one line per call on stderr
   bool profile = false;
   cudaEvent_t prof_e0 = nullptr, prof_e1 = nullptr;
@@ -98,6 +104,44 @@ struct tl_ctx {
   int32_t push_m = 0, push_dtype = 0;
   int64_t push_n = 0, push_tiles = 0;
 };
+
+// The stream of a launch whose CTAs may start while the kernels in front of it drain (programmatic stream serialization) and ask for
+// packed weights -- the CUDA-core kernel also for scales -- before they wait for those.  Nothing else that a kernel here computes is read
+// before the wait, and only the wait makes it certain that what was written is seen.  So a launch behind a kernel that may have written
+// its weights or scales is an ordinary one, which orders all that came before.  Packed weights are written by the quantizer and by
+// unpacking (a replayed graph or a program with the stream in hand may run them): a flag.  Scales may be any call's output: the
+// outputs since the last kernel that certainly saw all before it end.
+struct EarlyStream {
+  cudaStream_t stream;
+  unsigned attrs;  // of the launch: 1 with the attribute, 0 without
+  operator cudaStream_t() const { return stream; }
+};
+inline EarlyStream tl_early_stream(tl_ctx* ctx, const void* scales = nullptr, size_t scales_bytes = 0) {
+  bool wait = ctx->fresh_weights || (scales && ctx->n_written > tl_ctx::kWritten);
+  const uint8_t* s = static_cast<const uint8_t*>(scales);
+  for (int i = 0; scales && !wait && i < ctx->n_written; ++i) wait = ctx->written[i].begin < s + scales_bytes && s < ctx->written[i].end;
+  if (wait) {
+    ctx->fresh_weights = false;
+    ctx->n_written = 0;
+  }
+  return EarlyStream{ctx->stream, wait ? 0u : 1u};
+}
+// A call's output.  settled: its kernel saw all before it end, and starts nothing early itself.
+inline void tl_wrote(tl_ctx* ctx, const void* out, int64_t bytes, bool settled = false) {
+  if (settled) {
+    ctx->n_written = 0;
+    ctx->fresh_weights = false;
+  }
+  const uint8_t* p = static_cast<const uint8_t*>(out);
+  for (int i = 0; i < ctx->n_written && i < tl_ctx::kWritten; ++i)
+    if (ctx->written[i].begin == p) {
+      ctx->written[i].end = std::max(ctx->written[i].end, p + bytes);
+      return;
+    }
+  if (ctx->n_written < tl_ctx::kWritten) ctx->written[ctx->n_written] = {p, p + bytes};
+  ctx->n_written = std::min(ctx->n_written + 1, tl_ctx::kWritten + 1);  // one more than there is room for: some are not listed
+}
+inline void tl_wrote_some(tl_ctx* ctx) { ctx->n_written = tl_ctx::kWritten + 1; }
 
 int32_t tl_set_error(tl_ctx* ctx, int32_t code, const char* fmt, ...);
 int32_t tl_ensure_scratch(tl_ctx* ctx, size_t bytes, void** out);
@@ -365,8 +409,7 @@ __device__ __forceinline__ void tl_store_out(void* out, int out_dtype, int64_t i
 
 // The small ops of a step (norms, rotations, residual adds) are launched so that their CTAs may be set up while a kernel in front
 // that allows it drains; each waits for all of it before it reads or writes anything (every thread, or the kernel behind
-// could start before that one has ended), and allows no early start itself: the kernels behind prefetch what they take
-// for constant (weights, scales, biases), and that may be what an op has just made.
+// could start before that one has ended), and allows no early start itself, so that behind it all in front of it is settled (tl_wrote).
 __device__ __forceinline__ void tl_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 template <typename... P, typename... A>
 cudaError_t tl_launch_waiting(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t stream, A... args) {

@@ -164,6 +164,7 @@ int32_t tl_rmsnorm(tl_ctx* ctx, const void* x, int32_t x_dtype, const void* weig
                                    cols, eps));
   }
   ctx->counters[TL_COUNTER_KERNEL_LAUNCHES]++;
+  tl_wrote(ctx, out, rows * cols * tl_dtype_size(out_dtype), true);
   return TL_OK;
 }
 
@@ -183,6 +184,7 @@ int32_t tl_rope(tl_ctx* ctx, const void* qk, int32_t dtype, const float* cos_tab
   TL_CUDA(ctx, tl_launch_waiting(rope_kernel, dim3(unsigned(grid)), dim3(256), ctx->stream, qk, dtype, cos_table, sin_table, out, total, seq_len,
                                  head_dim, sin_scale, cos_offset, sin_offset));
   ctx->counters[TL_COUNTER_KERNEL_LAUNCHES]++;
+  tl_wrote(ctx, out, total * tl_dtype_size(dtype), true);
   return TL_OK;
 }
 

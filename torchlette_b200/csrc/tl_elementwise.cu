@@ -82,6 +82,7 @@ int32_t tl_unary_op(tl_ctx* ctx, int32_t op, const void* in, int32_t in_dtype, v
   TL_CUDA(ctx, tl_launch_waiting(unary_kernel, dim3(unsigned(grid_for(ctx, vec ? count / 4 + 1 : count))), dim3(256), ctx->stream, in, in_dtype, out,
                                  out_dtype, op, count, vec ? 1 : 0));
   ctx->counters[TL_COUNTER_KERNEL_LAUNCHES]++;
+  tl_wrote(ctx, out, count * tl_dtype_size(out_dtype), true);
   return TL_OK;
 }
 
@@ -96,6 +97,7 @@ int32_t tl_binary_op(tl_ctx* ctx, int32_t op, const void* a, int32_t a_dtype, co
   TL_CUDA(ctx, tl_launch_waiting(binary_kernel, dim3(unsigned(grid_for(ctx, rows * cols))), dim3(256), ctx->stream, a, a_dtype, b, b_dtype, out, out_dtype,
                                  op, rows, cols, b_is_row ? 1 : 0));
   ctx->counters[TL_COUNTER_KERNEL_LAUNCHES]++;
+  tl_wrote(ctx, out, rows * cols * tl_dtype_size(out_dtype), true);
   return TL_OK;
 }
 
@@ -113,6 +115,7 @@ int32_t tl_transpose2d(tl_ctx* ctx, const void* in, void* out, int64_t batch, in
   else transpose_kernel<uint8_t><<<grid, 256, 0, ctx->stream>>>(static_cast<const uint8_t*>(in), static_cast<uint8_t*>(out), rows, cols);
   TL_CUDA(ctx, cudaGetLastError());
   ctx->counters[TL_COUNTER_KERNEL_LAUNCHES]++;
+  tl_wrote(ctx, out, batch * rows * cols * elem_bytes, true);
   return TL_OK;
 }
 

@@ -480,12 +480,13 @@ cudaError_t int4_ring_at(tl_ctx* ctx, const Int4Args& p, const EpiParams& e, int
   cfg.gridDim = dim3(unsigned((p.n + 16 * RT - 1) / (16 * RT)));
   cfg.blockDim = dim3(warps * 32);
   cfg.dynamicSmemBytes = smem;
-  cfg.stream = ctx->stream;
+  const EarlyStream stream = tl_early_stream(ctx);
+  cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = stream.attrs;
   return cudaLaunchKernelEx(&cfg, kern, p, e);
 }
 template <typename AT, int NT, int RT, int FOLD>
@@ -624,6 +625,7 @@ int32_t tl_dequant_int4(tl_ctx* ctx, const void* packed, const void* scales, voi
     dequant_int4_kernel<__nv_bfloat16><<<grid, 256, 0, ctx->stream>>>(pk, scales, static_cast<__nv_bfloat16*>(out), n_words, qdesc->group_size, qdesc->scales_dtype, qdesc->scale_convention, vec);
   TL_CUDA(ctx, cudaGetLastError());
   ctx->counters[TL_COUNTER_KERNEL_LAUNCHES]++;
+  tl_wrote(ctx, out, n * k * tl_dtype_size(out_dtype), true);
   return TL_OK;
 }
 
@@ -636,6 +638,7 @@ int32_t tl_unpack_int4(tl_ctx* ctx, const void* packed, void* out_i8, int64_t n,
   DeviceGuard guard(ctx->device);
   const int grid = int(std::min<int64_t>((n_words + 255) / 256, int64_t(ctx->sm_count) * 16));
   unpack_int4_kernel<<<grid, 256, 0, ctx->stream>>>(static_cast<const uint32_t*>(packed), static_cast<int8_t*>(out_i8), n_words);
+  ctx->fresh_weights = true;  // its bytes are a packed int8 weight
   TL_CUDA(ctx, cudaGetLastError());
   ctx->counters[TL_COUNTER_KERNEL_LAUNCHES]++;
   return TL_OK;
@@ -703,6 +706,7 @@ int32_t tl_int4_matmul(tl_ctx* ctx, const char* who, int route, const void* a, i
     else launch_int4_m<__nv_bfloat16>(ctx, p, epi, int(m));
     TL_CUDA(ctx, cudaGetLastError());
     ctx->counters[TL_COUNTER_QGEMV]++;
+    tl_wrote(ctx, out, m * n * tl_dtype_size(out_dtype));
     if (has_ops) ctx->counters[TL_COUNTER_QGEMV_EPILOGUE]++;
     return TL_OK;
   }

@@ -331,5 +331,6 @@ extern "C" int32_t tl_matmul(tl_ctx* ctx, const void* a, const void* b, void* ou
   }
   TL_CUDA(ctx, cudaGetLastError());
   ctx->counters[TL_COUNTER_KERNEL_LAUNCHES]++;
+  tl_wrote(ctx, out, ((batch - 1) * stride_c + m * n) * tl_dtype_size(out_dtype));
   return TL_OK;
 }

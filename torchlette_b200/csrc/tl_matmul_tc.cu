@@ -527,5 +527,6 @@ int32_t tl_launch_dense_tc(tl_ctx* ctx, const void* a, const void* b, void* out,
     return tl_set_error(ctx, TL_ERR_CUDA, "tl_matmul: tensor-core launch failed: %s", cudaGetErrorString(e));
   }
   ctx->counters[TL_COUNTER_KERNEL_LAUNCHES]++;
+  tl_wrote(ctx, out, m * n * tl_dtype_size(out_dtype));
   return TL_OK;
 }

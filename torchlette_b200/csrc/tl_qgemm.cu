@@ -877,6 +877,7 @@ int32_t tl_launch_qgemm(tl_ctx* ctx, const tl_variant& v, const void* a, int32_t
     return tl_set_error(ctx, TL_ERR_CUDA, "qgemm: launch failed: %s", cudaGetErrorString(e));
   }
   ctx->counters[TL_COUNTER_KERNEL_LAUNCHES]++;
+  tl_wrote(ctx, out, m * n * tl_dtype_size(out_dtype));
   return TL_OK;
 }
 

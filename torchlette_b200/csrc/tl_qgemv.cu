@@ -259,7 +259,8 @@ __global__ void __launch_bounds__(256) qgemv_simt_kernel(GemvArgs p, EpiParams e
       for (int r = 0; r < R; ++r) sv[d][r] = tl_load_scale(p.scales, p.scales_dtype, srow[r] + g);
     }
   };
-  // weights and scales do not depend on the kernel before this one
+  // The host launches this early only where no kernel that may still be running, or whose writes may not be seen yet, wrote weights or
+  // scales (tl_early_stream).  Scales after the wait, their lines asked of L2 before it: 4096 x 4096, groups of 64, one token 7.2 -> 7.8 us.
 #pragma unroll
   for (int d = 0; d < D; ++d) fetch(d, d);
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -893,10 +894,9 @@ __device__ __forceinline__ void ring_tile(const GemvArgs& p, const EpiParams& ep
   }
   // The tile's per-channel scales and bias entries are read in the epilogue, at the very end of a
   // one-wave launch: a cold line there is an exposed DRAM round trip on every launch.  Ask for the
-  // lines early; no register stays live.
-  if (tid == 0 && !GROUPED) prefetch_l1(reinterpret_cast<const uint8_t*>(p.scales) + size_t(tile_row) * (p.scales_dtype == TL_F32 ? 4 : 2));
-  // weights and scales never depend on the previous kernel; activations (its output), a bias that may be one and our own stores do
+  // lines as soon as the kernel in front, whose output they may be, has ended; no register stays live.
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (tid == 0 && !GROUPED) prefetch_l1(reinterpret_cast<const uint8_t*>(p.scales) + size_t(tile_row) * (p.scales_dtype == TL_F32 ? 4 : 2));
   if (tid == 0 && epi.fast_bias) prefetch_l1(epi.fast_bias + tile_row);
   if (rin) reduce_in_prologue(*rin);  // the activations are written by CTAs of THIS grid: read them through L2
   uint32_t push2_half = 0, push2_epoch = 0;
@@ -1135,8 +1135,8 @@ __device__ __forceinline__ void ring_tile2(const GemvArgs& p, const EpiParams& e
     cp_async_commit();
   }
   // the epilogue's scales and bias entries: see ring_tile
-  if (tid == 0 && !GROUPED) prefetch_l1(reinterpret_cast<const uint8_t*>(p.scales) + size_t(tile_row) * (p.scales_dtype == TL_F32 ? 4 : 2));
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (tid == 0 && !GROUPED) prefetch_l1(reinterpret_cast<const uint8_t*>(p.scales) + size_t(tile_row) * (p.scales_dtype == TL_F32 ? 4 : 2));
   if (tid == 0 && epi.fast_bias) prefetch_l1(epi.fast_bias + tile_row);
 
   float total[2][NT][4];
@@ -1733,7 +1733,7 @@ __global__ void __launch_bounds__(17 * 32, 1) qgemv_bulk_kernel(GemvArgs p, EpiP
 // in the stream is still draining, prefetches its weights (which depend on nothing), and only
 // then waits (griddepcontrol.wait) for the predecessor before it touches activations or writes.
 template <typename K>
-void launch_with_smem(K kernel, int grid, int block, size_t smem, cudaStream_t s, const GemvArgs& p, const EpiParams& e) {
+void launch_with_smem(K kernel, int grid, int block, size_t smem, EarlyStream s, const GemvArgs& p, const EpiParams& e) {
   if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(grid);
@@ -1744,11 +1744,11 @@ void launch_with_smem(K kernel, int grid, int block, size_t smem, cudaStream_t s
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = s.attrs;
   cudaLaunchKernelEx(&cfg, kernel, p, e);
 }
 template <typename AT, int NT, bool GROUPED>
-void launch_ring_s(int depth, int grid, int block, cudaStream_t s, const GemvArgs& p, const EpiParams& e) {
+void launch_ring_s(int depth, int grid, int block, EarlyStream s, const GemvArgs& p, const EpiParams& e) {
   const size_t smem = size_t(depth >= 8 ? 8 : depth >= 6 ? 6 : depth >= 4 ? 4 : 2) * 2 * block * 16 + size_t(block / 32) * NT * 128 * 4;
   if (depth >= 8) launch_with_smem(qgemv_ring_kernel<AT, NT, GROUPED, 8>, grid, block, smem, s, p, e);
   else if (depth >= 6) launch_with_smem(qgemv_ring_kernel<AT, NT, GROUPED, 6>, grid, block, smem, s, p, e);
@@ -1756,7 +1756,7 @@ void launch_ring_s(int depth, int grid, int block, cudaStream_t s, const GemvArg
   else launch_with_smem(qgemv_ring_kernel<AT, NT, GROUPED, 2>, grid, block, smem, s, p, e);
 }
 template <typename AT>
-void launch_ring(bool two, bool grouped, int depth, int grid, int block, cudaStream_t s, const GemvArgs& p,
+void launch_ring(bool two, bool grouped, int depth, int grid, int block, EarlyStream s, const GemvArgs& p,
                  const EpiParams& e) {
   if (two) {
     if (grouped) launch_ring_s<AT, 2, true>(depth, grid, block, s, p, e);
@@ -1851,7 +1851,7 @@ void ring_pick_shape(tl_ctx* ctx, bool batched, int a_dtype, int m, bool grouped
 
 // wide (32-row) ring tiles: depths 2 and 4
 template <typename K>
-void launch_pdl(K kernel, int grid, int block, size_t smem, cudaStream_t s, const GemvArgs& p, const EpiParams& e) {
+void launch_pdl(K kernel, int grid, int block, size_t smem, EarlyStream s, const GemvArgs& p, const EpiParams& e) {
   if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(grid);
@@ -1862,20 +1862,20 @@ void launch_pdl(K kernel, int grid, int block, size_t smem, cudaStream_t s, cons
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = s.attrs;
   cudaLaunchKernelEx(&cfg, kernel, p, e);
 }
 inline size_t ring2_smem_bytes(int warps, int depth, bool two) {
   return size_t(depth) * 4 * warps * 32 * 16 + size_t(warps) * 2 * (two ? 2 : 1) * 128 * 4;
 }
 template <typename AT, int NT, bool GROUPED>
-void launch_ring2_s(int depth, int grid, int block, cudaStream_t s, const GemvArgs& p, const EpiParams& e) {
+void launch_ring2_s(int depth, int grid, int block, EarlyStream s, const GemvArgs& p, const EpiParams& e) {
   const size_t smem = ring2_smem_bytes(block / 32, depth >= 4 ? 4 : 2, NT == 2);
   if (depth >= 4) launch_pdl(qgemv_ring2_kernel<AT, NT, GROUPED, 4>, grid, block, smem, s, p, e);
   else launch_pdl(qgemv_ring2_kernel<AT, NT, GROUPED, 2>, grid, block, smem, s, p, e);
 }
 template <typename AT>
-void launch_ring2(bool two, bool grouped, int depth, int grid, int block, cudaStream_t s, const GemvArgs& p, const EpiParams& e) {
+void launch_ring2(bool two, bool grouped, int depth, int grid, int block, EarlyStream s, const GemvArgs& p, const EpiParams& e) {
   if (two) { if (grouped) launch_ring2_s<AT, 2, true>(depth, grid, block, s, p, e); else launch_ring2_s<AT, 2, false>(depth, grid, block, s, p, e); }
   else { if (grouped) launch_ring2_s<AT, 1, true>(depth, grid, block, s, p, e); else launch_ring2_s<AT, 1, false>(depth, grid, block, s, p, e); }
 }
@@ -1898,7 +1898,7 @@ void launch_sk(bool m16, bool grouped, int depth, int grid, cudaStream_t s, cons
 }
 
 template <typename AT, int MT, int R, int D, bool GROUPED>
-void launch_simt_staged(int grid, int block, cudaStream_t s, const GemvArgs& p, const EpiParams& e) {
+void launch_simt_staged(int grid, int block, EarlyStream s, const GemvArgs& p, const EpiParams& e) {
   const int steps = (p.k / 16 + 31) / 32, slice = std::min(simt_slice(MT, steps), (steps + D - 1) / D * D);
   const size_t smem = (steps > slice ? 2 : 1) * size_t(MT) * slice * 512 * sizeof(float);
   auto kern = qgemv_simt_kernel<AT, MT, R, D, GROUPED>;
@@ -1912,11 +1912,11 @@ void launch_simt_staged(int grid, int block, cudaStream_t s, const GemvArgs& p, 
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = s.attrs;
   cudaLaunchKernelEx(&cfg, kern, p, e, slice);
 }
 template <typename AT, int MT, int R, bool GROUPED>
-void launch_simt_g(int grid, int block, cudaStream_t s, const GemvArgs& p, const EpiParams& e) {
+void launch_simt_g(int grid, int block, EarlyStream s, const GemvArgs& p, const EpiParams& e) {
   if constexpr (MT == 1 && R == 4) {
     qgemv_simt_tall_kernel<AT, GROUPED><<<grid, block, 0, s>>>(p, e);
   } else if constexpr (MT == 1 && R == 1) {
@@ -1929,12 +1929,12 @@ void launch_simt_g(int grid, int block, cudaStream_t s, const GemvArgs& p, const
   }
 }
 template <typename AT, int MT, int R>
-void launch_simt(bool grouped, int grid, int block, cudaStream_t s, const GemvArgs& p, const EpiParams& e) {
+void launch_simt(bool grouped, int grid, int block, EarlyStream s, const GemvArgs& p, const EpiParams& e) {
   if (grouped) launch_simt_g<AT, MT, R, true>(grid, block, s, p, e);
   else launch_simt_g<AT, MT, R, false>(grid, block, s, p, e);
 }
 template <typename AT, int R>
-void launch_simt_m(int mt, bool grouped, int grid, int block, cudaStream_t s, const GemvArgs& p, const EpiParams& e) {
+void launch_simt_m(int mt, bool grouped, int grid, int block, EarlyStream s, const GemvArgs& p, const EpiParams& e) {
   switch (mt) {
     case 1: launch_simt<AT, 1, R>(grouped, grid, block, s, p, e); break;
     case 2: launch_simt<AT, 2, R>(grouped, grid, block, s, p, e); break;
@@ -1943,7 +1943,7 @@ void launch_simt_m(int mt, bool grouped, int grid, int block, cudaStream_t s, co
   }
 }
 template <typename AT>
-void launch_simt_r(int r, int mt, bool grouped, int grid, int block, cudaStream_t s, const GemvArgs& p, const EpiParams& e) {
+void launch_simt_r(int r, int mt, bool grouped, int grid, int block, EarlyStream s, const GemvArgs& p, const EpiParams& e) {
   if (r >= 4) launch_simt_m<AT, 4>(mt, grouped, grid, block, s, p, e);
   else if (r >= 2) launch_simt_m<AT, 2>(mt, grouped, grid, block, s, p, e);
   else launch_simt_m<AT, 1>(mt, grouped, grid, block, s, p, e);
@@ -2157,7 +2157,9 @@ int32_t tl_launch_qgemv(tl_ctx* ctx, const tl_variant& v, const void* a, int32_t
       return tl_set_error(ctx, TL_ERR_INVALID_ARG, "qgemv: %s needs 16-byte aligned weight and activation pointers",
                           tl_variant_name(&v));
   }
-  cudaStream_t s = ctx->stream;
+  const EarlyStream s = v.kernel == kSimt   ? tl_early_stream(ctx, scales, size_t(n) * p.groups_per_row * tl_dtype_size(q.scales_dtype))
+                        : v.kernel == kRing ? tl_early_stream(ctx)
+                                            : EarlyStream{ctx->stream, 0};
   if (v.kernel == kBulk) {
     ba.status = ctx->dev_status;
     const bool m16 = m > 8;
@@ -2257,6 +2259,7 @@ int32_t tl_launch_qgemv(tl_ctx* ctx, const tl_variant& v, const void* a, int32_t
   }
   TL_CUDA(ctx, cudaGetLastError());
   ctx->counters[TL_COUNTER_KERNEL_LAUNCHES] += launches;
+  tl_wrote(ctx, out, m * n * tl_dtype_size(out_dtype));
   return TL_OK;
 }
 
@@ -2378,6 +2381,7 @@ extern "C" int32_t tl_qgemv_nt_static_scratch(tl_ctx* ctx, const void* a, int32_
   else launch_tma_static<__nv_bfloat16>(m > 8, grouped, grid, block, smem, ctx->stream, wmap, p, epi, ta);
   TL_CUDA(ctx, cudaGetLastError());
   ctx->counters[TL_COUNTER_KERNEL_LAUNCHES]++;
+  tl_wrote(ctx, out, m * n * tl_dtype_size(out_dtype));
   ctx->counters[TL_COUNTER_QGEMV]++;
   if (has_ops) ctx->counters[TL_COUNTER_QGEMV_EPILOGUE]++;
   return TL_OK;
@@ -2389,7 +2393,7 @@ extern "C" int32_t tl_qgemv_nt_static_scratch(tl_ctx* ctx, const void* a, int32_
 // ---------------------------------------------------------------------------
 namespace {
 template <typename AT, int NT, bool GROUPED, int S>
-void launch_ring_batched(int grid, int block, cudaStream_t s, const RingBatchArgs& b) {
+void launch_ring_batched(int grid, int block, EarlyStream s, const RingBatchArgs& b) {
   const size_t smem = size_t(S) * 2 * block * 16 + size_t(block / 32) * NT * 128 * 4;
   auto kern = qgemv_ring_batched_kernel<AT, NT, GROUPED, S>;
   if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
@@ -2402,11 +2406,11 @@ void launch_ring_batched(int grid, int block, cudaStream_t s, const RingBatchArg
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = s.attrs;
   cudaLaunchKernelEx(&cfg, kern, b);
 }
 template <typename AT, int NT, bool GROUPED, int S>
-void launch_ring2_batched(int grid, int block, cudaStream_t s, const RingBatchArgs& b) {
+void launch_ring2_batched(int grid, int block, EarlyStream s, const RingBatchArgs& b) {
   const size_t smem = ring2_smem_bytes(block / 32, S, NT == 2);
   auto kern = qgemv_ring2_batched_kernel<AT, NT, GROUPED, S>;
   if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
@@ -2419,25 +2423,25 @@ void launch_ring2_batched(int grid, int block, cudaStream_t s, const RingBatchAr
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = s.attrs;
   cudaLaunchKernelEx(&cfg, kern, b);
 }
 template <typename AT>
-void launch_ring2_batched_at(bool two, bool grouped, int depth, int grid, int block, cudaStream_t s, const RingBatchArgs& b) {
+void launch_ring2_batched_at(bool two, bool grouped, int depth, int grid, int block, EarlyStream s, const RingBatchArgs& b) {
 #define TL_R2B(NT_, G_) { if (depth >= 4) launch_ring2_batched<AT, NT_, G_, 4>(grid, block, s, b); else launch_ring2_batched<AT, NT_, G_, 2>(grid, block, s, b); }
   if (two) { if (grouped) TL_R2B(2, true) else TL_R2B(2, false) }
   else { if (grouped) TL_R2B(1, true) else TL_R2B(1, false) }
 #undef TL_R2B
 }
 template <typename AT, int NT, bool GROUPED>
-void launch_ring_batched_s(int depth, int grid, int block, cudaStream_t s, const RingBatchArgs& b) {
+void launch_ring_batched_s(int depth, int grid, int block, EarlyStream s, const RingBatchArgs& b) {
   if (depth >= 8) launch_ring_batched<AT, NT, GROUPED, 8>(grid, block, s, b);
   else if (depth >= 6) launch_ring_batched<AT, NT, GROUPED, 6>(grid, block, s, b);
   else if (depth >= 4) launch_ring_batched<AT, NT, GROUPED, 4>(grid, block, s, b);
   else launch_ring_batched<AT, NT, GROUPED, 2>(grid, block, s, b);
 }
 template <typename AT>
-void launch_ring_batched_at(bool two, bool grouped, int depth, int grid, int block, cudaStream_t s, const RingBatchArgs& b) {
+void launch_ring_batched_at(bool two, bool grouped, int depth, int grid, int block, EarlyStream s, const RingBatchArgs& b) {
   if (two) { if (grouped) launch_ring_batched_s<AT, 2, true>(depth, grid, block, s, b); else launch_ring_batched_s<AT, 2, false>(depth, grid, block, s, b); }
   else { if (grouped) launch_ring_batched_s<AT, 1, true>(depth, grid, block, s, b); else launch_ring_batched_s<AT, 1, false>(depth, grid, block, s, b); }
 }
@@ -2527,12 +2531,13 @@ extern "C" int32_t tl_qgemv_nt_batched(tl_ctx* ctx, const void* a, int32_t a_dty
   const int block = warps * 32, grid = int(tiles);
   const bool grouped = qdesc->group_size != k;
   if (wide) {
-    if (a_dtype == TL_F16) launch_ring2_batched_at<__half>(m > 8, grouped, depth, grid, block, ctx->stream, b);
-    else launch_ring2_batched_at<__nv_bfloat16>(m > 8, grouped, depth, grid, block, ctx->stream, b);
-  } else if (a_dtype == TL_F16) launch_ring_batched_at<__half>(m > 8, grouped, depth, grid, block, ctx->stream, b);
-  else launch_ring_batched_at<__nv_bfloat16>(m > 8, grouped, depth, grid, block, ctx->stream, b);
+    if (a_dtype == TL_F16) launch_ring2_batched_at<__half>(m > 8, grouped, depth, grid, block, tl_early_stream(ctx), b);
+    else launch_ring2_batched_at<__nv_bfloat16>(m > 8, grouped, depth, grid, block, tl_early_stream(ctx), b);
+  } else if (a_dtype == TL_F16) launch_ring_batched_at<__half>(m > 8, grouped, depth, grid, block, tl_early_stream(ctx), b);
+  else launch_ring_batched_at<__nv_bfloat16>(m > 8, grouped, depth, grid, block, tl_early_stream(ctx), b);
   TL_CUDA(ctx, cudaGetLastError());
   ctx->counters[TL_COUNTER_KERNEL_LAUNCHES]++;
+  tl_wrote_some(ctx);
   ctx->counters[TL_COUNTER_QGEMV] += n_items;
   ctx->counters[TL_COUNTER_QGEMV_EPILOGUE] += n_epi;
   return TL_OK;
@@ -3088,6 +3093,7 @@ extern "C" int32_t tl_qgemv_chain_launch(tl_ctx* ctx, tl_chain* chain) {
     return tl_set_error(ctx, TL_ERR_CUDA, "tl_qgemv_chain_launch: %s", cudaGetErrorString(e));
   }
   ctx->counters[TL_COUNTER_KERNEL_LAUNCHES]++;
+  tl_wrote_some(ctx);
   ctx->counters[TL_COUNTER_QGEMV] += chain->n_items;
   ctx->counters[TL_COUNTER_QGEMV_EPILOGUE] += chain->n_epi;
   return TL_OK;
@@ -3099,7 +3105,7 @@ extern "C" int32_t tl_qgemv_chain_launch(tl_ctx* ctx, tl_chain* chain) {
 // ---------------------------------------------------------------------------
 namespace {
 template <typename AT, int NT, bool GROUPED>
-cudaError_t launch_ring_allreduce(int grid, int block, cudaStream_t s, const GemvArgs& p, const EpiParams& e, const PushArgs& q) {
+cudaError_t launch_ring_allreduce(int grid, int block, EarlyStream s, const GemvArgs& p, const EpiParams& e, const PushArgs& q) {
   constexpr int S = 4;
   const size_t smem = size_t(S) * 2 * block * 16 + size_t(block / 32) * NT * 128 * 4;
   auto kern = qgemv_ring_allreduce_kernel<AT, NT, GROUPED, S>;
@@ -3113,11 +3119,11 @@ cudaError_t launch_ring_allreduce(int grid, int block, cudaStream_t s, const Gem
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = s.attrs;
   return cudaLaunchKernelEx(&cfg, kern, p, e, q);
 }
 template <typename AT>
-cudaError_t launch_ring_allreduce_at(bool two, bool grouped, int grid, int block, cudaStream_t s, const GemvArgs& p,
+cudaError_t launch_ring_allreduce_at(bool two, bool grouped, int grid, int block, EarlyStream s, const GemvArgs& p,
                                      const EpiParams& e, const PushArgs& q) {
   if (two) return grouped ? launch_ring_allreduce<AT, 2, true>(grid, block, s, p, e, q) : launch_ring_allreduce<AT, 2, false>(grid, block, s, p, e, q);
   return grouped ? launch_ring_allreduce<AT, 1, true>(grid, block, s, p, e, q) : launch_ring_allreduce<AT, 1, false>(grid, block, s, p, e, q);
@@ -3170,14 +3176,15 @@ extern "C" int32_t tl_qgemv_nt_allreduce(tl_ctx* ctx, const void* a, int32_t a_d
     if (tiles <= int64_t(ctx->sm_count) * (1024 / (w * 32))) { warps = w; break; }
   const int block = warps * 32, grid = int(tiles);
   const bool grouped = qdesc->group_size != k;
-  cudaError_t e = a_dtype == TL_F16 ? launch_ring_allreduce_at<__half>(m > 8, grouped, grid, block, ctx->stream, p, epi, q)
-                                    : launch_ring_allreduce_at<__nv_bfloat16>(m > 8, grouped, grid, block, ctx->stream, p, epi, q);
+  cudaError_t e = a_dtype == TL_F16 ? launch_ring_allreduce_at<__half>(m > 8, grouped, grid, block, tl_early_stream(ctx), p, epi, q)
+                                    : launch_ring_allreduce_at<__nv_bfloat16>(m > 8, grouped, grid, block, tl_early_stream(ctx), p, epi, q);
   if (e != cudaSuccess) {
     ctx->async_errors++;
     return tl_set_error(ctx, TL_ERR_CUDA, "tl_qgemv_nt_allreduce: launch failed: %s", cudaGetErrorString(e));
   }
   ctx->fused_tiles = tiles;
   ctx->counters[TL_COUNTER_KERNEL_LAUNCHES]++;
+  tl_wrote_some(ctx);
   ctx->counters[TL_COUNTER_QGEMV]++;
   return TL_OK;
 }
@@ -3188,7 +3195,7 @@ extern "C" int32_t tl_qgemv_nt_allreduce(tl_ctx* ctx, const void* a, int32_t a_d
 // ---------------------------------------------------------------------------
 namespace {
 template <typename K, typename... Args>
-cudaError_t launch_pdl_args(K kern, int grid, int block, size_t smem, cudaStream_t s, Args... args) {
+cudaError_t launch_pdl_args(K kern, int grid, int block, size_t smem, EarlyStream s, Args... args) {
   if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(grid);
@@ -3199,7 +3206,7 @@ cudaError_t launch_pdl_args(K kern, int grid, int block, size_t smem, cudaStream
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = s.attrs;
   return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 constexpr int kTpStages = 4;  // ring depth of the tensor-parallel launches (their k loops are short)
@@ -3209,7 +3216,7 @@ inline size_t tp_smem(int block, int nt) { return size_t(kTpStages) * 2 * block 
   do {                                                                                            \
     auto kern = KERN_;                                                                            \
     const int block = tp_warps_for(ctx, kern, NT_, grid) * 32;                                    \
-    return launch_pdl_args(kern, grid, block, tp_smem(block, NT_), ctx->stream, __VA_ARGS__);     \
+    return launch_pdl_args(kern, grid, block, tp_smem(block, NT_), tl_early_stream(ctx), __VA_ARGS__);     \
   } while (0)
 template <typename AT>
 cudaError_t launch_push(tl_ctx* ctx, bool two, bool grouped, int grid, const GemvArgs& p, const EpiParams& e, const PushArgs& q) {
@@ -3333,6 +3340,7 @@ extern "C" int32_t tl_qgemv_nt_push(tl_ctx* ctx, const void* a, int32_t a_dtype,
   ctx->push_pending = true;
   ctx->push_dst = out; ctx->push_m = m; ctx->push_n = n; ctx->push_tiles = tiles; ctx->push_dtype = out_dtype;
   ctx->counters[TL_COUNTER_KERNEL_LAUNCHES]++;
+  tl_wrote_some(ctx);
   ctx->counters[TL_COUNTER_QGEMV]++;
   return TL_OK;
 }
@@ -3343,13 +3351,14 @@ extern "C" int32_t tl_reduce_pending(tl_ctx* ctx) {
   DeviceGuard guard(ctx->device);
   const int grid = 16;
   const ReduceIn r = make_reduce_in(ctx, ctx->push_dst, grid);
-  cudaError_t e = launch_pdl_args(reduce_pending_kernel, grid, 256, 0, ctx->stream, r);
+  cudaError_t e = launch_pdl_args(reduce_pending_kernel, grid, 256, 0, EarlyStream{ctx->stream, 1}, r);
   if (e != cudaSuccess) {
     ctx->async_errors++;
     return tl_set_error(ctx, TL_ERR_CUDA, "tl_reduce_pending: launch failed: %s", cudaGetErrorString(e));
   }
   ctx->push_pending = false;
   ctx->counters[TL_COUNTER_KERNEL_LAUNCHES]++;
+  tl_wrote_some(ctx);
   return TL_OK;
 }
 
@@ -3381,5 +3390,6 @@ int32_t tl_launch_qgemv_rin(tl_ctx* ctx, const void* a, int32_t a_dtype, const G
   }
   ctx->push_pending = false;
   ctx->counters[TL_COUNTER_KERNEL_LAUNCHES]++;
+  tl_wrote_some(ctx);
   return TL_OK;
 }

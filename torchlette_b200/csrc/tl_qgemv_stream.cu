@@ -548,7 +548,7 @@ __global__ void __launch_bounds__((C + 4) * 32, 2) qgemv_stream_kernel(const __g
 }
 
 template <typename AT, int NT, bool GROUPED>
-cudaError_t stream_launch_j(int cwarps, int jmax, int grid, int block, size_t smem, cudaStream_t s, const StreamArgs& p) {
+cudaError_t stream_launch_j(int cwarps, int jmax, int grid, int block, size_t smem, EarlyStream s, const StreamArgs& p) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(block);
@@ -558,7 +558,7 @@ cudaError_t stream_launch_j(int cwarps, int jmax, int grid, int block, size_t sm
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = s.attrs;
 #define TL_STREAM_GO(C_, J_)                                                                          \
   do {                                                                                               \
     auto kern = qgemv_stream_kernel<AT, NT, GROUPED, C_, J_>;                                         \
@@ -575,7 +575,7 @@ cudaError_t stream_launch_j(int cwarps, int jmax, int grid, int block, size_t sm
 }
 
 template <typename AT>
-cudaError_t stream_launch(bool two, bool grouped, int cwarps, int jmax, int grid, int block, size_t smem, cudaStream_t s, const StreamArgs& p) {
+cudaError_t stream_launch(bool two, bool grouped, int cwarps, int jmax, int grid, int block, size_t smem, EarlyStream s, const StreamArgs& p) {
   if (two) return grouped ? stream_launch_j<AT, 2, true>(cwarps, jmax, grid, block, smem, s, p) : stream_launch_j<AT, 2, false>(cwarps, jmax, grid, block, smem, s, p);
   return grouped ? stream_launch_j<AT, 1, true>(cwarps, jmax, grid, block, smem, s, p) : stream_launch_j<AT, 1, false>(cwarps, jmax, grid, block, smem, s, p);
 }
@@ -661,11 +661,12 @@ int32_t tl_launch_qgemv_stream(tl_ctx* ctx, const tl_variant& v, const void* a, 
   ctx->pf_last_grid = grid;
   const bool grouped = q.group_size != k;
   const int jmax = (v.p3 + v.p0 - 1) / v.p0;
-  cudaError_t e = a_dtype == TL_F16 ? stream_launch<__half>(nt == 2, grouped, v.p0, jmax, grid, block, smem, ctx->stream, p)
-                                    : stream_launch<__nv_bfloat16>(nt == 2, grouped, v.p0, jmax, grid, block, smem, ctx->stream, p);
+  cudaError_t e = a_dtype == TL_F16 ? stream_launch<__half>(nt == 2, grouped, v.p0, jmax, grid, block, smem, tl_early_stream(ctx), p)
+                                    : stream_launch<__nv_bfloat16>(nt == 2, grouped, v.p0, jmax, grid, block, smem, tl_early_stream(ctx), p);
   TL_CUDA(ctx, e);
   TL_CUDA(ctx, cudaGetLastError());
   ctx->counters[TL_COUNTER_KERNEL_LAUNCHES] += 1;
+  tl_wrote_some(ctx);
   return TL_OK;
 }
 

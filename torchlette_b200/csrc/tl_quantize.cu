@@ -178,6 +178,7 @@ int32_t tl_dequant_int8(tl_ctx* ctx, const void* packed, const void* scales, voi
         n_words, wpr, qdesc->group_size, gpr, qdesc->scales_dtype, qdesc->scale_convention);
   TL_CUDA(ctx, cudaGetLastError());
   ctx->counters[TL_COUNTER_KERNEL_LAUNCHES]++;
+  tl_wrote(ctx, out, n * k * tl_dtype_size(out_dtype), true);
   return TL_OK;
 }
 
@@ -194,6 +195,7 @@ int32_t tl_unpack_int8(tl_ctx* ctx, const void* packed, void* out_i8, int64_t n,
   const int block = 256;
   const int grid = int(std::min<int64_t>((n_words + block - 1) / block, int64_t(ctx->sm_count) * 16));
   unpack_int8_kernel<<<grid, block, 0, ctx->stream>>>((const uint32_t*)packed, (uint32_t*)out_i8, n_words);
+  ctx->fresh_weights = true;  // its bytes are a packed weight
   TL_CUDA(ctx, cudaGetLastError());
   ctx->counters[TL_COUNTER_KERNEL_LAUNCHES]++;
   return TL_OK;
@@ -374,6 +376,7 @@ extern "C" int32_t tl_quantize_linear_weight_device(tl_ctx* ctx, const float* we
   else if (group_size == 64) quantize_group_kernel<16><<<lin_grid, block, 0, ctx->stream>>>(w4, n_words, packed, scales);
   else if (group_size == 32) quantize_group_kernel<8><<<lin_grid, block, 0, ctx->stream>>>(w4, n_words, packed, scales);
   else quantize_kernel<<<grid, block, 0, ctx->stream>>>(weight, n_groups, group_size, packed, scales);
+  ctx->fresh_weights = true;
   TL_CUDA(ctx, cudaGetLastError());
   ctx->counters[TL_COUNTER_KERNEL_LAUNCHES]++;
   return TL_OK;
