@@ -3,7 +3,8 @@
 ``python -m torchlette_b200._build`` compiles every translation unit under
 ``csrc/`` to an object file (in parallel) and links the shared library next to
 the sources, where the ctypes binding looks for it; ``tl_pycall.cpp`` becomes the
-extension module ``_tlcall.so`` beside it.
+extension module ``_tlcall`` beside it, for the interpreter that builds it; without that interpreter's headers it is left out and
+the calls go through ctypes.
 """
 from __future__ import annotations
 
@@ -16,7 +17,7 @@ from concurrent.futures import ThreadPoolExecutor
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(CSRC, "libtlcuda.so")
-PYCALL = os.path.join(CSRC, "_tlcall.so")
+PYCALL = os.path.join(CSRC, "_tlcall" + sysconfig.get_config_var("EXT_SUFFIX"))
 SOURCES = ["tl_api.cu", "tl_pool.cu", "tl_quantize.cu", "tl_qgemv.cu", "tl_qgemv_stream.cu", "tl_qgemm.cu", "tl_matmul.cu", "tl_matmul_tc.cu", "tl_elementwise.cu", "tl_decode_ops.cu", "tl_attention.cu", "tl_attention_tc.cu", "tl_int4.cu", "tl_autotune.cu", "tl_comm.cu"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = [
@@ -61,8 +62,11 @@ def build(force: bool = False, verbose: bool = False) -> str:
     if jobs or _stale(LIB, objs):
         run([NVCC, "-shared", "-o", LIB, *objs, "-cudart", "static", "-ldl"])
     pysrc = os.path.join(CSRC, "tl_pycall.cpp")
-    if force or _stale(PYCALL, [pysrc, headers[-1]]):
-        run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", "-I", sysconfig.get_paths()["include"], "-o", PYCALL, pysrc])
+    include = sysconfig.get_paths()["include"]
+    if not os.path.exists(os.path.join(include, "Python.h")):
+        sys.stderr.write(f"{include} has no Python.h: {os.path.basename(PYCALL)} is not built, calls go through ctypes\n")
+    elif force or _stale(PYCALL, [pysrc, headers[-1]]):
+        run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", "-I", include, "-o", PYCALL, pysrc])
     return LIB
 
 

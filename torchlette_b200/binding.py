@@ -10,10 +10,13 @@ import ctypes as C
 import importlib.machinery
 import importlib.util
 import os
+import sysconfig
+import warnings
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.environ.get("TLCUDA_LIB") or os.path.join(_HERE, "csrc", "libtlcuda.so")
-PYCALL_PATH = os.path.join(_HERE, "csrc", "_tlcall.so")
+# one file per interpreter; the library's functions are handed to it by address, whichever library that is
+PYCALL_PATH = os.path.join(_HERE, "csrc", "_tlcall" + sysconfig.get_config_var("EXT_SUFFIX"))
 
 TL_OK = 0
 TL_ERR_INVALID_ARG, TL_ERR_UNSUPPORTED, TL_ERR_CUDA, TL_ERR_NCCL = -1, -2, -3, -4
@@ -198,10 +201,69 @@ def load():
     return lib
 
 
+CALLS = ("tl_alloc", "tl_free", "tl_copy2d", "tl_quantize_linear_weight_device", "tl_qmatmul_nt", "tl_matmul", "tl_unary_op", "tl_binary_op", "tl_rmsnorm",
+         "tl_rope", "tl_attention", "tl_decode_attention")
+
+
 class _Calls:
-    """The calls of the hot paths, one attribute per function of ``csrc/tl_pycall.cpp``: native argument conversion, an
-    exception instead of a status, ``tl_alloc(ctx, nbytes)`` with the address as its result.  ``quant`` and ``epilogue`` make the
-    descriptors those calls take (bytes)."""
+    """The calls of the hot paths, an attribute each: an exception instead of a status, ``tl_alloc(ctx, nbytes)`` with the
+    address as its result.  ``quant`` and ``epilogue`` make the descriptors those calls take (bytes).  Arguments are converted natively by
+    ``csrc/tl_pycall.cpp``; where that module has not been built, and for what it does not take, by ctypes."""
+
+
+def _through_ctypes(fn, kinds):
+    """The function with ctypes' own rules, descriptors (bytes of their size) as structures again."""
+    def argument(a, kind):
+        struct = getattr(kind, "_type_", None)
+        if isinstance(a, bytes) and isinstance(struct, type) and issubclass(struct, C.Structure) and len(a) == C.sizeof(struct):
+            return C.byref(struct.from_buffer_copy(a))
+        return a
+
+    def call(*args):
+        return fn(*(argument(a, kind) for a, kind in zip(args, kinds)), *args[len(kinds):])
+    return call
+
+
+def _alloc_through_ctypes(lib):
+    def alloc(ctx, nbytes):
+        p = C.c_void_p()
+        check(ctx, lib.tl_alloc(ctx, nbytes, C.byref(p)))
+        return p.value
+    return alloc
+
+
+def _ctypes_calls(lib) -> _Calls:
+    def checked(call):
+        def run(*args):
+            check(args[0] if args else None, call(*args))
+        return run
+
+    def quant(scheme, group_size, scales_dtype, scale_convention):
+        return bytes(QuantDesc(scheme, group_size, scales_dtype, scale_convention))
+
+    def epilogue(ops, inputs):
+        e = Epilogue()
+        if not isinstance(ops, tuple) or not isinstance(inputs, tuple) or len(ops) > TL_EPI_MAX_OPS or len(inputs) > TL_EPI_MAX_INPUTS or any(len(op) != 4 for op in ops):
+            raise TypeError("epilogue: tuples of integers")
+        e.n_ops, e.n_inputs = len(ops), len(inputs)
+        for i, op in enumerate(ops):
+            e.ops[i] = EpilogueOp(*op)
+        for i, at in enumerate(inputs):
+            e.inputs[i] = at
+        return bytes(e)
+
+    c = _Calls()
+    for name in CALLS:
+        setattr(c, name, _alloc_through_ctypes(lib) if name == "tl_alloc" else checked(_through_ctypes(getattr(lib, name), SIGNATURES[name][1])))
+    c.quant, c.epilogue = quant, epilogue
+    return c
+
+
+def _native_module():
+    loader = importlib.machinery.ExtensionFileLoader("_tlcall", PYCALL_PATH)
+    native = importlib.util.module_from_spec(importlib.util.spec_from_loader("_tlcall", loader))
+    loader.exec_module(native)
+    return native
 
 
 _calls = None
@@ -213,22 +275,15 @@ def calls() -> _Calls:
         return _calls
     lib = load()
     if not os.path.exists(PYCALL_PATH):
-        raise ImportError(f"{PYCALL_PATH} is missing: build it with `python -m torchlette_b200._build`")
-    loader = importlib.machinery.ExtensionFileLoader("_tlcall", PYCALL_PATH)
-    native = importlib.util.module_from_spec(importlib.util.spec_from_loader("_tlcall", loader))
-    loader.exec_module(native)
-
-    def through_ctypes(fn, kinds):
-        """The same call where an argument is not a plain number or address: ctypes' own rules, descriptors as structures again."""
-        def call(*args):
-            return fn(*(C.byref(kind._type_.from_buffer_copy(a)) if isinstance(a, bytes) and hasattr(kind, "_type_") and kind is not C.c_void_p else a
-                        for a, kind in zip(args, kinds)), *args[len(kinds):])
-        return call
-
+        warnings.warn(f"{PYCALL_PATH} has not been built (python -m torchlette_b200._build): calls take a few microseconds longer")
+        _calls = _ctypes_calls(lib)
+        return _calls
+    native = _native_module()
     c = _Calls()
-    for name in native.names:
+    for name in CALLS:
         fn = getattr(lib, name)
-        setattr(c, name, native.bind(name, C.cast(fn, C.c_void_p).value, through_ctypes(fn, SIGNATURES[name][1]), check))
+        slow = _alloc_through_ctypes(lib) if name == "tl_alloc" else _through_ctypes(fn, SIGNATURES[name][1])
+        setattr(c, name, native.bind(name, C.cast(fn, C.c_void_p).value, slow, check))
     c.quant, c.epilogue = native.quant, native.epilogue
     _calls = c
     return c

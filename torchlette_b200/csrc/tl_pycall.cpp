@@ -2,11 +2,11 @@
 // arguments (two to four microseconds a call, as long as the kernels of a small layer run).
 //
 // bind(name, address, slow, on_error) gives a callable for the library's function `name` at `address`.  The argument types come
-// from include/tlcuda.h.  Integers, floats and pointers given as int or None are converted here, as ctypes does; a call
-// with anything else (a ctypes pointer, an array, too few arguments) goes to `slow`, the ctypes function, whose rules then hold.  A
-// status other than TL_OK is handed to on_error(context, status), which raises.  The GIL is released around the call.
-// alloc(address, slow, on_error) is the same for tl_alloc with the block's address as the result.
-// epilogue(ops, inputs) gives the bytes of a tl_epilogue.
+// from include/tlcuda.h.  Integers, floats, pointers given as int or None and descriptors as bytes of their size are converted here, as
+// ctypes does; a call with anything else (a ctypes pointer, an array, another kind of integer, too few arguments) goes to `slow`, the
+// same call through ctypes, whose rules then hold.  A status other than TL_OK is handed to on_error(context, status), which raises.  The
+// GIL is released around the call.  For tl_alloc the call is (context, bytes) and its result, as that of `slow`, the block's address.
+// quant(scheme, group size, scales dtype, convention) and epilogue(ops, inputs) give the bytes of the descriptors.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
@@ -25,7 +25,10 @@ template <typename T> bool convert(PyObject* o, T* out) {
   if constexpr (std::is_pointer_v<T>) {
     if (o == Py_None) { *out = nullptr; return true; }
     if (PyLong_Check(o)) { *out = reinterpret_cast<T>(static_cast<uintptr_t>(PyLong_AsUnsignedLongLongMask(o))); return true; }
-    if (PyBytes_CheckExact(o)) { *out = reinterpret_cast<T>(PyBytes_AS_STRING(o)); return true; }  // a descriptor made by epilogue() or quant()
+    using Pointee = std::remove_const_t<std::remove_pointer_t<T>>;
+    if constexpr (std::is_same_v<Pointee, tl_quant_desc> || std::is_same_v<Pointee, tl_epilogue>) {
+      if (PyBytes_CheckExact(o) && PyBytes_GET_SIZE(o) == Py_ssize_t(sizeof(Pointee))) { *out = reinterpret_cast<T>(PyBytes_AS_STRING(o)); return true; }
+    }
     return false;
   } else if constexpr (std::is_floating_point_v<T>) {
     if (!PyFloat_Check(o)) return false;
@@ -36,6 +39,16 @@ template <typename T> bool convert(PyObject* o, T* out) {
     *out = static_cast<T>(PyLong_AsUnsignedLongLongMask(o));
     return true;
   }
+}
+
+// The same for what has no slow path: any object that is an integer by __index__.
+template <typename T> bool convert_index(PyObject* o, T* out) {
+  if (convert(o, out)) return true;
+  PyObject* i = PyNumber_Index(o);
+  if (!i) { PyErr_Clear(); return false; }
+  const bool ok = convert(i, out);
+  Py_DECREF(i);
+  return ok;
 }
 
 using Thunk = bool (*)(void* fn, PyObject* const* args, int32_t* status);  // false: an argument is not for here
@@ -59,7 +72,7 @@ struct Entry { const char* name; Thunk thunk; Py_ssize_t args; };
 const Entry kEntries[] = {TL_ENTRY(tl_free),     TL_ENTRY(tl_copy2d),    TL_ENTRY(tl_quantize_linear_weight_device),
                           TL_ENTRY(tl_qmatmul_nt), TL_ENTRY(tl_matmul),  TL_ENTRY(tl_unary_op),
                           TL_ENTRY(tl_binary_op), TL_ENTRY(tl_rmsnorm),  TL_ENTRY(tl_rope),
-                          TL_ENTRY(tl_attention), TL_ENTRY(tl_decode_attention), TL_ENTRY(tl_graph_launch)};
+                          TL_ENTRY(tl_attention), TL_ENTRY(tl_decode_attention)};
 
 struct Bound {
   PyObject_HEAD
@@ -96,10 +109,8 @@ PyObject* alloc_call(PyObject* callable, PyObject* const* args, size_t nargsf, P
   Bound* self = reinterpret_cast<Bound*>(callable);
   tl_ctx* ctx;
   size_t bytes;
-  if (kwnames || PyVectorcall_NARGS(nargsf) != 2 || !convert(args[0], &ctx) || !convert(args[1], &bytes)) {
-    PyErr_SetString(PyExc_TypeError, "alloc(context, bytes)");
-    return nullptr;
-  }
+  if (kwnames || PyVectorcall_NARGS(nargsf) != 2 || !convert(args[0], &ctx) || !convert(args[1], &bytes))
+    return PyObject_Vectorcall(self->slow, args, nargsf, kwnames);
   void* p = nullptr;
   int32_t status;
   Py_BEGIN_ALLOW_THREADS
@@ -152,8 +163,8 @@ PyObject* py_bind(PyObject*, PyObject* args) {
 // quant(scheme, group size, scales dtype, convention): a tl_quant_desc
 PyObject* py_quant(PyObject*, PyObject* const* args, Py_ssize_t n) {
   tl_quant_desc q{};
-  if (n != 4 || !convert(args[0], &q.scheme) || !convert(args[1], &q.group_size) || !convert(args[2], &q.scales_dtype) ||
-      !convert(args[3], &q.scale_convention)) {
+  if (n != 4 || !convert_index(args[0], &q.scheme) || !convert_index(args[1], &q.group_size) || !convert_index(args[2], &q.scales_dtype) ||
+      !convert_index(args[3], &q.scale_convention)) {
     PyErr_SetString(PyExc_TypeError, "quant: four integers");
     return nullptr;
   }
@@ -169,11 +180,11 @@ PyObject* py_epilogue(PyObject*, PyObject* const* args, Py_ssize_t n) {
     e.n_inputs = int32_t(PyTuple_GET_SIZE(args[1]));
     for (int i = 0; ok && i < e.n_ops; ++i) {
       PyObject* t = PyTuple_GET_ITEM(args[0], i);
-      ok = PyTuple_Check(t) && PyTuple_GET_SIZE(t) == 4 && convert(PyTuple_GET_ITEM(t, 0), &e.ops[i].kind) &&
-           convert(PyTuple_GET_ITEM(t, 1), &e.ops[i].op) && convert(PyTuple_GET_ITEM(t, 2), &e.ops[i].input_index) &&
-           convert(PyTuple_GET_ITEM(t, 3), &e.ops[i].to_dtype);
+      ok = PyTuple_Check(t) && PyTuple_GET_SIZE(t) == 4 && convert_index(PyTuple_GET_ITEM(t, 0), &e.ops[i].kind) &&
+           convert_index(PyTuple_GET_ITEM(t, 1), &e.ops[i].op) && convert_index(PyTuple_GET_ITEM(t, 2), &e.ops[i].input_index) &&
+           convert_index(PyTuple_GET_ITEM(t, 3), &e.ops[i].to_dtype);
     }
-    for (int i = 0; ok && i < e.n_inputs; ++i) ok = convert(PyTuple_GET_ITEM(args[1], i), &e.inputs[i]);
+    for (int i = 0; ok && i < e.n_inputs; ++i) ok = convert_index(PyTuple_GET_ITEM(args[1], i), &e.inputs[i]);
   }
   if (!ok) {
     PyErr_SetString(PyExc_TypeError, "epilogue: tuples of integers");
