@@ -32,6 +32,11 @@ int main() {
     q.group_size = group ? group : int(k);
     q.scales_dtype = TL_F16;
     tl_variant v;
+    if (bf16 == 2) {  // f32 activations, a small batch
+      tl_qgemv_default_variant(nullptr, int(m), n, k, TL_F32, q, &v);
+      std::printf("%d %d %d\\n", v.kernel, v.p0, v.p1);
+      continue;
+    }
     tl_qgemm_default_variant(nullptr, m, n, k, bf16 ? TL_BF16 : TL_F16, q, &v);
     std::printf("%d %d %d %d %d %d\\n", v.kernel, v.p0, v.p1, v.p2, v.p3, tl_dense_tc_choose(m, n, k, 148).parts);
   }
@@ -77,3 +82,12 @@ def test_an_int4_product_with_f32_output_keeps_its_short_sums(rule, n, k, group,
     """The forms with fewer warps a tile, hence longer sums, are for 16-bit outputs."""
     wide, half, bf16 = (r[:2] for r in rule((m, n, k, group, 0, B.DTYPE_ID["f32"]), (m, n, k, group, 0, B.DTYPE_ID["f16"]), (m, n, k, group, 1, B.DTYPE_ID["bf16"])))
     assert half == bf16 == fewer and wide == (warps, 1)
+
+
+@pytest.mark.parametrize("m,rows_a_warp,beyond", [(1, 1, (8, 2)), (2, 1, (8, 4)), (3, 2, (8, 4)), (4, 2, (4, 4)), (16, 2, (4, 4))])
+def test_f32_activations_take_more_rows_a_warp_where_one_wave_ends(rule, m, rows_a_warp, beyond):
+    """32 rows an SM: four CTAs of eight warps with a row each, or two with two."""
+    simt = 1
+    got = rule(*[(m, n, 4096, 64, 2) for n in (4200, 4736, 4737, 5328, 7103)])
+    assert got[:2] == [(simt, 8, rows_a_warp)] * 2
+    assert got[2:] == [(simt,) + beyond] * 3

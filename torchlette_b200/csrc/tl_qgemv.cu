@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(256) qgemv_simt_tall_kernel(GemvArgs p, EpiPar
 // lane's sixteen are 64 contiguous bytes, which straight from global memory are four 16-byte loads that touch four times the
 // lines they need (a 4096-row launch spent 8000 of its clocks on L1 wavefronts for them); here the quarters of a chunk are
 // swapped by the chunk ((c >> 1) & 3), so that no read has a bank conflict.
-// 4096 x 4096 with groups of 64, replayed: 7.1 us at m = 1 (9.9 with the activations met in the loop), 12.2 at 4 (16.9), 46 at 16 (65); 513 x 14336 16.8 (24.2).
+// 4096 x 4096 with groups of 64, replayed: 7.1 us at m = 1 (9.9 with the activations met in the loop), 12.2 at 4 (16.9), 46 at 16 (65); 513 x 14336 17.4 (24.2).
 // Steps of a slice, a multiple of D: all of K in one if that takes 32 KB, else two buffers of 16 to 32 KB (of 32 for one row, three CTAs fit an
 // SM and 4096 x 12288 took 29 us, the last of its 512 CTAs alone).
 constexpr int simt_slice(int mt, int steps) { return mt >= 3 ? 4 : mt == 2 ? (steps <= 8 ? 8 : 4) : steps <= 16 ? 16 : 8; }
@@ -1916,37 +1916,38 @@ void launch_simt_staged(int grid, int block, EarlyStream s, const GemvArgs& p, c
   cudaLaunchKernelEx(&cfg, kern, p, e, slice);
 }
 template <typename AT, int MT, int R, bool GROUPED>
-void launch_simt_g(int grid, int block, EarlyStream s, const GemvArgs& p, const EpiParams& e) {
+void launch_simt_g(int grid, int block, EarlyStream s, int sms, const GemvArgs& p, const EpiParams& e) {
   if constexpr (MT == 1 && R == 4) {
     qgemv_simt_tall_kernel<AT, GROUPED><<<grid, block, 0, s>>>(p, e);
   } else if constexpr (MT == 1 && R == 1) {
-    // Eight steps ahead where K is long enough for them (513 x 14336: 21.5 -> 18.8 us; 4096 x 4096, whose eight steps they are: 7.4 -> 10.2)
-    // and, with the registers of as many scales, where one wave still holds the CTAs (4096 x 12288, groups of 64, 512 of them: 31 us).
-    if (p.k >= 8192 && (!GROUPED || grid <= 384)) launch_simt_staged<AT, MT, R, 8, GROUPED>(grid, block, s, p, e);
+    // Eight steps ahead where K is long and, with the registers of as many scales, one wave holds the CTAs: three of eight warps an SM, 24
+    // rows.  us, four / eight ahead, groups of 64: 2368 x 8192 11.1 / 10.6, 3552 x 8192 12.9 / 11.7, 4096 x 8192 13.1 / 20.3; 512 x 14336
+    // 18.9 / 17.4, 3552 x 14336 23.5 / 20.9, 4096 x 14336 23.7 / 37.2; per channel 4096 x 8192 14.7 / 12.9, 4096 x 14336 25.8 / 22.9.
+    if (p.k >= 8192 && (!GROUPED || p.n <= 24 * sms)) launch_simt_staged<AT, MT, R, 8, GROUPED>(grid, block, s, p, e);
     else launch_simt_staged<AT, MT, R, 4, GROUPED>(grid, block, s, p, e);
   } else {
     launch_simt_staged<AT, MT, R, R == 4 ? 2 : 4, GROUPED>(grid, block, s, p, e);
   }
 }
 template <typename AT, int MT, int R>
-void launch_simt(bool grouped, int grid, int block, EarlyStream s, const GemvArgs& p, const EpiParams& e) {
-  if (grouped) launch_simt_g<AT, MT, R, true>(grid, block, s, p, e);
-  else launch_simt_g<AT, MT, R, false>(grid, block, s, p, e);
+void launch_simt(bool grouped, int grid, int block, EarlyStream s, int sms, const GemvArgs& p, const EpiParams& e) {
+  if (grouped) launch_simt_g<AT, MT, R, true>(grid, block, s, sms, p, e);
+  else launch_simt_g<AT, MT, R, false>(grid, block, s, sms, p, e);
 }
 template <typename AT, int R>
-void launch_simt_m(int mt, bool grouped, int grid, int block, EarlyStream s, const GemvArgs& p, const EpiParams& e) {
+void launch_simt_m(int mt, bool grouped, int grid, int block, EarlyStream s, int sms, const GemvArgs& p, const EpiParams& e) {
   switch (mt) {
-    case 1: launch_simt<AT, 1, R>(grouped, grid, block, s, p, e); break;
-    case 2: launch_simt<AT, 2, R>(grouped, grid, block, s, p, e); break;
-    case 3: launch_simt<AT, 3, R>(grouped, grid, block, s, p, e); break;
-    default: launch_simt<AT, 4, R>(grouped, grid, block, s, p, e); break;
+    case 1: launch_simt<AT, 1, R>(grouped, grid, block, s, sms, p, e); break;
+    case 2: launch_simt<AT, 2, R>(grouped, grid, block, s, sms, p, e); break;
+    case 3: launch_simt<AT, 3, R>(grouped, grid, block, s, sms, p, e); break;
+    default: launch_simt<AT, 4, R>(grouped, grid, block, s, sms, p, e); break;
   }
 }
 template <typename AT>
-void launch_simt_r(int r, int mt, bool grouped, int grid, int block, EarlyStream s, const GemvArgs& p, const EpiParams& e) {
-  if (r >= 4) launch_simt_m<AT, 4>(mt, grouped, grid, block, s, p, e);
-  else if (r >= 2) launch_simt_m<AT, 2>(mt, grouped, grid, block, s, p, e);
-  else launch_simt_m<AT, 1>(mt, grouped, grid, block, s, p, e);
+void launch_simt_r(int r, int mt, bool grouped, int grid, int block, EarlyStream s, int sms, const GemvArgs& p, const EpiParams& e) {
+  if (r >= 4) launch_simt_m<AT, 4>(mt, grouped, grid, block, s, sms, p, e);
+  else if (r >= 2) launch_simt_m<AT, 2>(mt, grouped, grid, block, s, sms, p, e);
+  else launch_simt_m<AT, 1>(mt, grouped, grid, block, s, sms, p, e);
 }
 
 template <typename AT, int NT>
@@ -2010,19 +2011,20 @@ int32_t tl_qgemv_default_variant(tl_ctx* ctx, int32_t m, int64_t n, int64_t k, i
   } else if (k % 16 == 0 && q.group_size % 16 == 0) {
     const int64_t sms = ctx ? ctx->sm_count : 148;
     v.kernel = kSimt;
-    // Rows a warp: the more, the fewer reads of the staged activations; the fewer, the more CTAs, as long as one wave holds them (three
-    // or four of eight warps an SM).  us with 1 / 2 / 4 rows and eight warps (f32, groups of 64): 4096 x 4096 m = 1 7.3 / 8.2 / 11.5, m = 3
-    // 11.7 / 10.9 / 15.1, m = 4 20.6 / 12.2 / 14.4; 7000 x 2048 m = 1 7.0 / 5.2 / 8.0, m = 3 11.0 / 10.8 / 9.6, m = 4 13.3 / 13.6 / 18.0 and 10.6 with
-    // four warps of four rows; 12288 x 4096 m = 1 19.1 / 16.8 / 15.4 (four warps, the tall form), m = 2 23.8 / 24.9 / 24.0, m = 3 30.4 / 30.5 / 27.4,
-    // m = 4 42.2 / 34.2 / 41.6; 1024 x 4096 m = 1 5.1 / 5.8 / 9.4, m = 16 41.8 / 39.2 / 48.8; 1000 x 1024 m = 4 4.0 / 4.5 / 6.6.
-    const bool tall = n >= 48 * sms;
+    // Rows a warp: the more, the fewer reads of the staged activations; the fewer, the more CTAs, as long as one wave holds them: four of
+    // eight warps an SM with one row a warp and up to three batch rows, two with two rows a warp and four batch rows, 32 rows an SM in both.
+    // us with 1 / 2 / 4 rows and eight warps (f32, groups of 64): 4096 x 4096 m = 1 7.1 / 8.1 / -, m = 3 11.6 / 10.7 / 15.6, m = 4 20.5 /
+    // 12.1 / 14.4; 4608 x 4096 m = 1 7.3 / 8.3 / -, m = 2 9.0 / 8.9 / 12.3; 5328 x 4096 m = 1 12.5 / 8.5 / -, m = 4 21.0 / 20.2 / 27.9 and 16.8 with four
+    // warps of four rows; 6144 x 4096 m = 2 15.2 / 15.8 / 12.7; 8192 x 4096 m = 1 13.3 / 15.0 / 14.4 (four warps, the tall form), m = 4 31.4 /
+    // 23.3 / 28.5; 12288 x 4096 m = 1 19.1 / 16.8 / 15.4, m = 4 42.2 / 34.1 / 41.8; 1776 x 4096 m = 2 8.5 / 8.1 / 11.0, m = 3 11.1 / 10.1 / 13.5.
+    const bool one_wave = n <= 32 * sms, tall = n >= 48 * sms;
     v.p0 = 8;
     if (m == 1) {
-      v.p1 = tall ? 4 : n > 28 * sms ? 2 : 1;
+      v.p1 = tall ? 4 : one_wave ? 1 : 2;
       if (tall) v.p0 = 4;
     } else if (m <= 3) {
-      v.p1 = n > 28 * sms ? 4 : m == 3 && n >= 12 * sms ? 2 : 1;
-    } else if (n > 36 * sms && !tall) {
+      v.p1 = !one_wave ? 4 : m == 3 && n >= 12 * sms ? 2 : 1;
+    } else if (!one_wave && !tall) {
       v.p0 = v.p1 = 4;
     } else {
       v.p1 = m >= 8 || n >= 12 * sms ? 2 : 1;
@@ -2237,9 +2239,9 @@ int32_t tl_launch_qgemv(tl_ctx* ctx, const tl_variant& v, const void* a, int32_t
       const int mt = std::min(4, m - m0);
       ps.m = mt; ps.row0 = m0;
       ps.a = reinterpret_cast<const uint8_t*>(a) + size_t(m0) * k * tl_dtype_size(a_dtype);
-      if (a_dtype == TL_F32) launch_simt_r<float>(v.p1, mt, grouped, grid, block, s, ps, epi);
-      else if (a_dtype == TL_F16) launch_simt_r<__half>(v.p1, mt, grouped, grid, block, s, ps, epi);
-      else launch_simt_r<__nv_bfloat16>(v.p1, mt, grouped, grid, block, s, ps, epi);
+      if (a_dtype == TL_F32) launch_simt_r<float>(v.p1, mt, grouped, grid, block, s, ctx->sm_count, ps, epi);
+      else if (a_dtype == TL_F16) launch_simt_r<__half>(v.p1, mt, grouped, grid, block, s, ctx->sm_count, ps, epi);
+      else launch_simt_r<__nv_bfloat16>(v.p1, mt, grouped, grid, block, s, ctx->sm_count, ps, epi);
     }
   } else if (v.kernel == kRing && v.p2 == 2) {
     if (a_dtype == TL_F16) launch_ring2<__half>(m > 8, grouped, v.p1, grid, block, s, p, epi);
