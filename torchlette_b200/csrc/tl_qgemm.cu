@@ -370,10 +370,9 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
       const int grp = gshift >= 0 ? k >> gshift : k / p.group;
       return (grp < p.groups_per_row ? tl_load_scale(p.scales, p.scales_dtype, grow * p.groups_per_row + grp) : 0.f) * p.wscale;
     };
-    auto slot_free = [&](int it) -> bool { return it < TS || mbar_wait(&slotfree_bar[it % TS], ((it / TS) - 1) & 1, &abort_flag); };
     auto convert = [&](int it, int ks, int n_tile) -> bool {
       const int s = it % STAGES;
-      if (kRing.slot_first && !slot_free(it)) return false;
+      if (kRing.slot_first && it >= TS && !mbar_wait(&slotfree_bar[it % TS], ((it / TS) - 1) & 1, &abort_flag)) return false;
       if (warp == 0 && lane == 0) TL_TR(2, it, 0);
       if (!mbar_wait(&full_bar[s], (it / STAGES) & 1, &abort_flag)) return false;
       if (warp == 0 && lane == 0) TL_TR(2, it, 1);
@@ -421,7 +420,7 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant_
         const int sl = it % TS;
         if (!convert(it, ks, n_tile)) { ok = false; break; }
         if (warp == 0 && lane == 0) TL_TR(2, it, 2);
-        if (!kRing.slot_first && !slot_free(it)) { ok = false; break; }
+        if (!kRing.slot_first && it >= TS && !mbar_wait(&slotfree_bar[sl], ((it / TS) - 1) & 1, &abort_flag)) { ok = false; break; }
         if (warp == 0 && lane == 0) TL_TR(2, it, 3);
         tc_fence_after();
         const uint32_t slot = tmem_base + lane_addr + uint32_t(2 * BN + sl * kSlotCols);
