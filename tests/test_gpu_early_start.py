@@ -121,3 +121,45 @@ def test_device_quantizer_and_the_product_behind_it(backend, act):
         for t in (full, y, w.scales, w):
             t.destroy()
     x.destroy()
+
+
+def test_small_ops_behind_copies_and_a_joined_stream_in_a_capture(backend):
+    """The attribute of an early launch where what is in front is no kernel, or more than one stream's work."""
+    from cuda.bindings import driver as cu
+
+    def ok(result):
+        assert result[0] == cu.CUresult.CUDA_SUCCESS, result
+        return result[1] if len(result) == 2 else result[1:]
+
+    be, n = backend, 1024
+    dt = tb.B.DTYPE_ID["f32"]
+    xv = np.linspace(-1, 1, n, dtype=np.float32)
+    x = be.ops.tensorFromArray(xv, [1, n], "f32")
+    row, y, z, w = (be.ops.empty([1, n], "f32") for _ in range(4))
+    s = be.stream()
+    side = ok(cu.cuStreamCreate(cu.CUstream_flags.CU_STREAM_NON_BLOCKING))
+    fork, join = (ok(cu.cuEventCreate(cu.CUevent_flags.CU_EVENT_DISABLE_TIMING)) for _ in range(2))
+    be.sync()
+    ok(cu.cuStreamBeginCapture(s, cu.CUstreamCaptureMode.CU_STREAM_CAPTURE_MODE_RELAXED))
+    try:
+        ok(cu.cuEventRecord(fork, s))
+        ok(cu.cuStreamWaitEvent(side, fork, 0))
+        ok(cu.cuMemsetD32Async(w.buffer, int(np.float32(2.0).view(np.uint32)), n, side))
+        ok(cu.cuEventRecord(join, side))
+        be._calls.tl_copy2d(be._handle, row.buffer, 4 * n, x.buffer, 4 * n, 4 * n, 1)
+        be._calls.tl_unary_op(be._handle, tb.B.TL_UNARY["relu"], row.buffer, dt, y.buffer, dt, n)  # behind a copy
+        ok(cu.cuStreamWaitEvent(s, join, 0))
+        be._calls.tl_binary_op(be._handle, tb.B.TL_BINARY["mul"], y.buffer, dt, w.buffer, dt, z.buffer, dt, 1, n, 0)  # behind a kernel and another stream
+    finally:
+        graph = ok(cu.cuStreamEndCapture(s))
+    run = ok(cu.cuGraphInstantiate(graph, 0))
+    ok(cu.cuGraphLaunch(run, s))
+    be.sync()
+    np.testing.assert_array_equal(be.ops.read(z).reshape(-1), np.maximum(xv, 0) * 2)
+    cu.cuGraphExecDestroy(run)
+    cu.cuGraphDestroy(graph)
+    cu.cuEventDestroy(fork)
+    cu.cuEventDestroy(join)
+    cu.cuStreamDestroy(side)
+    for t in (x, row, y, z, w):
+        t.destroy()
