@@ -231,10 +231,10 @@ void launch_int4_m(tl_ctx* ctx, Int4Args p, const EpiParams& epi, int m) {
 // A mask and an exclusive or with a magic exponent and the sign bits make the pair (q_x + 8, q_{x+4} + 8)
 // 16-bit floats 1024 + . (f16) or 128 + . (bf16), and one subtraction -- or, for the nibbles taken at bits 4-7, one
 // fused multiply-add -- gives (q_x, q_{x+4}) exactly (Nib::quad); the activations are paired the same way.
-// Bound: instruction issue (65 % of the slots, the ALU pipe 58 %, with a division and row arithmetic in every block) and a second wave
-// that fills half the chip, ahead of HBM.  14336 x 4096, groups of 128, bias + gelu, replayed: 15.0 us at m = 1, 15.3 at 4, 21.7 at 16
-// (16.2, 16.4, 22.9 with them; 20.3, 21.5, 33.5 with two blocks in registers and the activations met in the loop); groups of 32: 18.5,
-// 18.9, 28.8 (they took the CUDA cores' form).
+// Bound: instruction issue (66 % of the slots, the ALU pipe 59 %; 317 instructions a 16 x 128 block, 337 with a division and row
+// arithmetic in every block) and a second wave that fills half the chip, ahead of HBM.  14336 x 4096, groups of 128, bias + gelu,
+// replayed: 15.0 us at m = 1, 15.3 at 4, 21.7 at 16 (16.2, 16.4, 22.9 with that arithmetic; 20.3, 21.5, 33.5 with two blocks in registers
+// and the activations met in the loop); groups of 32: 18.5, 18.9, 28.8 (they took the CUDA cores' form).
 // ---------------------------------------------------------------------------
 // quad(u, v): the four MMA operand registers of one packed word u; the exclusive or that sets the exponent also turns
 // the two's complement nibble into n = q + 8:
